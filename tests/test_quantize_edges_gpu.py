@@ -1,0 +1,38 @@
+"""The activation quantizers at the edges of their kernels' tiles, bit for bit against the CPU oracle: rows held in registers
+(up to 4096 values, or 32768 in batches of up to 256 rows; 32 values to a thread)."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from crit_kernels_b200 import cabi
+from oracle import quantize_oracle as qo
+
+pytestmark = pytest.mark.gpu
+
+
+def _ptr(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def inputs(m, k):
+    g = torch.Generator().manual_seed(m * 7 + k)
+    x = torch.randn(m, k, generator=g) * torch.exp2(torch.randint(-9, 6, (m, 1), generator=g).float())
+    x[m // 2, : k // 3] = 0
+    return x.to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("m,k", [(1, 8), (3, 248), (9, 264), (33, 1016), (257, 1032), (5, 4096), (300, 4096), (300, 4104),
+                                 (256, 4104), (257, 5120), (2, 32768), (2, 32776), (1200, 1024)])
+def test_fp8_rows_at_the_edges_of_their_kernels(m, k):
+    x = inputs(m, k)
+    x[0, k - 1] = -448.0
+    xd = x.cuda()
+    q = torch.full((m, k), 0x55, dtype=torch.uint8, device="cuda")
+    scale = torch.empty(m, device="cuda")
+    assert cabi.load().dg_enqueue_quantize_fp8_rows(_ptr(xd), k, m, k, _ptr(q), k, _ptr(scale), None) == 0
+    torch.cuda.synchronize()
+    want_q, want_scale = qo.fp8_rows(x)
+    assert np.array_equal(scale.cpu().numpy().view(np.uint32), want_scale.view(np.uint32))
+    assert np.array_equal(q.cpu().numpy(), want_q)
