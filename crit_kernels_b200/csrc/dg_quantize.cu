@@ -12,8 +12,7 @@
 // Machine mapping (not the reference's): a row of the FP8 quantizer is read from HBM once: one bulk copy (TMA, 1-D)
 // brings it into shared memory, the CTA takes the maximum and quantizes from there, 16 output bytes per thread and
 // store; rows that do not fit or are not 16-byte aligned are read twice through L2 instead. The NVFP4 quantizer gives a
-// thread four consecutive blocks (128 input bytes, 32 code bytes, one 32-bit word of tiled scales) and converts with
-// the hardware E2M1 / E4M3 conversions.
+// lane a block and converts with the hardware E2M1 / E4M3 conversions.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -253,12 +252,6 @@ __global__ void __launch_bounds__(kRowThreads) fp8_rows_kernel(const __nv_bfloat
     quantize_row<false>(xr, reinterpret_cast<const uint4*>(row_smem), qr, K, sc, staged, aligned_in, vector_out, tid);
 }
 
-// Byte offset of block j of row n in cuBLASLt's 128 x 4 tiled scale layout with ct tiles per tile row.
-__device__ __forceinline__ size_t tiled_offset(int n, int j, int ct) {
-  const int r = n & 127;
-  return ((size_t)(n >> 7) * ct + (j >> 2)) * 512 + (size_t)(r & 31) * 16 + (r >> 5) * 4 + (j & 3);
-}
-
 // Two quotients -> two E2M1 codes in one byte (low nibble = lo). v + 0 turns a negative zero into +0 (code 0, as a
 // comparison with zero sees it); every other negative quotient keeps its sign bit, also when it rounds to zero.
 __device__ __forceinline__ uint32_t e2m1x2(float lo, float hi) {
@@ -269,72 +262,111 @@ __device__ __forceinline__ uint32_t e2m1x2(float lo, float hi) {
   return r;
 }
 
+// Packed FP32 pairs (each half IEEE, round to nearest).
+struct pair { unsigned long long v; };
+__device__ __forceinline__ pair pack(float lo, float hi) {
+  pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ pair mul2(pair a, pair b) {
+  pair r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ pair fma2(pair a, pair b, pair c) {
+  pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
 // 16 values (8 BF16 pairs) -> scale byte (returned) and 8 code bytes (lo, hi).
-__device__ __forceinline__ uint32_t nvfp4_block(const uint4& v0, const uint4& v1, float g, float g_rcp, uint32_t& lo,
-                                                uint32_t& hi) {
-  const float amax = amax_of(amax8(v1, amax8(v0, 0u)));
+__device__ __forceinline__ uint32_t nvfp4_block(const uint32_t (&w)[8], float g, float g_rcp, uint32_t& lo, uint32_t& hi) {
+  uint32_t m = 0u;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m = amax2(w[i], m);
+  const float amax = amax_of(m);
   float bs = (amax * kRcp6) * g;
   bs = bs > 448.f ? 448.f : bs;
   const uint32_t sbits = e4m3x2(bs, 0.f) & 0xffu;
   float d = e4m3_value(sbits) * g_rcp;
   const bool zero = !(d > 0.f);
   d = d < 1e-30f ? 1e-30f : d;
-  const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
   lo = hi = 0u;
   if (zero) return sbits;
-  // a block whose quotients cannot leave FP32's range takes the short division (a zero quotient's sign is dropped by
-  // the conversion's + 0 anyway); the rest (values near FP32's limits) the full one
+  uint32_t byte[8];
+  // a block whose quotients cannot leave FP32's range takes the short division, two values at once (a zero quotient's sign
+  // is dropped by the conversion's + 0 anyway); the rest (values near FP32's limits) the full one
   if (amax < 1e8f) {
     const float r = __frcp_rn(d);
+    const pair r2 = pack(r, r), d2 = pack(-d, -d);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint32_t byte = e2m1x2(quotient<true, false>(bf16_lo(w[i]), d, r), quotient<true, false>(bf16_hi(w[i]), d, r));
-      if (i < 4) lo |= byte << (8 * i);
-      else hi |= byte << (8 * (i - 4));
+      const pair x = pack(bf16_lo(w[i]), bf16_hi(w[i])), q0 = mul2(x, r2), q1 = fma2(fma2(d2, q0, x), r2, q0);
+      float a, b;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(q1.v));
+      byte[i] = e2m1x2(a, b);
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const uint32_t byte = e2m1x2(__fdiv_rn(bf16_lo(w[i]), d), __fdiv_rn(bf16_hi(w[i]), d));
-      if (i < 4) lo |= byte << (8 * i);
-      else hi |= byte << (8 * (i - 4));
-    }
+    for (int i = 0; i < 8; ++i) byte[i] = e2m1x2(__fdiv_rn(bf16_lo(w[i]), d), __fdiv_rn(bf16_hi(w[i]), d));
   }
+  lo = __byte_perm(__byte_perm(byte[0], byte[1], 0x0040), __byte_perm(byte[2], byte[3], 0x0040), 0x5410);
+  hi = __byte_perm(__byte_perm(byte[4], byte[5], 0x0040), __byte_perm(byte[6], byte[7], 0x0040), 0x5410);
   return sbits;
 }
 
-// One thread four consecutive blocks (one 32-bit word of the tiled scales) of the padded grid
-// [rows_padded][blocks_padded / 4].
+// A CTA quantizes 32 rows x 512 values of a 128-row tile of the scales: warp w the rows 8 i + w, 32 + 8 i + w, 64 + 8 i + w
+// and 96 + 8 i + w (i: which quarter), whose scale words lie side by side in the tiled layout. A lane takes one block of a
+// row: a warp reads 1024 and writes 256 consecutive bytes at a time, two rows' loads in flight at once, and the scale bytes
+// meet in shared memory and leave as 128 consecutive bytes per tile. (With four blocks to a thread a warp's load touched 32
+// lines.) The arithmetic bounds it, more than the memory: about 100 instructions a block, with the quotients in packed pairs.
+// 4096 x 8192: 22.3 us before, 18.9 now (13.1 at copy bandwidth); 16 x 28672: 5.0 and 1.9.
+constexpr int kQuantCols = 512, kQuantRows = 32;
 __global__ void __launch_bounds__(256) nvfp4_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int M, int K,
                                                     float g, float g_rcp, uint8_t* __restrict__ codes,
-                                                    uint8_t* __restrict__ scales, int rows_padded, int quads) {
+                                                    uint8_t* __restrict__ scales, int quads, int col_tiles, int wide_scales) {
+  __shared__ __align__(16) unsigned char tile[kQuantCols / 64 * 128];   // [quad][row % 8][row / 32][block % 4]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row_block = blockIdx.x / col_tiles, col_tile = blockIdx.x - row_block * col_tiles;
+  const int tile_row = row_block >> 2, eight = row_block & 3;
+  const int row0 = tile_row * 128 + eight * 8 + warp, k = col_tile * kQuantCols + lane * 16;
+  if (tid < kQuantCols / 64 * 8) reinterpret_cast<uint4*>(tile)[tid] = make_uint4(0u, 0u, 0u, 0u);   // padding rows and blocks
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= (long long)rows_padded * quads) return;
-  const int row = (int)(id / quads), quad = (int)(id - (long long)row * quads);
-  uint32_t word = 0;
-  const int blocks = K >> 4;
-  if (row < M) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * ldx + 64 * quad);
-    uint4 v[8];
+  uint4 v[4][2];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const bool in = 4 * quad + b < blocks;
-      v[2 * b] = in ? __ldg(src + 2 * b) : make_uint4(0u, 0u, 0u, 0u);
-      v[2 * b + 1] = in ? __ldg(src + 2 * b + 1) : make_uint4(0u, 0u, 0u, 0u);
-    }
-    uint2* dst = reinterpret_cast<uint2*>(codes + (size_t)row * (K >> 1) + 32 * quad);
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + 32 * i;
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * ldx + k);
+    const bool in = row < M && k < K;
+    v[i][0] = in ? __ldg(src) : make_uint4(0u, 0u, 0u, 0u);
+    v[i][1] = in ? __ldg(src + 1) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  __syncthreads();
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      if (4 * quad + b < blocks) {
-        uint32_t lo, hi;
-        word |= nvfp4_block(v[2 * b], v[2 * b + 1], g, g_rcp, lo, hi) << (8 * b);
-        dst[b] = make_uint2(lo, hi);
-      }
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + 32 * i;
+    if (row < M && k < K) {
+      const uint32_t w[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
+      uint32_t lo, hi;
+      const uint32_t scale = nvfp4_block(w, g, g_rcp, lo, hi);
+      *reinterpret_cast<uint2*>(codes + (size_t)row * (K >> 1) + (k >> 1)) = make_uint2(lo, hi);
+      tile[(lane >> 2) * 128 + warp * 16 + i * 4 + (lane & 3)] = (unsigned char)scale;
     }
   }
-  *reinterpret_cast<uint32_t*>(scales + tiled_offset(row, 4 * quad, quads)) = word;
+  __syncthreads();
+  const int quad = col_tile * (kQuantCols / 64) + (tid >> 3);
+  if (tid < kQuantCols / 64 * 8 && quad < quads) {
+    const uint4 s = reinterpret_cast<const uint4*>(tile)[tid];
+    uint8_t* dst = scales + ((size_t)tile_row * quads + quad) * 512 + (eight * 8 + (tid & 7)) * 16;
+    if (wide_scales) {
+      *reinterpret_cast<uint4*>(dst) = s;
+    } else {
+      uint32_t* d32 = reinterpret_cast<uint32_t*>(dst);
+      d32[0] = s.x; d32[1] = s.y; d32[2] = s.z; d32[3] = s.w;
+    }
+  }
 }
 
 bool aligned(const void* p, uintptr_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0; }
@@ -397,11 +429,12 @@ int dg_enqueue_quantize_nvfp4(const void* x, long long ldx, int M, int K, float 
   if (M < 1 || K < 16 || K % 16 || !x || !codes || !blocked_scales || ldx < K || ldx % 8 || !aligned(x, 16) ||
       !aligned(codes, 8) || !aligned(blocked_scales, 4) || !(input_scale > 0.f))
     return (int)cudaErrorInvalidValue;
-  const int rows_padded = (M + 127) / 128 * 128, quads = (K / 16 + 3) / 4;
-  const long long threads = (long long)rows_padded * quads;
-  return (int)launch_pdl(nvfp4_kernel, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0,
-                         static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x), ldx, M, K, input_scale,
-                         input_rcp, codes, blocked_scales, rows_padded, quads);
+  const int quads = (K / 16 + 3) / 4;
+  const int col_tiles = (K + kQuantCols - 1) / kQuantCols;
+  const long long ctas = ((long long)M + 127) / 128 * (128 / kQuantRows) * col_tiles;
+  return (int)launch_pdl(nvfp4_kernel, dim3((unsigned)ctas), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                         static_cast<const __nv_bfloat16*>(x), ldx, M, K, input_scale, input_rcp, codes, blocked_scales, quads, col_tiles,
+                         (int)aligned(blocked_scales, 16));
 }
 
 }  // extern "C"

@@ -1,5 +1,5 @@
 """The activation quantizers at the edges of their kernels' tiles, bit for bit against the CPU oracle: rows held in registers
-(up to 4096 values, or 32768 in batches of up to 256 rows; 32 values to a thread)."""
+(up to 4096 values, or 32768 in batches of up to 256 rows; 32 values to a thread), 32 x 512 tiles of NVFP4 blocks."""
 import ctypes
 
 import numpy as np
@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from crit_kernels_b200 import cabi
+from oracle import decode_gemv_oracle as oc
 from oracle import quantize_oracle as qo
 
 pytestmark = pytest.mark.gpu
@@ -36,3 +37,20 @@ def test_fp8_rows_at_the_edges_of_their_kernels(m, k):
     want_q, want_scale = qo.fp8_rows(x)
     assert np.array_equal(scale.cpu().numpy().view(np.uint32), want_scale.view(np.uint32))
     assert np.array_equal(q.cpu().numpy(), want_q)
+
+
+@pytest.mark.parametrize("m,k", [(1, 16), (8, 496), (31, 512), (33, 528), (127, 1040), (129, 560), (97, 64)])
+@pytest.mark.parametrize("offset", [0, 4])                         # of the tiled scales from 16 bytes
+def test_nvfp4_at_the_edges_of_its_tiles(m, k, offset):
+    x = inputs(m, k)
+    xd = x.cuda()
+    codes = torch.full((m, k // 2), 0x55, dtype=torch.uint8, device="cuda")
+    buffer = torch.full((oc.blocked_numel(m, k) + offset,), 0x55, dtype=torch.uint8, device="cuda")
+    scales = buffer[offset:]
+    g, r = ctypes.c_float(300.0), ctypes.c_float(np.float32(1.0) / np.float32(300.0))
+    assert cabi.load().dg_enqueue_quantize_nvfp4(_ptr(xd), k, m, k, g, r, _ptr(codes), _ptr(scales), None) == 0
+    torch.cuda.synchronize()
+    want_codes, want_blocked = qo.nvfp4_blocked(x, 300.0)
+    assert np.array_equal(codes.cpu().numpy(), want_codes)
+    assert np.array_equal(scales.cpu().numpy(), want_blocked)
+    assert bool((buffer[:offset] == 0x55).all())
