@@ -1,0 +1,28 @@
+"""The dequantizers at the edges of a CTA's run of 1024 output vectors (8 or 16 values each), which may start and end anywhere
+in a row: bit for bit against the CPU oracle."""
+import ctypes
+
+import pytest
+import torch
+
+from crit_kernels_b200 import cabi
+from oracle import decode_gemv_oracle as oc
+from oracle import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k", [(1, 8192), (1, 16384), (2, 8208), (3, 5472), (16, 512), (17, 1008), (1025, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float8_e4m3fn])
+def test_runs_that_cross_rows(n, k, dtype):
+    c, s, i = wl.cfg_nvfp4(n, k, seed=n + k)
+    i = i * (48.0 if dtype == torch.float8_e4m3fn else 1.0)
+    cd, sd, f = c.cuda(), s.cuda(), i.cuda()
+    out = torch.full((n * k * dtype.itemsize + 64,), 0x55, dtype=torch.uint8, device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    kind = 3 if dtype == torch.float8_e4m3fn else 1
+    assert cabi.load().dg_enqueue_dequantize(ptr(cd), ptr(sd), ptr(f), ptr(out), kind, n, k, None) == 0
+    torch.cuda.synchronize()
+    want = oc.dequantize(c, s, i, dtype)
+    assert torch.equal(out[:-64].cpu(), want.view(torch.uint8).flatten())
+    assert bool((out[-64:] == 0x55).all())
