@@ -46,37 +46,57 @@ EncodeTiled encode_tiled() {
   return fn;
 }
 
-// A map over `rows` rows of `row_bytes` bytes (a multiple of 16) as 8-byte elements, box = box_rows x box_bytes.
-// The encoded map is a function of these six values alone, and a decode loop asks for the same few maps token after
-// token: each host thread keeps the last ones it encoded (the driver call costs about as much as the launch).
-bool encode_rows(CUtensorMap* map, const void* base, int rows, int row_bytes, int box_rows, int box_bytes) {
-  EncodeTiled fn = encode_tiled();
-  if (!fn || row_bytes % 16 || box_bytes % 16 || box_bytes / 8 > 256 || box_rows > 256 || box_rows < 1) return false;
-  struct Kept {
-    const void* base = nullptr;
-    int rows = 0, row_bytes = 0, box_rows = 0, box_bytes = 0;
-    CUtensorMap map;
-  };
-  constexpr int kKept = 64;
+// Tensor maps. An encoded map is a function of the values it is asked for alone, and a decode loop asks for the same few
+// maps token after token: each host thread keeps the last ones it encoded (the driver call costs about as much as the
+// launch).
+struct MapKey {
+  const void* base;
+  long long a, b, c;       // the sizes the map is made from
+  bool operator==(const MapKey& o) const { return base == o.base && a == o.a && b == o.b && c == o.c; }
+};
+template <typename Encode>
+bool kept_map(CUtensorMap* map, const MapKey& key, const Encode& encode) {
+  struct Kept { MapKey key{}; CUtensorMap map; };
+  constexpr int kKept = 128;
   static thread_local Kept kept[kKept];
-  const uintptr_t mixed = reinterpret_cast<uintptr_t>(base) >> 8;
-  Kept& slot = kept[(mixed ^ (mixed >> 7) ^ (uintptr_t)rows ^ ((uintptr_t)box_rows << 3) ^ (uintptr_t)box_bytes) % kKept];
-  if (slot.base == base && slot.rows == rows && slot.row_bytes == row_bytes && slot.box_rows == box_rows &&
-      slot.box_bytes == box_bytes) {
-    *map = slot.map;
-    return true;
+  const uintptr_t mixed = reinterpret_cast<uintptr_t>(key.base) >> 8;
+  Kept& slot = kept[(mixed ^ (mixed >> 7) ^ (uintptr_t)key.a ^ (uintptr_t)(key.b * 5) ^ (uintptr_t)(key.c >> 4) ^ (uintptr_t)(key.c >> 12)) % kKept];
+  if (!(slot.key == key)) {
+    EncodeTiled fn = encode_tiled();
+    if (!fn || encode(fn, &slot.map) != CUDA_SUCCESS) {
+      slot.key = MapKey{};
+      return false;
+    }
+    slot.key = key;
   }
-  const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 8), (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 8), (cuuint32_t)box_rows};
-  const cuuint32_t elem[2] = {1, 1};
-  if (fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(base), dims, strides, box, elem,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
-  slot.base = base; slot.rows = rows; slot.row_bytes = row_bytes; slot.box_rows = box_rows; slot.box_bytes = box_bytes;
-  slot.map = *map;
+  *map = slot.map;
   return true;
+}
+// `rows` rows of `row_bytes` bytes (a multiple of 16) as 8-byte elements, box = box_rows rows x box_bytes.
+bool encode_rows(CUtensorMap* map, const void* base, int rows, int row_bytes, int box_rows, int box_bytes) {
+  return kept_map(map, MapKey{base, rows, row_bytes, box_rows * 4096 + box_bytes}, [&](EncodeTiled fn, CUtensorMap* out) {
+    const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 8), (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / 8), (cuuint32_t)box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(base), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
+}
+// The activations [M][K] (16-bit elements, rows ldx apart, K a multiple of 64) as [K / 64][M][64], box = `blocks` of them.
+bool encode_activations(CUtensorMap* map, const void* base, int M, int K, int ldx, int blocks, bool swizzled) {
+  const int row = M > 1 ? ldx : K;     // (one row may come with any distance to a next one)
+  return kept_map(map, MapKey{base, ((long long)M << 32) | K, row, swizzled ? -blocks : -blocks - 4096}, [&](EncodeTiled fn, CUtensorMap* out) {
+    const cuuint64_t dims[3] = {64, (cuuint64_t)M, (cuuint64_t)(K / 64)};
+    const cuuint64_t strides[2] = {(cuuint64_t)row * 2, 128};
+    const cuuint32_t box[3] = {64, (cuuint32_t)M, (cuuint32_t)blocks};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  });
 }
 DeviceState g_devices[kMaxDevices];
 std::atomic<int> g_static_weights{0};   // dg_set_static_weights
@@ -85,7 +105,7 @@ std::atomic<unsigned long long> g_wait_limit_ns{dg::kWaitLimitNs};   // dg_set_w
 std::atomic<unsigned long long*> g_trace_base{nullptr};
 std::atomic<int> g_trace_capacity{0}, g_trace_next{0};
 
-const void* const* const kTables[] = {dg_table_bf16,       dg_table_fp8_bf16,   dg_table_fp8_f16,  dg_table_mxfp8_bf16,
+const void* const (*const kTables[])[16] = {dg_table_bf16,       dg_table_fp8_bf16,   dg_table_fp8_f16,  dg_table_mxfp8_bf16,
                                       dg_table_mxfp8_f16,  dg_table_nvfp4_bf16, dg_table_nvfp4_f16};
 
 // Per device, once: SM count, the address of the status word, and the opt-in to 227 KB of dynamic shared memory for
@@ -102,15 +122,13 @@ DeviceState* device_state() {
   bool ok = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) == cudaSuccess && major == 10 &&
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0 &&
             cudaGetSymbolAddress(&status, dg_status_word) == cudaSuccess;
-  // (the carveout preference keeps the SM's whole shared memory available where two CTAs are to share it)
-  for (const void* const* table : kTables)
-    for (int m = 0; ok && m < 16; ++m)
-      ok = cudaFuncSetAttribute(table[m], cudaFuncAttributeMaxDynamicSharedMemorySize, dg::kSmemLimit) == cudaSuccess &&
-           cudaFuncSetAttribute(table[m], cudaFuncAttributePreferredSharedMemoryCarveout,
-                                cudaSharedmemCarveoutMaxShared) == cudaSuccess;
-  for (int m = 0; ok && m < 16; ++m)
-    ok = cudaFuncSetAttribute(dg_batch_table_nvfp4_bf16[m], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              dg::kSmemLimit) == cudaSuccess;
+  auto opt_in = [&](const void* const (*table)[16]) {
+    for (int i = 0; ok && i < 32; ++i)
+      ok = cudaFuncSetAttribute(table[i / 16][i % 16], cudaFuncAttributeMaxDynamicSharedMemorySize, dg::kSmemLimit) ==
+           cudaSuccess;
+  };
+  for (const void* const (*table)[16] : kTables) opt_in(table);
+  opt_in(dg_batch_table_nvfp4_bf16);
   if (!ok) {
     cudaGetLastError();
     st.ready.store(-1, std::memory_order_release);
@@ -123,99 +141,94 @@ DeviceState* device_state() {
 }
 
 struct FormatInfo {
-  int e, scb;   // elements per 16-byte block, scale bytes per 512-byte step
+  int e, step, x_row;   // elements per 16-byte block, bytes of a step of a weight row and of an activation row
 };
-constexpr FormatInfo kFormats[4] = {{8, 0}, {16, 0}, {16, 16}, {32, 64}};
+template <int FMT>
+constexpr FormatInfo info_of() { return {dg::Format<FMT>::E, dg::Format<FMT>::STEP, dg::Format<FMT>::XROW}; }
+constexpr FormatInfo kFormats[4] = {info_of<0>(), info_of<1>(), info_of<2>(), info_of<3>()};
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Bytes of the activations kept resident: whole steps of [M][x_row bytes], then a flag byte per step.
+int resident_bytes_of(int fmt, int M, int nblk) {
+  const int row_steps = ceil_div(nblk * 16, kFormats[fmt].step);
+  return row_steps * M * kFormats[fmt].x_row + ((row_steps + 15) & ~15);
+}
+
 // Launch shape: a speed choice from (format, M, N, K, SM count) only; no row's bits depend on it.
 //   CTAs            one per SM, fewer when the matrix has under four rows per SM
-//   rows per warp   the most the kernel holds (rows_max), less when a CTA's range is short
-//   steps           512-byte steps per ring stage: at least two (1 KB of every row per stage: 512-byte pieces cost
-//                   DRAM efficiency and per-row bulk copies are issue-limited), up to four when a tile has few rows;
-//                   activations under 32 KB per stage
+//   tile rows       64, 56 or 48 (less when a CTA's range is shorter): what takes the fewest mma groups of 16 rows, a tile
+//                   costing as much as half a group (its sums) plus, where its activations are converted on the way, as
+//                   much as these cost
+//   steps           512-byte steps per ring stage (BF16: one of 1 KB): two, one where the ring would have fewer than three
+//                   stages otherwise: a consumer warp's fixed costs per stage then weigh half
 //   stages          as many as fit in shared memory, at most kMaxStages
-// Dynamic shared memory a CTA may take: all of an SM's, or its share where several CTAs live on one SM together
-// (the system keeps 1 KB per CTA).
-int smem_limit(int fmt, int M) {
-  const int share = dg::ctas_per_sm(fmt, M);
-  return share == 1 ? dg::kSmemLimit : ((dg::kSmemLimit + 1024) / share - 1024) & ~127;
-}
-
-// Bytes of a row's activations kept resident: whole steps of [M][64 * e elements], then a flag byte per step.
-int resident_bytes_of(int fmt, int M, int nblk) {
-  const int row_steps = ceil_div(nblk, 32);
-  return row_steps * M * 64 * kFormats[fmt].e + ((row_steps + 15) & ~15);
-}
-
+// Activations stay resident where that leaves three stages of two steps (from three rows on, where they would take a fifth
+// and more of a stage, also with four stages of one); otherwise a window of them passes through every stage.
 // `grid` > 0: the launch is a batch's (that many CTAs whatever N; the caller sizes the ring for all its GEMVs and
-// decides about resident activations: `allow_resident` is its wish, and no stage rule is applied here).
+// decides about resident activations: `allow_resident` is its wish, and no rule about stages is applied here).
 bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int& smem, int grid = 0,
                bool allow_resident = true) {
   const FormatInfo f = kFormats[fmt];
-  const int cw = dg::consumer_warps(fmt, M);
   const long long row_bits = (long long)K * 128 / f.e;   // 16 bytes per e elements
   p.row_bytes = (int)(row_bits / 8);
   p.nblk = p.row_bytes / 16;
-  const int share = dg::ctas_per_sm(fmt, M);   // CTAs that live on one SM together
-  sms *= share;
+  p.M = M;
+  const int regions = p.pairs ? 2 : 1;    // N counts columns; gate_up matrices have two rows to a column
   ctas = grid > 0 ? grid : sms < ceil_div(N, 4) ? sms : ceil_div(N, 4);   // grid: the launch is shared (batch)
-  const int rows_per_cta = ceil_div(N, ctas);
-  const int per_warp = ceil_div(rows_per_cta, cw);
-  int rmax = dg::rows_max(fmt, M);
-  // Tuning aid: DG_FORCE_PLAN="rows,steps" caps the rows per warp and fixes the steps per stage (read once).
+  const int cols_per_cta = ceil_div(N, ctas), all_rows = regions * ceil_div(cols_per_cta, dg::kBoxRows) * dg::kBoxRows;
+  const int row_steps = ceil_div(p.row_bytes, f.step);
+  // Tuning aid: DG_FORCE_PLAN="rows,steps" fixes the rows of a tile and the steps of a stage (read once).
   static const char* forced = std::getenv("DG_FORCE_PLAN");
   int force_rows = 0, force_steps = 0;
-  if (forced && std::sscanf(forced, "%d,%d", &force_rows, &force_steps) >= 1 && force_rows >= 1 && force_rows < rmax)
-    rmax = force_rows;
-  p.rows_per_warp = per_warp < rmax ? per_warp : rmax;
-  if (p.pairs) p.rows_per_warp = p.rows_per_warp >= 4 ? 4 : 2;   // gate and up rows side by side: an even count
-  const int rows_cap = cw * p.rows_per_warp;
-  const int w_step = rows_cap * (dg::kStepBytes + f.scb);   // sizing estimate; the exact stage size is below
-  const int row_steps = ceil_div(p.nblk, 32);
-  // The ring for activations that pass through the stages (x_step bytes of every step) or stay resident behind it
-  // (x_step = 0, resident_bytes taken from the ring's room).
-  const int pairs_bytes = p.pairs ? dg::kMeetBytes : 0;   // the SwiGLU epilogue's meeting place, behind the ring
-  auto ring = [&](int x_step, int resident_bytes, int& steps, int& stage_bytes) {
-    steps = ceil_div(32768, w_step);
-    if (steps < 2) steps = 2;
-    if (steps > 4) steps = 4;   // a tensor-copy box is at most 256 eight-byte elements (2 KB) wide
-    // BF16 rows are the longest per K: 1.5 KB pieces in two deep stages measured up to 14 % faster than 1 KB pieces
-    // in three (8192 x 28672, M = 2: 82.9 -> 72.7 us; M = 1 unchanged), FP8 the other way round
-    if (fmt == dg::FMT_BF16 && dg::shape_class(fmt, M) == 0 && steps < 3) steps = 3;
-    if (steps > row_steps) steps = row_steps;
-    while (steps > 1 && steps * x_step > 32768) --steps;
-    if (force_steps >= 1) steps = force_steps < row_steps ? force_steps : row_steps;
-    if (steps > 8) steps = 8;
-    if (steps < 1) steps = 1;
-    stage_bytes = (steps * (rows_cap * dg::kStepBytes + x_step) +
-                   p.rows_per_warp * dg::scale_group_bytes(cw, steps, f.scb) + 127) & ~127;
-    int stages = (smem_limit(fmt, M) - dg::kSmemHeader - pairs_bytes - resident_bytes) / stage_bytes;
-    return stages > dg::kMaxStages ? dg::kMaxStages : stages;
-  };
-  int steps = 0, stage_bytes = 0;
-  int stages = ring(M * 64 * f.e, 0, steps, stage_bytes);
-  // Activations that are small enough stay in shared memory for the whole kernel instead of passing through the
-  // stages, unless that costs the ring its third stage.
+  if (forced) std::sscanf(forced, "%d,%d", &force_rows, &force_steps);
   const int resident_bytes = resident_bytes_of(fmt, M, p.nblk);
-  p.x_resident = 0;
   // (a batch shares one ring and one resident area between GEMVs of different K: only the smaller ones stay resident)
-  if (allow_resident && dg::resident_capable(fmt, M) &&
-      resident_bytes <= (grid > 0 ? dg::kResidentLimit / 2 - 15 * 1024 : dg::kResidentLimit)) {
-    int steps_r = 0, stage_bytes_r = 0;
-    const int stages_r = ring(0, resident_bytes, steps_r, stage_bytes_r);
-    if (grid > 0 || stages_r >= 3 || stages_r >= stages) {
-      p.x_resident = 1;
-      steps = steps_r; stage_bytes = stage_bytes_r; stages = stages_r;
+  // (one row's activations are a thirtieth of a stage: not worth a lower tile)
+  const int room = dg::kSmemLimit - dg::kSmemHeader;
+  const bool may_reside = allow_resident && dg::resident_capable(fmt, M) && K % 64 == 0 &&
+                          resident_bytes <= (grid > 0 ? dg::kResidentLimit / 2 - 15 * 1024 : dg::kResidentLimit) &&
+                          (M > 1 || 3 * 56 * (dg::weight_pitch(fmt, 2) + dg::scale_pitch(fmt, 2)) + resident_bytes <= room);
+  int best_cost = 0, best_rem = 0;
+  p.tile_rows = 0;
+  // resident with two steps, with one, not resident with two, with one: the first that has the stages it asks for
+  for (int attempt = may_reside ? 0 : 2; attempt < 4 && p.tile_rows == 0; ++attempt) {
+    const bool resident = attempt < 2;
+    const int steps = fmt == dg::FMT_BF16 ? 1 : 2 - attempt % 2;
+    // (a batch's GEMVs share one instance: the same steps for all, whatever their K)
+    if (grid > 0 ? steps != (M <= 4 ? 2 : 1) : force_steps > 0 ? steps != std::min(force_steps, row_steps)
+                                                               : steps == 2 && row_steps == 1 && fmt != dg::FMT_BF16) continue;
+    const int need = grid > 0 || force_steps > 0 ? 2 : attempt == 0 ? 3 : attempt == 1 ? (M >= 3 ? 4 : dg::kMaxStages + 1)
+                                                     : attempt == 2 ? 3 : 2;
+    const int convert = resident || fmt == dg::FMT_BF16 ? 0 : M <= 8 ? 5 : 7;   // of a tile, in halves of a group
+    for (int rows = 64; rows >= 40; rows -= 8) {
+      int tile_rows = std::min(force_rows >= 16 && force_rows <= 64 ? force_rows & ~7 : rows, all_rows);
+      if (p.pairs) tile_rows &= ~15;                            // the same for both regions
+      int stage_bytes = tile_rows * (dg::weight_pitch(fmt, steps) + dg::scale_pitch(fmt, steps));
+      if (!resident) stage_bytes = dg::x_offset(stage_bytes) + steps * M * f.x_row;
+      const int unit = resident ? 128 : 1024;
+      stage_bytes = (stage_bytes + unit - 1) / unit * unit;
+      const int stages = std::min((room - (resident ? resident_bytes : 0)) / stage_bytes, dg::kMaxStages);
+      if (stages < need) continue;
+      const int cap = tile_rows / regions, tiles = ceil_div(cols_per_cta, cap), rem = cols_per_cta - (tiles - 1) * cap;
+      const int eights = (tiles - 1) * tile_rows / 8 + ceil_div((regions - 1) * cap + rem, 8);
+      const int cost = eights + (1 + convert) * tiles;
+      // (of equals the one whose last tile is the fullest: a window of a few rows takes as long as its latency)
+      if (p.tile_rows == 0 || cost < best_cost || (cost == best_cost && rem > best_rem)) {
+        best_cost = cost;
+        best_rem = rem;
+        p.tile_rows = tile_rows;
+        p.last_rows = ceil_div(rem, dg::kBoxRows) * dg::kBoxRows;
+        p.steps = steps;
+        p.stage_bytes = stage_bytes;
+        p.stages = stages;
+        p.x_mode = resident ? dg::X_RESIDENT : K % 64 == 0 ? dg::X_TENSOR : dg::X_COPIED;
+      }
     }
   }
-  if (stages < 2) return false;
-  p.steps = steps;
-  p.stage_bytes = stage_bytes;
-  p.stages = stages;
-  p.x_res_off = dg::kSmemHeader + stages * stage_bytes + pairs_bytes;
-  smem = p.x_res_off + (p.x_resident ? resident_bytes : 0);
+  if (p.tile_rows == 0) return false;
+  p.x_res_off = dg::kSmemHeader + p.stages * p.stage_bytes;
+  smem = p.x_res_off + (p.x_mode == dg::X_RESIDENT ? resident_bytes : 0);
   return true;
 }
 
@@ -227,17 +240,25 @@ int prepare(int fmt, Params& p, int M, int& ctas, int& smem, int grid = 0, bool 
   if (!st) return (int)cudaErrorInvalidDevice;
   if (!make_plan(fmt, M, p.N, p.K, st->sms, p, ctas, smem, grid, allow_resident)) return (int)cudaErrorInvalidValue;
   p.status = st->status;
-  // Tensor maps for the 2-D copies of full row groups; without them every row travels as a 1-D bulk copy.
-  const int cw = dg::consumer_warps(fmt, M);
-  const int win_bytes = p.steps * dg::kStepBytes;
+  // Tensor maps for the copies of whole boxes and of the activations' windows.
   const int matrix_rows = p.pairs ? 2 * p.pairs : p.N;
-  p.use_2d = matrix_rows >= cw && encode_rows(&p.tmap_w, p.w, matrix_rows, p.row_bytes, cw, win_bytes);
-  if (p.use_2d && p.scale_mode == dg::SCALES_STAGED)
-    p.use_2d = encode_rows(&p.tmap_sc, p.scales, matrix_rows, p.scale_row_bytes, cw, p.steps * kFormats[fmt].scb);
+  const int full_rows = p.tile_rows / (p.pairs ? 2 : 1), w_box = dg::weight_pitch(fmt, p.steps), sc_box = dg::scale_pitch(fmt, p.steps);
+  if (!encode_rows(&p.tmap_w, p.w, matrix_rows, p.row_bytes, full_rows, w_box) ||
+      !encode_rows(&p.tmap_w_last, p.w, matrix_rows, p.row_bytes, p.last_rows, w_box) ||
+      (p.scale_mode == dg::SCALES_STAGED &&
+       (!encode_rows(&p.tmap_sc, p.scales, matrix_rows, p.scale_row_bytes, full_rows, sc_box) ||
+        !encode_rows(&p.tmap_sc_last, p.scales, matrix_rows, p.scale_row_bytes, p.last_rows, sc_box))))
+    return (int)cudaErrorNotSupported;
+  if (p.x_mode != dg::X_COPIED) {
+    const int step_blocks = kFormats[fmt].x_row / 128, steps = ceil_div(p.row_bytes, kFormats[fmt].step);
+    p.x_box_steps = std::min(steps, 256 / step_blocks);           // whole boxes only: the space ends with the last step
+    while (steps % p.x_box_steps) --p.x_box_steps;
+    const bool resident = p.x_mode == dg::X_RESIDENT;
+    if (!encode_activations(&p.tmap_x, p.x, M, p.K, p.ldx, (resident ? p.x_box_steps : p.steps) * step_blocks, !resident))
+      return (int)cudaErrorNotSupported;
+  }
   p.early_weights = g_static_weights.load(std::memory_order_relaxed);
   p.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
-  static const bool no_split = std::getenv("DG_NO_SPLIT_TAIL") != nullptr;   // tuning aid
-  p.split_tail = M == 1 && !no_split;
   return 0;
 }
 
@@ -269,8 +290,7 @@ int launch(int table, int fmt, Params& p, int M, cudaStream_t stream) {
       p.trace = base + (size_t)index * DG_TRACE_CTAS * dg::kTraceSlots;
   }
   void* args[] = {&p};
-  const int threads = 32 * (dg::consumer_warps(fmt, M) + dg::producer_warps(fmt, M));
-  return launch_pdl(kTables[table][M - 1], args, ctas, threads, smem, stream);
+  return launch_pdl(kTables[table][p.steps - 1][M - 1], args, ctas, dg::kThreads, smem, stream);
 }
 
 // Argument rules of the NVFP4 GEMV (dg_enqueue_nvfp4) and the fields they determine.
@@ -297,7 +317,7 @@ constexpr unsigned int kBatchMagic = 0x44474231u;   // "DGB1"
 constexpr size_t kBatchHead = 256;
 struct BatchHead {
   unsigned int magic;
-  int count, M, ctas, smem, threads, device;
+  int count, M, steps, ctas, smem, threads, device;
   const void* device_blob;
 };
 static_assert(sizeof(BatchHead) <= kBatchHead && kBatchHead % alignof(Params) == 0, "batch head layout");
@@ -424,9 +444,7 @@ int dg_enqueue_nvfp4_gate_up_swiglu(const void* x, int ldx, int x_is_bf16, const
     return (int)cudaErrorInvalidValue;
   p.out = out; p.ldo = ldo;
   p.pairs = I;
-  // the tiles walk whole blocks of gate rows and up rows in turn: N counts the rows in that order
-  const int cw = dg::consumer_warps(dg::FMT_NVFP4, M);
-  p.N = 2 * ((I + cw - 1) / cw) * cw;
+  p.N = I;                 // (output columns)
   return launch(x_is_bf16 ? 5 : 6, dg::FMT_NVFP4, p, M, static_cast<cudaStream_t>(stream));
 }
 
@@ -443,10 +461,9 @@ int dg_encode_nvfp4_batch(const DgNvfp4BatchItem* items, int count, int x_is_bf1
   BatchHead head{};
   Params* out = reinterpret_cast<Params*>(static_cast<unsigned char*>(host_blob) + kBatchHead);
   int stage_bytes = 0, resident_bytes = 0, stages = 0;
-  // One ring for all: the largest stage any GEMV needs, as many of them as fit. Behind the ring: room for one GEMV's
-  // parameters (kernels without producer warps keep them there), then room for the largest resident activations
-  // (every GEMV brings its own when its turn comes). If the resident ones cost the ring its third stage, once more
-  // without them.
+  // One ring for all: the largest stage any GEMV needs, as many of them as fit. Behind the ring: room for the largest
+  // resident activations (every GEMV brings its own when its turn comes). If the resident ones cost the ring its third
+  // stage, once more without them.
   for (int attempt = 0; attempt < 2; ++attempt) {
     stage_bytes = 0; resident_bytes = 0;
     for (int g = 0; g < count; ++g) {
@@ -470,14 +487,14 @@ int dg_encode_nvfp4_batch(const DgNvfp4BatchItem* items, int count, int x_is_bf1
       }
       int ctas = 0, smem = 0;
       // one grid for all: a CTA per SM, whatever a GEMV's size (a CTA without rows of a GEMV passes it by)
-      if (const int code = prepare(dg::FMT_NVFP4, p, M, ctas, smem, st->sms * dg::ctas_per_sm(dg::FMT_NVFP4, M),
+      if (const int code = prepare(dg::FMT_NVFP4, p, M, ctas, smem, st->sms,
                                    attempt == 0))
         return code;
-      if (p.stage_bytes > stage_bytes) stage_bytes = p.stage_bytes;
-      if (p.x_resident) resident_bytes = std::max(resident_bytes, resident_bytes_of(dg::FMT_NVFP4, M, p.nblk));
+      stage_bytes = std::max(stage_bytes, (p.stage_bytes + 1023) & ~1023);   // (where stages hold activations)
+      if (p.x_mode == dg::X_RESIDENT) resident_bytes = std::max(resident_bytes, resident_bytes_of(dg::FMT_NVFP4, M, p.nblk));
       out[g] = p;
     }
-    stages = (smem_limit(dg::FMT_NVFP4, M) - dg::kSmemHeader - (int)sizeof(Params) - resident_bytes) / stage_bytes;
+    stages = (dg::kSmemLimit - dg::kSmemHeader - resident_bytes) / stage_bytes;
     if (stages > dg::kMaxStages) stages = dg::kMaxStages;
     if (resident_bytes == 0 || stages >= 3) break;
   }
@@ -485,11 +502,11 @@ int dg_encode_nvfp4_batch(const DgNvfp4BatchItem* items, int count, int x_is_bf1
   for (int g = 0; g < count; ++g) {
     out[g].stage_bytes = stage_bytes;
     out[g].stages = stages;
-    out[g].x_res_off = dg::kSmemHeader + stages * stage_bytes + (int)sizeof(Params);
+    out[g].x_res_off = dg::kSmemHeader + stages * stage_bytes;
   }
-  head.magic = kBatchMagic; head.count = count; head.M = M; head.ctas = st->sms * dg::ctas_per_sm(dg::FMT_NVFP4, M);
-  head.smem = dg::kSmemHeader + stages * stage_bytes + (int)sizeof(Params) + resident_bytes;
-  head.threads = 32 * (dg::consumer_warps(dg::FMT_NVFP4, M) + dg::producer_warps(dg::FMT_NVFP4, M));
+  head.magic = kBatchMagic; head.count = count; head.M = M; head.steps = out[0].steps; head.ctas = st->sms;
+  head.smem = dg::kSmemHeader + stages * stage_bytes + resident_bytes;
+  head.threads = dg::kThreads;
   head.device_blob = device_blob;
   cudaGetDevice(&head.device);
   *reinterpret_cast<BatchHead*>(host_blob) = head;
@@ -500,14 +517,15 @@ int dg_enqueue_batch(const void* host_blob, void* stream) {
   if (!host_blob) return (int)cudaErrorInvalidValue;
   const BatchHead head = *reinterpret_cast<const BatchHead*>(host_blob);
   int device = -1;
-  if (head.magic != kBatchMagic || head.count < 1 || head.M < 1 || head.M > DG_MAX_ROWS ||
+  if (head.magic != kBatchMagic || head.count < 1 || head.M < 1 || head.M > DG_MAX_ROWS || head.steps < 1 ||
+      head.steps > 2 ||
       cudaGetDevice(&device) != cudaSuccess || device != head.device)
     return (int)cudaErrorInvalidValue;
   if (!device_state()) return (int)cudaErrorInvalidDevice;
   const Params* items = reinterpret_cast<const Params*>(static_cast<const unsigned char*>(head.device_blob) + kBatchHead);
   int count = head.count;
   void* args[] = {&items, &count};
-  return launch_pdl(dg_batch_table_nvfp4_bf16[head.M - 1], args, head.ctas, head.threads, head.smem,
+  return launch_pdl(dg_batch_table_nvfp4_bf16[head.steps - 1][head.M - 1], args, head.ctas, head.threads, head.smem,
                     static_cast<cudaStream_t>(stream));
 }
 
@@ -554,7 +572,7 @@ int dg_plan(int fmt, int M, int N, int K, int plan[6]) {
   p.N = N; p.K = K;
   int ctas = 0, smem = 0;
   if (!make_plan(fmt, M, N, K, sms, p, ctas, smem)) return (int)cudaErrorInvalidValue;
-  plan[0] = ctas; plan[1] = p.rows_per_warp; plan[2] = p.steps; plan[3] = p.stages; plan[4] = p.stage_bytes;
+  plan[0] = ctas; plan[1] = ceil_div(p.tile_rows, dg::kGroupRows); plan[2] = p.steps; plan[3] = p.stages; plan[4] = p.stage_bytes;
   plan[5] = smem;
   return 0;
 }

@@ -29,17 +29,16 @@ __device__ __forceinline__ float e4m3_to_f32(uint32_t byte) {
   return __half2float(*reinterpret_cast<const __half*>(&h));
 }
 
-__device__ __forceinline__ void unpack2(dg::pk2 a, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
-}
-
 // 8 codes (word c, element 2i in the low nibble of byte i) -> 8 FP32 values: (e2m1 * scale) * factor.
 __device__ __forceinline__ void values8(uint32_t c, float scale, float factor, float (&v)[8]) {
-  dg::pk2 w[4];
-  dg::decode_e2m1(c, w);                                   // (element 2q, element 2q + 1) of byte q
+  uint32_t h[4];
+  dg::decode_e2m1_h(c, h);                                 // (element 2q, element 2q + 1) of byte q
   const dg::pk2 s2 = dg::pack2(scale, scale), f2 = dg::pack2(factor, factor);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) unpack2(dg::fmul2(dg::fmul2(w[q], s2), f2), v[2 * q], v[2 * q + 1]);
+  for (int q = 0; q < 4; ++q) {
+    const float2 w = __half22float2(*reinterpret_cast<const __half2*>(&h[q]));
+    dg::unpack2(dg::fmul2(dg::fmul2(dg::pack2(w.x, w.y), s2), f2), v[2 * q], v[2 * q + 1]);
+  }
 }
 
 template <int OUT>

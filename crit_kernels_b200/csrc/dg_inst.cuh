@@ -1,18 +1,15 @@
-// Expands to the table of the sixteen kernels (M = 1..16) of one format and activation type.
+// Expands to the table of the kernels of one format and activation type, by steps per stage (1, 2) and activation rows
+// (1..16): instances for 1-4, 5-8 and 9-16 rows. BF16 has stages of one step only.
 #pragma once
 #include "dg_kernel.cuh"
 #include "dg_tables.h"
 
-#define DG_K(FMT, M, XT) reinterpret_cast<const void*>(&dg::gemv_kernel<FMT, M, XT>)
-#define DG_TABLE(NAME, FMT, XT)                                                                                     \
-  const void* const NAME[16] = {DG_K(FMT, 1, XT),  DG_K(FMT, 2, XT),  DG_K(FMT, 3, XT),  DG_K(FMT, 4, XT),          \
-                                DG_K(FMT, 5, XT),  DG_K(FMT, 6, XT),  DG_K(FMT, 7, XT),  DG_K(FMT, 8, XT),          \
-                                DG_K(FMT, 9, XT),  DG_K(FMT, 10, XT), DG_K(FMT, 11, XT), DG_K(FMT, 12, XT),         \
-                                DG_K(FMT, 13, XT), DG_K(FMT, 14, XT), DG_K(FMT, 15, XT), DG_K(FMT, 16, XT)};
-
-#define DG_KB(FMT, M, XT) reinterpret_cast<const void*>(&dg::gemv_batch_kernel<FMT, M, XT>)
-#define DG_BATCH_TABLE(NAME, FMT, XT)                                                                               \
-  const void* const NAME[16] = {DG_KB(FMT, 1, XT),  DG_KB(FMT, 2, XT),  DG_KB(FMT, 3, XT),  DG_KB(FMT, 4, XT),      \
-                                DG_KB(FMT, 5, XT),  DG_KB(FMT, 6, XT),  DG_KB(FMT, 7, XT),  DG_KB(FMT, 8, XT),      \
-                                DG_KB(FMT, 9, XT),  DG_KB(FMT, 10, XT), DG_KB(FMT, 11, XT), DG_KB(FMT, 12, XT),     \
-                                DG_KB(FMT, 13, XT), DG_KB(FMT, 14, XT), DG_KB(FMT, 15, XT), DG_KB(FMT, 16, XT)};
+#define DG_ROWS(A, B, C) {A, A, A, A, B, B, B, B, C, C, C, C, C, C, C, C}
+#define DG_K(KERNEL, FMT, NT, M, STEPS, XT)                                                                         \
+  reinterpret_cast<const void*>(&dg::KERNEL<FMT, NT, dg::resident_capable(FMT, M), (FMT) == dg::FMT_BF16 ? 1 : STEPS, XT>)
+#define DG_STEPS(KERNEL, FMT, STEPS, XT)                                                                            \
+  DG_ROWS(DG_K(KERNEL, FMT, 1, 1, STEPS, XT), DG_K(KERNEL, FMT, 1, 5, STEPS, XT), DG_K(KERNEL, FMT, 2, 9, STEPS, XT))
+#define DG_TABLE(NAME, FMT, XT) \
+  const void* const NAME[2][16] = {DG_STEPS(gemv_kernel, FMT, 1, XT), DG_STEPS(gemv_kernel, FMT, 2, XT)};
+#define DG_BATCH_TABLE(NAME, FMT, XT) \
+  const void* const NAME[2][16] = {DG_STEPS(gemv_batch_kernel, FMT, 1, XT), DG_STEPS(gemv_batch_kernel, FMT, 2, XT)};

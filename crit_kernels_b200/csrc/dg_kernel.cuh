@@ -5,24 +5,21 @@
 // :191 bf16_kernel, :285 fp8_kernel). Same formats, same contract (FP32 sums whose order never depends on the row
 // count), a different machine mapping:
 //
-//   * one persistent CTA per SM: C consumer warps + P producer warps (12 + 4 down to 8 + 0, by format and M). The matrix
-//     rows are split into one contiguous range per CTA; a range is walked in tiles of C*r rows (r rows per consumer
-//     warp) and each tile in K windows.
-//   * the producer warps stream every window of a tile into a shared-memory ring: one cp.async.bulk (TMA 1-D bulk
-//     copy, mbarrier complete_tx) per weight row (and per row of block scales), issued by the producers' lanes in
-//     parallel, plus the matching window of the activations as 16-byte cp.async copies into a bank-swizzled layout.
-//     Bytes in flight are set by the ring (up to ~200 KB per SM), not by registers. Where the arithmetic, not HBM,
-//     is the limit (larger M) the CTA has no producer warp: its consumer warps issue the same copies between stages.
-//   * consumer warp w owns rows w, w+C, ... of the tile. Lane l owns the 16-byte blocks l, l+32, ... of each row and
-//     keeps two FP32 chains per (row, m): even and odd elements, advanced together by one packed fma.rn.f32x2 or, where
-//     the arithmetic is the limit, by two mixed-precision fma.rn.f32.bf16 / .f16 (same bits: the products are exact).
-//     The chains visit the blocks in ascending order, the two chains are added, and one xor-shuffle tree (16, 8, 4, 2,
-//     1) adds the lanes; the row scale multiplies once and the result is rounded once to the output type.
+//   * one persistent CTA per SM: 8 consumer warps + 4 producer warps. The matrix rows are split into one contiguous
+//     range per CTA; a range is walked in tiles of up to 16 * kMaxGroups rows and each tile in K windows.
+//   * the producer warps stream every window of a tile into a shared-memory ring: whole boxes of 8 rows as one tensor
+//     copy (TMA, mbarrier complete_tx) each, a tile's last few rows as one 1-D bulk copy per row, block scales the same
+//     way, plus the matching window of the activations as 16-byte cp.async copies into a bank-swizzled layout. Bytes in
+//     flight are set by the ring (up to ~200 KB per SM), not by registers.
+//   * a 512-byte step of a row is eight chunks of 64 bytes; consumer warp w owns chunk w of every step, for all rows of
+//     the tile, and multiplies it on the tensor cores (dg_mma.cuh): the activations of a chunk are then loaded and
+//     converted by one warp, once per tile. At the end of a tile the eight warps' sums of every output meet in shared
+//     memory (in the ring stage just consumed) and are added in a fixed tree; the row scale multiplies once and the
+//     result is rounded once to the output type.
 //
 // A row's summation order is therefore a function of K and the format alone: it does not depend on M, on the rows a
-// warp holds, on the tile or window sizes the launch picked, on the CTA count, or on which slice of the matrix a
-// device holds. Every product is exact in FP32 (weights and block scales have few significant bits), NVFP4 block
-// scales multiply a 16-element partial sum (one fma per block and row instead of one multiply per weight).
+// tile holds, on the tile or window sizes the launch picked, on the CTA count, or on which slice of the matrix a
+// device holds.
 #pragma once
 
 #include <cuda.h>   // CUtensorMap (type only; the driver entry point is looked up at run time)
@@ -34,6 +31,8 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "dg_lane_reduce.cuh"
+#include "dg_mma.cuh"
 #include "dg_swiglu.cuh"
 
 namespace dg {
@@ -43,11 +42,17 @@ enum : int { SCALES_NONE = 0, SCALES_STAGED = 1, SCALES_DIRECT = 2, SCALES_BLOCK
 enum : int { OUT_F32 = 0, OUT_BF16 = 1, OUT_F16 = 2 };
 
 constexpr int kMaxStages = 12;
-constexpr int RMAX_ALL = 4;                // most rows a consumer warp holds in any kernel
-constexpr int kMeetBytes = 16 * RMAX_ALL * 16 * 4;   // SwiGLU epilogue: 16 warps x (4 rows x 16 activation rows) FP32
-constexpr int kStepBytes = 512;            // 32 lanes x 16 bytes of one weight row
+constexpr int kConsumers = 8;              // = chunks of a step: the slices of K whose sums are added at the end
+// Warps of a block: the consumers, one that feeds the ring, and three that finish tiles; in launches with something to copy
+// that bulk copies cannot bring, two of these copy instead.
+constexpr int kFeeder = kConsumers, kFinisher = kConsumers + 1, kFinishers = 3, kFirstCopier = kConsumers + 2, kCopyWarps = 2;
+constexpr int kThreads = 32 * (kConsumers + 1 + kFinishers);
+constexpr int kBoxRows = 8;                // tile rows come in multiples of these
+constexpr int kGroupRows = 16;             // rows of one mma tile
+constexpr int kMaxGroups = 4;              // mma tiles of rows a warp holds at most
 constexpr int kSmemHeader = 256;           // mbarriers + abort flag
-constexpr int kSmemLimit = 232448;         // 227 KB of dynamic shared memory per CTA on sm_100
+constexpr int kStaticSmem = 1024;          // room left for the kernels' static shared memory (kMaxMarks, kMaxStages)
+constexpr int kSmemLimit = 232448 - kStaticSmem;   // dynamic shared memory per CTA (sm_100 has 227 KB in all)
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;   // bounded waits give up after this (default; the host
                                                              // can set another limit, Params::wait_limit_ns)
 
@@ -61,108 +66,40 @@ constexpr int kMaxRanks = 8;
 constexpr int kTraceSlots = 8;
 enum : int { TRACE_ENTRY = 0, TRACE_DEP = 1, TRACE_FIRST_FULL = 2, TRACE_LAST_CONSUMED = 3, TRACE_EXIT = 4, TRACE_SM = 5 };
 
+// E: elements of a 16-byte block; STEP: bytes of one step of a row (eight chunks, one per consumer warp; BF16's are twice
+// as long, so that its sums take no more additions than the other formats'); SCB: scale bytes of one step; PAD: bytes a row's window is stored apart
+// beyond its length, so that the eight lanes of one shared-memory access phase fall into different banks (two rows'
+// 64-byte chunks, four rows' 32-byte blocks for MXFP8). The copies bring the padding from the next window.
 template <int FMT> struct Format;
-template <> struct Format<FMT_BF16>  { static constexpr int E = 8,  SCB = 0;  };   // elements / scale bytes per
-template <> struct Format<FMT_FP8>   { static constexpr int E = 16, SCB = 0;  };   // 16-byte block and per 512-byte
-template <> struct Format<FMT_MXFP8> { static constexpr int E = 16, SCB = 16; };   // step of one row
-template <> struct Format<FMT_NVFP4> { static constexpr int E = 32, SCB = 64; };
+template <> struct Format<FMT_BF16>  { static constexpr int STEP = 1024, E = 8,  SCB = 0,  PAD = 16;  static constexpr int XROW = STEP / 16 * E * 2; };
+template <> struct Format<FMT_FP8>   { static constexpr int STEP = 512, E = 16, SCB = 0,  PAD = 16;  static constexpr int XROW = STEP / 16 * E * 2; };
+template <> struct Format<FMT_MXFP8> { static constexpr int STEP = 512, E = 16, SCB = 16, PAD = 32;  static constexpr int XROW = STEP / 16 * E * 2; };
+template <> struct Format<FMT_NVFP4> { static constexpr int STEP = 512, E = 32, SCB = 64, PAD = 16;  static constexpr int XROW = STEP / 16 * E * 2; };
+constexpr int kScalePad = 16;
 
-// CTA shape per (format, M): a speed choice, never a row's bits. Register need decides it: the accumulators take
-// 2 * rows * M registers and the held operand (activations or decoded weights) 8-16 per activation row or weight row.
-//   class 0   M small: the kernel is HBM-bound. 12 consumer + 4 producer warps (14 + 2 where two_producers says so;
-//             128 registers each): as many warps
-//             as the register file gives, to hide shared-memory and conversion latencies; every SM sub-partition
-//             hosts the same number of consumers.
-//   class 1   M medium: 11 consumer + 1 producer warps, or 12 consumer warps that issue the copies themselves
-//             (168 registers each).
-//   class 2   M large: the kernel is FP32-FMA-bound. No producer warp; 8 to 16 consumer warps by (format, M), see
-//             class2_warps / class2_rows.
-//             In classes 1 and 2 the consumers' instruction issue is the limit and a sub-partition's time is that of
-//             the consumers it hosts, so the consumers should be spread evenly: one producer warp keeps up with the
-//             copies and leaves one sub-partition a consumer short (measured against 10 + 2 and 6 + 2 warps: 4-8 %
-//             and 10-17 % faster); no producer warp at all leaves none short but adds the copies to the consumers'
-//             instruction streams (measured against 11 + 1 and 7 + 1: class 2 up to 14 % faster, never slower;
-//             class 1 4-8 % faster for BF16 and MXFP8, 3-6 % slower for FP8 and NVFP4, which keep the producer).
-//             Moving the class limits either way measured 15-30 % slower.
-// Classes 0 and 1 hold the converted activations of a block and stream the rows past them; class 2 holds the rows'
-// decoded weights and streams the activation rows.
-// One warp issues a 1-D bulk copy only every ~60 clocks, so full groups of rows travel as one 2-D tensor copy and
-// only a tile's ragged remainder as per-row copies.
-__host__ __device__ constexpr int shape_class(int fmt, int m) {
-  return fmt == FMT_NVFP4 ? (m <= 2 ? 0 : m <= 4 ? 1 : 2) : (m <= 4 ? 0 : m <= 8 ? 1 : 2);
+// Shared-memory distance of two rows of a window of `steps` steps: weights, and staged scales.
+__host__ __device__ constexpr int step_bytes(int fmt) { return fmt == FMT_BF16 ? 1024 : 512; }
+__host__ __device__ constexpr int weight_pitch(int fmt, int steps) { return steps * step_bytes(fmt) + (fmt == FMT_MXFP8 ? 32 : 16); }
+__host__ __device__ constexpr int scale_pitch(int fmt, int steps) {
+  return fmt == FMT_NVFP4 ? steps * 64 + kScalePad : fmt == FMT_MXFP8 ? steps * 16 + kScalePad : 0;
 }
-// CTAs that share an SM (each with its share of the shared memory; the grid is this many per SM). BF16 class 0 runs
-// two CTAs of 7 + 1 warps: the next kernel's CTA moves in and starts its copies as soon as the first of the two
-// leaves (3-7 % faster over back-to-back calls at 8192 x 8192 than one CTA of 14 + 2; the other formats measured
-// 10-20 % slower as two CTAs of 6 + 2 than as one of 12 + 4).
-__host__ __device__ constexpr int ctas_per_sm(int fmt, int m) { return fmt == FMT_BF16 && shape_class(fmt, m) == 0 ? 2 : 1; }
-__host__ __device__ constexpr bool few_rows(int fmt, int m) { return shape_class(fmt, m) < 2; }
-// (BF16 weights, the lightest arithmetic per byte, measured 13-19 % faster with 14 + 2 warps per SM than with 12 + 4;
-// they run as two CTAs of 7 + 1, see ctas_per_sm.)
-// class 1 of the formats with the lighter arithmetic per byte (BF16, MXFP8) and class 2 of all: no producer warp.
-__host__ __device__ constexpr bool self_fed(int fmt, int m) {
-  return shape_class(fmt, m) == 2 || (shape_class(fmt, m) == 1 && (fmt == FMT_BF16 || fmt == FMT_MXFP8));
-}
-// Class 2 by (format, M), measured on 28672 x 8192 (16384 x 8192 for BF16) over the candidates 8 warps x 4 rows,
-// 12 x 3, 12 x 4 and 16 x 2 (255, 168, 168 and 128 registers per thread): up to 14 % between them. NVFP4 also on
-// 8192 x 8192, 8192 x 28672 and 57344 x 8192: at M = 8 the 16 x 2 shape is 2 % ahead of 8 x 4 on the large matrices
-// and 20-23 % on the two with 8192 rows (55 rows per CTA).
-// Class 0 with 14 + 2 warps instead of 12 + 4: FP8 and NVFP4 at M <= 2 measured 1.5-2 % faster at 28672 x 8192 and
-// NVFP4 7 % faster at 8192 x 8192 (M = 1); MXFP8 measured 10 % slower at M = 2 and stays.
-__host__ __device__ constexpr bool two_producers(int fmt, int m) { return (fmt == FMT_FP8 || fmt == FMT_NVFP4) && m <= 2; }
-__host__ __device__ constexpr int class2_warps(int fmt, int m) {
-  return fmt == FMT_FP8 ? (m <= 13 ? 12 : 8)
-         : fmt == FMT_BF16 ? (m <= 14 ? 12 : 8)
-         : fmt == FMT_NVFP4 ? (m == 8 || m >= 11 ? 16 : 12) : 8;
-}
-__host__ __device__ constexpr int class2_rows(int fmt, int m) {
-  return fmt == FMT_NVFP4 ? (m == 5 ? 4 : m == 8 || m >= 11 ? 2 : 3) : fmt == FMT_BF16 && m >= 12 && m <= 14 ? 3 : 4;
-}
-__host__ __device__ constexpr int consumer_warps(int fmt, int m) {
-  return shape_class(fmt, m) == 0 ? (fmt == FMT_BF16 ? 7 : two_producers(fmt, m) ? 14 : 12)
-         : shape_class(fmt, m) == 1 ? (self_fed(fmt, m) ? 12 : 11) : class2_warps(fmt, m);
-}
-__host__ __device__ constexpr int producer_warps(int fmt, int m) {
-  return shape_class(fmt, m) == 0 ? (fmt == FMT_BF16 ? 1 : two_producers(fmt, m) ? 2 : 4) : self_fed(fmt, m) ? 0 : 1;
-}
-// Kernels that advance their chains with the mixed-precision FMA instead of the packed FP32 FMA (same bits; see f2):
-// where the arithmetic is the limit, one issue slot per product without any conversion of the activations beats
-// half a slot per product plus the conversions. MXFP8 stays on the FP32 path: its weights carry their block scale,
-// and weight x 2^(e - 127) is not always a BF16 value.
-__host__ __device__ constexpr bool use_mixed(int fmt, int m) {
-  return fmt != FMT_MXFP8 && (shape_class(fmt, m) == 2 || (shape_class(fmt, m) == 1 && fmt != FMT_FP8) ||
-                              (fmt == FMT_BF16 && m <= 2));   // BF16 weights need no conversion at all: M FMAs per
-                                                              // weight against 1 + M / 2 instructions packed
-}
-// Rows a consumer warp holds at once (register budget).
-__host__ __device__ constexpr int rows_max(int fmt, int m) {
-  return shape_class(fmt, m) == 2 ? class2_rows(fmt, m) : 4;
-}
-// Resident activations (Params::x_resident, decided by the launch plan): class 0 of FP8 / NVFP4, where the whole
-// [M][K] activations are small, keeps them in shared memory behind the ring for the whole kernel instead of copying a
-// window of them into every ring stage: the consumer warps fetch them once, while the first weights are on their way.
-// (also NVFP4's class 1, M = 3 and 4: a mixed-FMA kernel whose FP16 steps spare it the weights' conversion to BF16)
-__host__ __device__ constexpr bool resident_capable(int fmt, int m) {
-  return ((fmt == FMT_FP8 || fmt == FMT_NVFP4) && shape_class(fmt, m) == 0) ||
-         (fmt == FMT_NVFP4 && shape_class(fmt, m) == 1);
-}
+// Columns (activation rows, in eights) an instance multiplies.
+__host__ __device__ constexpr int column_tiles(int m) { return m <= 8 ? 1 : 2; }
+__host__ __device__ constexpr bool split_columns(int fmt) { return fmt == FMT_BF16 || fmt == FMT_MXFP8; }   // see fragment_column
+// Ways of the activations into shared memory (Params::x_mode).
+enum : int { X_RESIDENT = 0, X_TENSOR = 1, X_COPIED = 2 };
+
+// Offset of the activations in a stage: the ring starts kSmemHeader bytes into shared memory, stages are multiples of 1024
+// bytes where they hold activations, which must start on such a multiple (the swizzle goes by address).
+__host__ __device__ constexpr int x_offset(int before) { return ((before + kSmemHeader + 1023) & ~1023) - kSmemHeader; }
+
+// Resident activations (X_RESIDENT, decided by the launch plan): FP8 / NVFP4 at up to 4 rows, where the whole
+// [M][K] activations are small, keep them in shared memory behind the ring for the whole kernel instead of copying a
+// window of them into every ring stage: one tensor copy brings them, and the consumer warps put them into the form the
+// tensor cores take (see prepare_resident) while the first weights are on their way.
+__host__ __device__ constexpr bool resident_capable(int fmt, int m) { return (fmt == FMT_FP8 || fmt == FMT_NVFP4) && m <= 4; }
 constexpr int kResidentLimit = 96 * 1024;   // bytes of activations (and their flags) a kernel keeps resident at most
-// How a kernel instance advances its chains, by the activations' type too.
-//   MIXED     the mixed-precision FMA throughout: use_mixed, and every FP16-activation kernel of the formats whose
-//             decoded weights are FP16 values already (E4M3, E2M1): nothing is converted at all.
-//   HALF_RES  BF16 activations of a resident_capable kernel: when the activations are resident, each 512-byte step
-//             of them (64 * E elements of every activation row) is kept as FP16 if every value of it is an FP16
-//             value too (|x| <= 65504, and FP16 carries BF16's 8 significant bits down to 2^-17), and the consumers
-//             run the FP16 mixed-FMA body on that step: about 2 instead of 3.5 instructions per weight at M = 1. A
-//             step with any other value (tiny, huge, infinite, NaN) stays BF16 and takes the kernel's other body
-//             (packed FP32, or the BF16 mixed FMA with converted weights). Every product is exact either way and the
-//             additions are the same, so are the bits.
-template <int FMT, int M, typename XT>
-struct Arithmetic {
-  static constexpr bool HALF_X = std::is_same<XT, __half>::value;
-  static constexpr bool MIXED = use_mixed(FMT, M) || (HALF_X && (FMT == FMT_FP8 || FMT == FMT_NVFP4));
-  static constexpr bool HALF_RES = !HALF_X && resident_capable(FMT, M);
-};
+constexpr int kMaxMarks = kResidentLimit / 2 / 64;   // marks of their (row, chunk)s: an FP8 chunk is 64 elements
 
 struct Params {
   const void* x;             // [M][ldx] BF16 or FP16
@@ -178,21 +115,22 @@ struct Params {
   int scale_row_bytes;       // bytes of one row-major scale row
   int scale_mode;            // SCALES_*
   int ct;                    // tiled scales: 4-block tiles per tile row
+  int M;                     // activation rows
   int steps;                 // 512-byte steps per ring stage
   int stages;                // ring depth
-  int rows_per_warp;         // r: a full tile is (consumer warps) * r rows
+  int tile_rows;             // rows of a full tile (a multiple of 8; gate_up: of 16, for both regions), at most 16 * kMaxGroups
   int stage_bytes;           // bytes of one ring stage
-  int use_2d;                // 1: tmap_w (and tmap_sc when scales are staged) are valid
   int early_weights;         // 1: weight copies may be issued before the previous kernel of the stream completed
-  int split_tail;            // 1: a short last tile and the tile before it are walked as two equal tiles (see Walk)
+  int last_rows;             // rows of the copies of a tile that is not full (per region; a multiple of 8)
   // SwiGLU epilogue (pairs > 0): the matrix is a gate_up projection of 2 * pairs rows, gate rows [0, pairs) and up rows
-  // [pairs, 2 pairs); N counts the rows as the tiles walk them (see Walk). A warp holds row k of both halves side by
-  // side and writes out[m][k] = silu(gate) * up (FP32, one rounding) instead of the two sums: `pairs` columns.
+  // [pairs, 2 pairs); N counts its output columns (= pairs). A tile holds row k of both halves and writes
+  // out[m][k] = silu(gate) * up (FP32, one rounding) instead of the two sums: `pairs` columns.
   int pairs;
-  // Resident activations (resident_capable kernels; 0 = the activations travel through the ring stages): the
-  // kernel's dynamic shared memory holds, x_res_off bytes in, ceil(nblk / 32) steps of [M][64 * E elements] laid out
-  // as in a stage, then one flag byte per step (1 = the step is held as FP16, see Arithmetic::HALF_RES).
-  int x_resident, x_res_off;
+  // Activations: X_RESIDENT (resident_capable; the kernel's dynamic shared memory holds, x_res_off bytes in, the steps of
+  // M x XROW bytes laid out as in a stage, then one flag byte per step, 1 = every chunk of the step is held as FP16), or a
+  // window of them in every ring stage, by one tensor copy (X_TENSOR) or, where K is no multiple of 64, by the copying
+  // warps (X_COPIED).
+  int x_mode, x_res_off;
   unsigned long long* trace; // diagnostic (dg_set_trace): kTraceSlots time stamps per CTA, or null
   unsigned long long wait_limit_ns;   // every wait in the kernel gives up after this long (status word, then leaves)
   // All-gather epilogue (world >= 1, 0 = off): this rank's [M][N] results go into slot `rank` of its own
@@ -203,127 +141,32 @@ struct Params {
   int world, rank, gather_slot, gather_nowait;   // nowait: signal only; dg_enqueue_gather_wait collects later
   void* peer_out[kMaxRanks];
   unsigned int* peer_flag[kMaxRanks];
-  // Tensor maps over the weight rows and the row-major scale rows as 8-byte elements: box = (consumer warps) rows
-  // x one window. Rows are 16-byte multiples apart, which the encoder requires.
-  alignas(64) CUtensorMap tmap_w;
-  alignas(64) CUtensorMap tmap_sc;
+  // Tensor maps over the weight rows and the row-major scale rows as 8-byte elements: box = one window and its padding of
+  // a full tile's rows (per region, see Walk), or of last_rows rows. Rows are 16-byte multiples apart, as the encoder asks.
+  alignas(64) CUtensorMap tmap_w, tmap_w_last, tmap_sc, tmap_sc_last;
+  int x_box_steps;           // X_RESIDENT: steps of one copy of the activations
+  // The activations as [K / 64][M][64 elements]. X_TENSOR: 128-byte swizzled, box = the blocks of one window; X_RESIDENT: as
+  // they are, box = those of x_box_steps steps.
+  alignas(64) CUtensorMap tmap_x;
 };
 
 // ---------------------------------------------------------------------------------------------------------------
 // PTX wrappers: mbarrier, 1-D bulk copy (TMA), 16-byte cp.async tied to an mbarrier.
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Shared-memory loads by 32-bit shared-space address: the ring is addressed with one base register per stage plus
-// constants, instead of 64-bit generic pointer arithmetic per load. Volatile keeps them after the barrier waits.
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
-  uint16_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ uint32_t lds_u8(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-__device__ __forceinline__ void sts_u8(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
 __device__ __forceinline__ uint4 ldg_nc128(const void* ptr) {   // memory nobody writes while the kernel runs
   uint4 v;
   asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(ptr));
   return v;
 }
-
-// Two FP32 values in one 64-bit register pair, the operand form of the packed fma.rn.f32x2 / mul.rn.f32x2. Operands
-// are packed once where they are produced and accumulators stay packed across the whole K loop, so that no
-// pack / unpack moves surround the FMAs (measured: almost one extra instruction per packed FMA otherwise).
-struct pk2 { unsigned long long v; };
-__device__ __forceinline__ pk2 pack2(float lo, float hi) {
-  pk2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ pk2 pack2_bits(uint32_t lo, uint32_t hi) {
-  pk2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "r"(lo), "r"(hi));
-  return r;
-}
-__device__ __forceinline__ float sum2(pk2 a) {   // low + high
-  float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
-  return lo + hi;
-}
-__device__ __forceinline__ pk2 ffma2(pk2 a, pk2 b, pk2 c) {   // (a.lo * b.lo + c.lo, a.hi * b.hi + c.hi), each IEEE RN
-  pk2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return d;
-}
-__device__ __forceinline__ pk2 fmul2(pk2 a, pk2 b) {
-  pk2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-  return d;
-}
-// The same two chains as two plain FP32 registers, for the kernels that advance them with the mixed-precision FMA
-// (16-bit operands, FP32 addend and result, one rounding: fma.rn.f32.bf16 / fma.rn.f32.f16). The product of two 16-bit
-// operands is exact in FP32, so the result is bit for bit that of the FP32 FMA on the converted operands; what the
-// mixed form saves is the conversion of the activations to FP32, which it reads as loaded. There is no packed mixed
-// form, so these kernels issue one FMA per product.
-struct f2 { float lo, hi; };
-__device__ __forceinline__ float sum2(f2 a) { return a.lo + a.hi; }
-template <typename XT> struct Mixed;
-template <> struct Mixed<__nv_bfloat16> {
-  // (w.lo * x.lo + acc.lo, w.hi * x.hi + acc.hi): two BF16 pairs in 32-bit registers
-  __device__ __forceinline__ static f2 fma2(uint32_t w, uint32_t x, f2 acc) {
-    asm("{\n\t.reg .b16 wl, wh, xl, xh;\n\t"
-        "mov.b32 {wl, wh}, %2;\n\tmov.b32 {xl, xh}, %3;\n\t"
-        "fma.rn.f32.bf16 %0, wl, xl, %0;\n\tfma.rn.f32.bf16 %1, wh, xh, %1;\n\t}"
-        : "+f"(acc.lo), "+f"(acc.hi) : "r"(w), "r"(x));
-    return acc;
-  }
-  // Two FP16 values that are exact in BF16 (decoded E4M3 / E2M1) as a BF16 pair: through FP32, every step exact.
-  __device__ __forceinline__ static uint32_t weights(uint32_t h) {
-    const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&h));
-    const __nv_bfloat162 p = __floats2bfloat162_rn(t.x, t.y);
-    return *reinterpret_cast<const uint32_t*>(&p);
-  }
-};
-template <> struct Mixed<__half> {
-  __device__ __forceinline__ static f2 fma2(uint32_t w, uint32_t x, f2 acc) {
-    asm("{\n\t.reg .b16 wl, wh, xl, xh;\n\t"
-        "mov.b32 {wl, wh}, %2;\n\tmov.b32 {xl, xh}, %3;\n\t"
-        "fma.rn.f32.f16 %0, wl, xl, %0;\n\tfma.rn.f32.f16 %1, wh, xh, %1;\n\t}"
-        : "+f"(acc.lo), "+f"(acc.hi) : "r"(w), "r"(x));
-    return acc;
-  }
-  __device__ __forceinline__ static uint32_t weights(uint32_t h) { return h; }   // decoded weights are FP16 already
-};
-template <typename XT>
-__device__ __forceinline__ f2 mixed_fma4(const uint32_t (&w)[4], const uint4& x, f2 a) {
-  a = Mixed<XT>::fma2(w[0], x.x, a);
-  a = Mixed<XT>::fma2(w[1], x.y, a);
-  a = Mixed<XT>::fma2(w[2], x.z, a);
-  return Mixed<XT>::fma2(w[3], x.w, a);
-}
-template <typename XT, int R, int M>
-__device__ __forceinline__ void mixed_rows(const uint32_t (&w)[R][4], const uint4& x, f2 (&acc)[R][M], int m) {
-#pragma unroll
-  for (int r = 0; r < R; ++r) acc[r][m] = mixed_fma4<XT>(w[r], x, acc[r][m]);
-}
-
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_count(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -352,13 +195,15 @@ __device__ __forceinline__ void trace_stamp(unsigned long long* trace, int slot)
 static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   const unsigned long long start = global_ns();
   const unsigned long long limit = *reinterpret_cast<const volatile unsigned long long*>(abort_flag + 2);
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255u) == 0u) {
-      if (*abort_flag) return false;
-      if (global_ns() - start > limit) break;
+  do {
+    if (*abort_flag) return false;
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (mbar_try_wait(bar, parity)) return true;
     }
-  }
+  } while (global_ns() - start <= limit);
   *abort_flag = 1;
   return false;
 }
@@ -377,139 +222,98 @@ __device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap* map,
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
                : "memory");
 }
+// The same box into L2 only.
+__device__ __forceinline__ void tensor_prefetch(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+// 3-D: from (0, 0, z) on.
+__device__ __forceinline__ void tensor3_g2s(uint32_t dst, const CUtensorMap* map, int z, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3}], [%4];"
+               ::"r"(dst), "l"(map), "r"(0), "r"(z), "r"(bar)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// `valid` of the bytes, zeros for the rest
+__device__ __forceinline__ void cp_async16_part(uint32_t dst, const void* src, int valid) {
+  const void* granule = reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(src) & ~(uintptr_t)15);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(granule), "r"(valid) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
 }
 __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// Element conversions. All exact.
-
-__device__ __forceinline__ pk2 half2_bits_to_f32(uint32_t h) {
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-  return pack2(f.x, f.y);
-}
-__device__ __forceinline__ pk2 pair_to_f32(uint32_t v, __nv_bfloat16) {   // two BF16 -> two FP32
-  // byte permute for the low element: keeps the shift off the FMA pipe, which the packed FMAs need
-  return pack2_bits(__byte_perm(v, 0u, 0x1044u), v & 0xffff0000u);
-}
-__device__ __forceinline__ pk2 pair_to_f32(uint32_t v, __half) {          // two FP16 -> two FP32
-  return half2_bits_to_f32(v);
-}
-__device__ __forceinline__ float2 e4m3x2_to_f32(uint32_t v) {                // low 16 bits: two E4M3 -> two FP32
-  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)v, __NV_E4M3);
-  return __half22float2(*reinterpret_cast<const __half2*>(&h));
-}
-// E8M0 exponent byte as FP32 2^(e-127); e = 0 is the FP32 subnormal 2^-127 and e = 255 is NaN, as the reference
-// decodes them (decode_gemv.cu:275-278).
-__device__ __forceinline__ float e8m0_to_f32(uint32_t e) {
-  return __uint_as_float(e == 0u ? 0x00400000u : e == 255u ? 0x7fc00000u : e << 23);
-}
 // Offset of the byte of 16-block j (j even) of row n in cuBLASLt's 128 x 4 tiled scale layout, ct tiles per tile
 // row: the layout the reference reads at decode_gemv.cu:78-82.
 __device__ __forceinline__ size_t tiled_scale_offset(int n, int j, int ct) {
   const int r = n & 127;
   return ((size_t)(n >> 7) * ct + (j >> 2)) * 512 + (size_t)(r & 31) * 16 + (r >> 5) * 4 + (j & 3);
 }
-
 __device__ __forceinline__ void store_out(void* out, int kind, size_t idx, float v) {
   if (kind == OUT_F32) reinterpret_cast<float*>(out)[idx] = v;
   else if (kind == OUT_BF16) reinterpret_cast<__nv_bfloat16*>(out)[idx] = __float2bfloat16_rn(v);
   else reinterpret_cast<__half*>(out)[idx] = __float2half_rn(v);
 }
 
-// ---------------------------------------------------------------------------------------------------------------
-// Tile walk shared by producers and consumers: CTA c owns rows [lo, hi); tiles of CW * r rows, the last one shorter.
+// A CTA's barriers (shared-memory addresses, 8 bytes per stage) and abort word. full: the stage's window has come; empty: its
+// eight consumers have left it (a tile's last window: the finishing warps have, for all eight); sums: in a tile's last
+// window, its eight consumers have left their sums in it.
+struct Bars {
+  uint32_t full, empty, sums, x;   // x (one for the CTA): the resident activations have come
+  volatile int* abort_flag;
+};
 
-template <int CW>
+// ---------------------------------------------------------------------------------------------------------------
+// Tile walk shared by all warps: CTA c owns the output columns [lo, hi), walked in tiles of `cap` columns, the last one what is
+// left. A tile's rows in the stage: its columns' matrix rows (regions = 1), or, for a gate_up matrix with the SwiGLU epilogue
+// (regions = 2), its columns' gate rows and, from row cap on, their up rows.
+
 struct Walk {
-  int lo, hi, tile_rows, ntiles, nwin, win_bytes;
-  int split_row0, split_first;   // split tail: first row and height of the last-but-one tile (split_first = 0: none)
+  int lo, hi, cap, regions, ntiles, nwin;
   int pairs;                     // SwiGLU epilogue: rows per half of the gate_up matrix (0: an ordinary matrix)
-  __device__ __forceinline__ Walk(const Params& p) {
+  __device__ __forceinline__ Walk(const Params& p, int window_bytes) {
     pairs = p.pairs;
-    if (pairs) {
-      // The tiles walk the rows in blocks of CW: block 2 b holds gate rows [b CW, (b + 1) CW), block 2 b + 1 the up
-      // rows of the same columns, so that a warp's rows 2 j and 2 j + 1 of a tile are gate and up of one column. A CTA
-      // owns whole pairs of blocks; [lo, hi) counts rows in that order (the last pair of blocks may be short).
-      const int blocks = (pairs + CW - 1) / CW;
-      lo = 2 * CW * (int)(((long long)blocks * blockIdx.x) / gridDim.x);
-      hi = 2 * CW * (int)(((long long)blocks * (blockIdx.x + 1)) / gridDim.x);
-    } else {
-      lo = (int)(((long long)p.N * blockIdx.x) / gridDim.x);
-      hi = (int)(((long long)p.N * (blockIdx.x + 1)) / gridDim.x);
-    }
-    tile_rows = CW * p.rows_per_warp;
-    ntiles = (hi - lo + tile_rows - 1) / tile_rows;
-    // A short last tile walks every K window for a few rows: with only `stages` windows in flight and almost no
-    // bytes in each, it runs at DRAM latency, not bandwidth. For one activation row (the only case where it
-    // measured faster: 8192 x 28672 NVFP4 45.5 -> 41.1 us) the last full tile and a remainder under a quarter of a
-    // tile are therefore walked as two tiles of equal height (48 + 7 -> 28 + 27).
-    split_first = 0;
-    split_row0 = 0;
-    const int rows = hi - lo, rem = rows % tile_rows;
-    if (p.split_tail && !pairs && rows > tile_rows && rem > 0 && 4 * rem < tile_rows) {
-      split_row0 = lo + (ntiles - 2) * tile_rows;
-      split_first = (tile_rows + rem + 1) / 2;
-    }
-    win_bytes = p.steps * kStepBytes;
-    nwin = (p.row_bytes + win_bytes - 1) / win_bytes;
+    lo = (int)(((long long)p.N * blockIdx.x) / gridDim.x);
+    hi = (int)(((long long)p.N * (blockIdx.x + 1)) / gridDim.x);
+    regions = pairs ? 2 : 1;
+    cap = p.tile_rows / regions;
+    ntiles = (hi - lo + cap - 1) / cap;
+    nwin = (p.row_bytes + window_bytes - 1) / window_bytes;
   }
-  // Group g of tile t (the rows a tile's consumer warps hold as their row g): first matrix row and row count (0..CW).
-  __device__ __forceinline__ void group(int t, int g, int& row0, int& rows) const {
-    if (pairs) {
-      const int first = lo + t * tile_rows + g * CW;         // in walking order
-      const int block = first / CW, k0 = (block >> 1) * CW;
-      rows = first < hi ? max(0, min(CW, pairs - k0)) : 0;
-      row0 = (block & 1) * pairs + k0;
-    } else {
-      int tile0, tile_n;
-      tile(t, tile0, tile_n);
-      row0 = tile0 + g * CW;
-      rows = max(0, min(CW, tile_n - g * CW));
-    }
+  // First column and width of tile t.
+  __device__ __forceinline__ void tile(int t, int& col0, int& cols) const {
+    col0 = lo + t * cap;
+    cols = min(cap, hi - col0);
   }
-  // First row and height of tile t (ordinary matrices).
-  __device__ __forceinline__ void tile(int t, int& row0, int& rows) const {
-    if (split_first && t >= ntiles - 2) {
-      row0 = t == ntiles - 2 ? split_row0 : split_row0 + split_first;
-      rows = t == ntiles - 2 ? split_first : hi - row0;
-    } else {
-      row0 = lo + t * tile_rows;
-      rows = min(tile_rows, hi - row0);
-    }
+  // Rows a tile of `cols` columns takes in the stage, and the matrix row of one of them (where there is one).
+  __device__ __forceinline__ int rows(int cols) const { return (regions - 1) * cap + cols; }
+  __device__ __forceinline__ int matrix_row(int col0, int cols, int r) const {
+    return r < cap ? col0 + min(r, cols - 1) : pairs + col0 + (r - cap);
   }
 };
 
-// Bytes of the scales of one group of `cw` rows in a stage, padded to the 128 bytes a tensor copy's destination
-// must be aligned to.
-__host__ __device__ constexpr int scale_group_bytes(int cw, int steps, int scb) { return (cw * steps * scb + 127) & ~127; }
-
-// Shared-memory stage: [weights rows_cap x win_bytes][scales: r groups of CW rows x steps*SCB, each group padded to
-// 128 bytes][x: steps x M x 64*E bytes, the activations of one 512-byte step of every activation row together]. Tile row t = w + CW * g is row w of group g.
-template <int FMT, int M, int CW>
+// Shared-memory stage: [weights, rows weight_pitch apart][scales, rows scale_pitch apart][x: per step XROW / 128 blocks of
+// K, each M rows of 128 bytes, on a multiple of 1024 bytes]. Boxes of kBoxRows rows start on 128 bytes, as tensor copies
+// ask.
+template <int FMT, int STEPS>
 struct StageLayout {
-  static constexpr int E = Format<FMT>::E, SCB = Format<FMT>::SCB;
-  int w_row, sc_row, sc_group, sc_off, x_off;
+  static constexpr int W_ROW = weight_pitch(FMT, STEPS), SC_ROW = scale_pitch(FMT, STEPS);
+  int sc_off, x_off;
   __device__ __forceinline__ StageLayout(const Params& p) {
-    const int rows_cap = CW * p.rows_per_warp;
-    w_row = p.steps * kStepBytes;
-    sc_row = p.steps * SCB;
-    sc_group = scale_group_bytes(CW, p.steps, SCB);
-    sc_off = rows_cap * w_row;
-    x_off = sc_off + p.rows_per_warp * sc_group;
+    sc_off = p.tile_rows * W_ROW;
+    x_off = x_offset(p.tile_rows * (W_ROW + SC_ROW));
   }
 };
 
-// 16-byte slot s of an activation row lands at slot s ^ ((s >> 3) & (NQ - 1)) (NQ = 16-byte slots a lane reads per
-// block): the eight lanes of a quarter warp then read eight different bank groups.
-template <int NQ>
-__device__ __forceinline__ int swizzle_slot(int s) { return s ^ ((s >> 3) & (NQ - 1)); }
+// Where 16-byte slot s (0..7) of row r of the activation blocks lies: the 128-byte swizzle of the tensor copies.
+__device__ __forceinline__ int x_slot(int r, int s) { return r * 128 + ((s ^ (r & 7)) << 4); }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Producer warps: `pl` is this thread's index among the 32 * PW producer lanes.
+// Producer warps.
 
 // Programmatic dependent launch: the next kernel of the stream may start while this one runs, and this one may have
 // started while the previous one ran. `griddep_wait` returns once the previous kernel has completed and its writes
@@ -517,865 +321,845 @@ __device__ __forceinline__ int swizzle_slot(int s) { return s ^ ((s >> 3) & (NQ 
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-template <int FMT, int M, int CW, int PW>
-struct Producer {
-  static constexpr int E = Format<FMT>::E, SCB = Format<FMT>::SCB, NQ = E / 8, PL = 32 * PW;
-  const Params& p;
-  const Params& maps;   // where the tensor maps are read from: kernel parameter or global memory, never shared memory
-                        // (p itself, unless p is a copy the CTA keeps in shared memory)
-  const Walk<CW> wk;
-  const StageLayout<FMT, M, CW> lay;
-  const uint32_t ring, full0, empty0;
-  const bool staged;
-  const int pl;
-
-  __device__ __forceinline__ Producer(const Params& p_, const Params& maps_, unsigned char* smem, uint32_t full0_,
-                                      uint32_t empty0_, int pl_)
-      : p(p_), maps(maps_), wk(p_), lay(p_), ring(smem_addr(smem) + kSmemHeader), full0(full0_), empty0(empty0_),
-        staged(SCB != 0 && p_.scale_mode == SCALES_STAGED), pl(pl_) {}
-  __device__ __forceinline__ Producer(const Params& p_, const Params& maps_, const Walk<CW>& wk_,
-                                      const StageLayout<FMT, M, CW>& lay_, unsigned char* smem, uint32_t full0_,
-                                      uint32_t empty0_, int pl_)
-      : p(p_), maps(maps_), wk(wk_), lay(lay_), ring(smem_addr(smem) + kSmemHeader), full0(full0_), empty0(empty0_),
-        staged(SCB != 0 && p_.scale_mode == SCALES_STAGED), pl(pl_) {}
-
-  // Weight (and scale) copies of iteration `it` (tile it / nwin, window it % nwin) into stage s.
-  // Full groups of CW rows travel as one 2-D tensor copy each (always the whole box: columns past the row's end are
-  // zero-filled and still counted), the remainder as one 1-D bulk copy per row. One arrival carries the byte count
-  // of them all; completions may land before it (the phase cannot end while this arrival and the producers'
-  // cp.async arrivals are outstanding).
-  __device__ __forceinline__ void weights(int it, int s) const {
-    const int t = it / wk.nwin, win = it - t * wk.nwin;
-    const uint32_t full = full0 + 8u * s;
-    const uint32_t stage = ring + (uint32_t)s * p.stage_bytes;
-    const int byte0 = win * wk.win_bytes;
-    const int wbytes = min(wk.win_bytes, p.row_bytes - byte0);
-    const int scbytes = staged ? (wbytes * SCB) >> 9 : 0;
-    if (!wk.pairs) {
-      // consecutive rows: the whole groups of CW rows as boxes, issued by as many lanes at once, the rest row by row
-      int row0, rows;
-      wk.tile(t, row0, rows);
-      const int boxes = p.use_2d ? rows / CW : 0;
-      const int box_rows = boxes * CW;
-      if (pl == 0)
-        mbar_arrive_expect_tx(full, (uint32_t)box_rows * (uint32_t)(lay.w_row + (staged ? lay.sc_row : 0)) +
-                                        (uint32_t)(rows - box_rows) * (uint32_t)(wbytes + scbytes));
-      if (pl < boxes) {
-        tensor_g2s(stage + pl * CW * lay.w_row, &maps.tmap_w, byte0 >> 3, row0 + pl * CW, full);
-        if (staged)
-          tensor_g2s(stage + lay.sc_off + pl * lay.sc_group, &maps.tmap_sc, (win * lay.sc_row) >> 3, row0 + pl * CW, full);
-      }
-      for (int r = box_rows + pl; r < rows; r += PL) {
-        const size_t n = (size_t)(row0 + r);
-        bulk_g2s(stage + r * lay.w_row, p.w + n * p.row_bytes + byte0, (uint32_t)wbytes, full);
-        if (staged)
-          bulk_g2s(stage + lay.sc_off + (r / CW) * lay.sc_group + (r % CW) * lay.sc_row,
-                   p.scales + n * p.scale_row_bytes + (size_t)win * lay.sc_row, (uint32_t)scbytes, full);
-      }
-      return;
-    }
-    // gate_up with the SwiGLU epilogue: groups of CW rows from the two halves in turn; a whole group is one box (one
-    // lane each, issued together), a short one goes row by row
-    uint32_t expect = 0;
-    for (int g = 0; g < p.rows_per_warp; ++g) {
-      int row0, rows;
-      wk.group(t, g, row0, rows);
-      expect += p.use_2d && rows == CW ? (uint32_t)CW * (uint32_t)(lay.w_row + (staged ? lay.sc_row : 0))
-                                       : (uint32_t)rows * (uint32_t)(wbytes + scbytes);
-    }
-    if (pl == 0) mbar_arrive_expect_tx(full, expect);
-    if (pl < p.rows_per_warp) {
-      int row0, rows;
-      wk.group(t, pl, row0, rows);
-      if (p.use_2d && rows == CW) {
-        tensor_g2s(stage + pl * CW * lay.w_row, &maps.tmap_w, byte0 >> 3, row0, full);
-        if (staged)
-          tensor_g2s(stage + lay.sc_off + pl * lay.sc_group, &maps.tmap_sc, (win * lay.sc_row) >> 3, row0, full);
-      }
-    }
-    for (int g = 0; g < p.rows_per_warp; ++g) {
-      int row0, rows;
-      wk.group(t, g, row0, rows);
-      if (rows == 0 || (p.use_2d && rows == CW)) continue;
-      for (int r = pl; r < rows; r += PL) {
-        const size_t n = (size_t)(row0 + r);
-        bulk_g2s(stage + (g * CW + r) * lay.w_row, p.w + n * p.row_bytes + byte0, (uint32_t)wbytes, full);
-        if (staged)
-          bulk_g2s(stage + lay.sc_off + g * lay.sc_group + r * lay.sc_row,
-                   p.scales + n * p.scale_row_bytes + (size_t)win * lay.sc_row, (uint32_t)scbytes, full);
-      }
-    }
-  }
-
-  // Activations of iteration `it`: wbytes / 16 blocks of E elements per row, 16 bytes (8 elements) per copy; then
-  // this lane's arrival, which fires when its copies have landed.
-  __device__ __forceinline__ void activations(int it, int s) const {
-    if constexpr (resident_capable(FMT, M)) {
-      if (p.x_resident) {   // nothing to copy: the lane's arrival alone
-        cp_async_arrive_noinc(full0 + 8u * s);
-        return;
-      }
-    }
-    const int win = it % wk.nwin;
-    const uint32_t full = full0 + 8u * s;
-    const uint32_t stage = ring + (uint32_t)s * p.stage_bytes;
-    const int byte0 = win * wk.win_bytes;
-    const int wbytes = min(wk.win_bytes, p.row_bytes - byte0);
-    const int slots = (wbytes >> 4) * NQ;
-    const size_t xbyte0 = (size_t)(byte0 >> 4) * E * 2;
-    const unsigned char* xg = reinterpret_cast<const unsigned char*>(p.x);
-    constexpr int STEP_SLOTS = 32 * NQ;              // 16-byte slots of one step of one activation row (64 * E bytes)
-#pragma unroll 1
-    for (int m = 0; m < M; ++m) {
-      const uint32_t dst = stage + lay.x_off + m * (64 * E);
-      const unsigned char* src = xg + (size_t)m * p.ldx * 2 + xbyte0;
-      for (int sl = pl; sl < slots; sl += PL) {
-        const int st = sl / STEP_SLOTS, in_step = sl - st * STEP_SLOTS;
-        cp_async16(dst + st * (M * 64 * E) + swizzle_slot<NQ>(in_step) * 16, src + (size_t)sl * 16);
-      }
-    }
-    cp_async_arrive_noinc(full);
-  }
-
-  // The same copies when all the CTA's threads share them (PL a multiple of a step's slots): a thread keeps one
-  // slot position of every step and every (PL / slots-per-step)-th activation row, so its addresses advance by
-  // constants.
-  __device__ __forceinline__ void activations_shared(int it, int s) const {
-    constexpr int STEP_SLOTS = 32 * NQ, MSTRIDE = PL / STEP_SLOTS;
-    static_assert(PL % STEP_SLOTS == 0 && MSTRIDE >= 1, "copying threads must cover whole steps");
-    const int win = it % wk.nwin;
-    const int byte0 = win * wk.win_bytes;
-    const int wbytes = min(wk.win_bytes, p.row_bytes - byte0);
-    const int slots = (wbytes >> 4) * NQ;
-    const int in_step = pl % STEP_SLOTS, m0 = pl / STEP_SLOTS;
-    uint32_t dst = ring + (uint32_t)s * p.stage_bytes + lay.x_off + swizzle_slot<NQ>(in_step) * 16;
-    const unsigned char* src =
-        reinterpret_cast<const unsigned char*>(p.x) + (size_t)(byte0 >> 4) * E * 2 + (size_t)in_step * 16;
-    const size_t xrow = (size_t)p.ldx * 2;
-    for (int sl = in_step; sl < slots; sl += STEP_SLOTS, dst += M * 64 * E, src += STEP_SLOTS * 16) {
-#pragma unroll
-      for (int k = 0; k < (M + MSTRIDE - 1) / MSTRIDE; ++k) {
-        const int m = m0 + k * MSTRIDE;
-        if (m < M) cp_async16(dst + m * (64 * E), src + m * xrow);
-      }
-    }
-    cp_async_arrive_noinc(full0 + 8u * s);
-  }
-
-  // One GEMV's iterations. The ring position (stage s, its phase parity) is the caller's and carries on from one
-  // GEMV of a batch to the next; `first` is the kernel's first GEMV: only there the previous kernel of the stream may
-  // still be running (wait before the activations; with static weights, after the first weight copies).
-  __device__ __forceinline__ bool run(volatile int* abort_flag, int& s, uint32_t& parity, bool first) const {
-    const int total = wk.ntiles * wk.nwin;
-    int it = 0;
-    if (first && p.early_weights) {
-      // The weights do not depend on the previous kernel of the stream: fill the ring with them before waiting for
-      // it; the activations (its output, typically) follow the wait. (First GEMV: the ring is empty, s = 0.)
-      const int ahead = min(p.stages, total);
-      for (int i = 0; i < ahead; ++i) weights(i, i);
-      griddep_wait();
-      for (int i = 0; i < ahead; ++i) activations(i, i);
-      it = ahead;
-      if (ahead == p.stages) parity ^= 1u;
-      else s = ahead;
-    } else if (first) {
-      griddep_wait();
-    }
-    for (; it < total; ++it) {
-      if (!mbar_wait(empty0 + 8u * s, parity ^ 1u, abort_flag)) {
-        if ((pl & 31) == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
-        return false;
-      }
-      weights(it, s);
-      activations(it, s);
-      if (++s == p.stages) { s = 0; parity ^= 1u; }
-    }
-    return true;
-  }
-};
-
-// ---------------------------------------------------------------------------------------------------------------
-// Consumer bodies: one 16-byte block of each of R rows times M activation rows. `wrow` points at the block of the
-// warp's first row in the stage, rows are `wstride` bytes apart; `xs` at the stage's activations.
-// acc[r][m] = (even chain, odd chain). With few activation rows (FEW) the activations of the block are converted
-// once and held while the rows stream past; otherwise the rows' weights are decoded once and held while the
-// activation rows stream past. Per (row, m) both issue the same operations in the same order.
-
-template <int NQ>
-struct XOffsets {   // byte offsets of the lane's NQ swizzled slots inside one step of one activation row
-  int off[NQ];
-  __device__ __forceinline__ XOffsets(int lane) {
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) off[j] = swizzle_slot<NQ>(lane * NQ + j) * 16;
-  }
-};
-
-template <typename XT>
-__device__ __forceinline__ void load_x8(uint32_t addr, pk2 (&x)[4]) {   // 8 activations -> 4 FP32 pairs
-  const uint4 v = lds128(addr);
-  x[0] = pair_to_f32(v.x, XT());
-  x[1] = pair_to_f32(v.y, XT());
-  x[2] = pair_to_f32(v.z, XT());
-  x[3] = pair_to_f32(v.w, XT());
-}
-__device__ __forceinline__ pk2 fma4(const pk2 (&w)[4], const pk2 (&x)[4], pk2 a) {
-  a = ffma2(w[0], x[0], a);
-  a = ffma2(w[1], x[1], a);
-  a = ffma2(w[2], x[2], a);
-  return ffma2(w[3], x[3], a);
+// Block scales that bulk copies cannot bring (row-major rows that are no multiples of 16 bytes or lie off 16 bytes, or
+// cuBLASLt's tiles): the activation producers copy them themselves.
+template <int FMT>
+__device__ __forceinline__ bool scales_gathered(const Params& p) {
+  return Format<FMT>::SCB != 0 && p.scale_mode != SCALES_STAGED;
 }
 
-// 8 weights of a sub-block as 4 FP32 pairs.
-__device__ __forceinline__ void decode_bf16(const uint4& v, pk2 (&w)[4]) {
-  w[0] = pair_to_f32(v.x, __nv_bfloat16());
-  w[1] = pair_to_f32(v.y, __nv_bfloat16());
-  w[2] = pair_to_f32(v.z, __nv_bfloat16());
-  w[3] = pair_to_f32(v.w, __nv_bfloat16());
-}
-// The conversions take their packed source from a 16-bit (E4M3 pair) or 8-bit (E2M1 pair) register; unpacking the
-// word in PTX lets the assembler select the sub-word instead of shifting it out first.
-__device__ __forceinline__ void decode_e4m3(uint32_t a, uint32_t b, pk2 (&w)[4]) {
-  uint32_t h0, h1, h2, h3;
-  asm("{\n\t.reg .b16 lo, hi;\n\t"
-      "mov.b32 {lo, hi}, %2;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %0, lo;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
-      : "=r"(h0), "=r"(h1) : "r"(a));
-  asm("{\n\t.reg .b16 lo, hi;\n\t"
-      "mov.b32 {lo, hi}, %2;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %0, lo;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
-      : "=r"(h2), "=r"(h3) : "r"(b));
-  w[0] = half2_bits_to_f32(h0);
-  w[1] = half2_bits_to_f32(h1);
-  w[2] = half2_bits_to_f32(h2);
-  w[3] = half2_bits_to_f32(h3);
-}
-__device__ __forceinline__ void decode_e2m1(uint32_t a, pk2 (&w)[4]) {
-  uint32_t h0, h1, h2, h3;
-  asm("{\n\t.reg .b8 c0, c1, c2, c3;\n\t"
-      "mov.b32 {c0, c1, c2, c3}, %4;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %0, c0;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %1, c1;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %2, c2;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %3, c3;\n\t}"
-      : "=r"(h0), "=r"(h1), "=r"(h2), "=r"(h3) : "r"(a));
-  w[0] = half2_bits_to_f32(h0);
-  w[1] = half2_bits_to_f32(h1);
-  w[2] = half2_bits_to_f32(h2);
-  w[3] = half2_bits_to_f32(h3);
-}
-
-template <bool FEW, int M, int R, typename XT>
-__device__ __forceinline__ void body_bf16(uint32_t wrow, const uint32_t (&woff)[R], uint32_t xs, pk2 (&acc)[R][M]) {
-  constexpr int XROW = 64 * Format<FMT_BF16>::E;   // bytes between activation rows inside a step
-  uint4 wv[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) wv[r] = lds128(wrow + woff[r]);
-  if constexpr (FEW) {
-    pk2 xf[M][4];
-#pragma unroll
-    for (int m = 0; m < M; ++m) load_x8<XT>(xs + m * XROW, xf[m]);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      pk2 wf[4];
-      decode_bf16(wv[r], wf);
-#pragma unroll
-      for (int m = 0; m < M; ++m) acc[r][m] = fma4(wf, xf[m], acc[r][m]);
-    }
-  } else {
-    pk2 wf[R][4];
-#pragma unroll
-    for (int r = 0; r < R; ++r) decode_bf16(wv[r], wf[r]);
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      pk2 xf[4];
-      load_x8<XT>(xs + m * XROW, xf);
-#pragma unroll
-      for (int r = 0; r < R; ++r) acc[r][m] = fma4(wf[r], xf, acc[r][m]);
-    }
-  }
-}
-
-// FP8 / MXFP8: the block is two sub-blocks of 8 weights (words 0-1, words 2-3). `sc` holds the MXFP8 scale of each
-// row's block (unused for FP8): every weight is multiplied by it (exact: a power of two).
-template <bool FEW, bool MX, int M, int R, typename XT>
-__device__ __forceinline__ void body_fp8(uint32_t wrow, const uint32_t (&woff)[R], const float (&sc)[R], uint32_t xs,
-                                         const XOffsets<2>& xo, pk2 (&acc)[R][M]) {
-  constexpr int XROW = 64 * Format<FMT_FP8>::E;   // bytes between activation rows inside a step
-  uint4 wv[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) wv[r] = lds128(wrow + woff[r]);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    if constexpr (FEW) {
-      pk2 xf[M][4];
-#pragma unroll
-      for (int m = 0; m < M; ++m) load_x8<XT>(xs + m * XROW + xo.off[j], xf[m]);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        pk2 wf[4];
-        decode_e4m3(j ? wv[r].z : wv[r].x, j ? wv[r].w : wv[r].y, wf);
-        if (MX) {
-          const pk2 s2 = pack2(sc[r], sc[r]);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) wf[q] = fmul2(wf[q], s2);
-        }
-#pragma unroll
-        for (int m = 0; m < M; ++m) acc[r][m] = fma4(wf, xf[m], acc[r][m]);
-      }
-    } else {
-      pk2 wf[R][4];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        decode_e4m3(j ? wv[r].z : wv[r].x, j ? wv[r].w : wv[r].y, wf[r]);
-        if (MX) {
-          const pk2 s2 = pack2(sc[r], sc[r]);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) wf[r][q] = fmul2(wf[r][q], s2);
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        pk2 xf[4];
-        load_x8<XT>(xs + m * XROW + xo.off[j], xf);
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r][m] = fma4(wf[r], xf, acc[r][m]);
-      }
-    }
-  }
-}
-
-// NVFP4: the block is 32 codes = two scale blocks of 16 (words 0-1 with scale .x, words 2-3 with scale .y). The 16
-// products of a scale block are summed first (two chains of 8, started by a multiply), then acc = fma(scale,
-// partial, acc).
-__device__ __forceinline__ pk2 dot16(const pk2 (&wa)[4], const pk2 (&wb)[4], const pk2 (&xa)[4],
-                                     const pk2 (&xb)[4]) {
-  pk2 part = fmul2(wa[0], xa[0]);
-  part = ffma2(wa[1], xa[1], part);
-  part = ffma2(wa[2], xa[2], part);
-  part = ffma2(wa[3], xa[3], part);
-  return fma4(wb, xb, part);
-}
-
-template <bool FEW, int M, int R, typename XT>
-__device__ __forceinline__ void body_nvfp4(uint32_t wrow, const uint32_t (&woff)[R], const float2 (&sc)[R], uint32_t xs,
-                                           const XOffsets<4>& xo, pk2 (&acc)[R][M]) {
-  constexpr int XROW = 64 * Format<FMT_NVFP4>::E;   // bytes between activation rows inside a step
-  uint4 wv[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) wv[r] = lds128(wrow + woff[r]);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    if constexpr (FEW) {
-      pk2 xa[M][4], xb[M][4];
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        load_x8<XT>(xs + m * XROW + xo.off[2 * h], xa[m]);
-        load_x8<XT>(xs + m * XROW + xo.off[2 * h + 1], xb[m]);
-      }
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        pk2 wa[4], wb[4];
-        decode_e2m1(h ? wv[r].z : wv[r].x, wa);
-        decode_e2m1(h ? wv[r].w : wv[r].y, wb);
-        const float s = h ? sc[r].y : sc[r].x;
-#pragma unroll
-        for (int m = 0; m < M; ++m)
-          acc[r][m] = ffma2(pack2(s, s), dot16(wa, wb, xa[m], xb[m]), acc[r][m]);
-      }
-    } else {
-      pk2 wa[R][4], wb[R][4];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        decode_e2m1(h ? wv[r].z : wv[r].x, wa[r]);
-        decode_e2m1(h ? wv[r].w : wv[r].y, wb[r]);
-      }
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        pk2 xa[4], xb[4];
-        load_x8<XT>(xs + m * XROW + xo.off[2 * h], xa);
-        load_x8<XT>(xs + m * XROW + xo.off[2 * h + 1], xb);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const float s = h ? sc[r].y : sc[r].x;
-          acc[r][m] = ffma2(pack2(s, s), dot16(wa[r], wb[r], xa, xb), acc[r][m]);
-        }
-      }
-    }
-  }
-}
-
-// The same blocks with the mixed-precision FMA (use_mixed): the rows' weights are brought to the activations' 16-bit
-// type once per block (BF16 weights as stored; decoded E4M3 / E2M1 are FP16, exact in BF16 too) and held, the
-// activation rows stream past as loaded. Per (row, m): the operations and order of the bodies above.
-__device__ __forceinline__ void decode_e4m3_h(uint32_t a, uint32_t b, uint32_t (&h)[4]) {   // 8 E4M3 -> 4 FP16 pairs
-  asm("{\n\t.reg .b16 lo, hi;\n\t"
-      "mov.b32 {lo, hi}, %2;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %0, lo;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
-      : "=r"(h[0]), "=r"(h[1]) : "r"(a));
-  asm("{\n\t.reg .b16 lo, hi;\n\t"
-      "mov.b32 {lo, hi}, %2;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %0, lo;\n\t"
-      "cvt.rn.f16x2.e4m3x2 %1, hi;\n\t}"
-      : "=r"(h[2]), "=r"(h[3]) : "r"(b));
-}
-__device__ __forceinline__ void decode_e2m1_h(uint32_t a, uint32_t (&h)[4]) {               // 8 E2M1 -> 4 FP16 pairs
-  asm("{\n\t.reg .b8 c0, c1, c2, c3;\n\t"
-      "mov.b32 {c0, c1, c2, c3}, %4;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %0, c0;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %1, c1;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %2, c2;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %3, c3;\n\t}"
-      : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]) : "r"(a));
-}
-
-template <int M, int R>
-__device__ __forceinline__ void body_bf16_mixed(uint32_t wrow, const uint32_t (&woff)[R], uint32_t xs, f2 (&acc)[R][M]) {
-  constexpr int XROW = 64 * Format<FMT_BF16>::E;
-  uint32_t w[R][4];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const uint4 v = lds128(wrow + woff[r]);
-    w[r][0] = v.x; w[r][1] = v.y; w[r][2] = v.z; w[r][3] = v.w;
-  }
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const uint4 xv = lds128(xs + m * XROW);
-    mixed_rows<__nv_bfloat16, R, M>(w, xv, acc, m);
-  }
-}
-
-template <int M, int R, typename XT>
-__device__ __forceinline__ void body_fp8_mixed(uint32_t wrow, const uint32_t (&woff)[R], uint32_t xs,
-                                               const XOffsets<2>& xo, f2 (&acc)[R][M]) {
-  constexpr int XROW = 64 * Format<FMT_FP8>::E;
-  uint4 wv[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) wv[r] = lds128(wrow + woff[r]);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    uint32_t w[R][4];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      decode_e4m3_h(j ? wv[r].z : wv[r].x, j ? wv[r].w : wv[r].y, w[r]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) w[r][q] = Mixed<XT>::weights(w[r][q]);
-    }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const uint4 xv = lds128(xs + m * XROW + xo.off[j]);
-      mixed_rows<XT, R, M>(w, xv, acc, m);
-    }
-  }
-}
-
-// NVFP4: the partial sum of a scale block starts as a product; fma(a, b, -0) is that product bit for bit.
-template <int M, int R, typename XT>
-__device__ __forceinline__ void body_nvfp4_mixed(uint32_t wrow, const uint32_t (&woff)[R], const float2 (&sc)[R],
-                                                 uint32_t xs, const XOffsets<4>& xo, f2 (&acc)[R][M]) {
-  constexpr int XROW = 64 * Format<FMT_NVFP4>::E;
-  uint4 wv[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) wv[r] = lds128(wrow + woff[r]);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t wa[R][4], wb[R][4];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      decode_e2m1_h(h ? wv[r].z : wv[r].x, wa[r]);
-      decode_e2m1_h(h ? wv[r].w : wv[r].y, wb[r]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        wa[r][q] = Mixed<XT>::weights(wa[r][q]);
-        wb[r][q] = Mixed<XT>::weights(wb[r][q]);
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const uint4 xa = lds128(xs + m * XROW + xo.off[2 * h]);
-      const uint4 xb = lds128(xs + m * XROW + xo.off[2 * h + 1]);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        f2 part;
-        part.lo = -0.0f;
-        part.hi = -0.0f;
-        part = mixed_fma4<XT>(wa[r], xa, part);
-        part = mixed_fma4<XT>(wb[r], xb, part);
-        const float s = h ? sc[r].y : sc[r].x;
-        acc[r][m].lo = fmaf(s, part.lo, acc[r][m].lo);
-        acc[r][m].hi = fmaf(s, part.hi, acc[r][m].hi);
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------------------------------------------
-// Lane reduction of V values per lane at once: the xor-shuffle tree 16, 8, 4, 2, 1 of every value, with the values
-// split between the two partners at each level so that a level costs one shuffle per value pair instead of one per
-// value. For each value the additions are those of the plain tree, pair by pair (a + b is commutative in IEEE
-// arithmetic), so the bits are the plain tree's. After the last level value v's total sits in lane (v % 32),
-// slot v / 32.
-template <int V, int OFFSET, int NOUT>
-struct LaneReduce {
-  static constexpr int H = (V + 1) / 2;   // values kept per lane after this level
-  __device__ __forceinline__ static void run(float (&val)[V], int lane, float (&out)[NOUT]) {
-    if constexpr (V == 1) {
-      float v = val[0];
-#pragma unroll
-      for (int o = OFFSET; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      out[0] = v;
-    } else if constexpr (OFFSET == 0) {
-      static_assert(V <= NOUT, "lane reduction output too small");
-#pragma unroll
-      for (int i = 0; i < V; ++i) out[i] = val[i];
-    } else {
-      // lanes with the OFFSET bit clear keep values [0, H) and send [H, V); the others keep [H, V) and send [0, H)
-      const bool upper = (lane & OFFSET) != 0;
-      float keep[H];
-#pragma unroll
-      for (int i = 0; i < H; ++i) {
-        const bool has_hi = H + i < V;
-        const float lo = val[i], hi = has_hi ? val[H + i] : 0.0f;
-        const float got = __shfl_xor_sync(0xffffffffu, upper ? lo : hi, OFFSET);
-        // a value without a partner slot (odd V) is finished by the lower lanes; the upper lanes carry a zero there
-        keep[i] = (upper ? hi : lo) + (has_hi || !upper ? got : 0.0f);
-      }
-      LaneReduce<H, OFFSET / 2, NOUT>::run(keep, lane, out);
-    }
-  }
-};
-
-// Which of the V values lane `lane` holds in output slot `slot` after LaneReduce<V, 16, .> (-1: none).
-template <int V>
-__device__ __forceinline__ int lane_value(int lane, int slot) {
-  int size = V, real = V, base = 0;   // entries [0, real) of this lane's array are values base, base + 1, ...
-  for (int o = 16; o > 0; o >>= 1) {
-    if (size == 1) return (real == 1 && slot == 0 && (lane & (2 * o - 1)) == 0) ? base : -1;
-    const int h = (size + 1) / 2;
-    if (lane & o) {
-      base += h;
-      real = real > h ? real - h : 0;
-    } else {
-      real = real < h ? real : h;
-    }
-    size = h;
-  }
-  return slot < real ? base + slot : -1;
-}
-
-// ---------------------------------------------------------------------------------------------------------------
-// One tile for one consumer warp holding up to R rows (nr of them real).
-
-// Eight BF16 values as eight FP16 values, and whether each converts exactly (what FP16 holds, its subnormals
-// included: the mixed FMA takes subnormal operands exactly, checked on a B200 over every subnormal pattern; values
-// beyond 65504 become infinite, NaN compares unequal, and both say no): the test of Arithmetic::HALF_RES.
-__device__ __forceinline__ bool bf16x2_fits_half(uint32_t v, uint32_t& h) {
-  const float lo = __uint_as_float(v << 16), hi = __uint_as_float(v & 0xffff0000u);
-  const __half2 t = __floats2half2_rn(lo, hi);
-  h = *reinterpret_cast<const uint32_t*>(&t);
-  const float2 back = __half22float2(t);
-  return back.x == lo && back.y == hi;
-}
-__device__ __forceinline__ bool bf16x8_fits_half(const uint4& v, uint4& h) {
-  const bool a = bf16x2_fits_half(v.x, h.x), b = bf16x2_fits_half(v.y, h.y);
-  const bool c = bf16x2_fits_half(v.z, h.z), d = bf16x2_fits_half(v.w, h.w);
-  return a && b && c && d;
-}
-
-// Resident activations: the consumer warps bring the whole [M][K] activations into shared memory, once per kernel.
-// Warp w takes steps w, w + CW, ...; of a step, lane l holds slots l, l + 32, ... (16 bytes each) of every activation
-// row and stores them where a ring stage would have them. BF16 activations (HALF) are tested on the way: the warp
-// stores a step as FP16 if all of its values allow it, as loaded otherwise, and says which in the step's flag byte.
-// Ends with a barrier of the consumer warps.
-template <int FMT, int M, int CW, bool HALF>
-__device__ __forceinline__ void fill_resident(const Params& p, unsigned char* smem) {
-  constexpr int E = Format<FMT>::E, NQ = E / 8;
-  const int nsteps = (p.nblk + 31) >> 5, slots = p.nblk * NQ;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t base = smem_addr(smem) + (uint32_t)p.x_res_off;
-  const uint32_t flags = base + (uint32_t)nsteps * (M * 64 * E);
-  const unsigned char* xg = reinterpret_cast<const unsigned char*>(p.x);
-  for (int st = warp; st < nsteps; st += CW) {
-    uint4 v[M][NQ];
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-#pragma unroll
-      for (int j = 0; j < NQ; ++j) {
-        const int sl = st * (32 * NQ) + j * 32 + lane;
-        v[m][j] = sl < slots ? ldg_nc128(xg + (size_t)m * p.ldx * 2 + (size_t)sl * 16) : make_uint4(0u, 0u, 0u, 0u);
-      }
-    bool fits = false;
-    if constexpr (HALF) {
-      uint4 h[M][NQ];
-      fits = true;
-#pragma unroll
-      for (int m = 0; m < M; ++m)
-#pragma unroll
-        for (int j = 0; j < NQ; ++j) fits &= bf16x8_fits_half(v[m][j], h[m][j]);   // (slots past the end hold zeros)
-      fits = __all_sync(0xffffffffu, fits);
-      if (fits) {
-#pragma unroll
-        for (int m = 0; m < M; ++m)
-#pragma unroll
-          for (int j = 0; j < NQ; ++j) v[m][j] = h[m][j];
-      }
-    }
-    const uint32_t dst = base + (uint32_t)st * (M * 64 * E);
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-#pragma unroll
-      for (int j = 0; j < NQ; ++j) sts128(dst + m * (64 * E) + swizzle_slot<NQ>(j * 32 + lane) * 16, v[m][j]);
-    if (lane == 0) sts_u8(flags + st, fits ? 1u : 0u);
-  }
-  asm volatile("bar.sync 1, %0;" ::"r"(CW * 32) : "memory");
-}
-
-// The two chains between their two forms (a step that could not be kept as FP16 takes the packed body).
-template <int R, int M>
-__device__ __forceinline__ void to_packed(const f2 (&a)[R][M], pk2 (&b)[R][M]) {
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int m = 0; m < M; ++m) b[r][m] = pack2(a[r][m].lo, a[r][m].hi);
-}
-template <int R, int M>
-__device__ __forceinline__ void from_packed(const pk2 (&b)[R][M], f2 (&a)[R][M]) {
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int m = 0; m < M; ++m) asm("mov.b64 {%0, %1}, %2;" : "=f"(a[r][m].lo), "=f"(a[r][m].hi) : "l"(b[r][m].v));
-}
-
-template <bool MIXED> struct Chains;   // accumulator pair type of a kernel
-template <> struct Chains<false> {
-  using type = pk2;
-  __device__ __forceinline__ static pk2 zero() { return pack2(0.f, 0.f); }
-};
-template <> struct Chains<true> {
-  using type = f2;
-  __device__ __forceinline__ static f2 zero() { f2 z; z.lo = 0.f; z.hi = 0.f; return z; }
-};
-
-// SELF: the CTA has no producer warps; its consumer warps share the copies. A warp that has finished iteration `it`
-// (stage s) refills the stage of iteration it - 1, which every warp has probably left by then, with iteration
-// it + stages - 1: nobody waits for the slowest warp of the iteration just finished, and the ring runs one stage
-// short of its depth. All threads share the activation copies; the warps take turns with the weight copies.
-template <int FMT, int M, int CW>
-__device__ __forceinline__ void self_fill(const Params& p, const Params& maps, const Walk<CW>& wk,
-                                          const StageLayout<FMT, M, CW>& lay,
-                                          unsigned char* smem, uint32_t full0, uint32_t empty0, int it, int s,
-                                          bool with_weights, bool with_activations) {
-  const int warp = threadIdx.x >> 5;
-  if (with_weights && warp == it % CW)
-    Producer<FMT, M, CW, 1>(p, maps, wk, lay, smem, full0, empty0, (int)(threadIdx.x & 31)).weights(it, s);
-  if (with_activations)
-    Producer<FMT, M, CW, CW>(p, maps, wk, lay, smem, full0, empty0, (int)threadIdx.x).activations_shared(it, s);
-}
-
-// RES: the activations are resident (Params::x_resident), not in the stages.
-template <int FMT, int M, int R, typename XT, int CW, bool SELF, bool RES = false>
-__device__ __forceinline__ bool consume_tile(const Params& p, const Params& maps, const Walk<CW>& wk,
-                                             const StageLayout<FMT, M, CW>& lay,
-                                             unsigned char* smem, uint32_t full0, uint32_t empty0,
-                                             volatile int* abort_flag, int t, int nr, int& s, uint32_t& parity,
-                                             int& it) {
-  constexpr int E = Format<FMT>::E, SCB = Format<FMT>::SCB, NQ = E / 8;
-  constexpr bool FEW = few_rows(FMT, M);
-  constexpr bool MIXED = Arithmetic<FMT, M, XT>::MIXED;
-  constexpr bool HALF = RES && Arithmetic<FMT, M, XT>::HALF_RES;   // steps flagged as FP16 take the mixed body
-  using Acc = typename Chains<MIXED || HALF>::type;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const XOffsets<NQ> xo(lane);
-  Acc acc[R][M];
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int m = 0; m < M; ++m) acc[r][m] = Chains<MIXED || HALF>::zero();
-  // Offsets of the warp's rows inside a stage (rows are CW tile rows and one scale group apart); rows the warp does
-  // not have alias its last real row (their sums are discarded).
-  uint32_t woff[R], scoff[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int rr = min(r, max(nr, 1) - 1);
-    woff[r] = (uint32_t)((warp + CW * rr) * lay.w_row + lane * 16);
-    scoff[r] = (uint32_t)(lay.sc_off + warp * lay.sc_row + rr * lay.sc_group + (SCB == 64 ? lane * 2 : lane >> 1));
-  }
+// The feeding warp: weight (and staged scale) copies of every window of one GEMV, in order, and the activations' tensor
+// copies. A tile's rows travel as ONE 2-D tensor copy per region (and one for their scales): a copy costs the SM about 150
+// clocks to start whatever its size (as boxes of 8 rows, 12 to 16 a window, or with single rows for a tile's remainder they
+// bounded the whole kernel at 1 us a window). A box is always brought whole: columns past the matrix row's end and rows past
+// the matrix come as zeros and count; rows past the tile are not used. One arrival carries the byte count of all copies;
+// completions may land before it (the phase cannot end while it is outstanding). `early`: the previous kernel of the stream
+// has not been waited for yet; the weights need not. The ring position (stage s, its phase parity) is the caller's and
+// carries on from one GEMV of a batch to the next (`first`: its first); `maps`: where the tensor maps are read from.
+template <int FMT, int STEPS>
+__device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars,
+                                             bool first, bool early, int& s, uint32_t& parity) {
+  constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP, SC_WIN = STEPS * SCB;
+  constexpr int W_ROW = weight_pitch(FMT, STEPS), SC_ROW = scale_pitch(FMT, STEPS), XROW = Format<FMT>::XROW;
+  const Walk wk(p, WIN);
+  const int lane = threadIdx.x & 31, stage_bytes = p.stage_bytes, stages = p.stages;
   const bool staged = SCB != 0 && p.scale_mode == SCALES_STAGED;
-  const uint32_t ring = smem_addr(smem) + kSmemHeader;
-  int rown[R];   // matrix row of each of the warp's rows (rows it does not have alias its last real one)
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    int group0, group_n;
-    wk.group(t, min(r, max(nr, 1) - 1), group0, group_n);
-    rown[r] = group0 + warp;
-  }
-
-  // row r's matrix row for an r known only at run time, without indexing the array (it stays in registers)
-  auto row_of = [&](int r) {
-    int n = rown[0];
-#pragma unroll
-    for (int q = 1; q < R; ++q) n = r == q ? rown[q] : n;
-    return n;
+  const uint32_t ring = smem_addr(smem) + kSmemHeader, sc_off = (uint32_t)(p.tile_rows * W_ROW);
+  // activations by tensor copy, a window at a time: with weights ahead of the wait for the previous kernel of the stream,
+  // those of the first windows follow once the ring is full of weights
+  constexpr int X_BLOCKS = STEPS * XROW / 128;
+  const uint32_t x_off = (uint32_t)x_offset(p.tile_rows * (W_ROW + SC_ROW));
+  const uint32_t x_bytes = p.x_mode == X_TENSOR ? (uint32_t)(X_BLOCKS * 128 * p.M) : 0u;
+  int behind = early ? 0 : -1;                   // windows issued without their activations
+  auto activations = [&](int at, int win) {
+    if (x_bytes && lane == 31) tensor3_g2s(ring + (uint32_t)at * stage_bytes + x_off, &maps.tmap_x, win * X_BLOCKS, bars.full + 8u * at);
   };
-
-  for (int win = 0; win < wk.nwin; ++win) {
-    if (!mbar_wait(full0 + 8u * s, parity, abort_flag)) return false;
-    if (it == 0 && threadIdx.x == 0) trace_stamp(p.trace, TRACE_FIRST_FULL);
-    if (nr > 0) {
-      const uint32_t stage = ring + (uint32_t)s * p.stage_bytes;
-      const int blk0 = win * p.steps * 32;
-      const int nsteps = min(p.steps, (p.nblk - blk0 + 31) >> 5);
-      for (int st = 0; st < nsteps; ++st) {
-        const int blk = blk0 + st * 32 + lane;
-        if (blk < p.nblk) {
-          const uint32_t wrow = stage + st * kStepBytes;
-          const int res_step = win * p.steps + st;   // the step's place among the resident ones
-          const uint32_t xs = RES ? smem_addr(smem) + (uint32_t)p.x_res_off + (uint32_t)res_step * (M * 64 * E)
-                                  : stage + lay.x_off + st * (M * 64 * E);
-          bool as_half = false;
-          if constexpr (HALF)
-            as_half = lds_u8(smem_addr(smem) + (uint32_t)p.x_res_off + (uint32_t)((p.nblk + 31) >> 5) * (M * 64 * E) +
-                             res_step) != 0;
-          if constexpr (FMT == FMT_BF16) {
-            if constexpr (MIXED) body_bf16_mixed<M, R>(wrow, woff, xs + lane * 16, acc);
-            else body_bf16<FEW, M, R, XT>(wrow, woff, xs + lane * 16, acc);
-          } else if constexpr (FMT == FMT_FP8) {
-            if constexpr (MIXED) {
-              body_fp8_mixed<M, R, XT>(wrow, woff, xs, xo, acc);
-            } else if constexpr (HALF) {
-              if (as_half) {
-                body_fp8_mixed<M, R, __half>(wrow, woff, xs, xo, acc);
-              } else {
-                float none[R];
-                pk2 packed[R][M];
-                to_packed<R, M>(acc, packed);
-                body_fp8<FEW, false, M, R, XT>(wrow, woff, none, xs, xo, packed);
-                from_packed<R, M>(packed, acc);
-              }
-            } else {
-              float none[R];
-              body_fp8<FEW, false, M, R, XT>(wrow, woff, none, xs, xo, acc);
-            }
-          } else if constexpr (FMT == FMT_MXFP8) {
-            float sc[R];
-            if (staged) {
-#pragma unroll
-              for (int r = 0; r < R; ++r) sc[r] = e8m0_to_f32(lds_u8(stage + scoff[r] + st * SCB));
-            } else {
-#pragma unroll
-              for (int r = 0; r < R; ++r) {
-                const int n = rown[r];
-                sc[r] = e8m0_to_f32(__ldg(p.scales + (size_t)n * p.scale_row_bytes + (blk >> 1)));
-              }
-            }
-            body_fp8<FEW, true, M, R, XT>(wrow, woff, sc, xs, xo, acc);
-          } else {
-            float2 sc[R];
-            if (staged) {
-#pragma unroll
-              for (int r = 0; r < R; ++r) sc[r] = e4m3x2_to_f32(lds_u16(stage + scoff[r] + st * SCB));
-            } else {
-#pragma unroll
-              for (int r = 0; r < R; ++r) {
-                const int n = rown[r];
-                const size_t off = p.scale_mode == SCALES_BLOCKED ? tiled_scale_offset(n, blk * 2, p.ct)
-                                                                   : (size_t)n * p.scale_row_bytes + blk * 2;
-                sc[r] = e4m3x2_to_f32(__ldg(reinterpret_cast<const uint16_t*>(p.scales + off)));
-              }
-            }
-            if constexpr (MIXED) {
-              if (HALF && as_half) body_nvfp4_mixed<M, R, __half>(wrow, woff, sc, xs, xo, acc);
-              else body_nvfp4_mixed<M, R, XT>(wrow, woff, sc, xs, xo, acc);
-            } else if constexpr (HALF) {
-              if (as_half) {
-                body_nvfp4_mixed<M, R, __half>(wrow, woff, sc, xs, xo, acc);
-              } else {
-                pk2 packed[R][M];
-                to_packed<R, M>(acc, packed);
-                body_nvfp4<FEW, M, R, XT>(wrow, woff, sc, xs, xo, packed);
-                from_packed<R, M>(packed, acc);
-              }
-            } else {
-              body_nvfp4<FEW, M, R, XT>(wrow, woff, sc, xs, xo, acc);
-            }
-          }
-        }
-      }
+  // or all at once: when nobody reads the previous GEMV's any more, which is known once the last of its stages is empty
+  bool x_due = p.x_mode == X_RESIDENT && wk.ntiles > 0;
+  auto resident = [&] {
+    if (x_due && lane == 31) {
+      const int steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP, bytes = p.M * XROW;
+      mbar_arrive_expect_tx(bars.x, (uint32_t)(steps * bytes));
+      for (int st = 0; st < steps; st += p.x_box_steps)
+        tensor3_g2s(smem_addr(smem) + (uint32_t)(p.x_res_off + st * bytes), &maps.tmap_x, st * (XROW / 128), bars.x);
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty0 + 8u * s);
-    if constexpr (SELF) {
-      const int next = it + p.stages - 1;
-      if (next < wk.ntiles * wk.nwin) {
-        const int sp = s == 0 ? p.stages - 1 : s - 1;   // stage of iteration it - 1 (never used yet when it = 0)
-        if (it > 0 && !mbar_wait(empty0 + 8u * sp, s == 0 ? parity ^ 1u : parity, abort_flag)) return false;
-        self_fill<FMT, M, CW>(p, maps, wk, lay, smem, full0, empty0, next, sp, true, true);
-      }
-    }
-    ++it;
-    if (++s == p.stages) { s = 0; parity ^= 1u; }
-  }
-
-  // the two chains, then the lanes (xor-shuffle tree 16, 8, 4, 2, 1); scale once; round once
-  constexpr int V = R * M;
-  float val[V];
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int m = 0; m < M; ++m) val[r * M + m] = sum2(acc[r][m]);
-  float total[(V + 31) / 32];
-  LaneReduce<V, 16, (V + 31) / 32>::run(val, lane, total);
-  if constexpr (FMT == FMT_NVFP4 && R % 2 == 0) {
-    if (p.pairs) {
-      // SwiGLU epilogue: the scaled sums of the warp's rows meet in the warp's corner of shared memory behind the
-      // ring; lane (j, m) then combines gate row 2 j and up row 2 j + 1 and writes one activation.
-      float* meet = reinterpret_cast<float*>(smem + kSmemHeader + (size_t)p.stages * p.stage_bytes) + warp * (RMAX_ALL * 16);
-#pragma unroll
-      for (int i = 0; i < (V + 31) / 32; ++i) {
-        const int v = lane_value<V>(lane, i);
-        if (v >= 0) meet[v] = total[i] * __ldg(p.row_scale + row_of(v / M));
-      }
+    x_due = false;
+  };
+  auto catch_up = [&] {
+    griddep_wait();
+    resident();
+    for (int i = 0; i < behind; ++i) activations(i, i % wk.nwin);
+    behind = -1;
+  };
+  auto wait_empty = [&](int at, uint32_t use) {
+    if (mbar_wait(bars.empty + 8u * at, use ^ 1u, bars.abort_flag)) return true;
+    if (lane == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
+    return false;
+  };
+  if (first && !early) resident();
+  int filled = 0;
+  for (int t = 0; t < wk.ntiles; ++t) {
+    int col0, cols;
+    wk.tile(t, col0, cols);
+    const bool full_tile = cols == wk.cap;
+    const CUtensorMap* const map_w = full_tile ? &maps.tmap_w : &maps.tmap_w_last;
+    const CUtensorMap* const map_sc = full_tile ? &maps.tmap_sc : &maps.tmap_sc_last;
+    const uint32_t bytes = x_bytes + wk.regions * (full_tile ? wk.cap : p.last_rows) * (uint32_t)(W_ROW + (staged ? SC_ROW : 0));
+    // lanes 0, 1: the regions' weights; 2, 3: their scales
+    const int region = lane & 1, n0 = region * wk.pairs + col0, row0 = region * wk.cap;
+    for (int win = 0; win < wk.nwin; ++win) {
+      if (behind == stages) catch_up();
+      if (!wait_empty(s, parity)) return false;
+      if (++filled == stages && !first) resident();
+      const uint32_t full = bars.full + 8u * s, stage = ring + (uint32_t)s * stage_bytes;
+      if (lane == 0) mbar_arrive_expect_tx(full, bytes);
       __syncwarp();
-      if (lane < (R / 2) * M) {
-        const int j = lane / M, m = lane - j * M;
-        if (2 * j < nr) {
-          const float result = swiglu_value(meet[2 * j * M + m], meet[(2 * j + 1) * M + m]);
-          store_out(p.out, p.out_kind, (size_t)m * p.ldo + row_of(2 * j), result);
-        }
+      if (behind < 0) activations(s, win);
+      if (region < wk.regions) {
+        if (lane < 2) tensor_g2s(stage + row0 * W_ROW, map_w, (win * WIN) >> 3, n0, full);
+        else if (lane < 4 && staged) tensor_g2s(stage + sc_off + row0 * SC_ROW, map_sc, (win * SC_WIN) >> 3, n0, full);
       }
-      __syncwarp();
-      return true;
+      if (behind >= 0) ++behind;
+      if (++s == stages) { s = 0; parity ^= 1u; }
     }
   }
-#pragma unroll
-  for (int i = 0; i < (V + 31) / 32; ++i) {
-    const int v = lane_value<V>(lane, i);
-    if (v >= 0) {
-      const int r = v / M, m = v - r * M;
-      if (r < nr) {
-        const int n = row_of(r);
-        const float sum = total[i];
-        const float result = p.row_scale ? sum * __ldg(p.row_scale + n) : sum;
-        if (p.world < 1) {
-          store_out(p.out, p.out_kind, (size_t)m * p.ldo + n, result);
-        } else {
-          store_out(p.out, p.out_kind, ((size_t)p.rank * M + m) * p.ldo + n, result);
-        }
+  if (behind >= 0) catch_up();
+  if (x_due) {                     // fewer windows than stages
+    int at = s;
+    uint32_t use = parity;
+    for (int i = filled; i < stages - 1; ++i)
+      if (++at == stages) { at = 0; use ^= 1u; }
+    if (!wait_empty(at, use)) return false;
+    resident();
+  }
+  return true;
+}
+
+// The first windows' weights (and staged scales) into L2, as many as the ring will hold, before the wait for the previous
+// kernel of the stream: what that kernel may still write reaches the same L2, so the copies after the wait read its
+// values, from L2 instead of HBM.
+template <int FMT, int STEPS>
+__device__ __forceinline__ void prefetch_weights(const Params& p) {
+  constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP, SC_WIN = STEPS * SCB;
+  if ((threadIdx.x & 31) != 0) return;
+  const Walk wk(p, WIN);
+  int left = p.stages;
+  for (int t = 0; t < wk.ntiles; ++t) {
+    int col0, cols;
+    wk.tile(t, col0, cols);
+    for (int win = 0; win < wk.nwin; ++win) {
+      for (int region = 0; region < wk.regions; ++region) {
+        const int n0 = region * wk.pairs + col0;
+        tensor_prefetch(cols == wk.cap ? &p.tmap_w : &p.tmap_w_last, (win * WIN) >> 3, n0);
+        if (SCB != 0 && p.scale_mode == SCALES_STAGED)
+          tensor_prefetch(cols == wk.cap ? &p.tmap_sc : &p.tmap_sc_last, (win * SC_WIN) >> 3, n0);
       }
+      if (--left == 0) return;
+    }
+  }
+}
+
+// The other producer warps, where they are needed: the windows' activations where no tensor copy can bring them, 16 bytes
+// (8 elements) per copy, and the scales that are gathered; then every lane's arrival, which fires when its copies have
+// landed.
+template <int FMT>
+__device__ __forceinline__ bool copies_needed(const Params& p) { return p.x_mode == X_COPIED || scales_gathered<FMT>(p); }
+
+// (zeros past the row's end, by stores, which the lane's arrival on the stage's barrier must follow: returns true then)
+template <int FMT, int STEPS>
+__device__ __forceinline__ bool copy_activations(const Params& p, uint32_t dst, int win, int warp, int lane) {
+  constexpr int SLOTS = STEPS * Format<FMT>::XROW / 16;
+  const int M = p.M, k0 = win * SLOTS * 8, slots = min(SLOTS, (p.K - k0) >> 3);
+  for (int m = warp; m < M; m += kCopyWarps) {
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(p.x) + ((size_t)m * p.ldx + k0) * 2;
+    for (int i = lane; i < SLOTS; i += 32) {
+      const uint32_t to = dst + x_slot((i >> 3) * M + m, i & 7);
+      if (i < slots) cp_async16(to, src + (size_t)i * 16);
+      else sts128(to, make_uint4(0u, 0u, 0u, 0u));
+    }
+  }
+  return slots < SLOTS;
+}
+
+// Whether gathered row-major scales travel in whole 16-byte granules: a row's place in the stage is then as far off 16 bytes
+// as its address is (scale_shift), which rows eight apart share (their distance is a multiple of 16 bytes; MXFP8: of 8).
+template <int FMT>
+__device__ __forceinline__ bool scale_granules(const Params& p) {
+  return Format<FMT>::SCB != 0 && p.scale_mode == SCALES_DIRECT && (((size_t)p.pairs * p.scale_row_bytes) & 15) == 0;
+}
+__device__ __forceinline__ uint32_t scale_shift(const Params& p, int n) {
+  return (uint32_t)(reinterpret_cast<uintptr_t>(p.scales) + (size_t)n * p.scale_row_bytes) & 15u;
+}
+
+// Scale bytes of the window for every row of the tile, zeros past the row's end. Row-major rows: 16 bytes at a time, from the
+// granule the window starts in on. Tiles: four blocks' bytes of a row at a time; a lane stays with its row. What neither fits
+// goes byte by byte through registers, to the places a bulk copy would use; the lane's arrival on the stage's barrier must
+// follow the stores (returns true then). One warp issues few instructions while the others compute, so the loops are kept
+// short: with addresses worked out anew for each four bytes, 20000 x 6016 took 30 us (now 21), and from rows off four bytes,
+// byte by byte, 40000 x 4128 took 137 us (now 36).
+template <int FMT, int STEPS>
+__device__ __forceinline__ bool gather_scales(const Params& p, const Walk& wk, uint32_t dst, int col0, int cols, int win,
+                                              int warp, int lane) {
+  constexpr int SCB = Format<FMT>::SCB, SC_ROW = scale_pitch(FMT, STEPS), WINDOW = STEPS * SCB;
+  const int rows = wk.rows(cols), byte0 = win * WINDOW, sc_bytes = p.row_bytes * SCB / Format<FMT>::STEP;   // of a row's scales
+  const bool tiled = p.scale_mode == SCALES_BLOCKED;
+  if (scale_granules<FMT>(p)) {
+    constexpr int GRANULES = WINDOW / 16 + 1;
+    const uint8_t* base = p.scales + byte0;
+    for (int i = warp * 32 + lane; i < rows * GRANULES; i += 32 * kCopyWarps) {
+      const int r = i / GRANULES, g = i - r * GRANULES;
+      const uint8_t* row = base + (size_t)wk.matrix_row(col0, cols, r) * p.scale_row_bytes;
+      const int off = 16 * g - (int)(reinterpret_cast<uintptr_t>(row) & 15);        // of the granule from the window's start
+      const int valid = max(0, min(16, sc_bytes - byte0 - off));
+      cp_async16_part(dst + (uint32_t)(r * SC_ROW + 16 * g), row + (valid > 0 ? off : 0), valid);
+    }
+    return false;
+  }
+  if (tiled && (reinterpret_cast<uintptr_t>(p.scales) & 3) == 0) {
+    for (int r = lane; r < rows; r += 32) {
+      const int n = wk.matrix_row(col0, cols, r);
+      const uint8_t* src = p.scales + tiled_scale_offset(n, byte0 + 4 * warp, p.ct);
+      uint32_t to = dst + (uint32_t)(r * SC_ROW + 4 * warp);
+      int left = sc_bytes - byte0 - 4 * warp;
+#pragma unroll 4
+      for (int u = warp; u < WINDOW / 4; u += kCopyWarps) {
+        cp_async4(to, left > 0 ? src : p.scales, max(0, min(4, left)));
+        src += 512 * kCopyWarps;
+        to += 4 * kCopyWarps;
+        left -= 4 * kCopyWarps;
+      }
+    }
+    return false;
+  }
+  for (int r = warp; r < rows; r += kCopyWarps) {
+    const int n = wk.matrix_row(col0, cols, r);
+    for (int b = lane; b < WINDOW; b += 32) {
+      const int j = byte0 + b;
+      const uint8_t* src = p.scales + (tiled ? tiled_scale_offset(n, j & ~1, p.ct) + (j & 1) : (size_t)n * p.scale_row_bytes + j);
+      sts_u8(dst + (uint32_t)(r * SC_ROW + b), j < sc_bytes ? (uint32_t)__ldg(src) : 0u);
     }
   }
   return true;
 }
 
+template <int FMT, int STEPS>
+__device__ __forceinline__ bool feed_activations(const Params& p, unsigned char* smem, const Bars& bars, int warp, int& s,
+                                                 uint32_t& parity) {
+  const Walk wk(p, STEPS * Format<FMT>::STEP);
+  const StageLayout<FMT, STEPS> lay(p);
+  const int lane = threadIdx.x & 31;
+  const bool gathered = scales_gathered<FMT>(p);
+  const uint32_t ring = smem_addr(smem) + kSmemHeader;
+  for (int t = 0; t < wk.ntiles; ++t) {
+    int col0, cols;
+    wk.tile(t, col0, cols);
+    for (int win = 0; win < wk.nwin; ++win) {
+      if (!mbar_wait(bars.empty + 8u * s, parity ^ 1u, bars.abort_flag)) {
+        if (lane == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
+        return false;
+      }
+      const uint32_t full = bars.full + 8u * s, stage = ring + (uint32_t)s * p.stage_bytes;
+      bool stored = false;
+      if constexpr (Format<FMT>::SCB != 0) {
+        if (gathered) stored = gather_scales<FMT, STEPS>(p, wk, stage + lay.sc_off, col0, cols, win, warp, lane);
+      }
+      if (p.x_mode == X_COPIED) stored |= copy_activations<FMT, STEPS>(p, stage + lay.x_off, win, warp, lane);
+      if (stored) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        mbar_arrive(full);
+      } else {
+        cp_async_arrive_noinc(full);
+      }
+      if (++s == p.stages) { s = 0; parity ^= 1u; }
+    }
+  }
+  return true;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Consumers.
+
+// What a consumer lane needs of the launch, held in registers or as constants of the tile.
+struct Lane {
+  int g, t, warp;              // lane / 4, lane % 4, consumer warp
+  __device__ __forceinline__ Lane() : g((threadIdx.x & 31) >> 2), t(threadIdx.x & 3), warp(threadIdx.x >> 5) {}
+};
+// Tile row (of eight) that lane group g supplies. Rows lie PAD bytes off a multiple of 128 apart: with 16 the rows that
+// share an access phase (g = 2q, 2q + 1) must be four apart to lie 64 bytes apart; with 32 (MXFP8, four rows a phase)
+// the natural order does.
+template <int FMT>
+__device__ __forceinline__ int fragment_row(int g) {
+  return FMT == FMT_MXFP8 ? g : (g >> 1) | ((g & 1) << 2);
+}
+
+// Activation row (of eight) that lane group g supplies, likewise: the two of a phase lie in 128-byte rows whose slots the
+// swizzle permutes by row; where a lane's slots are four apart (BF16, MXFP8) the two must differ in bit 2.
+template <int FMT>
+__device__ __forceinline__ int fragment_column(int g) {
+  return split_columns(FMT) ? (g >> 1) | ((g & 1) << 2) : g;
+}
+
+// A lane's share of one chunk of 16 rows: PIECES times 16 bytes of rows g and g + 8, with their scales (NVFP4: two E4M3
+// of the two 16-blocks in the low 16 bits; MXFP8: two E8M0 of the chunk's two blocks).
+template <int FMT> struct Fragment {
+  static constexpr int CHUNK = Format<FMT>::STEP / kConsumers, PIECES = CHUNK / 64;
+  static constexpr int NB = PIECES * Format<FMT>::E / 2, SUB = NB / 4;   // pairs a lane holds per row; eights of them
+};
+template <int FMT> struct RawRows { uint4 lo[Fragment<FMT>::PIECES], hi[Fragment<FMT>::PIECES]; uint32_t slo, shi; };
+
+template <int FMT>
+__device__ __forceinline__ uint4 load_piece(uint32_t row, int t, int piece) {   // `row`: the chunk of one row
+  if constexpr (FMT == FMT_MXFP8) {
+    const uint2 a = lds64(row + t * 8), b = lds64(row + 32 + t * 8);
+    return make_uint4(a.x, a.y, b.x, b.y);
+  } else {
+    return lds128(row + piece * 64 + t * 16);
+  }
+}
+
+// Weights of sub-block q (8 per row: four pairs) in the tensor cores' 16-bit type.
+template <int FMT>
+__device__ __forceinline__ void decode_sub(const uint4 (&v)[Fragment<FMT>::PIECES], uint32_t scale2, int q, uint32_t (&h)[4]) {
+  if constexpr (FMT == FMT_BF16) {
+    h[0] = v[q].x; h[1] = v[q].y; h[2] = v[q].z; h[3] = v[q].w;
+  } else if constexpr (FMT == FMT_NVFP4) {
+    decode_e2m1_h(q == 0 ? v[0].x : q == 1 ? v[0].y : q == 2 ? v[0].z : v[0].w, h);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = mul_half2(h[i], scale2);
+  } else {
+    decode_e4m3_h(q ? v[0].z : v[0].x, q ? v[0].w : v[0].y, h);
+  }
+}
+
+// One chunk of 16 rows into the running sums: acc[nt][0] rows g, acc[nt][1] rows g + 8, columns (2 t, 2 t + 1) + 8 nt.
+// SCALE: the activations' power of two comes off again: SCALE_NONE there is none, SCALE_WINDOW the usual one, SCALE_COLUMN
+// `unscale` per column.
+enum : int { SCALE_NONE = 0, SCALE_WINDOW = 1, SCALE_COLUMN = 2 };
+// HALF: there are no rows g + 8; their products are neither made nor added.
+template <int FMT, int NT, int SCALE, bool HALF>
+__device__ __forceinline__ void chunk_rows(const RawRows<FMT>& raw, const uint32_t (&b)[NT][Fragment<FMT>::NB],
+                                           const pk2 (&unscale)[NT], pk2 (&acc)[NT][2]) {
+  constexpr int SUB = Fragment<FMT>::SUB, PER = SUB / 2;   // two chains: of four steps (NVFP4) or two
+  constexpr bool BF = FMT == FMT_BF16;
+  uint32_t s2lo[2] = {0u, 0u}, s2hi[2] = {0u, 0u};
+  if constexpr (FMT == FMT_NVFP4) {
+    const uint32_t a = e4m3x2_to_half2(raw.slo);
+    s2lo[0] = __byte_perm(a, a, 0x1010); s2lo[1] = __byte_perm(a, a, 0x3232);
+    if constexpr (!HALF) {
+      const uint32_t c = e4m3x2_to_half2(raw.shi);
+      s2hi[0] = __byte_perm(c, c, 0x1010); s2hi[1] = __byte_perm(c, c, 0x3232);
+    }
+  }
+  float part[2][NT][4];
+#pragma unroll
+  for (int q = 0; q < SUB; ++q) {
+    const int chain = q / PER;
+    uint32_t lo[4], hi[4];
+    decode_sub<FMT>(raw.lo, s2lo[q >> 1 & 1], q, lo);
+    if constexpr (!HALF) {
+      decode_sub<FMT>(raw.hi, s2hi[q >> 1 & 1], q, hi);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) hi[i] = lo[i];
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      if (q % PER == 0) mma_step<BF, true>(part[chain][nt], lo[0], hi[0], lo[1], hi[1], b[nt][4 * q], b[nt][4 * q + 1]);
+      else mma_step<BF, false>(part[chain][nt], lo[0], hi[0], lo[1], hi[1], b[nt][4 * q], b[nt][4 * q + 1]);
+      mma_step<BF, false>(part[chain][nt], lo[2], hi[2], lo[3], hi[3], b[nt][4 * q + 2], b[nt][4 * q + 3]);
+    }
+  }
+  const pk2 window = pack2(kWindowUnscale, kWindowUnscale);
+  pk2 mx[2][2];                           // MXFP8: [block][rows g, g + 8] scales, powers of two
+  if constexpr (FMT == FMT_MXFP8) {
+    e8m0x2_to_f32(raw.slo, mx[0][0], mx[1][0]);
+    if constexpr (!HALF) e8m0x2_to_f32(raw.shi, mx[0][1], mx[1][1]);
+    if (SCALE == SCALE_WINDOW) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int half = 0; half < (HALF ? 1 : 2); ++half) mx[c][half] = fmul2(mx[c][half], window);
+    }
+  }
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int half = 0; half < (HALF ? 1 : 2); ++half) {
+      pk2 v0 = pack2(part[0][nt][2 * half], part[0][nt][2 * half + 1]);
+      pk2 v1 = pack2(part[1][nt][2 * half], part[1][nt][2 * half + 1]);
+      if constexpr (FMT == FMT_MXFP8) {
+        // (a column's power of two first: the product with the block's scale is then the true one)
+        if (SCALE == SCALE_COLUMN) { v0 = fmul2(v0, unscale[nt]); v1 = fmul2(v1, unscale[nt]); }
+        acc[nt][half] = ffma2(v1, mx[1][half], ffma2(v0, mx[0][half], acc[nt][half]));
+      } else {
+        v0 = fadd2(v0, v1);
+        acc[nt][half] = SCALE == SCALE_NONE ? fadd2(v0, acc[nt][half])
+                                            : ffma2(v0, SCALE == SCALE_WINDOW ? window : unscale[nt], acc[nt][half]);
+      }
+    }
+}
+
+// Where the lane's activations of its warp's chunk lie in a step: columns (fragment_column of g) + 8 nt, NJ slots of 16
+// bytes. Columns past the last activation row repeat it: nobody reads their sums.
+template <int FMT, int NT>
+struct XOffsets {
+  static constexpr int NJ = Fragment<FMT>::NB / 4;
+  uint32_t off[NT][NJ];
+  __device__ __forceinline__ XOffsets(const Lane& ln, int M) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int m = min(fragment_column<FMT>(ln.g) + 8 * nt, M - 1);
+        const int slot = ln.warp * 4 * NJ + (split_columns(FMT) ? 4 * j + ln.t : NJ * ln.t + j);   // of the step's
+        off[nt][j] = (uint32_t)x_slot((slot >> 3) * M + m, slot & 7);
+      }
+  }
+};
+// The activations as stored, NB pairs per column. (Past the row's end there are zeros, as in the weights and scales.)
+template <int FMT, int NT>
+__device__ __forceinline__ void load_x(uint32_t xs, const XOffsets<FMT, NT>& xo, uint32_t (&b)[NT][Fragment<FMT>::NB]) {
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int j = 0; j < Fragment<FMT>::NB / 4; ++j) {
+      const uint4 v = lds128(xs + xo.off[nt][j]);
+      b[nt][4 * j] = v.x; b[nt][4 * j + 1] = v.y; b[nt][4 * j + 2] = v.z; b[nt][4 * j + 3] = v.w;
+    }
+}
+
+// The same from global memory, step `step` of the rows; zeros past their end.
+template <int FMT, int NT>
+__device__ __forceinline__ void load_x_global(const Params& p, int step, const Lane& ln, uint32_t (&b)[NT][Fragment<FMT>::NB]) {
+  constexpr int NJ = Fragment<FMT>::NB / 4;
+  const unsigned char* x = reinterpret_cast<const unsigned char*>(p.x);
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int m = min(fragment_column<FMT>(ln.g) + 8 * nt, p.M - 1);
+      const int k = step * (Format<FMT>::XROW / 2) + (ln.warp * 4 * NJ + (split_columns(FMT) ? 4 * j + ln.t : NJ * ln.t + j)) * 8;
+      const uint4 v = k < p.K ? ldg_nc128(x + ((size_t)m * p.ldx + k) * 2) : make_uint4(0u, 0u, 0u, 0u);
+      b[nt][4 * j] = v.x; b[nt][4 * j + 1] = v.y; b[nt][4 * j + 2] = v.z; b[nt][4 * j + 3] = v.w;
+    }
+}
+
+// BF16 activations of a chunk (b, as stored) to FP16 in the usual way. Columns with a value outside the window are left out
+// (zeros); returns whether there are any, the same for all lanes of the warp.
+template <int NT, int NB>
+__device__ __forceinline__ bool window_chunk(uint32_t (&b)[NT][NB]) {
+  bool left_out = false;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    uint32_t outside = 0u;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) outside |= window_bits(b[nt][i]);
+    uint32_t misfit = 0u;
+    if (__any_sync(0xffffffffu, (outside & kOutside) != 0u)) misfit = __ballot_sync(0xffffffffu, !window_fits<NB>(b[nt]));
+#pragma unroll
+    for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(b[nt][i], kWindowScale);
+    if (misfit != 0u) {
+      left_out = true;
+      if (((misfit >> (threadIdx.x & 28)) & 0xfu) != 0u) {
+#pragma unroll
+        for (int i = 0; i < NB; ++i) b[nt][i] = 0u;
+      }
+    }
+  }
+  return left_out;
+}
+// The powers of two to take off the lane's sums' columns (2 t, 2 t + 1) again, from the lanes that hold these columns.
+__device__ __forceinline__ pk2 column_unscale(uint32_t e, const Lane& ln) {
+  return pack2(exp_unscale(__shfl_sync(0xffffffffu, e, 8 * ln.t)), exp_unscale(__shfl_sync(0xffffffffu, e, 8 * ln.t + 4)));
+}
+
+__device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumers) : "memory"); }
+// Resident activations have come as they are in global memory; every consumer warp puts its own slice of K into the form and
+// order the tiles read it in: BF16 values as FP16 in the usual way, a chunk with values outside the window as zeros (and
+// marked in `marks`: 1), FP16 ones as they are, the slots of a 128-byte row swizzled. No other warp reads that slice, so nobody
+// waits for anybody. The lanes of a group g take activation row g % M, chunks of 8 / M steps at a time. Returns whether there
+// are chunks outside the window.
+template <int FMT, bool HALF>
+__device__ __forceinline__ bool prepare_resident(const Params& p, unsigned char* smem, uint32_t marks) {
+  constexpr int XROW = Format<FMT>::XROW, NJ = Fragment<FMT>::NB / 4;
+  const Lane ln;
+  const int M = p.M, together = 8 / M, m = ln.g % M, steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP;
+  const uint32_t base = smem_addr(smem) + (uint32_t)p.x_res_off;
+  bool misfit = false;
+  for (int st0 = 0; st0 < steps; st0 += together) {
+    const int st = st0 + ln.g / M;
+    const bool mine = ln.g < together * M && st < steps;
+    uint4 v[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int slot = ln.warp * 4 * NJ + NJ * ln.t + j;
+      v[j] = mine ? lds128(base + (uint32_t)(st * M * XROW + ((slot >> 3) * M + m) * 128 + (slot & 7) * 16)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    bool out = false;
+    if constexpr (HALF) {
+      bool fits = true;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+        fits = fits && window_fits<4>(w);
+      }
+      out = ((__ballot_sync(0xffffffffu, !fits) >> (threadIdx.x & 28)) & 0xfu) != 0u;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        v[j] = out ? make_uint4(0u, 0u, 0u, 0u)
+                   : make_uint4(scaled_half2(v[j].x, kWindowScale), scaled_half2(v[j].y, kWindowScale),
+                                scaled_half2(v[j].z, kWindowScale), scaled_half2(v[j].w, kWindowScale));
+      misfit |= out;
+    }
+    __syncwarp();                  // (every lane has read its slots of the rows)
+    if (mine) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int slot = ln.warp * 4 * NJ + NJ * ln.t + j;
+        sts128(base + (uint32_t)(st * M * XROW + x_slot((slot >> 3) * M + m, slot & 7)), v[j]);
+      }
+      if (HALF && ln.t == 0) sts_u8(marks + (st * kConsumers + ln.warp) * M + m, out ? 1u : 0u);
+    }
+    __syncwarp();
+  }
+  return __any_sync(0xffffffffu, misfit);
+}
+
+// A row's two scale bytes of the lane. (Gathered MXFP8 rows may lie on odd addresses.)
+template <int FMT>
+__device__ __forceinline__ uint32_t load_scales(uint32_t at) {
+  return FMT == FMT_MXFP8 ? lds_u8(at) | lds_u8(at + 1) << 8 : lds_u16(at);
+}
+// Rows g and (unless HALF) g + 8, hi_row rows further on, of the chunk at wrow / srow; sc_hi: what the latter's scales lie
+// further off than srow's.
+template <int FMT, int STEPS, bool HALF>
+__device__ __forceinline__ void load_rows(RawRows<FMT>& raw, uint32_t wrow, uint32_t srow, int hi_row, int sc_hi, int t) {
+#pragma unroll
+  for (int i = 0; i < Fragment<FMT>::PIECES; ++i) {
+    raw.lo[i] = load_piece<FMT>(wrow, t, i);
+    if constexpr (!HALF) raw.hi[i] = load_piece<FMT>(wrow + hi_row * weight_pitch(FMT, STEPS), t, i);
+  }
+  if constexpr (Format<FMT>::SCB != 0) {
+    raw.slo = load_scales<FMT>(srow);
+    if constexpr (!HALF) raw.shi = load_scales<FMT>(srow + hi_row * scale_pitch(FMT, STEPS) + (FMT == FMT_MXFP8 ? sc_hi : 0));
+  }
+}
+
+// The columns of a chunk that were left out because of values outside the window, in as many passes as their values take:
+// into sums of their own, one set per row group. The chunk's activations lie at xs (as stored), or, where they are resident
+// (RES), in global memory, with their marks at `marked`.
+template <int FMT, int NT, int STEPS, bool RES>
+__device__ __noinline__ void extra_passes(const Params& p, pk2 (*acc)[NT][2], int groups, int last_hi, uint32_t xs, int step,
+                                          uint32_t wrow, uint32_t srow, int sc_hi, uint32_t marked) {
+  constexpr int NB = Fragment<FMT>::NB;
+  const Lane ln;
+  const int M = p.M;
+  const XOffsets<FMT, NT> xo(ln, M);
+  uint32_t high[NT];              // magnitudes from here on are done
+  bool more = true;
+  for (bool again = false; more; again = true) {
+    uint32_t b[NT][NB];
+    pk2 unscale[NT];
+    if constexpr (RES) load_x_global<FMT, NT>(p, step, ln, b);
+    else load_x<FMT, NT>(xs, xo, b);
+    more = false;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      if (!again) {
+        const bool mine = RES ? lds_u8(marked + min(fragment_column<FMT>(ln.g), M - 1)) != 0u
+                              : ((__ballot_sync(0xffffffffu, !window_fits<NB>(b[nt])) >> (threadIdx.x & 28)) & 0xfu) != 0u;
+        high[nt] = mine ? 0x8000u : 0u;
+      }
+#pragma unroll
+      for (int i = 0; i < NB; ++i) b[nt][i] = keep_range(b[nt][i], 0u, high[nt]);
+      uint32_t top = chunk_amax<NB>(b[nt]);
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+      top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+      const uint32_t e = chunk_exp(top), low = chunk_low(e);
+      more |= __any_sync(0xffffffffu, !chunk_fits<NB>(b[nt], low));
+      high[nt] = low;
+      const float scale = exp_scale(e);
+#pragma unroll
+      for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(keep_range(b[nt][i], low, 0x8000u), scale);
+      unscale[nt] = column_unscale(e, ln);
+    }
+#pragma unroll 1
+    for (int r = 0; r < groups; ++r) {
+      RawRows<FMT> raw;
+      load_rows<FMT, STEPS, false>(raw, wrow + r * kGroupRows * weight_pitch(FMT, STEPS), srow + r * kGroupRows * scale_pitch(FMT, STEPS),
+                            r + 1 == groups ? last_hi : 8, r + 1 == groups && last_hi == 0 ? 0 : sc_hi, ln.t);
+      chunk_rows<FMT, NT, SCALE_COLUMN, false>(raw, b, unscale, acc[r]);
+    }
+  }
+}
+
+// A tile is finished when every output's sums over the eight consumer warps have been added, in a fixed tree, multiplied by
+// the row's scale and rounded once to the output type. In units of 32 columns x four activation rows, one warp each; unit u:
+// columns 32 (u % 2) + lane (SwiGLU tiles have no more than 32), activation rows from 4 (u / 2) (SwiGLU: 4 u) on.
+__device__ __forceinline__ int finish_units(const Params& p, const Walk& wk) { return (p.M + 3) / 4 * (wk.pairs ? 1 : 2); }
+__device__ __forceinline__ int unit_column(const Walk& wk, int u) { return (threadIdx.x & 31) + (wk.pairs ? 0 : 32 * (u & 1)); }
+// Scale of the lane's column (SwiGLU: of its gate and up row).
+__device__ __forceinline__ void finish_scales(const Params& p, const Walk& wk, int col0, int cols, int u, float (&f)[2]) {
+  const int c = unit_column(wk, u);
+  f[0] = f[1] = 1.f;
+  if (p.row_scale && c < cols) {
+    f[0] = __ldg(p.row_scale + col0 + c);
+    if (wk.pairs) f[1] = __ldg(p.row_scale + wk.pairs + col0 + c);
+  }
+}
+template <int FMT, int STEPS>
+__device__ __forceinline__ void finish_unit(const Params& p, const Walk& wk, uint32_t stage, int col0, int cols, int u,
+                                            const float (&f)[2]) {
+  constexpr int W_ROW = weight_pitch(FMT, STEPS), CHUNK = Fragment<FMT>::CHUNK;
+  const int c = unit_column(wk, u), m = wk.pairs ? 4 * u : u / 2 * 4, M = p.M;
+  if (c >= cols) return;
+  auto sums = [&](int r, float scale, float (&v)[4]) {
+    float a[kConsumers][4];
+#pragma unroll
+    for (int w = 0; w < kConsumers; ++w) {
+      const uint4 q = lds128(stage + (uint32_t)(r * W_ROW + w * CHUNK + m * 4));
+      a[w][0] = __uint_as_float(q.x); a[w][1] = __uint_as_float(q.y); a[w][2] = __uint_as_float(q.z); a[w][3] = __uint_as_float(q.w);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      v[i] = (((a[0][i] + a[1][i]) + (a[2][i] + a[3][i])) + ((a[4][i] + a[5][i]) + (a[6][i] + a[7][i]))) * scale;
+  };
+  float v[4];
+  sums(c, f[0], v);
+  if constexpr (FMT == FMT_NVFP4) {
+    if (wk.pairs) {
+      float up[4];
+      sums(wk.cap + c, f[1], up);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = swiglu_value(v[i], up[i]);
+    }
+  }
+  const size_t at = (p.world < 1 ? 0 : (size_t)p.rank * M * p.ldo) + (size_t)m * p.ldo + col0 + c;
+  auto store = [&](auto kind) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (m + i < M) store_out(p.out, decltype(kind)::value, at + (size_t)i * p.ldo, v[i]);
+  };
+  if (p.out_kind == OUT_F32) store(std::integral_constant<int, OUT_F32>());
+  else if (p.out_kind == OUT_BF16) store(std::integral_constant<int, OUT_BF16>());
+  else store(std::integral_constant<int, OUT_F16>());
+}
+
+// One tile of up to 8 EIGHTS rows: the windows in turn; at the end the warp leaves its sums in the stage it has just consumed,
+// in its own chunk of each row (which no other warp reads), one FP32 per activation row, and tells the finishing warps, to
+// which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the activations are resident (`spread`: some chunk has values outside the window).
+template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool RES>
+__device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, const StageLayout<FMT, STEPS>& lay,
+                                             unsigned char* smem, int col0, int cols, bool last, uint32_t marks, bool spread, const Bars& bars, int& s, uint32_t& parity,
+                                             bool first_window, bool& ok) {
+  constexpr int SCB = Format<FMT>::SCB, STEP = Format<FMT>::STEP, XROW = Format<FMT>::XROW, WIN = STEPS * STEP;
+  constexpr int NB = Fragment<FMT>::NB, CHUNK = Fragment<FMT>::CHUNK, W_ROW = weight_pitch(FMT, STEPS), SC_ROW = scale_pitch(FMT, STEPS);
+  constexpr int G = (EIGHTS + 1) / 2;
+  constexpr bool ODD = EIGHTS % 2 != 0;       // the last group has no second half
+  // BF16 activations of the formats whose weights become FP16
+  constexpr bool CONVERT = FMT != FMT_BF16 && std::is_same<XT, __nv_bfloat16>::value;
+  const Lane ln;
+  const int M = p.M, stage_bytes = p.stage_bytes, stages = p.stages;
+  if (last && p.row_scale && unit_column(wk, ln.warp) < cols) {    // (needed at the tile's end)
+    const float* at = p.row_scale + col0 + unit_column(wk, ln.warp);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+    if (wk.pairs) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + wk.pairs));
+  }
+  const uint32_t ring = smem_addr(smem) + kSmemHeader;
+  const int frow = fragment_row<FMT>(ln.g);
+  // this lane's places in a stage: weights, scales, activations (or among the resident ones)
+  const uint32_t w_off = (uint32_t)(frow * W_ROW + ln.warp * CHUNK);
+  uint32_t sc_off = (uint32_t)(lay.sc_off + frow * SC_ROW + (FMT == FMT_NVFP4 ? ln.warp * 8 + ln.t * 2 : ln.warp * 2));
+  int sc_hi = 0;
+  if (scale_granules<FMT>(p)) {
+    const uint32_t shift = scale_shift(p, col0 + frow);
+    sc_off += shift;
+    if (FMT == FMT_MXFP8) sc_hi = (int)scale_shift(p, col0 + frow + 8) - (int)shift;
+  }
+  const XOffsets<FMT, NT> xo(ln, M);
+  uint32_t res = smem_addr(smem) + (uint32_t)p.x_res_off;    // of the next step
+  const uint32_t x_step = (uint32_t)(M * XROW);
+  pk2 acc[G][NT][2];
+#pragma unroll
+  for (int r = 0; r < G; ++r)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) acc[r][nt][0] = acc[r][nt][1] = pack2(0.f, 0.f);
+  pk2 extra[G][NT][2];            // sums of the columns left out in some step, in local memory
+  bool any_extra = false;
+
+  for (int win = 0, left = p.row_bytes;; ++win) {
+    // (after a wait that ran out the warp goes on without waiting: what it then reads and writes is not used)
+    ok &= mbar_wait(bars.full + 8u * s, parity, bars.abort_flag);
+    if (first_window && win == 0 && threadIdx.x == 0) trace_stamp(p.trace, TRACE_FIRST_FULL);
+    const uint32_t stage = ring + (uint32_t)s * stage_bytes;
+    uint32_t left_out = 0u;       // the steps in which columns were left out
+    // (not unrolled: the steps' code, twice, would not stay in the instruction caches)
+#pragma unroll 1
+    for (int st = 0; st < STEPS && left > st * STEP; ++st) {
+      const uint32_t wrow = stage + w_off + st * STEP, srow = stage + sc_off + st * SCB;
+      uint32_t b[NT][NB];
+      load_x<FMT, NT>(RES ? res + st * x_step : stage + lay.x_off + st * x_step, xo, b);
+      if constexpr (CONVERT && !RES) left_out |= window_chunk<NT, NB>(b) ? 1u << st : 0u;
+      pk2 none[NT] = {};
+      // the next group's rows are loaded while one's are multiplied
+      RawRows<FMT> raw[2];
+      load_rows<FMT, STEPS, ODD && G == 1>(raw[0], wrow, srow, 8, sc_hi, ln.t);
+#pragma unroll
+      for (int r = 0; r < G; ++r) {
+        constexpr int kRow = kGroupRows;
+        const int cur = r & 1;
+        if (r + 2 < G || (r + 2 == G && !ODD))
+          load_rows<FMT, STEPS, false>(raw[cur ^ 1], wrow + (r + 1) * kRow * W_ROW, srow + (r + 1) * kRow * SC_ROW, 8, sc_hi, ln.t);
+        else if (r + 2 == G)
+          load_rows<FMT, STEPS, true>(raw[cur ^ 1], wrow + (r + 1) * kRow * W_ROW, srow + (r + 1) * kRow * SC_ROW, 8, sc_hi, ln.t);
+        constexpr int SC = CONVERT ? SCALE_WINDOW : SCALE_NONE;
+        if (ODD && r == G - 1) chunk_rows<FMT, NT, SC, true>(raw[cur], b, none, acc[r]);
+        else chunk_rows<FMT, NT, SC, false>(raw[cur], b, none, acc[r]);
+      }
+    }
+    if constexpr (CONVERT) {
+      if (RES && spread) {
+#pragma unroll 1
+        for (int st = 0; st < STEPS; ++st)
+          if (left > st * STEP && __any_sync(0xffffffffu, lds_u8(marks + ((win * STEPS + st) * kConsumers + ln.warp) * M +
+                                                                 min(fragment_column<FMT>(ln.g), M - 1)) != 0u))
+            left_out |= 1u << st;
+      }
+      if (left_out != 0u) {
+        if (!any_extra) {
+#pragma unroll
+          for (int r = 0; r < G; ++r)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) extra[r][nt][0] = extra[r][nt][1] = pack2(0.f, 0.f);
+          any_extra = true;
+        }
+#pragma unroll 1
+        for (int st = 0; st < STEPS; ++st)
+          if (left_out >> st & 1u)
+            extra_passes<FMT, NT, STEPS, RES>(p, extra, G, ODD ? 0 : 8, stage + lay.x_off + st * x_step, win * STEPS + st,
+                                              stage + w_off + st * STEP, stage + sc_off + st * SCB, sc_hi,
+                                              marks + ((win * STEPS + st) * kConsumers + ln.warp) * M);
+      }
+    }
+    left -= WIN;
+    if (RES) res += STEPS * x_step;
+    __syncwarp();
+    if (left <= 0) break;
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bars.empty + 8u * s);
+    if (++s == stages) { s = 0; parity ^= 1u; }
+  }
+  if (CONVERT && any_extra) {
+#pragma unroll
+    for (int r = 0; r < G; ++r)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) acc[r][nt][half] = fadd2(acc[r][nt][half], extra[r][nt][half]);
+  }
+  float scales[2];
+  if (last) finish_scales(p, wk, col0, cols, ln.warp, scales);
+  const uint32_t at = ring + (uint32_t)s * stage_bytes + w_off;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    // the fragments' columns 2 t and 2 t + 1
+    const int m0 = 8 * nt + fragment_column<FMT>(2 * ln.t), m1 = 8 * nt + fragment_column<FMT>(2 * ln.t + 1);
+#pragma unroll
+    for (int r = 0; r < G; ++r)
+#pragma unroll
+      for (int half = 0; half < (ODD && r == G - 1 ? 1 : 2); ++half) {
+        float a, c;
+        unpack2(acc[r][nt][half], a, c);
+        const uint32_t row = at + (uint32_t)((r * kGroupRows + half * 8) * W_ROW);
+        if (m0 < M) sts_f32(row + m0 * 4, a);
+        if (m1 < M) sts_f32(row + m1 * 4, c);
+      }
+  }
+  if (last) {
+    consumer_barrier();
+    if (ln.warp < finish_units(p, wk)) finish_unit<FMT, STEPS>(p, wk, ring + (uint32_t)s * stage_bytes, col0, cols, ln.warp, scales);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the stage's next contents come by bulk copies
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive((last ? bars.empty : bars.sums) + 8u * s);
+  if (++s == stages) { s = 0; parity ^= 1u; }
+}
+
+// The consumer warps' walk over one GEMV, tile by tile. The ring position (s, parity) carries over from one GEMV of a
+// batch to the next; `first`: the kernel's first GEMV.
+template <int FMT, int NT, bool CAN_RES, int STEPS, typename XT>
+__device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* smem, unsigned char* marks, const Bars& bars,
+                                             int& s, uint32_t& parity, uint32_t& x_parity, bool first) {
+  const Walk wk(p, STEPS * Format<FMT>::STEP);
+  const StageLayout<FMT, STEPS> lay(p);
+  if (first) griddep_wait();   // consumers read scales and write results in global memory: after the previous kernel
+  bool resident = false, spread = false;
+  const uint32_t marks_at = smem_addr(marks);
+  bool ok = true;
+  if (first && threadIdx.x == 0) trace_stamp(p.trace, TRACE_DEP);
+  if constexpr (CAN_RES) {
+    resident = p.x_mode == X_RESIDENT;
+    if (resident && wk.ntiles > 0) {
+      ok = mbar_wait(bars.x, x_parity, bars.abort_flag);
+      x_parity ^= 1u;
+      spread = prepare_resident<FMT, std::is_same<XT, __nv_bfloat16>::value>(p, smem, marks_at);
+    }
+  }
+  for (int t = 0; t < wk.ntiles; ++t) {
+    int col0, cols;
+    wk.tile(t, col0, cols);
+    auto tile = [&](auto res) {
+      constexpr bool RES = decltype(res)::value;
+      auto run = [&](auto e) {
+        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, marks_at, spread, bars, s, parity, first && t == 0, ok);
+      };
+      switch ((wk.rows(cols) + 7) / 8) {
+        case 8: run(std::integral_constant<int, 8>()); break;
+        case 7: run(std::integral_constant<int, 7>()); break;
+        case 6: run(std::integral_constant<int, 6>()); break;
+        case 5: run(std::integral_constant<int, 5>()); break;
+        case 4: run(std::integral_constant<int, 4>()); break;
+        case 3: run(std::integral_constant<int, 3>()); break;
+        case 2: run(std::integral_constant<int, 2>()); break;
+        default: run(std::integral_constant<int, 1>());
+      }
+    };
+    if constexpr (CAN_RES) {
+      if (resident) tile(std::true_type());
+      else tile(std::false_type());
+    } else {
+      tile(std::false_type());
+    }
+  }
+  if (!ok && (threadIdx.x & 31) == 0 && p.status) atomicOr(p.status, kStatusConsumerTimeout);
+  return ok;
+}
+
+// The finishing warps' walk over one GEMV: every tile but the last, which the consumers finish themselves. They are at the
+// next tile's windows meanwhile (with the consumers finishing every tile between two barriers a tile of 64 rows took 0.6 us
+// longer). `team`: how many warps finish; `sums_parity`: a phase bit per stage.
+template <int FMT, int STEPS>
+__device__ __forceinline__ bool finish_gemv(const Params& p, unsigned char* smem, const Bars& bars, int worker, int team, int& s,
+                                            uint32_t& sums_parity) {
+  const Walk wk(p, STEPS * Format<FMT>::STEP);
+  const int lane = threadIdx.x & 31, stages = p.stages, skip = wk.nwin % stages;
+  // of the eight arrivals that a stage's return takes
+  const int arrivals = kConsumers / team + (worker < kConsumers % team ? 1 : 0);
+  for (int t = 0; t < wk.ntiles; ++t) {
+    int col0, cols;
+    wk.tile(t, col0, cols);
+    s += skip - 1;                 // the tile's last window
+    if (s < 0) s += stages;
+    if (s >= stages) s -= stages;
+    if (t + 1 < wk.ntiles) {
+      if (!mbar_wait(bars.sums + 8u * s, sums_parity >> s & 1u, bars.abort_flag)) {
+        if (lane == 0 && p.status) atomicOr(p.status, kStatusConsumerTimeout);
+        return false;
+      }
+      const uint32_t stage = smem_addr(smem) + kSmemHeader + (uint32_t)s * p.stage_bytes;
+      for (int u = worker; u < finish_units(p, wk); u += team) {
+        float f[2];
+        finish_scales(p, wk, col0, cols, u, f);
+        finish_unit<FMT, STEPS>(p, wk, stage, col0, cols, u, f);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the stage's next contents come by bulk copies
+      __syncwarp();
+      if (lane == 0) mbar_arrive_count(bars.empty + 8u * s, arrivals);
+      sums_parity ^= 1u << s;
+    }
+    if (++s == stages) s = 0;
+  }
+  return true;
+}
+
+// All-gather epilogue: all rows of the CTA have been written (every warp but the feeding one).
+__device__ __forceinline__ void finished_barrier() { asm volatile("bar.sync 3, %0;" ::"n"(kThreads - 32) : "memory"); }
+
 // All-gather epilogue, first half: the CTA's rows [lo, hi) of this rank's slot are complete in the local buffer; all
 // consumer threads copy them into the same place of every other rank's buffer: 16 bytes per store where the rows'
 // addresses allow it (every rank's buffer has the layout and alignment of this one), else element by element.
-template <int M, int CW>
 __device__ __forceinline__ void gather_copy(const Params& p) {
-  const int tid = threadIdx.x;                       // consumer threads are 0 .. CW * 32 - 1
-  asm volatile("bar.sync 1, %0;" ::"r"(CW * 32) : "memory");
+  const int tid = threadIdx.x, M = p.M;                       // consumer threads are 0 .. 255
+  finished_barrier();
   if (p.world < 2) return;
   const int lo = (int)(((long long)p.N * blockIdx.x) / gridDim.x);
   const int rows = (int)(((long long)p.N * (blockIdx.x + 1)) / gridDim.x) - lo;
@@ -1384,9 +1168,9 @@ __device__ __forceinline__ void gather_copy(const Params& p) {
   bool vector = true;                                // all buffers equally placed within 16 bytes
   for (int q = 0; q < p.world; ++q)
     vector &= ((reinterpret_cast<uintptr_t>(p.peer_out[q]) ^ reinterpret_cast<uintptr_t>(p.out)) & 15) == 0;
-  // warp w copies activation rows w, w + CW, ...; its lanes run along the CTA's rows (consecutive addresses)
+  // warp w copies activation rows w, w + 8, ...; its lanes run along the CTA's rows (consecutive addresses)
   const int lane = tid & 31, warp = tid >> 5;
-  for (int m = warp; m < M; m += CW) {
+  for (int m = warp; m < M; m += kConsumers) {
     const size_t byte0 = (slot0 + (size_t)m * p.ldo) * esize;
     const unsigned char* src = reinterpret_cast<const unsigned char*>(p.out) + byte0;
     const int bytes = rows * esize;
@@ -1426,9 +1210,8 @@ __device__ __forceinline__ void gather_copy(const Params& p) {
 
 // Second half: one thread publishes the CTA's copies and counts the CTA done; the rank's last CTA sends `arrivals`
 // arrivals to every rank (one per gathered GEMV) and waits, bounded, until its own counter holds arrivals x world.
-template <int CW>
 __device__ __forceinline__ void gather_signal(const Params& p, volatile int* abort_flag, unsigned int arrivals) {
-  asm volatile("bar.sync 1, %0;" ::"r"(CW * 32) : "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory");
   if (threadIdx.x != 0) return;
   // System-scope operations cost about a microsecond each and this is the kernel's tail, so the chain is kept short:
   // fence (the CTA's peer copies), one acquire-release count per CTA, then the last CTA fences once and sends one
@@ -1462,76 +1245,14 @@ __device__ __forceinline__ void gather_signal(const Params& p, volatile int* abo
     atomicOr(p.status, kStatusGatherTimeout);
 }
 
-// The consumer warps' walk over one GEMV: tiles in order, each for up to RMAX rows a warp. The ring position (s,
-// parity) carries over; `fresh`: the ring is empty and unfilled (a kernel's first GEMV, or any GEMV of a kernel
-// whose consumers feed themselves, which starts after all its warps have left the previous one).
-template <int FMT, int M, typename XT, int CW, bool SELF>
-__device__ __forceinline__ bool consume_gemv(const Params& p, const Params& maps, unsigned char* smem, uint32_t full0,
-                                             uint32_t empty0, volatile int* abort_flag, int& s, uint32_t& parity,
-                                             bool first) {
-  constexpr int RMAX = rows_max(FMT, M);
-  const int warp = threadIdx.x >> 5;
-  const Walk<CW> wk(p);
-  const StageLayout<FMT, M, CW> lay(p);
-  if constexpr (SELF) {
-    // the first stages - 1 iterations, into the stages after s; with static weights, in a kernel's first GEMV, their
-    // weight copies leave before the previous kernel of the stream has completed
-    const int ahead = min(p.stages - 1, wk.ntiles * wk.nwin);
-    const bool early = first && p.early_weights;
-    if (early)
-      for (int i = 0; i < ahead; ++i)
-        self_fill<FMT, M, CW>(p, maps, wk, lay, smem, full0, empty0, i, (s + i) % p.stages, true, false);
-    if (first) griddep_wait();
-    for (int i = 0; i < ahead; ++i)
-      self_fill<FMT, M, CW>(p, maps, wk, lay, smem, full0, empty0, i, (s + i) % p.stages, !early, true);
-  } else if (first) {
-    griddep_wait();   // consumers read scales and write results in global memory: after the previous kernel
-  }
-  bool resident = false;
-  if constexpr (resident_capable(FMT, M) && !SELF) {
-    resident = p.x_resident != 0;
-    if (resident) {
-      // (a later GEMV of a batch: nobody reads the previous one's activations any more)
-      if (!first) asm volatile("bar.sync 1, %0;" ::"r"(CW * 32) : "memory");
-      fill_resident<FMT, M, CW, Arithmetic<FMT, M, XT>::HALF_RES>(p, smem);
-    }
-  }
-  if (first && threadIdx.x == 0) trace_stamp(p.trace, TRACE_DEP);
-  int it = 0;
-  bool ok = true;
-  for (int t = 0; t < wk.ntiles && ok; ++t) {
-    int nr = 0;                      // rows this warp holds in the tile: one per group that reaches it
-    for (int g = 0; g < p.rows_per_warp; ++g) {
-      int group0, group_n;
-      wk.group(t, g, group0, group_n);
-      if (warp < group_n) nr = g + 1;
-    }
-    // three rows have their own code only where tiles of odd heights are made on purpose (split tails)
-    constexpr bool THREE = M == 1 && RMAX == 4;
-    auto tile = [&](auto res) {
-      constexpr bool RES = decltype(res)::value;
-      if (nr > (THREE ? 3 : 2))
-        return consume_tile<FMT, M, RMAX, XT, CW, SELF, RES>(p, maps, wk, lay, smem, full0, empty0, abort_flag, t, nr, s,
-                                                             parity, it);
-      if (THREE && nr > 2)
-        return consume_tile<FMT, M, THREE ? 3 : RMAX, XT, CW, SELF, RES>(p, maps, wk, lay, smem, full0, empty0, abort_flag,
-                                                                        t, nr, s, parity, it);
-      if (nr > 1)
-        return consume_tile<FMT, M, 2, XT, CW, SELF, RES>(p, maps, wk, lay, smem, full0, empty0, abort_flag, t, nr, s,
-                                                          parity, it);
-      return consume_tile<FMT, M, 1, XT, CW, SELF, RES>(p, maps, wk, lay, smem, full0, empty0, abort_flag, t, nr, s, parity,
-                                                        it);
-    };
-    if constexpr (resident_capable(FMT, M) && !SELF) ok = resident ? tile(std::true_type()) : tile(std::false_type());
-    else ok = tile(std::false_type());
-  }
-  if (!ok && (threadIdx.x & 31) == 0 && p.status) atomicOr(p.status, kStatusConsumerTimeout);
-  return ok;
-}
-
-// Barriers and the abort word of a CTA; the first thread sets them up.
-template <int CW, int COPY_WARPS>
-__device__ __forceinline__ void ring_setup(const Params& p, uint32_t full0, uint32_t empty0, volatile int* abort_flag) {
+// Barriers and the abort word of a CTA; the first thread sets them up. `copies`: the copying warps take part.
+__device__ __forceinline__ Bars ring_setup(const Params& p, bool copies, unsigned char* smem, uint64_t* sums) {
+  Bars bars;
+  bars.x = smem_addr(sums + kMaxStages);
+  bars.full = smem_addr(smem);
+  bars.empty = bars.full + 8u * kMaxStages;
+  bars.sums = smem_addr(sums);
+  bars.abort_flag = reinterpret_cast<volatile int*>(smem + 2 * kMaxStages * 8);
   if (threadIdx.x == 0) {
     if (p.trace) {
       unsigned int sm;
@@ -1540,47 +1261,59 @@ __device__ __forceinline__ void ring_setup(const Params& p, uint32_t full0, uint
       trace_stamp(p.trace, TRACE_ENTRY);
     }
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(full0 + 8u * s, 32 * COPY_WARPS + 1);   // the copying lanes' cp.async arrivals + the expect_tx arrival
-      mbar_init(empty0 + 8u * s, CW);
+      mbar_init(bars.full + 8u * s, 1 + (copies ? 32 * kCopyWarps : 0));   // the expect_tx arrival + the copying lanes'
+                                                                           // cp.async arrivals
+      mbar_init(bars.empty + 8u * s, kConsumers);
+      mbar_init(bars.sums + 8u * s, kConsumers);
     }
-    *abort_flag = 0;
-    *reinterpret_cast<volatile unsigned long long*>(abort_flag + 2) = p.wait_limit_ns;
+    mbar_init(bars.x, 1);
+    *bars.abort_flag = 0;
+    *reinterpret_cast<volatile unsigned long long*>(bars.abort_flag + 2) = p.wait_limit_ns;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
   griddep_launch_dependents();
+  return bars;
 }
 
-template <int FMT, int M, typename XT>
-__global__ void __launch_bounds__((consumer_warps(FMT, M) + producer_warps(FMT, M)) * 32, ctas_per_sm(FMT, M))
-    gemv_kernel(const __grid_constant__ Params p) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int CW = consumer_warps(FMT, M), PW = producer_warps(FMT, M);
-  constexpr bool SELF = PW == 0;             // no producer warps: the consumers issue the copies themselves
-  constexpr int COPY_WARPS = SELF ? CW : PW;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 2 * kMaxStages * 8);
-  const uint32_t full0 = smem_addr(bars), empty0 = full0 + 8u * kMaxStages;
-  ring_setup<CW, COPY_WARPS>(p, full0, empty0, abort_flag);
+// NT: column tiles of 8 activation rows; CAN_RES: the launch may keep the activations resident (resident_capable).
+template <int FMT, int NT, bool CAN_RES, int STEPS, typename XT>
+__global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant__ Params p) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ unsigned char marks[CAN_RES ? kMaxMarks : 1];
+  __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
+  const bool copies = copies_needed<FMT>(p);
+  const Bars bars = ring_setup(p, copies, smem, sums);
   int s = 0;
-  uint32_t parity = 0;
-  if ((int)(threadIdx.x >> 5) >= CW) {
-    if constexpr (!SELF)
-      Producer<FMT, M, CW, COPY_WARPS>(p, p, smem, full0, empty0, (int)threadIdx.x - CW * 32).run(abort_flag, s, parity,
-                                                                                                  true);
+  uint32_t parity = 0, x_parity = 0;
+  const int warp = (int)(threadIdx.x >> 5);
+  if (warp == kFeeder) {
+    if (!p.early_weights) {
+      prefetch_weights<FMT, STEPS>(p);
+      griddep_wait();
+    }
+    feed_weights<FMT, STEPS>(p, p, smem, bars, true, p.early_weights != 0, s, parity);
+  } else if (warp >= kFirstCopier && copies) {
+    griddep_wait();
+    feed_activations<FMT, STEPS>(p, smem, bars, warp - kFirstCopier, s, parity);
+    if (p.world >= 1) finished_barrier();
+  } else if (warp >= kFinisher) {
+    griddep_wait();   // reads scales and writes results in global memory: after the previous kernel
+    finish_gemv<FMT, STEPS>(p, smem, bars, warp - kFinisher, copies ? 1 : kFinishers, s, parity);
+    if (p.world >= 1) finished_barrier();
   } else {
-    consume_gemv<FMT, M, XT, CW, SELF>(p, p, smem, full0, empty0, abort_flag, s, parity, true);
+    consume_gemv<FMT, NT, CAN_RES, STEPS, XT>(p, smem, marks, bars, s, parity, x_parity, true);
     if ((threadIdx.x & 31) == 0) trace_stamp(p.trace, TRACE_LAST_CONSUMED);
     if (p.world >= 1) {
-      gather_copy<M, CW>(p);
-      gather_signal<CW>(p, abort_flag, 1u);
+      gather_copy(p);
+      gather_signal(p, bars.abort_flag, 1u);
     }
   }
   if ((threadIdx.x & 31) == 0) trace_stamp(p.trace, TRACE_EXIT);
   // A wait that ran out leaves copies in flight towards this CTA's shared memory: let them land before the CTA's
   // memory is handed to the next one (bounded sleep, error path only).
-  if (*abort_flag) {
+  if (*bars.abort_flag) {
 #pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
   }
@@ -1593,50 +1326,47 @@ __global__ void __launch_bounds__((consumer_warps(FMT, M) + producer_warps(FMT, 
 // next kernel's CTA can come). With the all-gather epilogue each CTA sends a GEMV's rows to the peers as soon as it has
 // finished them and goes on; the arrivals of all GEMVs are exchanged once, at the end. For GEMVs whose inputs do not
 // depend on each other's outputs only (all activations are read after one wait for the previous kernel).
-template <int FMT, int M, typename XT>
-__global__ void __launch_bounds__((consumer_warps(FMT, M) + producer_warps(FMT, M)) * 32, ctas_per_sm(FMT, M))
-    gemv_batch_kernel(const Params* __restrict__ items, int count) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  constexpr int CW = consumer_warps(FMT, M), PW = producer_warps(FMT, M);
-  constexpr bool SELF = PW == 0;
-  constexpr int COPY_WARPS = SELF ? CW : PW;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 2 * kMaxStages * 8);
-  const uint32_t full0 = smem_addr(bars), empty0 = full0 + 8u * kMaxStages;
-  ring_setup<CW, COPY_WARPS>(items[0], full0, empty0, abort_flag);
+template <int FMT, int NT, bool CAN_RES, int STEPS, typename XT>
+__global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* __restrict__ items, int count) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ unsigned char marks[CAN_RES ? kMaxMarks : 1];
+  __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
+  const Bars bars = ring_setup(items[0], true, smem, sums);
   int s = 0;
-  uint32_t parity = 0;
-  if ((int)(threadIdx.x >> 5) >= CW) {
-    if constexpr (!SELF) {
-      bool ok = true;
-      for (int g = 0; g < count && ok; ++g)
-        ok = Producer<FMT, M, CW, COPY_WARPS>(items[g], items[g], smem, full0, empty0, (int)threadIdx.x - CW * 32)
-                 .run(abort_flag, s, parity, g == 0);
+  uint32_t parity = 0, x_parity = 0;
+  const int warp = (int)(threadIdx.x >> 5);
+  if (warp == kFeeder) {
+    if (!items[0].early_weights) griddep_wait();
+    bool ok = true;
+    for (int g = 0; g < count && ok; ++g)
+      ok = feed_weights<FMT, STEPS>(items[g], items[g], smem, bars, g == 0, g == 0 && items[0].early_weights, s, parity);
+  } else if (warp == kFinisher) {
+    griddep_wait();
+    bool ok = true;
+    for (int g = 0; g < count; ++g) {
+      if (ok) ok = finish_gemv<FMT, STEPS>(items[g], smem, bars, 0, 1, s, parity);
+      if (items[g].world >= 1) finished_barrier();
+    }
+  } else if (warp >= kFirstCopier) {
+    griddep_wait();
+    bool ok = true;
+    for (int g = 0; g < count; ++g) {
+      if (ok) ok = feed_activations<FMT, STEPS>(items[g], smem, bars, warp - kFirstCopier, s, parity);
+      if (items[g].world >= 1) finished_barrier();
     }
   } else {
-    bool ok = true;
-    // Where the consumers feed themselves every warp of the CTA is on the same GEMV, and the kernels are short of
-    // registers: the GEMV's parameters are then kept in shared memory behind the ring (a read from there costs less
-    // than one from global memory; a kernel parameter would cost nothing, but a batch does not fit there).
-    Params* held = reinterpret_cast<Params*>(smem + kSmemHeader + (size_t)items[0].stages * items[0].stage_bytes);
-    for (int g = 0; g < count && ok; ++g) {
-      if constexpr (SELF) {
-        asm volatile("bar.sync 1, %0;" ::"r"(CW * 32) : "memory");
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(items + g);
-        for (int i = threadIdx.x; i < (int)(sizeof(Params) / 4); i += CW * 32) reinterpret_cast<uint32_t*>(held)[i] = src[i];
-        asm volatile("bar.sync 1, %0;" ::"r"(CW * 32) : "memory");
-      }
-      const Params& p = SELF ? *held : items[g];
-      ok = consume_gemv<FMT, M, XT, CW, SELF>(p, items[g], smem, full0, empty0, abort_flag, s, parity, g == 0);
-      // the CTA's rows of this GEMV go to the peers now (and, without producer warps, every warp has left the ring
-      // before the next GEMV refills it: the copy starts with a barrier of the consumer warps)
-      if (p.world >= 1 || SELF) gather_copy<M, CW>(p);
+    // (every warp passes every GEMV's barriers, also after a wait that ran out)
+    for (int g = 0; g < count; ++g) {
+      consume_gemv<FMT, NT, CAN_RES, STEPS, XT>(items[g], smem, marks, bars, s, parity, x_parity, g == 0);
+      if (items[g].world >= 1) gather_copy(items[g]);   // the CTA's rows of this GEMV go to the peers now
     }
     if ((threadIdx.x & 31) == 0) trace_stamp(items[0].trace, TRACE_LAST_CONSUMED);
-    if (items[0].world >= 1) gather_signal<CW>(items[0], abort_flag, (unsigned int)count);
+    if (items[0].world >= 1) gather_signal(items[0], bars.abort_flag, (unsigned int)count);
   }
   if ((threadIdx.x & 31) == 0) trace_stamp(items[0].trace, TRACE_EXIT);
-  if (*abort_flag) {
+  // A wait that ran out leaves copies in flight towards this CTA's shared memory: let them land before the CTA's
+  // memory is handed to the next one (bounded sleep, error path only).
+  if (*bars.abort_flag) {
 #pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
   }
