@@ -328,6 +328,10 @@ __device__ __forceinline__ bool scales_gathered(const Params& p) {
   return Format<FMT>::SCB != 0 && p.scale_mode != SCALES_STAGED;
 }
 
+// The ring's first filling is paced, at a rate of all SMs together somewhat above HBM's: asked for all at once, the first
+// windows came as late as the last, up to 3 us later on some SMs than on others (8192 x 8192 NVFP4, one row: 12.4 us, now 12.0).
+constexpr int kUnpaced = 32 * 1024, kPace = 22;   // bytes at once, bytes per clock
+
 // The feeding warp: weight (and staged scale) copies of every window of one GEMV, in order, and the activations' tensor
 // copies. A tile's rows travel as ONE 2-D tensor copy per region (and one for their scales): a copy costs the SM about 150
 // clocks to start whatever its size (as boxes of 8 rows, 12 to 16 a window, or with single rows for a tile's remainder they
@@ -378,6 +382,7 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
   };
   if (first && !early) resident();
   int filled = 0;
+  const long long start = clock64();
   for (int t = 0; t < wk.ntiles; ++t) {
     int col0, cols;
     wk.tile(t, col0, cols);
@@ -391,6 +396,10 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
       if (behind == stages) catch_up();
       if (!wait_empty(s, parity)) return false;
       if (++filled == stages && !first) resident();
+      if (first && filled > 1 && filled <= stages) {   // (see kPace)
+        const int due = ((filled - 1) * stage_bytes - kUnpaced) / kPace;
+        while ((int)(clock64() - start) < due) {}
+      }
       const uint32_t full = bars.full + 8u * s, stage = ring + (uint32_t)s * stage_bytes;
       if (lane == 0) mbar_arrive_expect_tx(full, bytes);
       __syncwarp();
@@ -415,27 +424,28 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
   return true;
 }
 
-// The first windows' weights (and staged scales) into L2, as many as the ring will hold, before the wait for the previous
-// kernel of the stream: what that kernel may still write reaches the same L2, so the copies after the wait read its
-// values, from L2 instead of HBM.
+// The first window's weights (and staged scales) into L2, before the wait for the previous kernel of the stream: what that
+// kernel may still write reaches the same L2, so the copies after the wait read its values, from L2 instead of HBM. (Further
+// windows would come late for the kernels still running. Small windows are not worth the traffic: 2048 x 2048 FP8 takes 4.7 us
+// without and 5.0 with, 8192 x 8192 NVFP4 13.4 and 12.4.) And the tensor maps, on their way to be used.
+constexpr int kPrefetchFrom = 32 * 1024;   // bytes of a stage
 template <int FMT, int STEPS>
 __device__ __forceinline__ void prefetch_weights(const Params& p) {
-  constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP, SC_WIN = STEPS * SCB;
-  if ((threadIdx.x & 31) != 0) return;
+  constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP;
+  const int lane = threadIdx.x & 31;
+  if (lane < 5 && (lane < 4 || p.x_mode != X_COPIED)) {    // the maps themselves: half a microsecond at their first use
+    const CUtensorMap* map = lane == 0 ? &p.tmap_w : lane == 1 ? &p.tmap_w_last : lane == 2 ? &p.tmap_sc : lane == 3 ? &p.tmap_sc_last : &p.tmap_x;
+    if (lane < 2 || lane == 4 || (SCB != 0 && p.scale_mode == SCALES_STAGED)) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+  }
+  if (lane != 0 || p.stage_bytes < kPrefetchFrom) return;
   const Walk wk(p, WIN);
-  int left = p.stages;
-  for (int t = 0; t < wk.ntiles; ++t) {
-    int col0, cols;
-    wk.tile(t, col0, cols);
-    for (int win = 0; win < wk.nwin; ++win) {
-      for (int region = 0; region < wk.regions; ++region) {
-        const int n0 = region * wk.pairs + col0;
-        tensor_prefetch(cols == wk.cap ? &p.tmap_w : &p.tmap_w_last, (win * WIN) >> 3, n0);
-        if (SCB != 0 && p.scale_mode == SCALES_STAGED)
-          tensor_prefetch(cols == wk.cap ? &p.tmap_sc : &p.tmap_sc_last, (win * SC_WIN) >> 3, n0);
-      }
-      if (--left == 0) return;
-    }
+  if (wk.ntiles == 0) return;
+  int col0, cols;
+  wk.tile(0, col0, cols);
+  for (int region = 0; region < wk.regions; ++region) {
+    const int n0 = region * wk.pairs + col0;
+    tensor_prefetch(cols == wk.cap ? &p.tmap_w : &p.tmap_w_last, 0, n0);
+    if (SCB != 0 && p.scale_mode == SCALES_STAGED) tensor_prefetch(cols == wk.cap ? &p.tmap_sc : &p.tmap_sc_last, 0, n0);
   }
 }
 
@@ -681,7 +691,8 @@ __device__ __forceinline__ void chunk_rows(const RawRows<FMT>& raw, const uint32
 
 // Where the lane's activations of its warp's chunk lie in a step: columns (fragment_column of g) + 8 nt, NJ slots of 16
 // bytes. Columns past the last activation row repeat it: nobody reads their sums.
-template <int FMT, int NT>
+// (Window by window they are swizzled, see x_slot; resident ones lie as they came.)
+template <int FMT, int NT, bool RES>
 struct XOffsets {
   static constexpr int NJ = Fragment<FMT>::NB / 4;
   uint32_t off[NT][NJ];
@@ -692,13 +703,13 @@ struct XOffsets {
       for (int j = 0; j < NJ; ++j) {
         const int m = min(fragment_column<FMT>(ln.g) + 8 * nt, M - 1);
         const int slot = ln.warp * 4 * NJ + (split_columns(FMT) ? 4 * j + ln.t : NJ * ln.t + j);   // of the step's
-        off[nt][j] = (uint32_t)x_slot((slot >> 3) * M + m, slot & 7);
+        off[nt][j] = (uint32_t)(RES ? ((slot >> 3) * M + m) * 128 + (slot & 7) * 16 : x_slot((slot >> 3) * M + m, slot & 7));
       }
   }
 };
 // The activations as stored, NB pairs per column. (Past the row's end there are zeros, as in the weights and scales.)
-template <int FMT, int NT>
-__device__ __forceinline__ void load_x(uint32_t xs, const XOffsets<FMT, NT>& xo, uint32_t (&b)[NT][Fragment<FMT>::NB]) {
+template <int FMT, int NT, bool RES>
+__device__ __forceinline__ void load_x(uint32_t xs, const XOffsets<FMT, NT, RES>& xo, uint32_t (&b)[NT][Fragment<FMT>::NB]) {
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -754,53 +765,56 @@ __device__ __forceinline__ pk2 column_unscale(uint32_t e, const Lane& ln) {
 }
 
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumers) : "memory"); }
-// Resident activations have come as they are in global memory; every consumer warp puts its own slice of K into the form and
-// order the tiles read it in: BF16 values as FP16 in the usual way, a chunk with values outside the window as zeros (and
-// marked in `marks`: 1), FP16 ones as they are, the slots of a 128-byte row swizzled. No other warp reads that slice, so nobody
-// waits for anybody. The lanes of a group g take activation row g % M, chunks of 8 / M steps at a time. Returns whether there
-// are chunks outside the window.
-template <int FMT, bool HALF>
+// Resident activations have come as they are in global memory. BF16 ones: every consumer warp puts its own slice of K into the
+// form the tiles read, FP16 in the usual way, a chunk with values outside the window as zeros (and marked in `marks`: 1). No
+// other warp reads that slice, so nobody waits for anybody. The lanes of a group g take activation row g % M, chunks of 8 / M
+// steps at a time, slot by slot in place. Returns whether there are chunks outside the window. (Rolled loops: this runs once
+// per kernel, from cold instruction caches; unrolled over a lane's slots it took 1.0 us for a single step, now 0.6.)
+template <int FMT>
 __device__ __forceinline__ bool prepare_resident(const Params& p, unsigned char* smem, uint32_t marks) {
   constexpr int XROW = Format<FMT>::XROW, NJ = Fragment<FMT>::NB / 4;
   const Lane ln;
   const int M = p.M, together = 8 / M, m = ln.g % M, steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP;
-  const uint32_t base = smem_addr(smem) + (uint32_t)p.x_res_off;
+  const int slot0 = ln.warp * 4 * NJ + NJ * ln.t;
+  const uint32_t at0 = smem_addr(smem) + (uint32_t)(p.x_res_off + ((slot0 >> 3) * M + m) * 128 + (slot0 & 7) * 16);
   bool misfit = false;
+#pragma unroll 1
   for (int st0 = 0; st0 < steps; st0 += together) {
     const int st = st0 + ln.g / M;
     const bool mine = ln.g < together * M && st < steps;
-    uint4 v[NJ];
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const int slot = ln.warp * 4 * NJ + NJ * ln.t + j;
-      v[j] = mine ? lds128(base + (uint32_t)(st * M * XROW + ((slot >> 3) * M + m) * 128 + (slot & 7) * 16)) : make_uint4(0u, 0u, 0u, 0u);
-    }
-    bool out = false;
-    if constexpr (HALF) {
-      bool fits = true;
-#pragma unroll
+    const uint32_t at = at0 + (uint32_t)(st * M * XROW);
+    uint32_t outside = 0u;
+    if (mine) {
+#pragma unroll 1
       for (int j = 0; j < NJ; ++j) {
-        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-        fits = fits && window_fits<4>(w);
+        const uint4 v = lds128(at + 16 * j);
+        outside |= window_bits(v.x) | window_bits(v.y) | window_bits(v.z) | window_bits(v.w);
+        sts128(at + 16 * j, make_uint4(scaled_half2(v.x, kWindowScale), scaled_half2(v.y, kWindowScale),
+                                       scaled_half2(v.z, kWindowScale), scaled_half2(v.w, kWindowScale)));
+      }
+    }
+    // (a bit may be a zero's: the values once more, from global memory, decide)
+    bool out = false;
+    if (__any_sync(0xffffffffu, (outside & kOutside) != 0u)) {
+      bool fits = true;
+      if (mine) {
+#pragma unroll 1
+        for (int j = 0; j < NJ; ++j) {
+          const int kk = st * (XROW / 2) + (slot0 + j) * 8;
+          if (kk >= p.K) break;
+          const uint4 v = ldg_nc128(reinterpret_cast<const unsigned char*>(p.x) + ((size_t)m * p.ldx + kk) * 2);
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+          fits = fits && window_fits<4>(w);
+        }
       }
       out = ((__ballot_sync(0xffffffffu, !fits) >> (threadIdx.x & 28)) & 0xfu) != 0u;
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-        v[j] = out ? make_uint4(0u, 0u, 0u, 0u)
-                   : make_uint4(scaled_half2(v[j].x, kWindowScale), scaled_half2(v[j].y, kWindowScale),
-                                scaled_half2(v[j].z, kWindowScale), scaled_half2(v[j].w, kWindowScale));
+      if (mine && out) {
+#pragma unroll 1
+        for (int j = 0; j < NJ; ++j) sts128(at + 16 * j, make_uint4(0u, 0u, 0u, 0u));
+      }
       misfit |= out;
     }
-    __syncwarp();                  // (every lane has read its slots of the rows)
-    if (mine) {
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const int slot = ln.warp * 4 * NJ + NJ * ln.t + j;
-        sts128(base + (uint32_t)(st * M * XROW + x_slot((slot >> 3) * M + m, slot & 7)), v[j]);
-      }
-      if (HALF && ln.t == 0) sts_u8(marks + (st * kConsumers + ln.warp) * M + m, out ? 1u : 0u);
-    }
-    __syncwarp();
+    if (mine && ln.t == 0) sts_u8(marks + (st * kConsumers + ln.warp) * M + m, out ? 1u : 0u);
   }
   return __any_sync(0xffffffffu, misfit);
 }
@@ -834,14 +848,14 @@ __device__ __noinline__ void extra_passes(const Params& p, pk2 (*acc)[NT][2], in
   constexpr int NB = Fragment<FMT>::NB;
   const Lane ln;
   const int M = p.M;
-  const XOffsets<FMT, NT> xo(ln, M);
+  const XOffsets<FMT, NT, RES> xo(ln, M);
   uint32_t high[NT];              // magnitudes from here on are done
   bool more = true;
   for (bool again = false; more; again = true) {
     uint32_t b[NT][NB];
     pk2 unscale[NT];
     if constexpr (RES) load_x_global<FMT, NT>(p, step, ln, b);
-    else load_x<FMT, NT>(xs, xo, b);
+    else load_x<FMT, NT, RES>(xs, xo, b);
     more = false;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
@@ -956,7 +970,7 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
     sc_off += shift;
     if (FMT == FMT_MXFP8) sc_hi = (int)scale_shift(p, col0 + frow + 8) - (int)shift;
   }
-  const XOffsets<FMT, NT> xo(ln, M);
+  const XOffsets<FMT, NT, RES> xo(ln, M);
   uint32_t res = smem_addr(smem) + (uint32_t)p.x_res_off;    // of the next step
   const uint32_t x_step = (uint32_t)(M * XROW);
   pk2 acc[G][NT][2];
@@ -978,7 +992,7 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
     for (int st = 0; st < STEPS && left > st * STEP; ++st) {
       const uint32_t wrow = stage + w_off + st * STEP, srow = stage + sc_off + st * SCB;
       uint32_t b[NT][NB];
-      load_x<FMT, NT>(RES ? res + st * x_step : stage + lay.x_off + st * x_step, xo, b);
+      load_x<FMT, NT, RES>(RES ? res + st * x_step : stage + lay.x_off + st * x_step, xo, b);
       if constexpr (CONVERT && !RES) left_out |= window_chunk<NT, NB>(b) ? 1u << st : 0u;
       pk2 none[NT] = {};
       // the next group's rows are loaded while one's are multiplied
@@ -1081,7 +1095,8 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     if (resident && wk.ntiles > 0) {
       ok = mbar_wait(bars.x, x_parity, bars.abort_flag);
       x_parity ^= 1u;
-      spread = prepare_resident<FMT, std::is_same<XT, __nv_bfloat16>::value>(p, smem, marks_at);
+      if constexpr (std::is_same<XT, __nv_bfloat16>::value) spread = prepare_resident<FMT>(p, smem, marks_at);
+      __syncwarp();
     }
   }
   for (int t = 0; t < wk.ntiles; ++t) {
