@@ -328,6 +328,36 @@ __device__ __forceinline__ bool scales_gathered(const Params& p) {
   return Format<FMT>::SCB != 0 && p.scale_mode != SCALES_STAGED;
 }
 
+// Resident activations: all of them, in as few copies as boxes allow (one thread).
+template <int FMT>
+__device__ __forceinline__ void copy_resident(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars) {
+  constexpr int XROW = Format<FMT>::XROW;
+  const int steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP, bytes = p.M * XROW;
+  mbar_arrive_expect_tx(bars.x, (uint32_t)(steps * bytes));
+  for (int st = 0; st < steps; st += p.x_box_steps)
+    tensor3_g2s(smem_addr(smem) + (uint32_t)(p.x_res_off + st * bytes), &maps.tmap_x, st * (XROW / 128), bars.x);
+}
+
+// A kernel's first activations, the moment the previous kernel of the stream has finished (the finishing warp has nothing else
+// to do then): the resident ones, or those of the windows that fill the ring.
+template <int FMT, int STEPS>
+__device__ __forceinline__ void start_activations(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars) {
+  constexpr int X_BLOCKS = STEPS * Format<FMT>::XROW / 128;
+  if ((threadIdx.x & 31) == 0 && p.x_mode != X_COPIED) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.tmap_x) : "memory");
+  griddep_wait();
+  if ((threadIdx.x & 31) != 0) return;
+  const Walk wk(p, STEPS * Format<FMT>::STEP);
+  if (p.x_mode == X_RESIDENT && wk.ntiles > 0) copy_resident<FMT>(p, maps, smem, bars);
+  if (p.x_mode != X_TENSOR) return;
+  const uint32_t at = smem_addr(smem) + kSmemHeader +
+                      (uint32_t)x_offset(p.tile_rows * (weight_pitch(FMT, STEPS) + scale_pitch(FMT, STEPS)));
+  const int windows = min(p.stages, wk.ntiles * wk.nwin);
+  for (int i = 0, win = 0; i < windows; ++i) {
+    tensor3_g2s(at + (uint32_t)i * p.stage_bytes, &maps.tmap_x, win * X_BLOCKS, bars.full + 8u * i);
+    if (++win == wk.nwin) win = 0;
+  }
+}
+
 // The ring's first filling is paced, at a rate of all SMs together somewhat above HBM's: asked for all at once, the first
 // windows came as late as the last, up to 3 us later on some SMs than on others (8192 x 8192 NVFP4, one row: 12.4 us, now 12.0).
 constexpr int kUnpaced = 32 * 1024, kPace = 22;   // bytes at once, bytes per clock
@@ -337,50 +367,37 @@ constexpr int kUnpaced = 32 * 1024, kPace = 22;   // bytes at once, bytes per cl
 // clocks to start whatever its size (as boxes of 8 rows, 12 to 16 a window, or with single rows for a tile's remainder they
 // bounded the whole kernel at 1 us a window). A box is always brought whole: columns past the matrix row's end and rows past
 // the matrix come as zeros and count; rows past the tile are not used. One arrival carries the byte count of all copies;
-// completions may land before it (the phase cannot end while it is outstanding). `early`: the previous kernel of the stream
-// has not been waited for yet; the weights need not. The ring position (stage s, its phase parity) is the caller's and
+// completions may land before it (the phase cannot end while it is outstanding). The activations of a kernel's first windows
+// are not its business (see start_activations): the previous kernel of the stream may not have been waited for yet when
+// the ring fills. The ring position (stage s, its phase parity) is the caller's and
 // carries on from one GEMV of a batch to the next (`first`: its first); `maps`: where the tensor maps are read from.
 template <int FMT, int STEPS>
 __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars,
-                                             bool first, bool early, int& s, uint32_t& parity) {
+                                             bool first, int& s, uint32_t& parity) {
   constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP, SC_WIN = STEPS * SCB;
   constexpr int W_ROW = weight_pitch(FMT, STEPS), SC_ROW = scale_pitch(FMT, STEPS), XROW = Format<FMT>::XROW;
   const Walk wk(p, WIN);
   const int lane = threadIdx.x & 31, stage_bytes = p.stage_bytes, stages = p.stages;
   const bool staged = SCB != 0 && p.scale_mode == SCALES_STAGED;
   const uint32_t ring = smem_addr(smem) + kSmemHeader, sc_off = (uint32_t)(p.tile_rows * W_ROW);
-  // activations by tensor copy, a window at a time: with weights ahead of the wait for the previous kernel of the stream,
-  // those of the first windows follow once the ring is full of weights
+  // activations by tensor copy: a window at a time
   constexpr int X_BLOCKS = STEPS * XROW / 128;
   const uint32_t x_off = (uint32_t)x_offset(p.tile_rows * (W_ROW + SC_ROW));
   const uint32_t x_bytes = p.x_mode == X_TENSOR ? (uint32_t)(X_BLOCKS * 128 * p.M) : 0u;
-  int behind = early ? 0 : -1;                   // windows issued without their activations
   auto activations = [&](int at, int win) {
     if (x_bytes && lane == 31) tensor3_g2s(ring + (uint32_t)at * stage_bytes + x_off, &maps.tmap_x, win * X_BLOCKS, bars.full + 8u * at);
   };
   // or all at once: when nobody reads the previous GEMV's any more, which is known once the last of its stages is empty
-  bool x_due = p.x_mode == X_RESIDENT && wk.ntiles > 0;
+  bool x_due = p.x_mode == X_RESIDENT && wk.ntiles > 0 && !first;
   auto resident = [&] {
-    if (x_due && lane == 31) {
-      const int steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP, bytes = p.M * XROW;
-      mbar_arrive_expect_tx(bars.x, (uint32_t)(steps * bytes));
-      for (int st = 0; st < steps; st += p.x_box_steps)
-        tensor3_g2s(smem_addr(smem) + (uint32_t)(p.x_res_off + st * bytes), &maps.tmap_x, st * (XROW / 128), bars.x);
-    }
+    if (x_due && lane == 31) copy_resident<FMT>(p, maps, smem, bars);
     x_due = false;
-  };
-  auto catch_up = [&] {
-    griddep_wait();
-    resident();
-    for (int i = 0; i < behind; ++i) activations(i, i % wk.nwin);
-    behind = -1;
   };
   auto wait_empty = [&](int at, uint32_t use) {
     if (mbar_wait(bars.empty + 8u * at, use ^ 1u, bars.abort_flag)) return true;
     if (lane == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
     return false;
   };
-  if (first && !early) resident();
   int filled = 0;
   const long long start = clock64();
   for (int t = 0; t < wk.ntiles; ++t) {
@@ -393,9 +410,9 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
     // lanes 0, 1: the regions' weights; 2, 3: their scales
     const int region = lane & 1, n0 = region * wk.pairs + col0, row0 = region * wk.cap;
     for (int win = 0; win < wk.nwin; ++win) {
-      if (behind == stages) catch_up();
       if (!wait_empty(s, parity)) return false;
-      if (++filled == stages && !first) resident();
+      if (++filled == stages) resident();
+      if (first && filled == stages + 1) griddep_wait();   // (passed by now, but not by this warp)
       if (first && filled > 1 && filled <= stages) {   // (see kPace)
         const int due = ((filled - 1) * stage_bytes - kUnpaced) / kPace;
         while ((int)(clock64() - start) < due) {}
@@ -403,16 +420,14 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
       const uint32_t full = bars.full + 8u * s, stage = ring + (uint32_t)s * stage_bytes;
       if (lane == 0) mbar_arrive_expect_tx(full, bytes);
       __syncwarp();
-      if (behind < 0) activations(s, win);
+      if (!first || filled > stages) activations(s, win);
       if (region < wk.regions) {
         if (lane < 2) tensor_g2s(stage + row0 * W_ROW, map_w, (win * WIN) >> 3, n0, full);
         else if (lane < 4 && staged) tensor_g2s(stage + sc_off + row0 * SC_ROW, map_sc, (win * SC_WIN) >> 3, n0, full);
       }
-      if (behind >= 0) ++behind;
       if (++s == stages) { s = 0; parity ^= 1u; }
     }
   }
-  if (behind >= 0) catch_up();
   if (x_due) {                     // fewer windows than stages
     int at = s;
     uint32_t use = parity;
@@ -433,9 +448,9 @@ template <int FMT, int STEPS>
 __device__ __forceinline__ void prefetch_weights(const Params& p) {
   constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP;
   const int lane = threadIdx.x & 31;
-  if (lane < 5 && (lane < 4 || p.x_mode != X_COPIED)) {    // the maps themselves: half a microsecond at their first use
-    const CUtensorMap* map = lane == 0 ? &p.tmap_w : lane == 1 ? &p.tmap_w_last : lane == 2 ? &p.tmap_sc : lane == 3 ? &p.tmap_sc_last : &p.tmap_x;
-    if (lane < 2 || lane == 4 || (SCB != 0 && p.scale_mode == SCALES_STAGED)) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+  if (lane < 4) {               // the maps themselves: half a microsecond at their first use
+    const CUtensorMap* map = lane == 0 ? &p.tmap_w : lane == 1 ? &p.tmap_w_last : lane == 2 ? &p.tmap_sc : &p.tmap_sc_last;
+    if (lane < 2 || (SCB != 0 && p.scale_mode == SCALES_STAGED)) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
   }
   if (lane != 0 || p.stage_bytes < kPrefetchFrom) return;
   const Walk wk(p, WIN);
@@ -1308,13 +1323,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
       prefetch_weights<FMT, STEPS>(p);
       griddep_wait();
     }
-    feed_weights<FMT, STEPS>(p, p, smem, bars, true, p.early_weights != 0, s, parity);
+    feed_weights<FMT, STEPS>(p, p, smem, bars, true, s, parity);
   } else if (warp >= kFirstCopier && copies) {
     griddep_wait();
     feed_activations<FMT, STEPS>(p, smem, bars, warp - kFirstCopier, s, parity);
     if (p.world >= 1) finished_barrier();
   } else if (warp >= kFinisher) {
-    griddep_wait();   // reads scales and writes results in global memory: after the previous kernel
+    // (reads scales and writes results in global memory: after the previous kernel)
+    if (warp == kFinisher) start_activations<FMT, STEPS>(p, p, smem, bars);
+    else griddep_wait();
     finish_gemv<FMT, STEPS>(p, smem, bars, warp - kFinisher, copies ? 1 : kFinishers, s, parity);
     if (p.world >= 1) finished_barrier();
   } else {
@@ -1354,9 +1371,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* _
     if (!items[0].early_weights) griddep_wait();
     bool ok = true;
     for (int g = 0; g < count && ok; ++g)
-      ok = feed_weights<FMT, STEPS>(items[g], items[g], smem, bars, g == 0, g == 0 && items[0].early_weights, s, parity);
+      ok = feed_weights<FMT, STEPS>(items[g], items[g], smem, bars, g == 0, s, parity);
   } else if (warp == kFinisher) {
-    griddep_wait();
+    start_activations<FMT, STEPS>(items[0], items[0], smem, bars);
     bool ok = true;
     for (int g = 0; g < count; ++g) {
       if (ok) ok = finish_gemv<FMT, STEPS>(items[g], smem, bars, 0, 1, s, parity);
