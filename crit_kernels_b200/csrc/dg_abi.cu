@@ -122,13 +122,16 @@ DeviceState* device_state() {
   bool ok = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) == cudaSuccess && major == 10 &&
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0 &&
             cudaGetSymbolAddress(&status, dg_status_word) == cudaSuccess;
-  auto opt_in = [&](const void* const (*table)[16]) {
-    for (int i = 0; ok && i < 32; ++i)
+  // (the whole of an SM's 228 KB as shared memory: two small blocks, or one, and no change between launches)
+  auto opt_in = [&](const void* const (*table)[16], int rows) {
+    for (int i = 0; ok && i < 16 * rows; ++i)
       ok = cudaFuncSetAttribute(table[i / 16][i % 16], cudaFuncAttributeMaxDynamicSharedMemorySize, dg::kSmemLimit) ==
-           cudaSuccess;
+               cudaSuccess &&
+           cudaFuncSetAttribute(table[i / 16][i % 16], cudaFuncAttributePreferredSharedMemoryCarveout,
+                                cudaSharedmemCarveoutMaxShared) == cudaSuccess;
   };
-  for (const void* const (*table)[16] : kTables) opt_in(table);
-  opt_in(dg_batch_table_nvfp4_bf16);
+  for (const void* const (*table)[16] : kTables) opt_in(table, 4);
+  opt_in(dg_batch_table_nvfp4_bf16, 2);
   if (!ok) {
     cudaGetLastError();
     st.ready.store(-1, std::memory_order_release);
@@ -177,6 +180,8 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
   const int regions = p.pairs ? 2 : 1;    // N counts columns; gate_up matrices have two rows to a column
   ctas = grid > 0 ? grid : sms < ceil_div(N, 4) ? sms : ceil_div(N, 4);   // grid: the launch is shared (batch)
   const int cols_per_cta = ceil_div(N, ctas), all_rows = regions * ceil_div(cols_per_cta, dg::kBoxRows) * dg::kBoxRows;
+  p.cols_each = N / ctas;
+  p.cols_more = N % ctas;
   const int row_steps = ceil_div(p.row_bytes, f.step);
   // Tuning aid: DG_FORCE_PLAN="rows,steps" fixes the rows of a tile and the steps of a stage (read once).
   static const char* forced = std::getenv("DG_FORCE_PLAN");
@@ -227,6 +232,26 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
     }
   }
   if (p.tile_rows == 0) return false;
+  // Small launches: a stage for every window, in half of the shared memory, so that the next launch's CTA fits beside.
+  if (grid == 0 && dg::column_tiles(M) == 1 && all_rows <= dg::kSmallRows && K % 64 == 0 && p.scale_mode != dg::SCALES_DIRECT &&
+      p.scale_mode != dg::SCALES_BLOCKED && force_steps == 0) {
+    const int steps = fmt == dg::FMT_BF16 || row_steps == 1 ? 1 : 2, windows = std::max(2, ceil_div(row_steps, steps));
+    const int rows = regions * ceil_div(all_rows / regions, dg::kBoxRows) * dg::kBoxRows;
+    const bool resident = may_reside;
+    int stage_bytes = rows * (dg::weight_pitch(fmt, steps) + dg::scale_pitch(fmt, steps));
+    if (!resident) stage_bytes = (dg::x_offset(stage_bytes) + steps * M * f.x_row + 1023) / 1024 * 1024;
+    stage_bytes = (stage_bytes + 127) / 128 * 128;
+    if (windows <= dg::kMaxStages &&
+        dg::kSmemHeader + windows * stage_bytes + (resident ? resident_bytes : 0) <= dg::kSmallSmem) {
+      p.small = 1;
+      p.tile_rows = rows;
+      p.last_rows = rows / regions;
+      p.steps = steps;
+      p.stage_bytes = stage_bytes;
+      p.stages = windows;
+      p.x_mode = resident ? dg::X_RESIDENT : dg::X_TENSOR;
+    }
+  }
   p.x_res_off = dg::kSmemHeader + p.stages * p.stage_bytes;
   smem = p.x_res_off + (p.x_mode == dg::X_RESIDENT ? resident_bytes : 0);
   return true;
@@ -290,7 +315,8 @@ int launch(int table, int fmt, Params& p, int M, cudaStream_t stream) {
       p.trace = base + (size_t)index * DG_TRACE_CTAS * dg::kTraceSlots;
   }
   void* args[] = {&p};
-  return launch_pdl(kTables[table][p.steps - 1][M - 1], args, ctas, dg::kThreads, smem, stream);
+  return launch_pdl(kTables[table][p.steps - 1 + 2 * p.small][M - 1], args, ctas, p.small ? dg::kSmallThreads : dg::kThreads, smem,
+                    stream);
 }
 
 // Argument rules of the NVFP4 GEMV (dg_enqueue_nvfp4) and the fields they determine.

@@ -47,11 +47,17 @@ constexpr int kConsumers = 8;              // = chunks of a step: the slices of 
 // that bulk copies cannot bring, two of these copy instead.
 constexpr int kFeeder = kConsumers, kFinisher = kConsumers + 1, kFinishers = 3, kFirstCopier = kConsumers + 2, kCopyWarps = 2;
 constexpr int kThreads = 32 * (kConsumers + 1 + kFinishers);
+// Small launches: a CTA's whole share is one tile of at most 32 rows, brought by bulk copies alone, and fits in half of the
+// SM's shared memory. Their blocks have fewer warps (the finisher only starts the activations) and fewer registers, so that
+// two fit on an SM: the next launch of the stream then waits there for this one to finish, its barriers set up and its weights
+// on their way into L2.
+constexpr int kSmallThreads = 32 * (kConsumers + 2), kSmallRows = 32;
+constexpr int kSmallSmem = 111 * 1024;     // dynamic shared memory: 228 KB for two, less 1 KB and the static part each
 constexpr int kBoxRows = 8;                // tile rows come in multiples of these
 constexpr int kGroupRows = 16;             // rows of one mma tile
 constexpr int kMaxGroups = 4;              // mma tiles of rows a warp holds at most
 constexpr int kSmemHeader = 256;           // mbarriers + abort flag
-constexpr int kStaticSmem = 1024;          // room left for the kernels' static shared memory (kMaxMarks, kMaxStages)
+constexpr int kStaticSmem = 1024;          // room left for the kernels' static shared memory
 constexpr int kSmemLimit = 232448 - kStaticSmem;   // dynamic shared memory per CTA (sm_100 has 227 KB in all)
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;   // bounded waits give up after this (default; the host
                                                              // can set another limit, Params::wait_limit_ns)
@@ -99,7 +105,6 @@ __host__ __device__ constexpr int x_offset(int before) { return ((before + kSmem
 // tensor cores take (see prepare_resident) while the first weights are on their way.
 __host__ __device__ constexpr bool resident_capable(int fmt, int m) { return (fmt == FMT_FP8 || fmt == FMT_NVFP4) && m <= 4; }
 constexpr int kResidentLimit = 96 * 1024;   // bytes of activations (and their flags) a kernel keeps resident at most
-constexpr int kMaxMarks = kResidentLimit / 2 / 64;   // marks of their (row, chunk)s: an FP8 chunk is 64 elements
 
 struct Params {
   const void* x;             // [M][ldx] BF16 or FP16
@@ -116,6 +121,8 @@ struct Params {
   int scale_mode;            // SCALES_*
   int ct;                    // tiled scales: 4-block tiles per tile row
   int M;                     // activation rows
+  int cols_each, cols_more;  // the CTAs' output columns (see Walk)
+  int small;                 // 1: a small launch (see kSmallThreads)
   int steps;                 // 512-byte steps per ring stage
   int stages;                // ring depth
   int tile_rows;             // rows of a full tile (a multiple of 8; gate_up: of 16, for both regions), at most 16 * kMaxGroups
@@ -272,16 +279,19 @@ struct Bars {
 // left. A tile's rows in the stage: its columns' matrix rows (regions = 1), or, for a gate_up matrix with the SwiGLU epilogue
 // (regions = 2), its columns' gate rows and, from row cap on, their up rows.
 
+// First column of CTA c: the first cols_more CTAs have cols_each + 1, the others cols_each.
+__device__ __forceinline__ int first_column(const Params& p, unsigned c) { return (int)c * p.cols_each + min((int)c, p.cols_more); }
+
 struct Walk {
   int lo, hi, cap, regions, ntiles, nwin;
   int pairs;                     // SwiGLU epilogue: rows per half of the gate_up matrix (0: an ordinary matrix)
   __device__ __forceinline__ Walk(const Params& p, int window_bytes) {
     pairs = p.pairs;
-    lo = (int)(((long long)p.N * blockIdx.x) / gridDim.x);
-    hi = (int)(((long long)p.N * (blockIdx.x + 1)) / gridDim.x);
+    lo = first_column(p, blockIdx.x);
+    hi = first_column(p, blockIdx.x + 1);
     regions = pairs ? 2 : 1;
-    cap = p.tile_rows / regions;
-    ntiles = (hi - lo + cap - 1) / cap;
+    cap = pairs ? p.tile_rows >> 1 : p.tile_rows;
+    ntiles = (int)((unsigned)(hi - lo + cap - 1) / (unsigned)cap);
     nwin = (p.row_bytes + window_bytes - 1) / window_bytes;
   }
   // First column and width of tile t.
@@ -344,9 +354,9 @@ template <int FMT, int STEPS>
 __device__ __forceinline__ void start_activations(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars) {
   constexpr int X_BLOCKS = STEPS * Format<FMT>::XROW / 128;
   if ((threadIdx.x & 31) == 0 && p.x_mode != X_COPIED) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.tmap_x) : "memory");
+  const Walk wk(p, STEPS * Format<FMT>::STEP);
   griddep_wait();
   if ((threadIdx.x & 31) != 0) return;
-  const Walk wk(p, STEPS * Format<FMT>::STEP);
   if (p.x_mode == X_RESIDENT && wk.ntiles > 0) copy_resident<FMT>(p, maps, smem, bars);
   if (p.x_mode != X_TENSOR) return;
   const uint32_t at = smem_addr(smem) + kSmemHeader +
@@ -370,10 +380,11 @@ constexpr int kUnpaced = 32 * 1024, kPace = 22;   // bytes at once, bytes per cl
 // completions may land before it (the phase cannot end while it is outstanding). The activations of a kernel's first windows
 // are not its business (see start_activations): the previous kernel of the stream may not have been waited for yet when
 // the ring fills. The ring position (stage s, its phase parity) is the caller's and
-// carries on from one GEMV of a batch to the next (`first`: its first); `maps`: where the tensor maps are read from.
+// carries on from one GEMV of a batch to the next (`first`: its first; `wait`: the previous kernel of the stream has to be
+// waited for); `maps`: where the tensor maps are read from.
 template <int FMT, int STEPS>
 __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars,
-                                             bool first, int& s, uint32_t& parity) {
+                                             bool first, bool wait, int& s, uint32_t& parity) {
   constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP, SC_WIN = STEPS * SCB;
   constexpr int W_ROW = weight_pitch(FMT, STEPS), SC_ROW = scale_pitch(FMT, STEPS), XROW = Format<FMT>::XROW;
   const Walk wk(p, WIN);
@@ -398,6 +409,7 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
     if (lane == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
     return false;
   };
+  if (wait) griddep_wait();   // (with everything worked out)
   int filled = 0;
   const long long start = clock64();
   for (int t = 0; t < wk.ntiles; ++t) {
@@ -413,7 +425,7 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
       if (!wait_empty(s, parity)) return false;
       if (++filled == stages) resident();
       if (first && filled == stages + 1) griddep_wait();   // (passed by now, but not by this warp)
-      if (first && filled > 1 && filled <= stages) {   // (see kPace)
+      if (first && filled > 1 && filled <= stages && !p.small) {   // (see kPace)
         const int due = ((filled - 1) * stage_bytes - kUnpaced) / kPace;
         while ((int)(clock64() - start) < due) {}
       }
@@ -439,9 +451,9 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
   return true;
 }
 
-// The first window's weights (and staged scales) into L2, before the wait for the previous kernel of the stream: what that
-// kernel may still write reaches the same L2, so the copies after the wait read its values, from L2 instead of HBM. (Further
-// windows would come late for the kernels still running. Small windows are not worth the traffic: 2048 x 2048 FP8 takes 4.7 us
+// The first window's weights (and staged scales; a small launch: all of them) into L2, before the wait for the previous kernel
+// of the stream: what that kernel may still write reaches the same L2, so the copies after the wait read its values, from L2
+// instead of HBM. (Further windows would come late for the kernels still running. Small windows are not worth the traffic: 2048 x 2048 FP8 takes 4.7 us
 // without and 5.0 with, 8192 x 8192 NVFP4 13.4 and 12.4.) And the tensor maps, on their way to be used.
 constexpr int kPrefetchFrom = 32 * 1024;   // bytes of a stage
 template <int FMT, int STEPS>
@@ -452,16 +464,18 @@ __device__ __forceinline__ void prefetch_weights(const Params& p) {
     const CUtensorMap* map = lane == 0 ? &p.tmap_w : lane == 1 ? &p.tmap_w_last : lane == 2 ? &p.tmap_sc : &p.tmap_sc_last;
     if (lane < 2 || (SCB != 0 && p.scale_mode == SCALES_STAGED)) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
   }
-  if (lane != 0 || p.stage_bytes < kPrefetchFrom) return;
+  if (lane != 0 || (!p.small && p.stage_bytes < kPrefetchFrom)) return;
   const Walk wk(p, WIN);
   if (wk.ntiles == 0) return;
   int col0, cols;
   wk.tile(0, col0, cols);
-  for (int region = 0; region < wk.regions; ++region) {
-    const int n0 = region * wk.pairs + col0;
-    tensor_prefetch(cols == wk.cap ? &p.tmap_w : &p.tmap_w_last, 0, n0);
-    if (SCB != 0 && p.scale_mode == SCALES_STAGED) tensor_prefetch(cols == wk.cap ? &p.tmap_sc : &p.tmap_sc_last, 0, n0);
-  }
+  for (int win = 0; win < (p.small ? wk.nwin : 1); ++win)
+    for (int region = 0; region < wk.regions; ++region) {
+      const int n0 = region * wk.pairs + col0;
+      tensor_prefetch(cols == wk.cap ? &p.tmap_w : &p.tmap_w_last, (win * WIN) >> 3, n0);
+      if (SCB != 0 && p.scale_mode == SCALES_STAGED)
+        tensor_prefetch(cols == wk.cap ? &p.tmap_sc : &p.tmap_sc_last, (win * STEPS * SCB) >> 3, n0);
+    }
 }
 
 // The other producer warps, where they are needed: the windows' activations where no tensor copy can bring them, 16 bytes
@@ -781,22 +795,23 @@ __device__ __forceinline__ pk2 column_unscale(uint32_t e, const Lane& ln) {
 
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumers) : "memory"); }
 // Resident activations have come as they are in global memory. BF16 ones: every consumer warp puts its own slice of K into the
-// form the tiles read, FP16 in the usual way, a chunk with values outside the window as zeros (and marked in `marks`: 1). No
+// form the tiles read, FP16 in the usual way, a chunk with values outside the window as zeros (see extra_tile). No
 // other warp reads that slice, so nobody waits for anybody. The lanes of a group g take activation row g % M, chunks of 8 / M
 // steps at a time, slot by slot in place. Returns whether there are chunks outside the window. (Rolled loops: this runs once
 // per kernel, from cold instruction caches; unrolled over a lane's slots it took 1.0 us for a single step, now 0.6.)
 template <int FMT>
-__device__ __forceinline__ bool prepare_resident(const Params& p, unsigned char* smem, uint32_t marks) {
+__device__ __forceinline__ uint32_t prepare_resident(const Params& p, unsigned char* smem) {
   constexpr int XROW = Format<FMT>::XROW, NJ = Fragment<FMT>::NB / 4;
   const Lane ln;
-  const int M = p.M, together = 8 / M, m = ln.g % M, steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP;
+  const int M = p.M, by = M == 1 ? 32 : M == 2 ? 16 : M == 3 ? 11 : 8, q = ln.g * by >> 5, m = ln.g - q * M;   // q: g / M
+  const int together = M == 1 ? 8 : M == 2 ? 4 : 2, steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP;
   const int slot0 = ln.warp * 4 * NJ + NJ * ln.t;
   const uint32_t at0 = smem_addr(smem) + (uint32_t)(p.x_res_off + ((slot0 >> 3) * M + m) * 128 + (slot0 & 7) * 16);
-  bool misfit = false;
+  uint32_t misfit = 0u;
 #pragma unroll 1
   for (int st0 = 0; st0 < steps; st0 += together) {
-    const int st = st0 + ln.g / M;
-    const bool mine = ln.g < together * M && st < steps;
+    const int st = st0 + q;
+    const bool mine = q < together && st < steps;
     const uint32_t at = at0 + (uint32_t)(st * M * XROW);
     uint32_t outside = 0u;
     if (mine) {
@@ -827,11 +842,10 @@ __device__ __forceinline__ bool prepare_resident(const Params& p, unsigned char*
 #pragma unroll 1
         for (int j = 0; j < NJ; ++j) sts128(at + 16 * j, make_uint4(0u, 0u, 0u, 0u));
       }
-      misfit |= out;
+      if (out) misfit |= 1u << (st & 31);
     }
-    if (mine && ln.t == 0) sts_u8(marks + (st * kConsumers + ln.warp) * M + m, out ? 1u : 0u);
   }
-  return __any_sync(0xffffffffu, misfit);
+  return __reduce_or_sync(0xffffffffu, misfit);
 }
 
 // A row's two scale bytes of the lane. (Gathered MXFP8 rows may lie on odd addresses.)
@@ -854,50 +868,102 @@ __device__ __forceinline__ void load_rows(RawRows<FMT>& raw, uint32_t wrow, uint
   }
 }
 
-// The columns of a chunk that were left out because of values outside the window, in as many passes as their values take:
-// into sums of their own, one set per row group. The chunk's activations lie at xs (as stored), or, where they are resident
-// (RES), in global memory, with their marks at `marked`.
-template <int FMT, int NT, int STEPS, bool RES>
-__device__ __noinline__ void extra_passes(const Params& p, pk2 (*acc)[NT][2], int groups, int last_hi, uint32_t xs, int step,
-                                          uint32_t wrow, uint32_t srow, int sc_hi, uint32_t marked) {
+// A lane's share of a chunk of one weight row, and its scales, from global memory (zeros past the row's end).
+template <int FMT>
+__device__ __forceinline__ void load_row_global(const Params& p, int n, int step, const Lane& ln, uint4 (&v)[Fragment<FMT>::PIECES],
+                                                uint32_t& sc) {
+  constexpr int STEP = Format<FMT>::STEP, SCB = Format<FMT>::SCB, CHUNK = Fragment<FMT>::CHUNK;
+  const uint8_t* row = p.w + (size_t)n * p.row_bytes;
+#pragma unroll
+  for (int i = 0; i < Fragment<FMT>::PIECES; ++i) {
+    const int at = step * STEP + ln.warp * CHUNK + (FMT == FMT_MXFP8 ? ln.t * 8 : i * 64 + ln.t * 16);
+    if constexpr (FMT == FMT_MXFP8) {
+      const uint2 z = make_uint2(0u, 0u);
+      const uint2 a = at < p.row_bytes ? __ldg(reinterpret_cast<const uint2*>(row + at)) : z;
+      const uint2 c = at + 32 < p.row_bytes ? __ldg(reinterpret_cast<const uint2*>(row + at + 32)) : z;
+      v[i] = make_uint4(a.x, a.y, c.x, c.y);
+    } else {
+      v[i] = at < p.row_bytes ? ldg_nc128(row + at) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  sc = 0u;
+  if constexpr (SCB != 0) {
+    const int sc_bytes = p.row_bytes * SCB / STEP, j = step * SCB + (FMT == FMT_NVFP4 ? ln.warp * 8 + ln.t * 2 : ln.warp * 2);
+    const uint8_t* src = p.scales + (p.scale_mode == SCALES_BLOCKED ? tiled_scale_offset(n, j, p.ct) : (size_t)n * p.scale_row_bytes + j);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (j + i < sc_bytes) sc |= (uint32_t)__ldg(src + i) << (8 * i);
+  }
+}
+
+// The columns that were left out of some chunks because of values outside the window, after the tile: their products, in as
+// many passes as the values take, are added to the sums the warp has left in the stage (`sums`: the lane's row 0 there).
+// `steps`: bit i, one of the steps i + 32 n. Everything comes from global memory again: such values are rare, and a call inside
+// the tile's loop cost every launch registers (NVFP4 4096 x 4096, one row: 6.7 us, and 5.9 for FP16, which has none).
+template <int FMT, int NT>
+__device__ __noinline__ void extra_tile(const Params& p, int col0, int cols, uint32_t sums, uint32_t pitch,
+                                        uint32_t steps) {
   constexpr int NB = Fragment<FMT>::NB;
   const Lane ln;
-  const int M = p.M;
-  const XOffsets<FMT, NT, RES> xo(ln, M);
-  uint32_t high[NT];              // magnitudes from here on are done
-  bool more = true;
-  for (bool again = false; more; again = true) {
-    uint32_t b[NT][NB];
-    pk2 unscale[NT];
-    if constexpr (RES) load_x_global<FMT, NT>(p, step, ln, b);
-    else load_x<FMT, NT, RES>(xs, xo, b);
-    more = false;
+  const Walk wk(p, Format<FMT>::STEP);
+  const int M = p.M, rows = wk.rows(cols), all = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP;
+#pragma unroll 1
+  for (int r0 = 0; r0 < rows; r0 += kGroupRows) {
+    pk2 acc[NT][2];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = pack2(0.f, 0.f);
+    const int lo = r0 + fragment_row<FMT>(ln.g), hi = lo + 8;
+    const int n_lo = wk.matrix_row(col0, cols, min(lo, rows - 1)), n_hi = wk.matrix_row(col0, cols, min(hi, rows - 1));
+#pragma unroll 1
+    for (int step = 0; step < all; ++step) {
+      if ((steps >> (step & 31) & 1u) == 0u) continue;
+      uint32_t high[NT];              // magnitudes from here on are done
+      bool more = true;
+      for (bool again = false; more; again = true) {
+        uint32_t b[NT][NB];
+        pk2 unscale[NT];
+        load_x_global<FMT, NT>(p, step, ln, b);
+        more = false;
+        bool any = again;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          if (!again) {
+            const uint32_t misfit = __ballot_sync(0xffffffffu, !window_fits<NB>(b[nt]));
+            high[nt] = ((misfit >> (threadIdx.x & 28)) & 0xfu) != 0u ? 0x8000u : 0u;
+            any |= misfit != 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < NB; ++i) b[nt][i] = keep_range(b[nt][i], 0u, high[nt]);
+          uint32_t top = chunk_amax<NB>(b[nt]);
+          top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+          top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+          const uint32_t e = chunk_exp(top), low = chunk_low(e);
+          more |= __any_sync(0xffffffffu, !chunk_fits<NB>(b[nt], low));
+          high[nt] = low;
+          const float scale = exp_scale(e);
+#pragma unroll
+          for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(keep_range(b[nt][i], low, 0x8000u), scale);
+          unscale[nt] = column_unscale(e, ln);
+        }
+        if (!any) break;
+        RawRows<FMT> raw;
+        load_row_global<FMT>(p, n_lo, step, ln, raw.lo, raw.slo);
+        load_row_global<FMT>(p, n_hi, step, ln, raw.hi, raw.shi);
+        chunk_rows<FMT, NT, SCALE_COLUMN, false>(raw, b, unscale, acc);
+      }
+    }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      if (!again) {
-        const bool mine = RES ? lds_u8(marked + min(fragment_column<FMT>(ln.g), M - 1)) != 0u
-                              : ((__ballot_sync(0xffffffffu, !window_fits<NB>(b[nt])) >> (threadIdx.x & 28)) & 0xfu) != 0u;
-        high[nt] = mine ? 0x8000u : 0u;
+      const int m0 = 8 * nt + fragment_column<FMT>(2 * ln.t), m1 = 8 * nt + fragment_column<FMT>(2 * ln.t + 1);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        float a, c;
+        unpack2(acc[nt][half], a, c);
+        const uint32_t at = sums + (uint32_t)(r0 + half * 8) * pitch;
+        if (r0 + half * 8 >= rows) continue;     // (an eighth without rows has no sums)
+        if (m0 < M) sts_f32(at + m0 * 4, lds_f32(at + m0 * 4) + a);
+        if (m1 < M) sts_f32(at + m1 * 4, lds_f32(at + m1 * 4) + c);
       }
-#pragma unroll
-      for (int i = 0; i < NB; ++i) b[nt][i] = keep_range(b[nt][i], 0u, high[nt]);
-      uint32_t top = chunk_amax<NB>(b[nt]);
-      top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
-      top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
-      const uint32_t e = chunk_exp(top), low = chunk_low(e);
-      more |= __any_sync(0xffffffffu, !chunk_fits<NB>(b[nt], low));
-      high[nt] = low;
-      const float scale = exp_scale(e);
-#pragma unroll
-      for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(keep_range(b[nt][i], low, 0x8000u), scale);
-      unscale[nt] = column_unscale(e, ln);
-    }
-#pragma unroll 1
-    for (int r = 0; r < groups; ++r) {
-      RawRows<FMT> raw;
-      load_rows<FMT, STEPS, false>(raw, wrow + r * kGroupRows * weight_pitch(FMT, STEPS), srow + r * kGroupRows * scale_pitch(FMT, STEPS),
-                            r + 1 == groups ? last_hi : 8, r + 1 == groups && last_hi == 0 ? 0 : sc_hi, ln.t);
-      chunk_rows<FMT, NT, SCALE_COLUMN, false>(raw, b, unscale, acc[r]);
     }
   }
 }
@@ -959,7 +1025,7 @@ __device__ __forceinline__ void finish_unit(const Params& p, const Walk& wk, uin
 // which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the activations are resident (`spread`: some chunk has values outside the window).
 template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool RES>
 __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, const StageLayout<FMT, STEPS>& lay,
-                                             unsigned char* smem, int col0, int cols, bool last, uint32_t marks, bool spread, const Bars& bars, int& s, uint32_t& parity,
+                                             unsigned char* smem, int col0, int cols, bool last, uint32_t spread, const Bars& bars, int& s, uint32_t& parity,
                                              bool first_window, bool& ok) {
   constexpr int SCB = Format<FMT>::SCB, STEP = Format<FMT>::STEP, XROW = Format<FMT>::XROW, WIN = STEPS * STEP;
   constexpr int NB = Fragment<FMT>::NB, CHUNK = Fragment<FMT>::CHUNK, W_ROW = weight_pitch(FMT, STEPS), SC_ROW = scale_pitch(FMT, STEPS);
@@ -993,22 +1059,21 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
   for (int r = 0; r < G; ++r)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[r][nt][0] = acc[r][nt][1] = pack2(0.f, 0.f);
-  pk2 extra[G][NT][2];            // sums of the columns left out in some step, in local memory
-  bool any_extra = false;
+  uint32_t left_out = 0u;         // the steps (modulo 32) in which columns were left out
 
   for (int win = 0, left = p.row_bytes;; ++win) {
     // (after a wait that ran out the warp goes on without waiting: what it then reads and writes is not used)
     ok &= mbar_wait(bars.full + 8u * s, parity, bars.abort_flag);
     if (first_window && win == 0 && threadIdx.x == 0) trace_stamp(p.trace, TRACE_FIRST_FULL);
     const uint32_t stage = ring + (uint32_t)s * stage_bytes;
-    uint32_t left_out = 0u;       // the steps in which columns were left out
     // (not unrolled: the steps' code, twice, would not stay in the instruction caches)
 #pragma unroll 1
     for (int st = 0; st < STEPS && left > st * STEP; ++st) {
       const uint32_t wrow = stage + w_off + st * STEP, srow = stage + sc_off + st * SCB;
       uint32_t b[NT][NB];
       load_x<FMT, NT, RES>(RES ? res + st * x_step : stage + lay.x_off + st * x_step, xo, b);
-      if constexpr (CONVERT && !RES) left_out |= window_chunk<NT, NB>(b) ? 1u << st : 0u;
+      if constexpr (CONVERT && !RES)
+        if (window_chunk<NT, NB>(b)) left_out |= 1u << ((win * STEPS + st) & 31);
       pk2 none[NT] = {};
       // the next group's rows are loaded while one's are multiplied
       RawRows<FMT> raw[2];
@@ -1026,44 +1091,12 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
         else chunk_rows<FMT, NT, SC, false>(raw[cur], b, none, acc[r]);
       }
     }
-    if constexpr (CONVERT) {
-      if (RES && spread) {
-#pragma unroll 1
-        for (int st = 0; st < STEPS; ++st)
-          if (left > st * STEP && __any_sync(0xffffffffu, lds_u8(marks + ((win * STEPS + st) * kConsumers + ln.warp) * M +
-                                                                 min(fragment_column<FMT>(ln.g), M - 1)) != 0u))
-            left_out |= 1u << st;
-      }
-      if (left_out != 0u) {
-        if (!any_extra) {
-#pragma unroll
-          for (int r = 0; r < G; ++r)
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) extra[r][nt][0] = extra[r][nt][1] = pack2(0.f, 0.f);
-          any_extra = true;
-        }
-#pragma unroll 1
-        for (int st = 0; st < STEPS; ++st)
-          if (left_out >> st & 1u)
-            extra_passes<FMT, NT, STEPS, RES>(p, extra, G, ODD ? 0 : 8, stage + lay.x_off + st * x_step, win * STEPS + st,
-                                              stage + w_off + st * STEP, stage + sc_off + st * SCB, sc_hi,
-                                              marks + ((win * STEPS + st) * kConsumers + ln.warp) * M);
-      }
-    }
     left -= WIN;
     if (RES) res += STEPS * x_step;
     __syncwarp();
     if (left <= 0) break;
     if ((threadIdx.x & 31) == 0) mbar_arrive(bars.empty + 8u * s);
     if (++s == stages) { s = 0; parity ^= 1u; }
-  }
-  if (CONVERT && any_extra) {
-#pragma unroll
-    for (int r = 0; r < G; ++r)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) acc[r][nt][half] = fadd2(acc[r][nt][half], extra[r][nt][half]);
   }
   float scales[2];
   if (last) finish_scales(p, wk, col0, cols, ln.warp, scales);
@@ -1083,6 +1116,10 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
         if (m1 < M) sts_f32(row + m1 * 4, c);
       }
   }
+  if constexpr (CONVERT) {
+    if (RES) left_out = spread;
+    if (left_out != 0u) extra_tile<FMT, NT>(p, col0, cols, at, W_ROW, left_out);
+  }
   if (last) {
     consumer_barrier();
     if (ln.warp < finish_units(p, wk)) finish_unit<FMT, STEPS>(p, wk, ring + (uint32_t)s * stage_bytes, col0, cols, ln.warp, scales);
@@ -1095,14 +1132,14 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
 
 // The consumer warps' walk over one GEMV, tile by tile. The ring position (s, parity) carries over from one GEMV of a
 // batch to the next; `first`: the kernel's first GEMV.
-template <int FMT, int NT, bool CAN_RES, int STEPS, typename XT>
-__device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* smem, unsigned char* marks, const Bars& bars,
+template <int FMT, int NT, bool CAN_RES, int STEPS, bool SMALL, typename XT>
+__device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* smem, const Bars& bars,
                                              int& s, uint32_t& parity, uint32_t& x_parity, bool first) {
   const Walk wk(p, STEPS * Format<FMT>::STEP);
   const StageLayout<FMT, STEPS> lay(p);
   if (first) griddep_wait();   // consumers read scales and write results in global memory: after the previous kernel
-  bool resident = false, spread = false;
-  const uint32_t marks_at = smem_addr(marks);
+  bool resident = false;
+  uint32_t spread = 0u;           // steps (modulo 32) with activations outside the window
   bool ok = true;
   if (first && threadIdx.x == 0) trace_stamp(p.trace, TRACE_DEP);
   if constexpr (CAN_RES) {
@@ -1110,7 +1147,7 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     if (resident && wk.ntiles > 0) {
       ok = mbar_wait(bars.x, x_parity, bars.abort_flag);
       x_parity ^= 1u;
-      if constexpr (std::is_same<XT, __nv_bfloat16>::value) spread = prepare_resident<FMT>(p, smem, marks_at);
+      if constexpr (std::is_same<XT, __nv_bfloat16>::value) spread = prepare_resident<FMT>(p, smem);
       __syncwarp();
     }
   }
@@ -1120,18 +1157,20 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     auto tile = [&](auto res) {
       constexpr bool RES = decltype(res)::value;
       auto run = [&](auto e) {
-        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, marks_at, spread, bars, s, parity, first && t == 0, ok);
+        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
+                                                                  first && t == 0, ok);
       };
-      switch ((wk.rows(cols) + 7) / 8) {
-        case 8: run(std::integral_constant<int, 8>()); break;
-        case 7: run(std::integral_constant<int, 7>()); break;
-        case 6: run(std::integral_constant<int, 6>()); break;
-        case 5: run(std::integral_constant<int, 5>()); break;
-        case 4: run(std::integral_constant<int, 4>()); break;
-        case 3: run(std::integral_constant<int, 3>()); break;
-        case 2: run(std::integral_constant<int, 2>()); break;
-        default: run(std::integral_constant<int, 1>());
+      const int eights = (wk.rows(cols) + 7) / 8;
+      if constexpr (!SMALL) {
+        if (eights == 8) return run(std::integral_constant<int, 8>());
+        if (eights == 7) return run(std::integral_constant<int, 7>());
+        if (eights == 6) return run(std::integral_constant<int, 6>());
+        if (eights == 5) return run(std::integral_constant<int, 5>());
       }
+      if (eights >= 4) return run(std::integral_constant<int, 4>());
+      if (eights == 3) return run(std::integral_constant<int, 3>());
+      if (eights == 2) return run(std::integral_constant<int, 2>());
+      run(std::integral_constant<int, 1>());
     };
     if constexpr (CAN_RES) {
       if (resident) tile(std::true_type());
@@ -1182,7 +1221,7 @@ __device__ __forceinline__ bool finish_gemv(const Params& p, unsigned char* smem
 }
 
 // All-gather epilogue: all rows of the CTA have been written (every warp but the feeding one).
-__device__ __forceinline__ void finished_barrier() { asm volatile("bar.sync 3, %0;" ::"n"(kThreads - 32) : "memory"); }
+__device__ __forceinline__ void finished_barrier() { asm volatile("bar.sync 3, %0;" ::"r"(blockDim.x - 32) : "memory"); }
 
 // All-gather epilogue, first half: the CTA's rows [lo, hi) of this rank's slot are complete in the local buffer; all
 // consumer threads copy them into the same place of every other rank's buffer: 16 bytes per store where the rows'
@@ -1191,8 +1230,7 @@ __device__ __forceinline__ void gather_copy(const Params& p) {
   const int tid = threadIdx.x, M = p.M;                       // consumer threads are 0 .. 255
   finished_barrier();
   if (p.world < 2) return;
-  const int lo = (int)(((long long)p.N * blockIdx.x) / gridDim.x);
-  const int rows = (int)(((long long)p.N * (blockIdx.x + 1)) / gridDim.x) - lo;
+  const int lo = first_column(p, blockIdx.x), rows = first_column(p, blockIdx.x + 1) - lo;
   const int esize = p.out_kind == OUT_F32 ? 4 : 2;
   const size_t slot0 = (size_t)p.rank * M * p.ldo + lo;
   bool vector = true;                                // all buffers equally placed within 16 bytes
@@ -1308,12 +1346,11 @@ __device__ __forceinline__ Bars ring_setup(const Params& p, bool copies, unsigne
 }
 
 // NT: column tiles of 8 activation rows; CAN_RES: the launch may keep the activations resident (resident_capable).
-template <int FMT, int NT, bool CAN_RES, int STEPS, typename XT>
-__global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant__ Params p) {
+template <int FMT, int NT, bool CAN_RES, int STEPS, bool SMALL, typename XT>
+__global__ void __launch_bounds__(SMALL ? kSmallThreads : kThreads, SMALL ? 2 : 1) gemv_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ unsigned char marks[CAN_RES ? kMaxMarks : 1];
   __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
-  const bool copies = copies_needed<FMT>(p);
+  const bool copies = !SMALL && copies_needed<FMT>(p);
   const Bars bars = ring_setup(p, copies, smem, sums);
   int s = 0;
   uint32_t parity = 0, x_parity = 0;
@@ -1321,10 +1358,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
   if (warp == kFeeder) {
     if (!p.early_weights) {
       prefetch_weights<FMT, STEPS>(p);
-      griddep_wait();
     }
-    feed_weights<FMT, STEPS>(p, p, smem, bars, true, s, parity);
-  } else if (warp >= kFirstCopier && copies) {
+    feed_weights<FMT, STEPS>(p, p, smem, bars, true, !p.early_weights, s, parity);
+  } else if (!SMALL && warp >= kFirstCopier && copies) {
     griddep_wait();
     feed_activations<FMT, STEPS>(p, smem, bars, warp - kFirstCopier, s, parity);
     if (p.world >= 1) finished_barrier();
@@ -1332,10 +1368,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
     // (reads scales and writes results in global memory: after the previous kernel)
     if (warp == kFinisher) start_activations<FMT, STEPS>(p, p, smem, bars);
     else griddep_wait();
-    finish_gemv<FMT, STEPS>(p, smem, bars, warp - kFinisher, copies ? 1 : kFinishers, s, parity);
+    if (!SMALL) finish_gemv<FMT, STEPS>(p, smem, bars, warp - kFinisher, copies ? 1 : kFinishers, s, parity);
     if (p.world >= 1) finished_barrier();
   } else {
-    consume_gemv<FMT, NT, CAN_RES, STEPS, XT>(p, smem, marks, bars, s, parity, x_parity, true);
+    consume_gemv<FMT, NT, CAN_RES, STEPS, SMALL, XT>(p, smem, bars, s, parity, x_parity, true);
     if ((threadIdx.x & 31) == 0) trace_stamp(p.trace, TRACE_LAST_CONSUMED);
     if (p.world >= 1) {
       gather_copy(p);
@@ -1361,17 +1397,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant
 template <int FMT, int NT, bool CAN_RES, int STEPS, typename XT>
 __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* __restrict__ items, int count) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ unsigned char marks[CAN_RES ? kMaxMarks : 1];
   __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
   const Bars bars = ring_setup(items[0], true, smem, sums);
   int s = 0;
   uint32_t parity = 0, x_parity = 0;
   const int warp = (int)(threadIdx.x >> 5);
   if (warp == kFeeder) {
-    if (!items[0].early_weights) griddep_wait();
     bool ok = true;
     for (int g = 0; g < count && ok; ++g)
-      ok = feed_weights<FMT, STEPS>(items[g], items[g], smem, bars, g == 0, s, parity);
+      ok = feed_weights<FMT, STEPS>(items[g], items[g], smem, bars, g == 0, g == 0 && !items[0].early_weights, s, parity);
   } else if (warp == kFinisher) {
     start_activations<FMT, STEPS>(items[0], items[0], smem, bars);
     bool ok = true;
@@ -1389,7 +1423,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* _
   } else {
     // (every warp passes every GEMV's barriers, also after a wait that ran out)
     for (int g = 0; g < count; ++g) {
-      consume_gemv<FMT, NT, CAN_RES, STEPS, XT>(items[g], smem, marks, bars, s, parity, x_parity, g == 0);
+      consume_gemv<FMT, NT, CAN_RES, STEPS, false, XT>(items[g], smem, bars, s, parity, x_parity, g == 0);
       if (items[g].world >= 1) gather_copy(items[g]);   // the CTA's rows of this GEMV go to the peers now
     }
     if ((threadIdx.x & 31) == 0) trace_stamp(items[0].trace, TRACE_LAST_CONSUMED);

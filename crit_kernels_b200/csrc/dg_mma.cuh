@@ -26,7 +26,7 @@
 //
 // Activations. BF16 weights multiply BF16 activations as they are. Decoded E4M3 and E2M1 x E4M3 weights are FP16 values
 // (at most 6 significant bits, 2^-10 .. 2688), so FP16 activations are used as they are too. BF16 activations of these
-// formats become FP16 times 2^5: exact for zero and for magnitudes of [2^-22, 2^10) (FP16 holds BF16's eight bits down to
+// formats become FP16 times 2^7: exact for zero and for magnitudes of [2^-24, 2^8) (FP16 holds BF16's eight bits down to
 // 2^-17, its subnormals included); the power of two comes off in the FP32 FMA. A chunk of a row with any other value is
 // multiplied apart, in as many passes as its values take: each pass takes the values within 28 binades of the largest that
 // is left, times a power of two of its own, and zeros for the rest.
@@ -173,11 +173,11 @@ __device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// BF16 activations times 2^5 as FP16: the usual way. A value fits when (|v| - 2^-22) as 15-bit patterns lies within 32
+// BF16 activations times 2^7 as FP16: the usual way. A value fits when (|v| - 2^-24) as 15-bit patterns lies within 32
 // binades; `window_bits` has a bit of kOutside set where one of a pair does not (zeros do not either: window_fits looks
 // closer). v * 2 drops the upper half's sign and puts the lower half's where it does no harm.
-constexpr uint32_t kWindowLow = 105u << 7, kWindowSize = 32u << 7, kOutside = 0xe000e000u;
-constexpr float kWindowScale = 32.0f, kWindowUnscale = 1.0f / 32.0f;
+constexpr uint32_t kWindowLow = 103u << 7, kWindowSize = 32u << 7, kOutside = 0xe000e000u;
+constexpr float kWindowScale = 128.0f, kWindowUnscale = 1.0f / 128.0f;
 __device__ __forceinline__ uint32_t window_bits(uint32_t v) { return v * 2u - 2u * (kWindowLow << 16 | kWindowLow); }
 template <int NB>
 __device__ __forceinline__ bool window_fits(const uint32_t (&v)[NB]) {
