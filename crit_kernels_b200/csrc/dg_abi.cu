@@ -152,7 +152,7 @@ constexpr FormatInfo kFormats[4] = {info_of<0>(), info_of<1>(), info_of<2>(), in
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Bytes of the activations kept resident: whole steps of [M][x_row bytes], then a flag byte per step.
+// Bytes of the activations kept resident: whole steps of [M][x_row bytes], and 16-byte padding.
 int resident_bytes_of(int fmt, int M, int nblk) {
   const int row_steps = ceil_div(nblk * 16, kFormats[fmt].step);
   return row_steps * M * kFormats[fmt].x_row + ((row_steps + 15) & ~15);
@@ -160,8 +160,8 @@ int resident_bytes_of(int fmt, int M, int nblk) {
 
 // Launch shape: a speed choice from (format, M, N, K, SM count) only; no row's bits depend on it.
 //   CTAs            one per SM, fewer when the matrix has under four rows per SM
-//   tile rows       64, 56 or 48 (less when a CTA's range is shorter): what takes the fewest mma groups of 16 rows, a tile
-//                   costing as much as half a group (its sums) plus, where its activations are converted on the way, as
+//   tile rows       64 to 40 (less when a CTA's range is shorter): what takes the fewest eighths of 8 rows, a tile
+//                   costing as much as one eighth (its sums) plus, where its activations are converted on the way, as
 //                   much as these cost
 //   steps           512-byte steps per ring stage (BF16: one of 1 KB): two, one where the ring would have fewer than three
 //                   stages otherwise: a consumer warp's fixed costs per stage then weigh half

@@ -5,17 +5,16 @@
 // :191 bf16_kernel, :285 fp8_kernel). Same formats, same contract (FP32 sums whose order never depends on the row
 // count), a different machine mapping:
 //
-//   * one persistent CTA per SM: 8 consumer warps + 4 producer warps. The matrix rows are split into one contiguous
-//     range per CTA; a range is walked in tiles of up to 16 * kMaxGroups rows and each tile in K windows.
-//   * the producer warps stream every window of a tile into a shared-memory ring: whole boxes of 8 rows as one tensor
-//     copy (TMA, mbarrier complete_tx) each, a tile's last few rows as one 1-D bulk copy per row, block scales the same
-//     way, plus the matching window of the activations as 16-byte cp.async copies into a bank-swizzled layout. Bytes in
+//   * one persistent CTA per SM: 8 consumer warps, a warp that feeds the ring and 3 that finish tiles. The matrix rows are
+//     split into one contiguous range per CTA; a range is walked in tiles of up to 64 rows and each tile in K windows.
+//   * the feeding warp streams every window of a tile into a shared-memory ring, one tensor copy (TMA, mbarrier
+//     complete_tx) for the weights and one for the block scales, plus the matching window of the activations. Bytes in
 //     flight are set by the ring (up to ~200 KB per SM), not by registers.
 //   * a 512-byte step of a row is eight chunks of 64 bytes; consumer warp w owns chunk w of every step, for all rows of
 //     the tile, and multiplies it on the tensor cores (dg_mma.cuh): the activations of a chunk are then loaded and
 //     converted by one warp, once per tile. At the end of a tile the eight warps' sums of every output meet in shared
-//     memory (in the ring stage just consumed) and are added in a fixed tree; the row scale multiplies once and the
-//     result is rounded once to the output type.
+//     memory (in the ring stage just consumed), where the finishing warps add them in a fixed tree; the row scale
+//     multiplies once and the result is rounded once to the output type.
 //
 // A row's summation order is therefore a function of K and the format alone: it does not depend on M, on the rows a
 // tile holds, on the tile or window sizes the launch picked, on the CTA count, or on which slice of the matrix a
@@ -136,7 +135,7 @@ struct Params {
   // out[m][k] = silu(gate) * up (FP32, one rounding) instead of the two sums: `pairs` columns.
   int pairs;
   // Activations: X_RESIDENT (resident_capable; the kernel's dynamic shared memory holds, x_res_off bytes in, the steps of
-  // M x XROW bytes laid out as in a stage, then one flag byte per step, 1 = every chunk of the step is held as FP16), or a
+  // M x XROW bytes, unswizzled, FP16), or a
   // window of them in every ring stage, by one tensor copy (X_TENSOR) or, where K is no multiple of 64, by the copying
   // warps (X_COPIED).
   int x_mode, x_res_off;

@@ -27,6 +27,12 @@ _TRITON_SIDE = {"DOT_ROWS", "TRITON_ROWS", "dot_partial_elements", "fp8_dot_tile
                 "hardware"}
 
 
+def _bytes(t: torch.Tensor) -> torch.Tensor:
+    """t as the ops take it: they ask for one byte an element, not for a type (a view of every argument cost a call about
+    half a microsecond of its five)."""
+    return t if t.element_size() == 1 else t.view(torch.uint8)
+
+
 def gemv(x: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor, inverse: torch.Tensor, out: torch.Tensor,
          blocked: bool = False):
     """NVFP4 projection. Writes x @ W^T into out and returns it. x: [M][K], 1 <= M <= 16, BF16 or FP16, every row on
@@ -40,7 +46,7 @@ def gemv_fp8(x: torch.Tensor, codes: torch.Tensor, scales: torch.Tensor, out: to
     """FP8 projection. Writes x @ W^T into out and returns it. codes: [N][K] E4M3 (float8_e4m3fn or raw uint8),
     K % 16 == 0. The dtype of `scales` picks the flavour: FP32 [N] multiplies each finished sum by its channel's
     scale; uint8 [N][K / 32] are MXFP8 exponents, each weight counting 2^(e - 127) times its code (K % 32 == 0)."""
-    ops.gemv_fp8(x, codes.view(torch.uint8), scales, out)
+    ops.gemv_fp8(x, _bytes(codes), scales, out)
     return out
 
 
@@ -81,7 +87,7 @@ def quantize_fp8_rows(x: torch.Tensor, q: torch.Tensor, scale: torch.Tensor):
     """BF16 rows to FP8: q [rows][K] (float8_e4m3fn or uint8) = x / scale rounded to E4M3, with scale [rows] FP32 =
     max(|row|) / 448 (at least 1e-12) written too. Any number of rows and any K. The arithmetic and bits of the
     reference's mma_rows.quantize_fp8_rows (mma-rows/torch-ext/mma_rows/__init__.py:124-128). Returns (q, scale)."""
-    ops.quantize_fp8_rows(x, q.view(torch.uint8), scale)
+    ops.quantize_fp8_rows(x, _bytes(q), scale)
     return q, scale
 
 
