@@ -798,7 +798,7 @@ __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %
 // Resident activations have come as they are in global memory. BF16 ones: every consumer warp puts its own slice of K into the
 // form the tiles read, FP16 in the usual way, a chunk with values outside the window as zeros (see extra_tile). No
 // other warp reads that slice, so nobody waits for anybody. The lanes of a group g take activation row g % M, chunks of 8 / M
-// steps at a time, slot by slot in place. Returns whether there are chunks outside the window. (Rolled loops: this runs once
+// steps at a time, slot by slot in place. Returns the steps (modulo 32) with chunks outside. (Rolled loops: this runs once
 // per kernel, from cold instruction caches; unrolled over a lane's slots it took 1.0 us for a single step, now 0.6.)
 template <int FMT>
 __device__ __forceinline__ uint32_t prepare_resident(const Params& p, unsigned char* smem) {
@@ -1023,7 +1023,8 @@ __device__ __forceinline__ void finish_unit(const Params& p, const Walk& wk, uin
 
 // One tile of up to 8 EIGHTS rows: the windows in turn; at the end the warp leaves its sums in the stage it has just consumed,
 // in its own chunk of each row (which no other warp reads), one FP32 per activation row, and tells the finishing warps, to
-// which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the activations are resident (`spread`: some chunk has values outside the window).
+// which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the
+// activations are resident (`spread`: the steps, modulo 32, with values outside the window).
 template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool RES>
 __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, const StageLayout<FMT, STEPS>& lay,
                                              unsigned char* smem, int col0, int cols, bool last, uint32_t spread, const Bars& bars, int& s, uint32_t& parity,
