@@ -124,11 +124,15 @@ DeviceState* device_state() {
             cudaGetSymbolAddress(&status, dg_status_word) == cudaSuccess;
   // (the whole of an SM's 228 KB as shared memory: two small blocks, or one, and no change between launches)
   auto opt_in = [&](const void* const (*table)[16], int rows) {
-    for (int i = 0; ok && i < 16 * rows; ++i)
-      ok = cudaFuncSetAttribute(table[i / 16][i % 16], cudaFuncAttributeMaxDynamicSharedMemorySize, dg::kSmemLimit) ==
+    const void* done = nullptr;    // (a table's neighbours share their kernel)
+    for (int i = 0; ok && i < 16 * rows; ++i) {
+      if (table[i / 16][i % 16] == done) continue;
+      done = table[i / 16][i % 16];
+      ok = cudaFuncSetAttribute(done, cudaFuncAttributeMaxDynamicSharedMemorySize, dg::kSmemLimit) ==
                cudaSuccess &&
-           cudaFuncSetAttribute(table[i / 16][i % 16], cudaFuncAttributePreferredSharedMemoryCarveout,
+           cudaFuncSetAttribute(done, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+    }
   };
   for (const void* const (*table)[16] : kTables) opt_in(table, 4);
   opt_in(dg_batch_table_nvfp4_bf16, 2);
