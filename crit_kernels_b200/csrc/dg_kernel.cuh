@@ -105,7 +105,10 @@ __host__ __device__ constexpr int x_offset(int before) { return ((before + kSmem
 // window of them into every ring stage: one tensor copy brings them, and the consumer warps put them into the form the
 // tensor cores take (see prepare_resident) while the first weights are on their way.
 __host__ __device__ constexpr bool resident_capable(int fmt, int m) { return (fmt == FMT_FP8 || fmt == FMT_NVFP4) && m <= 4; }
-constexpr int kResidentLimit = 96 * 1024;   // bytes of activations (and their flags) a kernel keeps resident at most
+constexpr int kResidentLimit = 96 * 1024;   // bytes of activations (and padding) a kernel keeps resident at most
+// The exponents of resident BF16 activations (see prepare_resident): a byte per consumer warp, step and row.
+constexpr int kResidentExps = kResidentLimit / Format<FMT_FP8>::XROW * kConsumers;
+static_assert(kResidentExps + (kMaxStages + 1) * 8 <= kStaticSmem, "static shared memory");
 
 struct Params {
   const void* x;             // [M][ldx] BF16 or FP16
@@ -162,11 +165,6 @@ struct Params {
 // PTX wrappers: mbarrier, 1-D bulk copy (TMA), 16-byte cp.async tied to an mbarrier.
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint4 ldg_nc128(const void* ptr) {   // memory nobody writes while the kernel runs
-  uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(ptr));
-  return v;
-}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -272,6 +270,7 @@ __device__ __forceinline__ void store_out(void* out, int kind, size_t idx, float
 // window, its eight consumers have left their sums in it.
 struct Bars {
   uint32_t full, empty, sums, x;   // x (one for the CTA): the resident activations have come
+  uint32_t exps;                   // the resident activations' exponents (kResidentExps bytes)
   volatile int* abort_flag;
 };
 
@@ -652,15 +651,15 @@ __device__ __forceinline__ void decode_sub(const uint4 (&v)[Fragment<FMT>::PIECE
 }
 
 // One chunk of 16 rows into the running sums: acc[nt][0] rows g, acc[nt][1] rows g + 8, columns (2 t, 2 t + 1) + 8 nt.
-// SCALE: the activations' power of two comes off again: SCALE_NONE there is none, SCALE_WINDOW the usual one, SCALE_COLUMN
-// `unscale` per column.
-enum : int { SCALE_NONE = 0, SCALE_WINDOW = 1, SCALE_COLUMN = 2 };
+// ACTS: the activations are used as they came (ACTS_PLAIN), are FP16 times the usual power of two (ACTS_USUAL) or one of their
+// column, which `unscale` takes off again (ACTS_SCALED), or are BF16 beside weights that decode to FP16 (ACTS_WIDE).
+enum : int { ACTS_PLAIN = 0, ACTS_USUAL = 1, ACTS_SCALED = 2, ACTS_WIDE = 3 };
 // HALF: there are no rows g + 8; their products are neither made nor added.
-template <int FMT, int NT, int SCALE, bool HALF>
+template <int FMT, int NT, int ACTS, bool HALF>
 __device__ __forceinline__ void chunk_rows(const RawRows<FMT>& raw, const uint32_t (&b)[NT][Fragment<FMT>::NB],
                                            const pk2 (&unscale)[NT], pk2 (&acc)[NT][2]) {
   constexpr int SUB = Fragment<FMT>::SUB, PER = SUB / 2;   // two chains: of four steps (NVFP4) or two
-  constexpr bool BF = FMT == FMT_BF16;
+  constexpr bool BF = FMT == FMT_BF16 || ACTS == ACTS_WIDE;
   uint32_t s2lo[2] = {0u, 0u}, s2hi[2] = {0u, 0u};
   if constexpr (FMT == FMT_NVFP4) {
     const uint32_t a = e4m3x2_to_half2(raw.slo);
@@ -682,6 +681,10 @@ __device__ __forceinline__ void chunk_rows(const RawRows<FMT>& raw, const uint32
 #pragma unroll
       for (int i = 0; i < 4; ++i) hi[i] = lo[i];
     }
+    if constexpr (ACTS == ACTS_WIDE) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { lo[i] = half2_to_bf162(lo[i]); hi[i] = half2_to_bf162(hi[i]); }
+    }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       if (q % PER == 0) mma_step<BF, true>(part[chain][nt], lo[0], hi[0], lo[1], hi[1], b[nt][4 * q], b[nt][4 * q + 1]);
@@ -689,16 +692,16 @@ __device__ __forceinline__ void chunk_rows(const RawRows<FMT>& raw, const uint32
       mma_step<BF, false>(part[chain][nt], lo[2], hi[2], lo[3], hi[3], b[nt][4 * q + 2], b[nt][4 * q + 3]);
     }
   }
-  const pk2 window = pack2(kWindowUnscale, kWindowUnscale);
+  const pk2 usual = pack2(kWindowUnscale, kWindowUnscale);
   pk2 mx[2][2];                           // MXFP8: [block][rows g, g + 8] scales, powers of two
   if constexpr (FMT == FMT_MXFP8) {
     e8m0x2_to_f32(raw.slo, mx[0][0], mx[1][0]);
     if constexpr (!HALF) e8m0x2_to_f32(raw.shi, mx[0][1], mx[1][1]);
-    if (SCALE == SCALE_WINDOW) {
+    if (ACTS == ACTS_USUAL) {
 #pragma unroll
       for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int half = 0; half < (HALF ? 1 : 2); ++half) mx[c][half] = fmul2(mx[c][half], window);
+        for (int half = 0; half < (HALF ? 1 : 2); ++half) mx[c][half] = fmul2(mx[c][half], usual);
     }
   }
 #pragma unroll
@@ -709,12 +712,13 @@ __device__ __forceinline__ void chunk_rows(const RawRows<FMT>& raw, const uint32
       pk2 v1 = pack2(part[1][nt][2 * half], part[1][nt][2 * half + 1]);
       if constexpr (FMT == FMT_MXFP8) {
         // (a column's power of two first: the product with the block's scale is then the true one)
-        if (SCALE == SCALE_COLUMN) { v0 = fmul2(v0, unscale[nt]); v1 = fmul2(v1, unscale[nt]); }
+        if (ACTS == ACTS_SCALED) { v0 = fmul2(v0, unscale[nt]); v1 = fmul2(v1, unscale[nt]); }
         acc[nt][half] = ffma2(v1, mx[1][half], ffma2(v0, mx[0][half], acc[nt][half]));
       } else {
         v0 = fadd2(v0, v1);
-        acc[nt][half] = SCALE == SCALE_NONE ? fadd2(v0, acc[nt][half])
-                                            : ffma2(v0, SCALE == SCALE_WINDOW ? window : unscale[nt], acc[nt][half]);
+        acc[nt][half] = ACTS == ACTS_USUAL || ACTS == ACTS_SCALED
+                            ? ffma2(v0, ACTS == ACTS_USUAL ? usual : unscale[nt], acc[nt][half])
+                            : fadd2(v0, acc[nt][half]);
       }
     }
 }
@@ -749,104 +753,90 @@ __device__ __forceinline__ void load_x(uint32_t xs, const XOffsets<FMT, NT, RES>
     }
 }
 
-// The same from global memory, step `step` of the rows; zeros past their end.
-template <int FMT, int NT>
-__device__ __forceinline__ void load_x_global(const Params& p, int step, const Lane& ln, uint32_t (&b)[NT][Fragment<FMT>::NB]) {
-  constexpr int NJ = Fragment<FMT>::NB / 4;
-  const unsigned char* x = reinterpret_cast<const unsigned char*>(p.x);
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const int m = min(fragment_column<FMT>(ln.g) + 8 * nt, p.M - 1);
-      const int k = step * (Format<FMT>::XROW / 2) + (ln.warp * 4 * NJ + (split_columns(FMT) ? 4 * j + ln.t : NJ * ln.t + j)) * 8;
-      const uint4 v = k < p.K ? ldg_nc128(x + ((size_t)m * p.ldx + k) * 2) : make_uint4(0u, 0u, 0u, 0u);
-      b[nt][4 * j] = v.x; b[nt][4 * j + 1] = v.y; b[nt][4 * j + 2] = v.z; b[nt][4 * j + 3] = v.w;
-    }
-}
-
-// BF16 activations of a chunk (b, as stored) to FP16 in the usual way. Columns with a value outside the window are left out
-// (zeros); returns whether there are any, the same for all lanes of the warp.
-template <int NT, int NB>
-__device__ __forceinline__ bool window_chunk(uint32_t (&b)[NT][NB]) {
-  bool left_out = false;
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-    uint32_t outside = 0u;
-#pragma unroll
-    for (int i = 0; i < NB; ++i) outside |= window_bits(b[nt][i]);
-    uint32_t misfit = 0u;
-    if (__any_sync(0xffffffffu, (outside & kOutside) != 0u)) misfit = __ballot_sync(0xffffffffu, !window_fits<NB>(b[nt]));
-#pragma unroll
-    for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(b[nt][i], kWindowScale);
-    if (misfit != 0u) {
-      left_out = true;
-      if (((misfit >> (threadIdx.x & 28)) & 0xfu) != 0u) {
-#pragma unroll
-        for (int i = 0; i < NB; ++i) b[nt][i] = 0u;
-      }
-    }
-  }
-  return left_out;
-}
 // The powers of two to take off the lane's sums' columns (2 t, 2 t + 1) again, from the lanes that hold these columns.
 __device__ __forceinline__ pk2 column_unscale(uint32_t e, const Lane& ln) {
+  e = e == kWide ? kWindowExp : e;          // (such a column is zeros)
   return pack2(exp_unscale(__shfl_sync(0xffffffffu, e, 8 * ln.t)), exp_unscale(__shfl_sync(0xffffffffu, e, 8 * ln.t + 4)));
 }
 
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumers) : "memory"); }
 // Resident activations have come as they are in global memory. BF16 ones: every consumer warp puts its own slice of K into the
-// form the tiles read, FP16 in the usual way, a chunk with values outside the window as zeros (see extra_tile). No
-// other warp reads that slice, so nobody waits for anybody. The lanes of a group g take activation row g % M, chunks of 8 / M
-// steps at a time, slot by slot in place. Returns the steps (modulo 32) with chunks outside. (Rolled loops: this runs once
-// per kernel, from cold instruction caches; unrolled over a lane's slots it took 1.0 us for a single step, now 0.6.)
+// form the tiles read, FP16 times 2^7 or the chunk's own power of two, whose exponent it then leaves in `exps`, one byte
+// per warp, step and row (kWide: the chunk stays BF16). No other warp reads that slice, so nobody waits for anybody. The lanes of
+// a group g take activation row g % M, chunks of 8 / M steps at a time, slot by slot in place. Returns the steps (modulo 32)
+// with another exponent than the usual one. (Rolled loops: this runs once per kernel, from cold instruction caches; unrolled
+// over a lane's slots it took 1.0 us for a single step, now 0.6.)
 template <int FMT>
-__device__ __forceinline__ uint32_t prepare_resident(const Params& p, unsigned char* smem) {
+__device__ __forceinline__ uint32_t prepare_resident(const Params& p, unsigned char* smem, uint32_t exps) {
   constexpr int XROW = Format<FMT>::XROW, NJ = Fragment<FMT>::NB / 4;
   const Lane ln;
   const int M = p.M, by = M == 1 ? 32 : M == 2 ? 16 : M == 3 ? 11 : 8, q = ln.g * by >> 5, m = ln.g - q * M;   // q: g / M
   const int together = M == 1 ? 8 : M == 2 ? 4 : 2, steps = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP;
   const int slot0 = ln.warp * 4 * NJ + NJ * ln.t;
   const uint32_t at0 = smem_addr(smem) + (uint32_t)(p.x_res_off + ((slot0 >> 3) * M + m) * 128 + (slot0 & 7) * 16);
-  uint32_t misfit = 0u;
+  const uint32_t mine0 = exps + (uint32_t)(ln.warp * steps * M);
+  uint32_t spread = 0u;
+  bool noted = false;             // the exponents have been set to the usual one
 #pragma unroll 1
   for (int st0 = 0; st0 < steps; st0 += together) {
     const int st = st0 + q;
     const bool mine = q < together && st < steps;
     const uint32_t at = at0 + (uint32_t)(st * M * XROW);
-    uint32_t outside = 0u;
+    uint32_t left = 0u;          // bit j: slot j is as it came
     if (mine) {
 #pragma unroll 1
       for (int j = 0; j < NJ; ++j) {
         const uint4 v = lds128(at + 16 * j);
-        outside |= window_bits(v.x) | window_bits(v.y) | window_bits(v.z) | window_bits(v.w);
-        sts128(at + 16 * j, make_uint4(scaled_half2(v.x, kWindowScale), scaled_half2(v.y, kWindowScale),
-                                       scaled_half2(v.z, kWindowScale), scaled_half2(v.w, kWindowScale)));
+        if ((window_bits(v.x) | window_bits(v.y) | window_bits(v.z) | window_bits(v.w)) & kOutside)
+          left |= 1u << j;
+        else
+          sts128(at + 16 * j, make_uint4(scaled_half2(v.x, kWindowScale), scaled_half2(v.y, kWindowScale),
+                                         scaled_half2(v.z, kWindowScale), scaled_half2(v.w, kWindowScale)));
       }
     }
-    // (a bit may be a zero's: the values once more, from global memory, decide)
-    bool out = false;
-    if (__any_sync(0xffffffffu, (outside & kOutside) != 0u)) {
-      bool fits = true;
+    if (__any_sync(0xffffffffu, left != 0u)) {
+      auto slot = [&](int j, uint32_t (&v)[4]) {     // as it came
+        const uint4 h = lds128(at + 16 * j);
+        v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = h.w;
+        if ((left >> j & 1u) == 0u) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[i] = window_back(v[i]);
+        }
+      };
+      uint32_t range = 0u;
       if (mine) {
 #pragma unroll 1
         for (int j = 0; j < NJ; ++j) {
-          const int kk = st * (XROW / 2) + (slot0 + j) * 8;
-          if (kk >= p.K) break;
-          const uint4 v = ldg_nc128(reinterpret_cast<const unsigned char*>(p.x) + ((size_t)m * p.ldx + kk) * 2);
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-          fits = fits && window_fits<4>(w);
+          uint32_t v[4];
+          slot(j, v);
+          range = __vmaxu2(range, chunk_range<4>(v));
         }
       }
-      out = ((__ballot_sync(0xffffffffu, !fits) >> (threadIdx.x & 28)) & 0xfu) != 0u;
-      if (mine && out) {
+      const uint32_t e = chunk_exp(range);
+      if (mine) {
 #pragma unroll 1
-        for (int j = 0; j < NJ; ++j) sts128(at + 16 * j, make_uint4(0u, 0u, 0u, 0u));
+        for (int j = 0; j < NJ; ++j) {
+          uint32_t v[4];
+          slot(j, v);
+          if (e != kWide) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = scaled_half2(v[i], exp_scale(e));
+          }
+          sts128(at + 16 * j, make_uint4(v[0], v[1], v[2], v[3]));
+        }
       }
-      if (out) misfit |= 1u << (st & 31);
+      if (!noted) {
+        noted = true;
+        for (int i = threadIdx.x & 31; i < steps * M; i += 32) sts_u8(mine0 + i, kWindowExp);
+        __syncwarp();
+      }
+      if (mine && e != kWindowExp) {
+        spread |= 1u << (st & 31);
+        if (ln.t == 0) sts_u8(mine0 + st * M + m, e);
+      }
     }
   }
-  return __reduce_or_sync(0xffffffffu, misfit);
+  return __reduce_or_sync(0xffffffffu, spread);
 }
 
 // A row's two scale bytes of the lane. (Gathered MXFP8 rows may lie on odd addresses.)
@@ -866,106 +856,6 @@ __device__ __forceinline__ void load_rows(RawRows<FMT>& raw, uint32_t wrow, uint
   if constexpr (Format<FMT>::SCB != 0) {
     raw.slo = load_scales<FMT>(srow);
     if constexpr (!HALF) raw.shi = load_scales<FMT>(srow + hi_row * scale_pitch(FMT, STEPS) + (FMT == FMT_MXFP8 ? sc_hi : 0));
-  }
-}
-
-// A lane's share of a chunk of one weight row, and its scales, from global memory (zeros past the row's end).
-template <int FMT>
-__device__ __forceinline__ void load_row_global(const Params& p, int n, int step, const Lane& ln, uint4 (&v)[Fragment<FMT>::PIECES],
-                                                uint32_t& sc) {
-  constexpr int STEP = Format<FMT>::STEP, SCB = Format<FMT>::SCB, CHUNK = Fragment<FMT>::CHUNK;
-  const uint8_t* row = p.w + (size_t)n * p.row_bytes;
-#pragma unroll
-  for (int i = 0; i < Fragment<FMT>::PIECES; ++i) {
-    const int at = step * STEP + ln.warp * CHUNK + (FMT == FMT_MXFP8 ? ln.t * 8 : i * 64 + ln.t * 16);
-    if constexpr (FMT == FMT_MXFP8) {
-      const uint2 z = make_uint2(0u, 0u);
-      const uint2 a = at < p.row_bytes ? __ldg(reinterpret_cast<const uint2*>(row + at)) : z;
-      const uint2 c = at + 32 < p.row_bytes ? __ldg(reinterpret_cast<const uint2*>(row + at + 32)) : z;
-      v[i] = make_uint4(a.x, a.y, c.x, c.y);
-    } else {
-      v[i] = at < p.row_bytes ? ldg_nc128(row + at) : make_uint4(0u, 0u, 0u, 0u);
-    }
-  }
-  sc = 0u;
-  if constexpr (SCB != 0) {
-    const int sc_bytes = p.row_bytes * SCB / STEP, j = step * SCB + (FMT == FMT_NVFP4 ? ln.warp * 8 + ln.t * 2 : ln.warp * 2);
-    const uint8_t* src = p.scales + (p.scale_mode == SCALES_BLOCKED ? tiled_scale_offset(n, j, p.ct) : (size_t)n * p.scale_row_bytes + j);
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (j + i < sc_bytes) sc |= (uint32_t)__ldg(src + i) << (8 * i);
-  }
-}
-
-// The columns that were left out of some chunks because of values outside the window, after the tile: their products, in as
-// many passes as the values take, are added to the sums the warp has left in the stage (`sums`: the lane's row 0 there).
-// `steps`: bit i, one of the steps i + 32 n. Everything comes from global memory again: such values are rare, and a call inside
-// the tile's loop cost every launch registers (NVFP4 4096 x 4096, one row: 6.7 us, and 5.9 for FP16, which has none).
-template <int FMT, int NT>
-__device__ __noinline__ void extra_tile(const Params& p, int col0, int cols, uint32_t sums, uint32_t pitch,
-                                        uint32_t steps) {
-  constexpr int NB = Fragment<FMT>::NB;
-  const Lane ln;
-  const Walk wk(p, Format<FMT>::STEP);
-  const int M = p.M, rows = wk.rows(cols), all = (p.row_bytes + Format<FMT>::STEP - 1) / Format<FMT>::STEP;
-#pragma unroll 1
-  for (int r0 = 0; r0 < rows; r0 += kGroupRows) {
-    pk2 acc[NT][2];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = pack2(0.f, 0.f);
-    const int lo = r0 + fragment_row<FMT>(ln.g), hi = lo + 8;
-    const int n_lo = wk.matrix_row(col0, cols, min(lo, rows - 1)), n_hi = wk.matrix_row(col0, cols, min(hi, rows - 1));
-#pragma unroll 1
-    for (int step = 0; step < all; ++step) {
-      if ((steps >> (step & 31) & 1u) == 0u) continue;
-      uint32_t high[NT];              // magnitudes from here on are done
-      bool more = true;
-      for (bool again = false; more; again = true) {
-        uint32_t b[NT][NB];
-        pk2 unscale[NT];
-        load_x_global<FMT, NT>(p, step, ln, b);
-        more = false;
-        bool any = again;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          if (!again) {
-            const uint32_t misfit = __ballot_sync(0xffffffffu, !window_fits<NB>(b[nt]));
-            high[nt] = ((misfit >> (threadIdx.x & 28)) & 0xfu) != 0u ? 0x8000u : 0u;
-            any |= misfit != 0u;
-          }
-#pragma unroll
-          for (int i = 0; i < NB; ++i) b[nt][i] = keep_range(b[nt][i], 0u, high[nt]);
-          uint32_t top = chunk_amax<NB>(b[nt]);
-          top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
-          top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
-          const uint32_t e = chunk_exp(top), low = chunk_low(e);
-          more |= __any_sync(0xffffffffu, !chunk_fits<NB>(b[nt], low));
-          high[nt] = low;
-          const float scale = exp_scale(e);
-#pragma unroll
-          for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(keep_range(b[nt][i], low, 0x8000u), scale);
-          unscale[nt] = column_unscale(e, ln);
-        }
-        if (!any) break;
-        RawRows<FMT> raw;
-        load_row_global<FMT>(p, n_lo, step, ln, raw.lo, raw.slo);
-        load_row_global<FMT>(p, n_hi, step, ln, raw.hi, raw.shi);
-        chunk_rows<FMT, NT, SCALE_COLUMN, false>(raw, b, unscale, acc);
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int m0 = 8 * nt + fragment_column<FMT>(2 * ln.t), m1 = 8 * nt + fragment_column<FMT>(2 * ln.t + 1);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        float a, c;
-        unpack2(acc[nt][half], a, c);
-        const uint32_t at = sums + (uint32_t)(r0 + half * 8) * pitch;
-        if (r0 + half * 8 >= rows) continue;     // (an eighth without rows has no sums)
-        if (m0 < M) sts_f32(at + m0 * 4, lds_f32(at + m0 * 4) + a);
-        if (m1 < M) sts_f32(at + m1 * 4, lds_f32(at + m1 * 4) + c);
-      }
-    }
   }
 }
 
@@ -1021,11 +911,20 @@ __device__ __forceinline__ void finish_unit(const Params& p, const Walk& wk, uin
   else store(std::integral_constant<int, OUT_F16>());
 }
 
+enum : int { RES_NONE = 0, RES_USUAL = 1, RES_MIXED = 2 };
+// Where chunks with values outside the usual window are multiplied: nowhere (there are none); in kernels for up to four rows by
+// the usual chunks' code, which then has the columns' powers of two in registers; from five rows up in code of its own (with
+// the powers in registers for every chunk, 28672 x 8192 NVFP4 with 8 rows took 38.4 us, without 37.4; but the code of its own is
+// one more thing to fetch, which a launch for few rows pays for with a single such chunk: 4096 x 4096, one row, 7.1 and 6.4 us).
+// NVFP4 28672 x 8192 at 1 / 8 / 16 rows, us: N(0, 1) activations 31.0 / 37.4 / 53.5, one value of 300 in each row 33.2 / 38.1 /
+// 54.9, all above 2^8 36.1 / 45.8 / 68, chunks over more than 32 binades 56 / 55 / 74. (As passes after the tile, from global
+// memory, they took 68 / 72 / 117, 320 / 316 / 645 and 949 / 1087 / 2158.)
+enum : int { ODD_NONE = 0, ODD_SHARED = 1, ODD_APART = 2 };
 // One tile of up to 8 EIGHTS rows: the windows in turn; at the end the warp leaves its sums in the stage it has just consumed,
 // in its own chunk of each row (which no other warp reads), one FP32 per activation row, and tells the finishing warps, to
 // which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the
-// activations are resident (`spread`: the steps, modulo 32, with values outside the window).
-template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool RES>
+// activations are resident (RES_MIXED: `spread` has the steps, modulo 32, with chunks of another exponent than the usual one).
+template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool CAN_RES, int RES>
 __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, const StageLayout<FMT, STEPS>& lay,
                                              unsigned char* smem, int col0, int cols, bool last, uint32_t spread, const Bars& bars, int& s, uint32_t& parity,
                                              bool first_window, bool& ok) {
@@ -1035,6 +934,7 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
   constexpr bool ODD = EIGHTS % 2 != 0;       // the last group has no second half
   // BF16 activations of the formats whose weights become FP16
   constexpr bool CONVERT = FMT != FMT_BF16 && std::is_same<XT, __nv_bfloat16>::value;
+  constexpr int ODDITIES = !CONVERT || RES == RES_USUAL ? ODD_NONE : CAN_RES ? ODD_SHARED : ODD_APART;
   const Lane ln;
   const int M = p.M, stage_bytes = p.stage_bytes, stages = p.stages;
   if (last && p.row_scale && unit_column(wk, ln.warp) < cols) {    // (needed at the tile's end)
@@ -1053,7 +953,7 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
     sc_off += shift;
     if (FMT == FMT_MXFP8) sc_hi = (int)scale_shift(p, col0 + frow + 8) - (int)shift;
   }
-  const XOffsets<FMT, NT, RES> xo(ln, M);
+  const XOffsets<FMT, NT, RES != RES_NONE> xo(ln, M);
   uint32_t res = smem_addr(smem) + (uint32_t)p.x_res_off;    // of the next step
   const uint32_t x_step = (uint32_t)(M * XROW);
   pk2 acc[G][NT][2];
@@ -1061,7 +961,6 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
   for (int r = 0; r < G; ++r)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[r][nt][0] = acc[r][nt][1] = pack2(0.f, 0.f);
-  uint32_t left_out = 0u;         // the steps (modulo 32) in which columns were left out
 
   for (int win = 0, left = p.row_bytes;; ++win) {
     // (after a wait that ran out the warp goes on without waiting: what it then reads and writes is not used)
@@ -1073,24 +972,156 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
     for (int st = 0; st < STEPS && left > st * STEP; ++st) {
       const uint32_t wrow = stage + w_off + st * STEP, srow = stage + sc_off + st * SCB;
       uint32_t b[NT][NB];
-      load_x<FMT, NT, RES>(RES ? res + st * x_step : stage + lay.x_off + st * x_step, xo, b);
-      if constexpr (CONVERT && !RES)
-        if (window_chunk<NT, NB>(b)) left_out |= 1u << ((win * STEPS + st) & 31);
-      pk2 none[NT] = {};
-      // the next group's rows are loaded while one's are multiplied
+      const uint32_t xs = (RES ? res : stage + lay.x_off) + st * x_step;
+      load_x<FMT, NT, RES != RES_NONE>(xs, xo, b);
       RawRows<FMT> raw[2];
-      load_rows<FMT, STEPS, ODD && G == 1>(raw[0], wrow, srow, 8, sc_hi, ln.t);
+      pk2 unscale[NT] = {};
+      auto first_rows = [&] { load_rows<FMT, STEPS, ODD && G == 1>(raw[0], wrow, srow, 8, sc_hi, ln.t); };
+      // the groups' products in turn: the next group's rows are loaded while one's are multiplied
+      auto multiply = [&](auto acts) {
+        constexpr int ACTS = decltype(acts)::value;
 #pragma unroll
-      for (int r = 0; r < G; ++r) {
-        constexpr int kRow = kGroupRows;
-        const int cur = r & 1;
-        if (r + 2 < G || (r + 2 == G && !ODD))
-          load_rows<FMT, STEPS, false>(raw[cur ^ 1], wrow + (r + 1) * kRow * W_ROW, srow + (r + 1) * kRow * SC_ROW, 8, sc_hi, ln.t);
-        else if (r + 2 == G)
-          load_rows<FMT, STEPS, true>(raw[cur ^ 1], wrow + (r + 1) * kRow * W_ROW, srow + (r + 1) * kRow * SC_ROW, 8, sc_hi, ln.t);
-        constexpr int SC = CONVERT ? SCALE_WINDOW : SCALE_NONE;
-        if (ODD && r == G - 1) chunk_rows<FMT, NT, SC, true>(raw[cur], b, none, acc[r]);
-        else chunk_rows<FMT, NT, SC, false>(raw[cur], b, none, acc[r]);
+        for (int r = 0; r < G; ++r) {
+          constexpr int kRow = kGroupRows;
+          const int cur = r & 1;
+          if (r + 2 < G || (r + 2 == G && !ODD))
+            load_rows<FMT, STEPS, false>(raw[cur ^ 1], wrow + (r + 1) * kRow * W_ROW, srow + (r + 1) * kRow * SC_ROW, 8, sc_hi, ln.t);
+          else if (r + 2 == G)
+            load_rows<FMT, STEPS, true>(raw[cur ^ 1], wrow + (r + 1) * kRow * W_ROW, srow + (r + 1) * kRow * SC_ROW, 8, sc_hi, ln.t);
+          if (ODD && r == G - 1) chunk_rows<FMT, NT, ACTS, true>(raw[cur], b, unscale, acc[r]);
+          else chunk_rows<FMT, NT, ACTS, false>(raw[cur], b, unscale, acc[r]);
+        }
+      };
+      using Wide = std::integral_constant<int, ACTS_WIDE>;
+      using Scaled = std::integral_constant<int, ACTS_SCALED>;
+      using Usual = std::integral_constant<int, CONVERT ? ACTS_USUAL : ACTS_PLAIN>;
+      // of a chunk as stored: has it values outside the usual window (zeros among them)
+      auto outside = [&] {
+        uint32_t bits = 0u;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int i = 0; i < NB; ++i) bits |= window_bits(b[nt][i]);
+        return __any_sync(0xffffffffu, (bits & kOutside) != 0u);
+      };
+      // columns that stay BF16, or the others
+      auto keep = [&](const uint32_t (&e)[NT], bool wide) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int i = 0; i < NB; ++i) b[nt][i] = (e[nt] == kWide) == wide ? b[nt][i] : 0u;
+      };
+      if constexpr (ODDITIES == ODD_SHARED) {
+        first_rows();                       // (on their way meanwhile)
+        float scale[NT];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          unscale[nt] = pack2(kWindowUnscale, kWindowUnscale);
+          scale[nt] = kWindowScale;
+        }
+        const int step = win * STEPS + st;
+        bool odd;
+        if constexpr (RES == RES_NONE) odd = outside();
+        else odd = (spread >> (step & 31) & 1u) != 0u;
+        if (__builtin_expect(odd, 0)) {
+          uint32_t e[NT];
+          bool any = false, all = true;      // are kWide
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            if constexpr (RES == RES_NONE) {
+              e[nt] = chunk_exp(chunk_range<NB>(b[nt]));
+            } else {
+              const int steps = (p.row_bytes + STEP - 1) / STEP;
+              e[nt] = lds_u8(bars.exps + (uint32_t)((ln.warp * steps + step) * M + min(fragment_column<FMT>(ln.g), M - 1)));
+            }
+            const uint32_t wide = __ballot_sync(0xffffffffu, e[nt] == kWide);
+            any |= wide != 0u;
+            all &= wide == 0xffffffffu;
+          }
+          if (any) {
+            keep(e, true);
+            // (rolled: its registers and its instructions would be taken from the other chunks. An odd tile's last group has its
+            // lower rows twice.)
+#pragma unroll 1
+            for (int r = 0; r < G; ++r) {
+              pk2 sum[NT][2];
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) sum[nt][0] = sum[nt][1] = pack2(0.f, 0.f);
+              const bool half = ODD && r == G - 1;
+              load_rows<FMT, STEPS, false>(raw[0], wrow + r * kGroupRows * W_ROW, srow + r * kGroupRows * SC_ROW, half ? 0 : 8, half ? 0 : sc_hi, ln.t);
+              chunk_rows<FMT, NT, ACTS_WIDE, false>(raw[0], b, unscale, sum);
+#pragma unroll
+              for (int i = 0; i < G; ++i)
+                if (i == r) {
+#pragma unroll
+                  for (int nt = 0; nt < NT; ++nt) {
+                    acc[i][nt][0] = fadd2(sum[nt][0], acc[i][nt][0]);
+                    acc[i][nt][1] = fadd2(sum[nt][1], acc[i][nt][1]);
+                  }
+                }
+            }
+            if (all) continue;
+            load_x<FMT, NT, RES != RES_NONE>(xs, xo, b);
+            first_rows();
+            keep(e, false);
+          }
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            unscale[nt] = column_unscale(e[nt], ln);
+            scale[nt] = exp_scale(e[nt] == kWide ? kWindowExp : e[nt]);
+          }
+        }
+        if constexpr (RES == RES_NONE) {
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(b[nt][i], scale[nt]);
+        }
+        multiply(Scaled());
+      } else {
+        if constexpr (ODDITIES == ODD_APART) {
+          if (__builtin_expect(outside(), 0)) {
+            uint32_t e[NT];
+            bool odd = false, any = false, all = true;       // not the usual exponent; are kWide
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+              e[nt] = chunk_exp(chunk_range<NB>(b[nt]));
+              odd |= e[nt] != kWindowExp;
+            }
+            if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) {
+                const uint32_t wide = __ballot_sync(0xffffffffu, e[nt] == kWide);
+                any |= wide != 0u;
+                all &= wide == 0xffffffffu;
+              }
+              if (any) {
+                keep(e, true);
+                first_rows();
+                multiply(Wide());
+                if (all) continue;
+                load_x<FMT, NT, false>(xs, xo, b);           // (registers for both would be taken from every chunk)
+              }
+              first_rows();
+              keep(e, false);
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt) {
+                unscale[nt] = column_unscale(e[nt], ln);
+                const float scale = exp_scale(e[nt] == kWide ? kWindowExp : e[nt]);
+#pragma unroll
+                for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(b[nt][i], scale);
+              }
+              multiply(Scaled());
+              continue;
+            }
+          }
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(b[nt][i], kWindowScale);
+        }
+        first_rows();
+        multiply(Usual());
       }
     }
     left -= WIN;
@@ -1118,10 +1149,6 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
         if (m1 < M) sts_f32(row + m1 * 4, c);
       }
   }
-  if constexpr (CONVERT) {
-    if (RES) left_out = spread;
-    if (left_out != 0u) extra_tile<FMT, NT>(p, col0, cols, at, W_ROW, left_out);
-  }
   if (last) {
     consumer_barrier();
     if (ln.warp < finish_units(p, wk)) finish_unit<FMT, STEPS>(p, wk, ring + (uint32_t)s * stage_bytes, col0, cols, ln.warp, scales);
@@ -1141,7 +1168,7 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
   const StageLayout<FMT, STEPS> lay(p);
   if (first) griddep_wait();   // consumers read scales and write results in global memory: after the previous kernel
   bool resident = false;
-  uint32_t spread = 0u;           // steps (modulo 32) with activations outside the window
+  uint32_t spread = 0u;           // (see prepare_resident)
   bool ok = true;
   if (first && threadIdx.x == 0) trace_stamp(p.trace, TRACE_DEP);
   if constexpr (CAN_RES) {
@@ -1149,7 +1176,7 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     if (resident && wk.ntiles > 0) {
       ok = mbar_wait(bars.x, x_parity, bars.abort_flag);
       x_parity ^= 1u;
-      if constexpr (std::is_same<XT, __nv_bfloat16>::value) spread = prepare_resident<FMT>(p, smem);
+      if constexpr (std::is_same<XT, __nv_bfloat16>::value) spread = prepare_resident<FMT>(p, smem, bars.exps);
       __syncwarp();
     }
   }
@@ -1157,9 +1184,9 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     int col0, cols;
     wk.tile(t, col0, cols);
     auto tile = [&](auto res) {
-      constexpr bool RES = decltype(res)::value;
+      constexpr int RES = decltype(res)::value;
       auto run = [&](auto e) {
-        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
+        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, CAN_RES, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
                                                                   first && t == 0, ok);
       };
       const int eights = (wk.rows(cols) + 7) / 8;
@@ -1175,10 +1202,12 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
       run(std::integral_constant<int, 1>());
     };
     if constexpr (CAN_RES) {
-      if (resident) tile(std::true_type());
-      else tile(std::false_type());
+      // (the usual case in code of its own: what a launch fetches of the other costs it 0.6 us)
+      if (resident && spread == 0u) tile(std::integral_constant<int, RES_USUAL>());
+      else if (resident && std::is_same<XT, __nv_bfloat16>::value) tile(std::integral_constant<int, RES_MIXED>());
+      else tile(std::integral_constant<int, RES_NONE>());
     } else {
-      tile(std::false_type());
+      tile(std::integral_constant<int, RES_NONE>());
     }
   }
   if (!ok && (threadIdx.x & 31) == 0 && p.status) atomicOr(p.status, kStatusConsumerTimeout);
@@ -1316,8 +1345,9 @@ __device__ __forceinline__ void gather_signal(const Params& p, volatile int* abo
 }
 
 // Barriers and the abort word of a CTA; the first thread sets them up. `copies`: the copying warps take part.
-__device__ __forceinline__ Bars ring_setup(const Params& p, bool copies, unsigned char* smem, uint64_t* sums) {
+__device__ __forceinline__ Bars ring_setup(const Params& p, bool copies, unsigned char* smem, uint64_t* sums, const uint8_t* exps) {
   Bars bars;
+  bars.exps = smem_addr(exps);
   bars.x = smem_addr(sums + kMaxStages);
   bars.full = smem_addr(smem);
   bars.empty = bars.full + 8u * kMaxStages;
@@ -1352,8 +1382,9 @@ template <int FMT, int NT, bool CAN_RES, int STEPS, bool SMALL, typename XT>
 __global__ void __launch_bounds__(SMALL ? kSmallThreads : kThreads, SMALL ? 2 : 1) gemv_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
+  __shared__ uint8_t exps[CAN_RES ? kResidentExps : 1];
   const bool copies = !SMALL && copies_needed<FMT>(p);
-  const Bars bars = ring_setup(p, copies, smem, sums);
+  const Bars bars = ring_setup(p, copies, smem, sums, exps);
   int s = 0;
   uint32_t parity = 0, x_parity = 0;
   const int warp = (int)(threadIdx.x >> 5);
@@ -1400,7 +1431,8 @@ template <int FMT, int NT, bool CAN_RES, int STEPS, typename XT>
 __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* __restrict__ items, int count) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
-  const Bars bars = ring_setup(items[0], true, smem, sums);
+  __shared__ uint8_t exps[CAN_RES ? kResidentExps : 1];
+  const Bars bars = ring_setup(items[0], true, smem, sums, exps);
   int s = 0;
   uint32_t parity = 0, x_parity = 0;
   const int warp = (int)(threadIdx.x >> 5);

@@ -26,10 +26,10 @@
 //
 // Activations. BF16 weights multiply BF16 activations as they are. Decoded E4M3 and E2M1 x E4M3 weights are FP16 values
 // (at most 6 significant bits, 2^-10 .. 2688), so FP16 activations are used as they are too. BF16 activations of these
-// formats become FP16 times 2^7: exact for zero and for magnitudes of [2^-24, 2^8) (FP16 holds BF16's eight bits down to
-// 2^-17, its subnormals included); the power of two comes off in the FP32 FMA. A chunk of a row with any other value is
-// multiplied apart, in as many passes as its values take: each pass takes the values within 28 binades of the largest that
-// is left, times a power of two of its own, and zeros for the rest.
+// formats become FP16 times a power of two, exactly; it comes off in the FP32 FMA. The power is 2^7 for a chunk of a row
+// whose magnitudes lie in [2^-24, 2^8) or are zero, the one that fits for any other chunk within 32 binades. A chunk that
+// spans more (or holds infinities or NaNs) stays BF16: its products are made with the weights converted to BF16, which is
+// exact too and takes about twice as long.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -173,70 +173,69 @@ __device__ __forceinline__ void mma_step(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// BF16 activations times 2^7 as FP16: the usual way. A value fits when (|v| - 2^-24) as 15-bit patterns lies within 32
-// binades; `window_bits` has a bit of kOutside set where one of a pair does not (zeros do not either: window_fits looks
-// closer). v * 2 drops the upper half's sign and puts the lower half's where it does no harm.
-constexpr uint32_t kWindowLow = 103u << 7, kWindowSize = 32u << 7, kOutside = 0xe000e000u;
+// BF16 activations as FP16. FP16 holds BF16's eight bits over 32 binades, [2^-17, 2^15) (the lower ones as subnormals): a
+// chunk of an activation row whose values lie within 32 binades is multiplied by the power of two that takes them there,
+// 2^(141 - e), e being a biased exponent: the usual 2^7 (e = kWindowExp) for zeros and magnitudes of [2^-24, 2^8), else that
+// of the chunk's largest magnitude (from kExpLow on: below it the power would leave FP32's range, and everything down to
+// BF16's subnormals fits under 2^121).
+constexpr uint32_t kWindowExp = 134, kExpLow = 20, kExpInf = 255, kExpSpan = 31;
+constexpr uint32_t kWindowLow = (kWindowExp - kExpSpan) << 7, kOutside = 0xe000e000u;
 constexpr float kWindowScale = 128.0f, kWindowUnscale = 1.0f / 128.0f;
+// Has a bit of kOutside set where one of a pair is not in the usual window: (|v| - 2^-24) as 15-bit patterns lies within 32
+// binades there. (Zeros set one too: chunk_range looks closer.) v * 2 drops the upper half's sign and puts the lower half's
+// where it does no harm.
 __device__ __forceinline__ uint32_t window_bits(uint32_t v) { return v * 2u - 2u * (kWindowLow << 16 | kWindowLow); }
-template <int NB>
-__device__ __forceinline__ bool window_fits(const uint32_t (&v)[NB]) {
-  bool ok = true;
-#pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    const uint32_t lo = v[i] & 0x7fffu, hi = (v[i] >> 16) & 0x7fffu;
-    ok = ok && (lo == 0u || lo - kWindowLow < kWindowSize) && (hi == 0u || hi - kWindowLow < kWindowSize);
-  }
-  return ok;
-}
-// The other way: times 2^(141 - e) for a chunk whose largest magnitude has the biased exponent e, which takes that
-// magnitude to [2^14, 2^15). Below kExpLow the power would leave FP32's range; everything down to BF16's subnormals still
-// fits under 2^121. Infinities and NaNs (e = 255) survive the product.
-constexpr uint32_t kExpLow = 20, kExpInf = 255, kExpSpan = 28;
 __device__ __forceinline__ float exp_scale(uint32_t e) { return __uint_as_float((268u - e) << 23); }      // 2^(141 - e)
 __device__ __forceinline__ float exp_unscale(uint32_t e) { return __uint_as_float((e - 14u) << 23); }     // 2^(e - 141)
-// e of a chunk with largest magnitude `top` (15-bit BF16 pattern), and the smallest magnitude that goes with it: a
-// normal FP16 value after scaling.
-__device__ __forceinline__ uint32_t chunk_exp(uint32_t top) { return max(top >> 7, kExpLow); }
-__device__ __forceinline__ uint32_t chunk_low(uint32_t e) {
-  return e >= kExpInf ? kExpInf << 7 : e > kExpSpan ? (e - kExpSpan) << 7 : 0u;
+
+// Range of NB pairs: the largest magnitude's 15-bit pattern in the upper half; in the lower 0xffff less (the pattern of the
+// smallest magnitude that is not zero, less one), 0 where all are zeros. The ranges of two parts join as their larger halves.
+template <int NB>
+__device__ __forceinline__ uint32_t chunk_range(const uint32_t (&v)[NB]) {
+  uint32_t hi[NB], lo[NB];
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    hi[i] = v[i] & 0x7fff7fffu;
+    lo[i] = hi[i] + 0x7fff7fffu;              // (zero: the largest of signed halves; else the smaller the lower)
+  }
+#pragma unroll
+  for (int n = NB / 2; n > 0; n /= 2)         // (a chain would cost its latency)
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      hi[i] = __vmaxu2(hi[i], hi[i + n]);
+      lo[i] = __vmins2(lo[i], lo[i + n]);
+    }
+  const uint32_t top = max(hi[0] & 0xffffu, hi[0] >> 16), low = ~(lo[0] ^ 0x80008000u);
+  return top << 16 | max(low & 0xffffu, low >> 16);
+}
+// The chunk's exponent e from the ranges of the four lanes that hold it; kWide: its values span more than FP16 holds, or are
+// not all finite.
+constexpr uint32_t kWide = 0;
+__device__ __forceinline__ uint32_t chunk_exp(uint32_t range) {
+  range = __vmaxu2(range, __shfl_xor_sync(0xffffffffu, range, 1));
+  range = __vmaxu2(range, __shfl_xor_sync(0xffffffffu, range, 2));
+  const uint32_t top = range >> 16, smallest = 0x10000u - (range & 0xffffu);
+  const uint32_t e = top >> 7 <= kWindowExp && smallest >= kWindowLow ? kWindowExp : max(top >> 7, kExpLow);
+  return e < kExpInf && (e <= kExpSpan || smallest >= (e - kExpSpan) << 7) ? e : kWide;
 }
 
-// Per half: the larger magnitude (NaN kept), in the low 15 bits.
-__device__ __forceinline__ uint32_t amax_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
 __device__ __forceinline__ uint32_t scaled_half2(uint32_t v, float s) {   // two BF16 times s as two FP16
   float lo, hi;
   unpack2(fmul2(pack2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)), pack2(s, s)), lo, hi);
   const __half2 t = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&t);
 }
-// Largest magnitude of NB pairs as a 15-bit BF16 pattern (above 0x7f80: a NaN).
-template <int NB>
-__device__ __forceinline__ uint32_t chunk_amax(const uint32_t (&v)[NB]) {
-  uint32_t m = v[0];
-#pragma unroll
-  for (int i = 1; i < NB; ++i) m = amax_bf16x2(m, v[i]);
-  return max(m & 0x7fffu, (m >> 16) & 0x7fffu);
+// A pair that fitted the usual window, from FP16 times 2^7 back to BF16.
+__device__ __forceinline__ uint32_t window_back(uint32_t h) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+  const __nv_bfloat162 t = __floats2bfloat162_rn(f.x * kWindowUnscale, f.y * kWindowUnscale);
+  return *reinterpret_cast<const uint32_t*>(&t);
 }
-// Whether every value that is not zero is at least `low` (15-bit patterns).
-template <int NB>
-__device__ __forceinline__ bool chunk_fits(const uint32_t (&v)[NB], uint32_t low) {
-  bool ok = true;
-#pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    const uint32_t lo = v[i] & 0x7fffu, hi = (v[i] >> 16) & 0x7fffu;
-    ok = ok && (lo == 0u || lo >= low) && (hi == 0u || hi >= low);
-  }
-  return ok;
-}
-// The values of a pair with low <= magnitude < high, zeros for the others.
-__device__ __forceinline__ uint32_t keep_range(uint32_t v, uint32_t low, uint32_t high) {
-  const uint32_t lo = v & 0x7fffu, hi = (v >> 16) & 0x7fffu;
-  return (lo >= low && lo < high ? v & 0xffffu : 0u) | (hi >= low && hi < high ? v & 0xffff0000u : 0u);
+// A pair of decoded weights (FP16 with at most 6 significant bits) as BF16: exact.
+__device__ __forceinline__ uint32_t half2_to_bf162(uint32_t h) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+  const __nv_bfloat162 t = __floats2bfloat162_rn(f.x, f.y);
+  return *reinterpret_cast<const uint32_t*>(&t);
 }
 
 }  // namespace dg
