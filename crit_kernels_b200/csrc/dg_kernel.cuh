@@ -555,7 +555,7 @@ __device__ __forceinline__ bool gather_scales(const Params& p, const Walk& wk, u
     for (int b = lane; b < WINDOW; b += 32) {
       const int j = byte0 + b;
       const uint8_t* src = p.scales + (tiled ? tiled_scale_offset(n, j & ~1, p.ct) + (j & 1) : (size_t)n * p.scale_row_bytes + j);
-      sts_u8(dst + (uint32_t)(r * SC_ROW + b), j < sc_bytes ? (uint32_t)__ldg(src) : 0u);
+      sts_u8(dst + (uint32_t)(r * SC_ROW + b), j < sc_bytes ? (uint32_t)*src : 0u);
     }
   }
   return true;
@@ -869,8 +869,8 @@ __device__ __forceinline__ void finish_scales(const Params& p, const Walk& wk, i
   const int c = unit_column(wk, u);
   f[0] = f[1] = 1.f;
   if (p.row_scale && c < cols) {
-    f[0] = __ldg(p.row_scale + col0 + c);
-    if (wk.pairs) f[1] = __ldg(p.row_scale + wk.pairs + col0 + c);
+    f[0] = p.row_scale[col0 + c];
+    if (wk.pairs) f[1] = p.row_scale[wk.pairs + col0 + c];
   }
 }
 template <int FMT, int STEPS>

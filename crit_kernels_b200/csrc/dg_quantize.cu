@@ -92,18 +92,18 @@ __device__ __forceinline__ void quantize_row(const __nv_bfloat16* xr, const uint
     const uint4* rv = staged ? row_smem : reinterpret_cast<const uint4*>(xr);
     if (vector_out && (K & 15) == 0) {   // 16 values -> one 16-byte store
       for (int i = tid; i < (K >> 4); i += kRowThreads) {
-        const uint4 a = staged ? rv[2 * i] : __ldg(rv + 2 * i), b = staged ? rv[2 * i + 1] : __ldg(rv + 2 * i + 1);
+        const uint4 a = rv[2 * i], b = rv[2 * i + 1];
         reinterpret_cast<uint4*>(qr)[i] = make_uint4(fp8_quad<SAFE>(a.x, a.y, d, r), fp8_quad<SAFE>(a.z, a.w, d, r),
                                                      fp8_quad<SAFE>(b.x, b.y, d, r), fp8_quad<SAFE>(b.z, b.w, d, r));
       }
     } else if (vector_out) {             // 8 values -> one 8-byte store
       for (int i = tid; i < (K >> 3); i += kRowThreads) {
-        const uint4 a = staged ? rv[i] : __ldg(rv + i);
+        const uint4 a = rv[i];
         reinterpret_cast<uint2*>(qr)[i] = make_uint2(fp8_quad<SAFE>(a.x, a.y, d, r), fp8_quad<SAFE>(a.z, a.w, d, r));
       }
     } else {
       for (int i = tid; i < (K >> 3); i += kRowThreads) {
-        const uint4 a = staged ? rv[i] : __ldg(rv + i);
+        const uint4 a = rv[i];
         const uint32_t lo = fp8_quad<SAFE>(a.x, a.y, d, r), hi = fp8_quad<SAFE>(a.z, a.w, d, r);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -125,7 +125,7 @@ __device__ __forceinline__ void quantize_row(const __nv_bfloat16* xr, const uint
 // 3.3 us, now 2.8; 1 x 4096: 1.65, now 1.35). From about 5000 values on in batches that fill the chip the bulk copy is the
 // faster way (4096 x 28672: 54 us, at copy bandwidth; 96 here, with one CTA of 1024 threads waiting at its barrier).
 constexpr int kHeld = 4;
-__global__ void __launch_bounds__(1024) fp8_held_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int M, int K,
+__global__ void __launch_bounds__(1024) fp8_held_rows_kernel(const __nv_bfloat16* x, long long ldx, int M, int K,
                                                                 uint8_t* __restrict__ q, long long ldq, float* __restrict__ scale,
                                                                 int group) {
   __shared__ float part[32];
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(1024) fp8_held_rows_kernel(const __nv_bfloat16
   uint32_t m2 = 0u;
 #pragma unroll
   for (int i = 0; i < kHeld; ++i)
-    v[i] = in && t + i * group < (K >> 3) ? __ldg(xr + t + i * group) : make_uint4(0u, 0u, 0u, 0u);
+    v[i] = in && t + i * group < (K >> 3) ? xr[t + i * group] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
   for (int i = 0; i < kHeld; ++i) m2 = amax8(v[i], m2);
   float m = amax_of(m2);
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(1024) fp8_held_rows_kernel(const __nv_bfloat16
 }
 
 // Other rows, one CTA each. `staged`: the row (K a multiple of 8, 16-byte aligned, within shared memory) arrives by one bulk copy.
-__global__ void __launch_bounds__(kRowThreads) fp8_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int K,
+__global__ void __launch_bounds__(kRowThreads) fp8_rows_kernel(const __nv_bfloat16* x, long long ldx, int K,
                                                                uint8_t* __restrict__ q, long long ldq,
                                                                float* __restrict__ scale, int staged, int vector_out) {
   extern __shared__ __align__(128) unsigned char row_smem[];
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kRowThreads) fp8_rows_kernel(const __nv_bfloat
     m = amax_of(m2);
   } else if ((K & 7) == 0 && (ldx & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     const uint4* rv = reinterpret_cast<const uint4*>(xr);
-    for (int i = tid; i < (K >> 3); i += kRowThreads) m2 = amax8(__ldg(rv + i), m2);
+    for (int i = tid; i < (K >> 3); i += kRowThreads) m2 = amax8(rv[i], m2);
     m = amax_of(m2);
   } else {
     for (int k = tid; k < K; k += kRowThreads) m = nanmax(m, fabsf(__bfloat162float(xr[k])));
@@ -323,7 +323,7 @@ __device__ __forceinline__ uint32_t nvfp4_block(const uint32_t (&w)[8], float g,
 // lines.) The arithmetic bounds it, more than the memory: about 100 instructions a block, with the quotients in packed pairs.
 // 4096 x 8192: 22.3 us before, 18.9 now (13.1 at copy bandwidth); 16 x 28672: 5.0 and 1.9.
 constexpr int kQuantCols = 512, kQuantRows = 32;
-__global__ void __launch_bounds__(256) nvfp4_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int M, int K,
+__global__ void __launch_bounds__(256) nvfp4_kernel(const __nv_bfloat16* x, long long ldx, int M, int K,
                                                     float g, float g_rcp, uint8_t* __restrict__ codes,
                                                     uint8_t* __restrict__ scales, int quads, int col_tiles, int wide_scales) {
   __shared__ __align__(16) unsigned char tile[kQuantCols / 64 * 128];   // [quad][row % 8][row / 32][block % 4]
@@ -340,8 +340,8 @@ __global__ void __launch_bounds__(256) nvfp4_kernel(const __nv_bfloat16* __restr
     const int row = row0 + 32 * i;
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * ldx + k);
     const bool in = row < M && k < K;
-    v[i][0] = in ? __ldg(src) : make_uint4(0u, 0u, 0u, 0u);
-    v[i][1] = in ? __ldg(src + 1) : make_uint4(0u, 0u, 0u, 0u);
+    v[i][0] = in ? src[0] : make_uint4(0u, 0u, 0u, 0u);
+    v[i][1] = in ? src[1] : make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
 #pragma unroll

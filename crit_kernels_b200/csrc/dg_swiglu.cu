@@ -14,7 +14,7 @@
 namespace {
 
 template <bool IN_F32, bool OUT_F32>
-__global__ void __launch_bounds__(256) swiglu_kernel(const void* __restrict__ gate_up, long long ldg, int rows, int inter,
+__global__ void __launch_bounds__(256) swiglu_kernel(const void* gate_up, long long ldg, int rows, int inter,
                                                      void* __restrict__ out, long long ldo, int vector) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

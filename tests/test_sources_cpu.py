@@ -1,0 +1,31 @@
+"""Rules of the kernel sources that no run shows reliably."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "crit_kernels_b200", "csrc")
+
+
+def code(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def early_starters():
+    """Sources of the kernels that are resident while the previous kernel of the stream still runs."""
+    names = [n for n in sorted(os.listdir(CSRC)) if "griddepcontrol.wait" in code(n)]
+    assert {"dg_kernel.cuh", "dg_quantize.cu", "dg_swiglu.cu"} <= set(names)
+    return names
+
+
+@pytest.mark.parametrize("name", early_starters())
+def test_kernels_that_start_early_read_nothing_through_the_read_only_path(name):
+    """Loads through the non-coherent path (ld.global.nc, __ldg, const __restrict__ parameters, which the compiler turns into
+    such loads) are for memory nobody writes during a kernel's whole life. The previous kernel may write what these read: its
+    outputs are their activations, and scales unless the caller has declared them static. (A batch's launch parameters are
+    read before the wait as it is, so they have to be there before the previous kernel starts.)"""
+    text = code(name)
+    assert not re.findall(r"ld\.global\.nc|\b__ldg\s*\(|\bldg_nc\w*", text)
+    restricted = re.findall(r"const\s+(\w+)\s*\*\s*__restrict__\s+(\w+)", text)
+    assert set(restricted) <= {("Params", "items")}, restricted
