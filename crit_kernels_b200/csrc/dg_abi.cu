@@ -530,6 +530,7 @@ int dg_encode_nvfp4_batch(const DgNvfp4BatchItem* items, int count, int x_is_bf1
   }
   if (stages < 2) return (int)cudaErrorInvalidValue;
   for (int g = 0; g < count; ++g) {
+    out[0].batch_copies |= out[g].x_mode == dg::X_COPIED || out[g].scale_mode != dg::SCALES_STAGED;
     out[g].stage_bytes = stage_bytes;
     out[g].stages = stages;
     out[g].x_res_off = dg::kSmemHeader + stages * stage_bytes;

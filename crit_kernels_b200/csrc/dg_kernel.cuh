@@ -127,6 +127,7 @@ struct Params {
   int M;                     // activation rows
   int cols_each, cols_more;  // the CTAs' output columns (see Walk)
   int small;                 // 1: a small launch (see kSmallThreads)
+  int batch_copies;          // batched launches, first GEMV: some GEMV of the batch needs the copying warps (copies_needed)
   int steps;                 // 512-byte steps per ring stage
   int stages;                // ring depth
   int tile_rows;             // rows of a full tile (a multiple of 8; gate_up: of 16, for both regions), at most 16 * kMaxGroups
@@ -1432,7 +1433,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* _
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
   __shared__ uint8_t exps[CAN_RES ? kResidentExps : 1];
-  const Bars bars = ring_setup(items[0], true, smem, sums, exps);
+  const bool copies = items[0].batch_copies != 0;
+  const Bars bars = ring_setup(items[0], copies, smem, sums, exps);
   int s = 0;
   uint32_t parity = 0, x_parity = 0;
   const int warp = (int)(threadIdx.x >> 5);
@@ -1440,11 +1442,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* _
     bool ok = true;
     for (int g = 0; g < count && ok; ++g)
       ok = feed_weights<FMT, STEPS>(items[g], items[g], smem, bars, g == 0, g == 0 && !items[0].early_weights, s, parity);
-  } else if (warp == kFinisher) {
-    start_activations<FMT, STEPS>(items[0], items[0], smem, bars);
+  } else if (warp >= kFinisher && !(copies && warp >= kFirstCopier)) {
+    if (warp == kFinisher) start_activations<FMT, STEPS>(items[0], items[0], smem, bars);
+    else griddep_wait();
     bool ok = true;
     for (int g = 0; g < count; ++g) {
-      if (ok) ok = finish_gemv<FMT, STEPS>(items[g], smem, bars, 0, 1, s, parity);
+      if (ok) ok = finish_gemv<FMT, STEPS>(items[g], smem, bars, warp - kFinisher, copies ? 1 : kFinishers, s, parity);
       if (items[g].world >= 1) finished_barrier();
     }
   } else if (warp >= kFirstCopier) {
