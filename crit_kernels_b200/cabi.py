@@ -67,10 +67,11 @@ def load() -> ctypes.CDLL:
 
 
 def plan(fmt: str, m: int, n: int, k: int) -> dict:
-    """The launch shape a call of these sizes gets (host only)."""
+    """The launch shape a call of these sizes gets (host only). `rows_per_warp` is the name that `row_groups` had while a consumer
+    warp took a part of a tile's rows (before version 1.03)."""
     out = (ctypes.c_int * 6)()
     code = load().dg_plan(FMT[fmt], m, n, k, out)
     if code:
         raise ValueError(f"dg_plan refused fmt={fmt} M={m} N={n} K={k} (cudaError {code})")
-    keys = ("ctas", "rows_per_warp", "steps", "stages", "stage_bytes", "smem_bytes")
-    return dict(zip(keys, out))
+    keys = ("ctas", "row_groups", "steps", "stages", "stage_bytes", "smem_bytes")
+    return {**dict(zip(keys, out)), "rows_per_warp": out[1]}

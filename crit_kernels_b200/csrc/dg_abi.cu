@@ -644,6 +644,6 @@ int dg_set_trace(void* buffer, int launches) {
   return 0;
 }
 
-int dg_version(void) { return 102; }
+int dg_version(void) { return 103; }
 
 }  // extern "C"

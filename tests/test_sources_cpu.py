@@ -29,3 +29,13 @@ def test_kernels_that_start_early_read_nothing_through_the_read_only_path(name):
     assert not re.findall(r"ld\.global\.nc|\b__ldg\s*\(|\bldg_nc\w*", text)
     restricted = re.findall(r"const\s+(\w+)\s*\*\s*__restrict__\s+(\w+)", text)
     assert set(restricted) <= {("Params", "items")}, restricted
+
+
+def test_the_plan_is_what_its_description_says_and_the_version_tells_it_from_the_earlier_one():
+    """plan[1] used to be the rows per consumer warp; since every consumer warp takes all rows of a tile it is a tile's groups of
+    16 rows, under its own name and a library version of its own."""
+    from crit_kernels_b200 import cabi
+    assert cabi.load().dg_version() >= 103
+    for fmt, n, k, row in (("nvfp4", 8192, 8192, 2 * 512 + 16 + 2 * 64 + 16), ("fp8", 28672, 8192, 2 * 512 + 16)):
+        p = cabi.plan(fmt, 1, n, k)                  # (resident activations: a stage is rows of weights and scales)
+        assert p["row_groups"] == -(-(p["stage_bytes"] // row) // 16) and p["row_groups"] == p["rows_per_warp"]
