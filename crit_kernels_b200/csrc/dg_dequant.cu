@@ -14,6 +14,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/decode_gemv_b200.h"
 #include "dg_kernel.cuh"
@@ -22,7 +23,7 @@ namespace {
 
 enum : int { DQ_BF16 = 1, DQ_F16 = 2, DQ_E4M3 = 3 };
 constexpr int kThreads = 256;
-constexpr int kBatch = 4;   // 16-byte output units a thread has in flight
+constexpr int kBatch = 4;   // 16-byte output units a thread has in flight in a large matrix
 
 __device__ __forceinline__ float e4m3_to_f32(uint32_t byte) {
   const __half_raw h = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)byte, __NV_E4M3);
@@ -63,17 +64,20 @@ __device__ __forceinline__ uint32_t round4_e4m3(float a, float b, float c, float
 // scale block) for FP8. `unit` counts such units from the start of the matrix.
 template <int OUT> struct Unit { static constexpr int WORDS = OUT == DQ_E4M3 ? 2 : 1; };
 
-// The matrix is one run of units, kBatch x kThreads to a CTA, whatever its rows: the rows of codes, scales and values follow
+// The matrix is one run of units, BATCH x kThreads to a CTA, whatever its rows: the rows of codes, scales and values follow
 // each other without gaps. As many CTAs as that takes: a CTA that is done makes room for the next, so that loads and stores
 // of different CTAs overlap all the time (eight persistent CTAs per SM, walking whole rows, took 33.5 us for 8192 x 8192 to
 // BF16; this 30.7, the rate of a device-to-device copy of as many bytes; stores alone take 24.5; 28672 x 8192: 105.7 and 92.2).
-template <int OUT>
+// BATCH is kBatch where that makes a CTA for every SM, else one unit per thread: a small matrix is bound by a CTA's latency and by
+// the SMs without one (256 x 512 to BF16 2.03 us with four, 1.52 with one, and 1.74 with a CTA per row; 1024 x 1024 to FP8 2.84,
+// 2.37 and 2.65; from a CTA per SM on both are the same).
+template <int OUT, int BATCH>
 __global__ void __launch_bounds__(kThreads)
     dequantize_kernel(const uint32_t* __restrict__ codes, const uint8_t* __restrict__ scales,
                       const float* __restrict__ factor, uint4* __restrict__ out, long long total, int units) {
   constexpr int WORDS = Unit<OUT>::WORDS;
-  const long long first = (long long)blockIdx.x * (kThreads * kBatch);
-  const int count = (int)min((long long)(kThreads * kBatch), total - first);
+  const long long first = (long long)blockIdx.x * (kThreads * BATCH);
+  const int count = (int)min((long long)(kThreads * BATCH), total - first);
   // row and place within the row of the CTA's first unit (units: per row)
   const long long row0 = total <= 0xffffffffll ? (long long)((uint32_t)first / (uint32_t)units) : first / units;
   const int place0 = (int)(first - row0 * units);
@@ -81,10 +85,10 @@ __global__ void __launch_bounds__(kThreads)
   scales += (first * WORDS) >> 1;                           // (first is even)
   factor += row0;
   out += first;
-  uint32_t c[kBatch][WORDS] = {}, sb[kBatch] = {};
-  float f[kBatch] = {};
+  uint32_t c[BATCH][WORDS] = {}, sb[BATCH] = {};
+  float f[BATCH] = {};
 #pragma unroll
-  for (int b = 0; b < kBatch; ++b) {
+  for (int b = 0; b < BATCH; ++b) {
     const int u = b * kThreads + threadIdx.x;
     if (u < count) {
       if constexpr (WORDS == 2) {
@@ -100,7 +104,7 @@ __global__ void __launch_bounds__(kThreads)
     }
   }
 #pragma unroll
-  for (int b = 0; b < kBatch; ++b) {
+  for (int b = 0; b < BATCH; ++b) {
     const int u = b * kThreads + threadIdx.x;
     if (u < count) {
       const float scale = e4m3_to_f32(sb[b]);
@@ -154,12 +158,17 @@ extern "C" DG_API int dg_enqueue_dequantize(const uint8_t* codes, const uint8_t*
   if (sms < 1) return (int)cudaErrorInvalidDevice;
   const int units = K / (out_kind == DQ_E4M3 ? 16 : 8);      // 16-byte output vectors per row
   const long long total = (long long)N * units;
-  const dim3 grid((unsigned)((total + kThreads * kBatch - 1) / (kThreads * kBatch))), block(kThreads);
-  const uint32_t* c32 = reinterpret_cast<const uint32_t*>(codes);
-  uint4* o = static_cast<uint4*>(out);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (out_kind == DQ_BF16) dequantize_kernel<DQ_BF16><<<grid, block, 0, s>>>(c32, scales, factor, o, total, units);
-  else if (out_kind == DQ_F16) dequantize_kernel<DQ_F16><<<grid, block, 0, s>>>(c32, scales, factor, o, total, units);
-  else dequantize_kernel<DQ_E4M3><<<grid, block, 0, s>>>(c32, scales, factor, o, total, units);
+  auto launch = [&](auto out_type) {
+    constexpr int OUT = decltype(out_type)::value;
+    const bool batched = total >= (long long)sms * kThreads * kBatch;
+    const int run = kThreads * (batched ? kBatch : 1);
+    const dim3 grid((unsigned)((total + run - 1) / run));
+    const uint32_t* c32 = reinterpret_cast<const uint32_t*>(codes);
+    (batched ? dequantize_kernel<OUT, kBatch> : dequantize_kernel<OUT, 1>)<<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        c32, scales, factor, static_cast<uint4*>(out), total, units);
+  };
+  if (out_kind == DQ_BF16) launch(std::integral_constant<int, DQ_BF16>());
+  else if (out_kind == DQ_F16) launch(std::integral_constant<int, DQ_F16>());
+  else launch(std::integral_constant<int, DQ_E4M3>());
   return (int)cudaGetLastError();
 }

@@ -26,3 +26,10 @@ def test_runs_that_cross_rows(n, k, dtype):
     want = oc.dequantize(c, s, i, dtype)
     assert torch.equal(out[:-64].cpu(), want.view(torch.uint8).flatten())
     assert bool((out[-64:] == 0x55).all())
+
+
+@pytest.mark.parametrize("n,k,dtype", [(n, k, d) for d, k in ((torch.bfloat16, 8192), (torch.float8_e4m3fn, 16384))
+                                       for n in (147, 148, 149)] + [(1, 16, torch.bfloat16), (255, 16, torch.float8_e4m3fn)])
+def test_matrices_around_one_run_per_sm(n, k, dtype):
+    """Below 1024 output vectors per SM a CTA takes 256 of them."""
+    test_runs_that_cross_rows(n, k, dtype)
