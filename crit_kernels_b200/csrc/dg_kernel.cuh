@@ -30,7 +30,6 @@
 #include <cstdint>
 #include <type_traits>
 
-#include "dg_lane_reduce.cuh"
 #include "dg_mma.cuh"
 #include "dg_swiglu.cuh"
 
@@ -163,7 +162,7 @@ struct Params {
 };
 
 // ---------------------------------------------------------------------------------------------------------------
-// PTX wrappers: mbarrier, 1-D bulk copy (TMA), 16-byte cp.async tied to an mbarrier.
+// PTX wrappers: mbarriers, tensor copies (TMA), cp.async tied to an mbarrier.
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -217,11 +216,6 @@ static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, abort_flag);
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
 }
 // 2-D tiled tensor copy: box of the tensor map at element column x, row y.
 __device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
