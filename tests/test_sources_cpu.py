@@ -39,3 +39,9 @@ def test_the_plan_is_what_its_description_says_and_the_version_tells_it_from_the
     for fmt, n, k, row in (("nvfp4", 8192, 8192, 2 * 512 + 16 + 2 * 64 + 16), ("fp8", 28672, 8192, 2 * 512 + 16)):
         p = cabi.plan(fmt, 1, n, k)                  # (resident activations: a stage is rows of weights and scales)
         assert p["row_groups"] == -(-(p["stage_bytes"] // row) // 16) and p["row_groups"] == p["rows_per_warp"]
+
+
+def test_the_build_description_names_every_source():
+    with open(os.path.join(os.path.dirname(CSRC), "build.toml")) as f:
+        named = re.findall(r'"csrc/([^"]+)"', f.read())
+    assert sorted(named) == sorted(os.listdir(CSRC))
