@@ -17,7 +17,7 @@ The line rank 0 prints carries
   roofline      for the kernel with the largest share of the step (NVFP4, M = 16, gate_up), timed live; per_m = the
                 passes; per_config (N = 1) = the single-GPU configurations C0-C3 (NVFP4 4096^2, FP8 28672x8192, MXFP8
                 13824x5120, BF16 8192^2): median / min / max of 7 trials of graph replays over rotating weight copies,
-                against the HBM peak and the FP32-FMA ceiling, each checked against the CPU oracle on sampled rows, with
+                against the HBM peak, each checked against the CPU oracle on sampled rows, with
                 the reference's own sm_100a kernel timed beside it where that comparator was built (gpu_reference_us)
   parity        after the timed region: N > 1: every rank recomputes the last layer's four projections from the whole
                 matrices on its own GPU and compares them bit for bit with what the sharded pass gathered; N = 1: the
@@ -45,7 +45,6 @@ import torch  # noqa: E402
 STACK_MS = (1, 8, 16)
 METRIC = "decode_gemv_weight_stream"
 UNIT = "TB/s"
-FMA_PER_CLK = 148 * 128
 # single-GPU configurations: id, format, N, K, row counts timed here (the tests sweep every M)
 CONFIGS = (("C0", "nvfp4", 4096, 4096, (1,)),
            ("C1", "fp8", 28672, 8192, (1, 2, 4, 8, 16)),
@@ -423,7 +422,7 @@ def make_copies(fmt, n, k, dev, copies):
     return out
 
 
-def run_configs(dev, hbm_gbs, sm_mhz):
+def run_configs(dev, hbm_gbs):
     """C0-C3 on one GPU: per (configuration, M) the time of a call (graph replays over rotating weight copies larger
     than L2 in total), the same for the reference's sm_100a kernel when oracle/_ref holds it, and an oracle check."""
     import crit_kernels_b200
@@ -496,7 +495,6 @@ def run_configs(dev, hbm_gbs, sm_mhz):
                      "us_max": t_ours["us_max"], "trials": TRIALS, "ms_per_trial": t_ours["ms_per_trial"],
                      "weight_bytes": nbytes, "copies_in_rotation": copies,
                      "GBps": nbytes / t_ours["us"] / 1e3, "frac_hbm": nbytes / t_ours["us"] / 1e3 / hbm_gbs,
-                     "frac_fp32_fma": m * n * k / (t_ours["us"] * 1e-6) / (FMA_PER_CLK * sm_mhz * 1e6),
                      "oracle_max_rel_err": err, "gpu_reference_us": None, "speedup_vs_gpu_reference": None}
             if ref is not None:
                 g = graph_of(many(theirs), dev)
@@ -638,7 +636,6 @@ def main():
     hbm_gbs, peak_kind = measured_peaks()
 
     r = run_stack(args, dev, rank, world)
-    sm_mhz = r["clocks"]["sm_mhz"] or 1965.0
     detail = []
     for m, t in zip(STACK_MS, r["per_m"]):
         gbs = r["pass_bytes"] / (t["us"] * 1e-6) / 1e9
@@ -653,9 +650,8 @@ def main():
                 "traffic": ncu_traffic(f"nvfp4:16:{n_top}:8192"), "peak_kind": peak_kind,
                 "us": top_us, "us_minmax": [r["top_kernel"]["us_min"], r["top_kernel"]["us_max"]],
                 "algorithmic_bytes": r["top_bytes"],
-                "frac_fp32_fma_ceiling": 16 * n_top * 8192 / (top_us * 1e-6) / (FMA_PER_CLK * sm_mhz * 1e6),
-                "note": "M = 16 on CUDA cores is bound by FP32 FMA issue, not HBM (16 FMAs per 4-bit weight): the FMA "
-                        "floor of this call is 16 N K / (148 x 128 x clock)",
+                "note": "the weights are decoded in registers for mma.sync: neither HBM nor the tensor pipe is saturated "
+                        "(profiles/gemv_tensor_cores.md)",
                 "per_m": detail}
     model, runs = r.pop("model"), r.pop("runs")
     per_config, host_us = None, None
@@ -667,7 +663,7 @@ def main():
         torch.cuda.empty_cache()
         host_us = host_cost(dev)
         if not args.no_configs:
-            per_config = run_configs(dev, hbm_gbs, sm_mhz)
+            per_config = run_configs(dev, hbm_gbs)
             roofline["per_config"] = per_config
     if rank != 0:
         if world > 1:

@@ -156,7 +156,8 @@ constexpr FormatInfo kFormats[4] = {info_of<0>(), info_of<1>(), info_of<2>(), in
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Bytes of the activations kept resident: whole steps of [M][x_row bytes], and 16-byte padding.
+// Bytes kept behind the ring for resident activations: whole steps of [M][x_row bytes], and a byte per step, in sixteens, which
+// nothing uses (the exponents lie in static shared memory); it stays in the plans that callers know.
 int resident_bytes_of(int fmt, int M, int nblk) {
   const int row_steps = ceil_div(nblk * 16, kFormats[fmt].step);
   return row_steps * M * kFormats[fmt].x_row + ((row_steps + 15) & ~15);
@@ -335,8 +336,8 @@ bool fill_nvfp4(Params& p, const void* x, int ldx, int x_is_bf16, const uint8_t*
   p.N = N; p.K = K;
   p.scale_row_bytes = K / 16;
   p.ct = blocked ? (K / 16 + 3) / 4 : 0;
-  // Scale rows travel by bulk copy when every window of every row starts on 16 bytes and is a multiple of 16 bytes
-  // long (K a multiple of 256, base on 16 bytes); otherwise, and for the tiled layout, lanes read them directly.
+  // Scale rows travel by tensor copy when every window of every row starts on 16 bytes and is a multiple of 16 bytes
+  // long (K a multiple of 256, base on 16 bytes); otherwise, and for the tiled layout, two warps copy them into the stage.
   p.scale_mode = blocked ? dg::SCALES_BLOCKED
                          : (K % 256 == 0 && aligned(scales, 16)) ? dg::SCALES_STAGED : dg::SCALES_DIRECT;
   return true;

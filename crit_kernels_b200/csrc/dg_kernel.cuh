@@ -104,7 +104,7 @@ __host__ __device__ constexpr int x_offset(int before) { return ((before + kSmem
 // window of them into every ring stage: one tensor copy brings them, and the consumer warps put them into the form the
 // tensor cores take (see prepare_resident) while the first weights are on their way.
 __host__ __device__ constexpr bool resident_capable(int fmt, int m) { return (fmt == FMT_FP8 || fmt == FMT_NVFP4) && m <= 4; }
-constexpr int kResidentLimit = 96 * 1024;   // bytes of activations (and padding) a kernel keeps resident at most
+constexpr int kResidentLimit = 96 * 1024;   // bytes behind the ring that resident activations take at most
 // The exponents of resident BF16 activations (see prepare_resident): a byte per consumer warp, step and row.
 constexpr int kResidentExps = kResidentLimit / Format<FMT_FP8>::XROW * kConsumers;
 static_assert(kResidentExps + (kMaxStages + 1) * 8 <= kStaticSmem, "static shared memory");
@@ -363,8 +363,12 @@ __device__ __forceinline__ void start_activations(const Params& p, const Params&
   }
 }
 
-// The ring's first filling is paced, at a rate of all SMs together somewhat above HBM's: asked for all at once, the first
-// windows came as late as the last, up to 3 us later on some SMs than on others (8192 x 8192 NVFP4, one row: 12.4 us, now 12.0).
+// The ring's first filling is paced: asked for all at once, the first windows came as late as the last, up to 3 us later on some
+// SMs than on others. 22 bytes per clock and SM are 6.4 TB/s from 148 SMs at 1965 MHz, just under what HBM gives (6.55); fewer SMs
+// or a lower clock ask for less, and so do weights that lie in L2, for the first filling only. Measured at 1965 MHz, us with 19 /
+// 22 / 26 bytes and without pacing: NVFP4 10240 x 8192, one row 13.6 / 13.8 / 14.2 / 14.2, 8192 x 8192, 8 rows 12.7 / 12.6 / 12.2 /
+// 12.5; FP8 4096 x 4096, one row 5.62 / 5.74 / 5.87 / 5.88, 8 rows 7.1 / 6.6 / 6.2 / 6.7, 4096 x 14336, one row 13.5 / 13.0 / 12.5 /
+// 12.6; BF16 4096 x 2048, one row 5.24 / 5.27 / 5.39 / 5.45, 8 rows 5.87 / 5.51 / 5.20 / 5.49: few rows like it slower, many faster.
 constexpr int kUnpaced = 32 * 1024, kPace = 22;   // bytes at once, bytes per clock
 
 // The feeding warp: weight (and staged scale) copies of every window of one GEMV, in order, and the activations' tensor

@@ -61,7 +61,7 @@ __device__ __forceinline__ float e4m3_value(uint32_t byte) {
 //
 // x / d, correctly rounded, for many x over one d whose quotients stay within FP32's normal range (SAFE): with
 // r = RN(1 / d) computed once, q0 = RN(x r), the exact residual e = x - d q0 (one FMA) and q = RN(q0 + e r) give the
-// IEEE quotient: the tail of the usual division sequence without its per-element reciprocal refinement. A zero
+// IEEE quotient (P. Markstein, Computation of elementary functions on the IBM RISC System/6000, 1990). A zero
 // quotient keeps its own sign where that matters (KEEP_ZERO: the correction would turn -0 into +0). Quotients too
 // small for an exact residual convert to zero whatever their last bits are. Otherwise the full division runs.
 template <bool SAFE, bool KEEP_ZERO>

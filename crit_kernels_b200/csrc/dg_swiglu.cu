@@ -1,8 +1,8 @@
 // SwiGLU between the gate_up and down projections: out[row][k] = silu(gate_up[row][k]) * gate_up[row][inter + k], FP32
 // arithmetic as the reference declares it (dg_swiglu.cuh; int-block-experts/int_block_cuda/int_block.cu:275-282 and its
 // entry point :326-331), inputs and outputs FP32 or BF16 (one rounding to BF16 where the output is the next GEMV's
-// activations). One thread eight values where rows are 16-byte aligned, else one. The NVFP4 GEMV can also form these
-// activations itself while it stages them (dg_enqueue_nvfp4_swiglu), which this kernel serves as the unfused form of.
+// activations). One thread eight values where rows are 16-byte aligned, else one. The gate_up GEMV can also form
+// these activations in its epilogue (dg_enqueue_nvfp4_gate_up_swiglu), which this kernel is the unfused form of.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

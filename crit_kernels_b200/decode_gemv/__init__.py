@@ -1,7 +1,7 @@
 """Weight-only decode projections for B200: y = x W^T for 1 to 16 activation rows x (BF16 or FP16) and a weight matrix
 W kept in its checkpoint format: NVFP4 (4-bit E2M1 codes with an E4M3 scale per 16 inputs), FP8 E4M3 with one FP32
 scale per output channel, MXFP8 (E4M3 with a power-of-two E8M0 scale per 32 inputs) or plain BF16. The products are
-summed in FP32 on CUDA cores in an order that depends only on K and the format, so an output row has the same bits
+made on the tensor cores and summed in FP32 in an order that depends only on K and the format, so an output row has the same bits
 whether it is computed alone, among other rows, or from a slice of W's rows on another GPU.
 
 This module is what `get_kernel("crit-labs/decode-gemv")` hands out: `gemv`, `gemv_fp8`, `gemv_bf16`,

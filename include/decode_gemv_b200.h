@@ -120,8 +120,8 @@ DG_API int dg_enqueue_swiglu(const void* gate_up, long long ldg, int in_is_f32, 
 /* The gate_up projection with SwiGLU in its epilogue: the NVFP4 matrix holds 2 I rows, gate rows [0, I) and up rows
  * [I, 2 I) (codes [2 I][K / 2], scales, inverse [2 I] as dg_enqueue_nvfp4), and out [M][ldo] receives the I activations
  * of the down projection, out[m][k] = silu(g) * u with g, u the two finished FP32 sums times their inverse scales, in the
- * arithmetic of dg_enqueue_swiglu, rounded once to out's type (out_kind 0 FP32, 1 x's type). A warp holds row k of both
- * halves side by side, so nothing but the activations is written: no [M][2 I] intermediate, no second launch. The bits
+ * arithmetic of dg_enqueue_swiglu, rounded once to out's type (out_kind 0 FP32, 1 x's type). A tile holds row k of both
+ * halves, so nothing but the activations is written: no [M][2 I] intermediate, no second launch. The bits
  * are those of dg_enqueue_nvfp4 with FP32 output followed by dg_enqueue_swiglu. No counterpart in the reference (it
  * runs the steps as separate kernels: int_block.cu:275-282 is its SwiGLU). */
 DG_API int dg_enqueue_nvfp4_gate_up_swiglu(const void* x, int ldx, int x_is_bf16, const uint8_t* codes,

@@ -1,7 +1,7 @@
 """The GEMV kernels at the edges of their tiles and dispatch rules, against the CPU oracle's exact products: shares of a CTA of
 one tile and of several, windows that end with the row and short of it, activations that no tensor copy can bring (K no
-multiple of 64), gathered scales, and chunks with activations outside the range that FP16 holds after scaling (above 2^8,
-below 2^-24), which are multiplied after the tile. Every row's bits are those it has alone."""
+multiple of 64), gathered scales, and chunks with activations outside the range that FP16 holds after the usual
+scaling (above 2^8, below 2^-24). Every row's bits are those it has alone."""
 import pytest
 import torch
 
