@@ -863,13 +863,20 @@ __device__ __forceinline__ void load_rows(RawRows<FMT>& raw, uint32_t wrow, uint
 // columns 32 (u % 2) + lane (SwiGLU tiles have no more than 32), activation rows from 4 (u / 2) (SwiGLU: 4 u) on.
 __device__ __forceinline__ int finish_units(const Params& p, const Walk& wk) { return (p.M + 3) / 4 * (wk.pairs ? 1 : 2); }
 __device__ __forceinline__ int unit_column(const Walk& wk, int u) { return (threadIdx.x & 31) + (wk.pairs ? 0 : 32 * (u & 1)); }
+// (Behind the wait for the previous kernel, as it is written: a load that the compiler places cost the resident kernels up to 5 %,
+// 28672 x 8192 NVFP4 with four rows 35.6 and 34.8 us.)
+__device__ __forceinline__ float load_f32(const float* at) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(at));
+  return v;
+}
 // Scale of the lane's column (SwiGLU: of its gate and up row).
 __device__ __forceinline__ void finish_scales(const Params& p, const Walk& wk, int col0, int cols, int u, float (&f)[2]) {
   const int c = unit_column(wk, u);
   f[0] = f[1] = 1.f;
   if (p.row_scale && c < cols) {
-    f[0] = p.row_scale[col0 + c];
-    if (wk.pairs) f[1] = p.row_scale[wk.pairs + col0 + c];
+    f[0] = load_f32(p.row_scale + col0 + c);
+    if (wk.pairs) f[1] = load_f32(p.row_scale + wk.pairs + col0 + c);
   }
 }
 template <int FMT, int STEPS>
