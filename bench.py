@@ -650,8 +650,7 @@ def main():
                 "traffic": ncu_traffic(f"nvfp4:16:{n_top}:8192"), "peak_kind": peak_kind,
                 "us": top_us, "us_minmax": [r["top_kernel"]["us_min"], r["top_kernel"]["us_max"]],
                 "algorithmic_bytes": r["top_bytes"],
-                "note": "the weights are decoded in registers for mma.sync: neither HBM nor the tensor pipe is saturated "
-                        "(profiles/gemv_tensor_cores.md)",
+                "note": "the weights are decoded in registers for mma.sync: neither HBM nor the tensor pipe is saturated",
                 "per_m": detail}
     model, runs = r.pop("model"), r.pop("runs")
     per_config, host_us = None, None
