@@ -919,18 +919,19 @@ __device__ __forceinline__ void finish_unit(const Params& p, const Walk& wk, uin
 
 enum : int { RES_NONE = 0, RES_USUAL = 1, RES_MIXED = 2 };
 // Where chunks with values outside the usual window are multiplied: nowhere (there are none); in kernels for up to four rows by
-// the usual chunks' code, which then has the columns' powers of two in registers; from five rows up in code of its own (with
-// the powers in registers for every chunk, 28672 x 8192 NVFP4 with 8 rows took 38.4 us, without 37.4; but the code of its own is
-// one more thing to fetch, which a launch for few rows pays for with a single such chunk: 4096 x 4096, one row, 7.1 and 6.4 us).
-// NVFP4 28672 x 8192 at 1 / 8 / 16 rows, us: N(0, 1) activations 31.0 / 37.4 / 53.5, one value of 300 in each row 33.2 / 38.1 /
-// 54.9, all above 2^8 36.1 / 45.8 / 68, chunks over more than 32 binades 56 / 55 / 74. (As passes after the tile, from global
+// the usual chunks' code, which then has the columns' powers of two in registers; from five rows up, and in batched kernels unless
+// the activations are resident, in code of its own (with the powers in registers for every chunk, 28672 x 8192 NVFP4 with 8 rows
+// took 38.4 us, without 37.4, a batched pass over 32 GEMVs at one row 849, without 831; but the code of its own is one more thing
+// to fetch, which a launch for few rows pays for with a single such chunk: 4096 x 4096, one row, 7.1 and 6.4 us).
+// NVFP4 28672 x 8192 at 1 / 8 / 16 rows, us: N(0, 1) activations 31.1 / 37.6 / 53.4, one value of 300 in each row 33.2 / 38.5 /
+// 54.3, all above 2^8 36.5 / 45.0 / 67.3, chunks over more than 32 binades 56.6 / 64.9 / 80.8. (As passes after the tile, from global
 // memory, they took 68 / 72 / 117, 320 / 316 / 645 and 949 / 1087 / 2158.)
 enum : int { ODD_NONE = 0, ODD_SHARED = 1, ODD_APART = 2 };
 // One tile of up to 8 EIGHTS rows: the windows in turn; at the end the warp leaves its sums in the stage it has just consumed,
 // in its own chunk of each row (which no other warp reads), one FP32 per activation row, and tells the finishing warps, to
 // which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the
 // activations are resident (RES_MIXED: `spread` has the steps, modulo 32, with chunks of another exponent than the usual one).
-template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool CAN_RES, int RES>
+template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool SHARED, int RES>
 __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, const StageLayout<FMT, STEPS>& lay,
                                              unsigned char* smem, int col0, int cols, bool last, uint32_t spread, const Bars& bars, int& s, uint32_t& parity,
                                              bool first_window, bool& ok) {
@@ -940,7 +941,7 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
   constexpr bool ODD = EIGHTS % 2 != 0;       // the last group has no second half
   // BF16 activations of the formats whose weights become FP16
   constexpr bool CONVERT = FMT != FMT_BF16 && std::is_same<XT, __nv_bfloat16>::value;
-  constexpr int ODDITIES = !CONVERT || RES == RES_USUAL ? ODD_NONE : CAN_RES ? ODD_SHARED : ODD_APART;
+  constexpr int ODDITIES = !CONVERT || RES == RES_USUAL ? ODD_NONE : SHARED || RES == RES_MIXED ? ODD_SHARED : ODD_APART;
   const Lane ln;
   const int M = p.M, stage_bytes = p.stage_bytes, stages = p.stages;
   if (last && p.row_scale && unit_column(wk, ln.warp) < cols) {    // (needed at the tile's end)
@@ -1169,7 +1170,7 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
 
 // The consumer warps' walk over one GEMV, tile by tile. The ring position (s, parity) carries over from one GEMV of a
 // batch to the next; `first`: the kernel's first GEMV.
-template <int FMT, int NT, bool CAN_RES, int STEPS, bool SMALL, typename XT>
+template <int FMT, int NT, bool CAN_RES, int STEPS, bool SMALL, bool BATCH, typename XT>
 __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* smem, const Bars& bars,
                                              int& s, uint32_t& parity, uint32_t& x_parity, bool first) {
   const Walk wk(p, STEPS * Format<FMT>::STEP);
@@ -1194,7 +1195,7 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     auto tile = [&](auto res) {
       constexpr int RES = decltype(res)::value;
       auto run = [&](auto e) {
-        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, CAN_RES, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
+        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, CAN_RES && !BATCH, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
                                                                   first && t == 0, ok);
       };
       const int eights = (wk.rows(cols) + 7) / 8;
@@ -1412,7 +1413,7 @@ __global__ void __launch_bounds__(SMALL ? kSmallThreads : kThreads, SMALL ? 2 : 
     if (!SMALL) finish_gemv<FMT, STEPS>(p, smem, bars, warp - kFinisher, copies ? 1 : kFinishers, s, parity);
     if (p.world >= 1) finished_barrier();
   } else {
-    consume_gemv<FMT, NT, CAN_RES, STEPS, SMALL, XT>(p, smem, bars, s, parity, x_parity, true);
+    consume_gemv<FMT, NT, CAN_RES, STEPS, SMALL, false, XT>(p, smem, bars, s, parity, x_parity, true);
     if ((threadIdx.x & 31) == 0) trace_stamp(p.trace, TRACE_LAST_CONSUMED);
     if (p.world >= 1) {
       gather_copy(p);
@@ -1467,7 +1468,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* _
   } else {
     // (every warp passes every GEMV's barriers, also after a wait that ran out)
     for (int g = 0; g < count; ++g) {
-      consume_gemv<FMT, NT, CAN_RES, STEPS, false, XT>(items[g], smem, bars, s, parity, x_parity, g == 0);
+      consume_gemv<FMT, NT, CAN_RES, STEPS, false, true, XT>(items[g], smem, bars, s, parity, x_parity, g == 0);
       if (items[g].world >= 1) gather_copy(items[g]);   // the CTA's rows of this GEMV go to the peers now
     }
     if ((threadIdx.x & 31) == 0) trace_stamp(items[0].trace, TRACE_LAST_CONSUMED);
