@@ -165,11 +165,16 @@ int resident_bytes_of(int fmt, int M, int nblk) {
 
 // Launch shape: a speed choice from (format, M, N, K, SM count) only; no row's bits depend on it.
 //   CTAs            one per SM, fewer when the matrix has under four rows per SM
-//   tile rows       64 to 40 (less when a CTA's range is shorter): what takes the fewest eighths of 8 rows, a tile
-//                   costing as much as one eighth (its sums) plus, where its activations are converted on the way, as
-//                   much as these cost
+//   tile rows       64 to 40 (less when a CTA's range is shorter): what takes the fewest eighths of 8 rows, a tile costing as much
+//                   as one eighth (its sums) plus, where its activations are converted on the way, as much as these cost
+//                   (57344 x 8192 NVFP4 in tiles of 56 and of 64 rows, both seven: 8 rows 64.8 and 63.8 us, 16 rows 93.3 and 91)
 //   steps           512-byte steps per ring stage (BF16: one of 1 KB): two, one where the ring would have fewer than three
-//                   stages otherwise: a consumer warp's fixed costs per stage then weigh half
+//                   stages otherwise: a consumer warp's fixed costs per stage then weigh half. A CTA's whole range in one tile
+//                   is worth more than two steps (8192 x 8192 NVFP4, 2 / 3 / 4 rows, 56 matrix rows per CTA: tiles of 40 and 16
+//                   in two steps 12.65 / 14.35 / 14.9 us, one tile in one step 11.7 / 12.45 / 13.15; FP8 with 4 rows 17.3 and
+//                   14.8), and from 16 steps of K on two steps are worth more than a third stage where the ring does not have
+//                   to hold a finished tile's sums as well (8192 x 28672 NVFP4, 4 rows: three stages of 40 rows 41.8, two of 56
+//                   31.2; 8 rows: one step 32.6, two 31.7)
 //   stages          as many as fit in shared memory, at most kMaxStages
 // Activations stay resident where that leaves three stages of two steps (from three rows on, where they would take a fifth
 // and more of a stage, also with four stages of one); otherwise a window of them passes through every stage.
@@ -199,8 +204,15 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
   const bool may_reside = allow_resident && dg::resident_capable(fmt, M) && K % 64 == 0 &&
                           resident_bytes <= (grid > 0 ? dg::kResidentLimit / 2 - 15 * 1024 : dg::kResidentLimit) &&
                           (M > 1 || 3 * 56 * (dg::weight_pitch(fmt, 2) + dg::scale_pitch(fmt, 2)) + resident_bytes <= room);
-  int best_cost = 0, best_rem = 0;
+  int best_cost = 0, best_merit = 0;
   p.tile_rows = 0;
+  // whether stages of the range's only tile fit, `need` of them
+  auto one_tile_fits = [&](bool resident, int steps, int need) {
+    if (all_rows > 64 || grid > 0 || force_steps > 0 || p.pairs) return false;
+    int bytes = all_rows * (dg::weight_pitch(fmt, steps) + dg::scale_pitch(fmt, steps));
+    if (!resident) bytes = (dg::x_offset(bytes) + steps * M * f.x_row + 1023) & ~1023;
+    return need * ((bytes + 127) & ~127) <= room - (resident ? resident_bytes : 0);
+  };
   // resident with two steps, with one, not resident with two, with one: the first that has the stages it asks for
   for (int attempt = may_reside ? 0 : 2; attempt < 4 && p.tile_rows == 0; ++attempt) {
     const bool resident = attempt < 2;
@@ -208,8 +220,14 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
     // (a batch's GEMVs share one instance: the same steps for all, whatever their K)
     if (grid > 0 ? steps != (M <= 4 ? 2 : 1) : force_steps > 0 ? steps != std::min(force_steps, row_steps)
                                                                : steps == 2 && row_steps == 1 && fmt != dg::FMT_BF16) continue;
-    const int need = grid > 0 || force_steps > 0 ? 2 : attempt == 0 ? 3 : attempt == 1 ? (M >= 3 ? 4 : dg::kMaxStages + 1)
-                                                     : attempt == 2 ? 3 : 2;
+    int need = grid > 0 || force_steps > 0 ? 2 : attempt == 0 ? 3 : attempt == 1 ? (M >= 3 ? 4 : dg::kMaxStages + 1)
+                                               : attempt == 2 ? 3 : 2;
+    const bool one_step_tile = fmt != dg::FMT_BF16 && one_tile_fits(resident, 1, resident ? 4 : 3);
+    if (steps == 2 && fmt != dg::FMT_BF16 && row_steps > 1 && !one_tile_fits(resident, 2, 3)) {
+      if (!resident && row_steps >= 16 && one_tile_fits(false, 2, 2)) need = 2;
+      else if (one_step_tile) continue;
+    }
+    if (attempt == 1 && one_step_tile) need = 4;
     const int convert = resident || fmt == dg::FMT_BF16 ? 0 : M <= 8 ? 5 : 7;   // of a tile, in halves of a group
     for (int rows = 64; rows >= 40; rows -= 8) {
       int tile_rows = std::min(force_rows >= 16 && force_rows <= 64 ? force_rows & ~7 : rows, all_rows);
@@ -222,11 +240,14 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
       if (stages < need) continue;
       const int cap = tile_rows / regions, tiles = ceil_div(cols_per_cta, cap), rem = cols_per_cta - (tiles - 1) * cap;
       const int eights = (tiles - 1) * tile_rows / 8 + ceil_div((regions - 1) * cap + rem, 8);
+      // of equals the one with the fewest tiles of an odd number of eighths where NVFP4's activations come in windows (their last
+      // group's products are made whole), then the one whose last tile is the fullest: a window of a few rows takes as long as its latency
+      const int odd = resident || fmt != dg::FMT_NVFP4 ? 0 : (tiles - 1) * (tile_rows / 8 & 1) + (ceil_div((regions - 1) * cap + rem, 8) & 1);
+      const int merit = 64 * (64 - std::min(odd, 63)) + rem;
       const int cost = eights + (1 + convert) * tiles;
-      // (of equals the one whose last tile is the fullest: a window of a few rows takes as long as its latency)
-      if (p.tile_rows == 0 || cost < best_cost || (cost == best_cost && rem > best_rem)) {
+      if (p.tile_rows == 0 || cost < best_cost || (cost == best_cost && merit > best_merit)) {
         best_cost = cost;
-        best_rem = rem;
+        best_merit = merit;
         p.tile_rows = tile_rows;
         p.last_rows = ceil_div(rem, dg::kBoxRows) * dg::kBoxRows;
         p.steps = steps;
@@ -320,7 +341,12 @@ int launch(int table, int fmt, Params& p, int M, cudaStream_t stream) {
       p.trace = base + (size_t)index * DG_TRACE_CTAS * dg::kTraceSlots;
   }
   void* args[] = {&p};
-  return launch_pdl(kTables[table][p.steps - 1 + 2 * p.small][M - 1], args, ctas, p.small ? dg::kSmallThreads : dg::kThreads, smem,
+  // Up to four rows whose activations come in windows run the kernel for five to eight, the bits being the same: its code for such
+  // windows is the better one (NVFP4 8192 x 28672, one row 32.5 us in the kernel for up to four and 30.5 in this one, 2731 x 5152 7.72
+  // and 7.09), but for copied windows in more than one tile per CTA (9000 x 8224, one row 16.3 and 16.45).
+  const bool windows = p.x_mode == dg::X_TENSOR || (p.x_mode == dg::X_COPIED && ceil_div(p.N, ctas) <= p.tile_rows);
+  const int rows = windows ? std::max(M, 5) : M;
+  return launch_pdl(kTables[table][p.steps - 1 + 2 * p.small][rows - 1], args, ctas, p.small ? dg::kSmallThreads : dg::kThreads, smem,
                     stream);
 }
 
