@@ -252,13 +252,11 @@ __global__ void __launch_bounds__(kRowThreads) fp8_rows_kernel(const __nv_bfloat
     quantize_row<false>(xr, reinterpret_cast<const uint4*>(row_smem), qr, K, sc, staged, aligned_in, vector_out, tid);
 }
 
-// Two quotients -> two E2M1 codes in one byte (low nibble = lo). v + 0 turns a negative zero into +0 (code 0, as a
-// comparison with zero sees it); every other negative quotient keeps its sign bit, also when it rounds to zero.
+// Two quotients -> two E2M1 codes in one byte (low nibble = lo): every negative quotient's sign bit is set, also when it rounds to
+// zero, and a negative zero's.
 __device__ __forceinline__ uint32_t e2m1x2(float lo, float hi) {
   uint16_t r;
-  asm("{\n\t.reg .b8 t;\n\tcvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\n\tcvt.u16.u8 %0, t;\n\t}"
-      : "=h"(r)
-      : "f"(hi + 0.0f), "f"(lo + 0.0f));
+  asm("{\n\t.reg .b8 t;\n\tcvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\n\tcvt.u16.u8 %0, t;\n\t}" : "=h"(r) : "f"(hi), "f"(lo));
   return r;
 }
 
@@ -280,8 +278,41 @@ __device__ __forceinline__ pair fma2(pair a, pair b, pair c) {
   return r;
 }
 
+// A launch has at most 127 scales (an input scale times an E4M3 value each): their d and 1 / d, worked out once per CTA. d = 0: all
+// codes are 0 (e4m3(s) is not > 0).
+struct Scale { float d, r; };
+__device__ __forceinline__ Scale scale_of(uint32_t byte, float g_rcp) {
+  float d = e4m3_value(byte) * g_rcp;
+  if (!(d > 0.f)) return {0.f, 0.f};
+  d = d < 1e-30f ? 1e-30f : d;
+  return {d, __frcp_rn(d)};
+}
+
+// Codes of 8 BF16 pairs. SHORT: no quotient can leave FP32's range, so they take the short division, two values at once. ZEROS: a
+// negative zero quotient becomes +0 first (code 0, as a comparison with zero sees it). The short division does that by
+// itself where no quotient underflows: the residual of -0 is +0, and so is its sum with it.
+template <bool SHORT, bool ZEROS>
+__device__ __forceinline__ void codes16(const uint32_t (&w)[8], const Scale& sc, uint32_t& lo, uint32_t& hi) {
+  uint32_t byte[8];
+  const pair r2 = pack(sc.r, sc.r), d2 = pack(-sc.d, -sc.d);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float a, b;
+    if constexpr (SHORT) {
+      const pair x = pack(bf16_lo(w[i]), bf16_hi(w[i])), q0 = mul2(x, r2), q1 = fma2(fma2(d2, q0, x), r2, q0);
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(q1.v));
+    } else {
+      a = __fdiv_rn(bf16_lo(w[i]), sc.d);
+      b = __fdiv_rn(bf16_hi(w[i]), sc.d);
+    }
+    byte[i] = ZEROS ? e2m1x2(a + 0.f, b + 0.f) : e2m1x2(a, b);
+  }
+  lo = __byte_perm(__byte_perm(byte[0], byte[1], 0x0040), __byte_perm(byte[2], byte[3], 0x0040), 0x5410);
+  hi = __byte_perm(__byte_perm(byte[4], byte[5], 0x0040), __byte_perm(byte[6], byte[7], 0x0040), 0x5410);
+}
+
 // 16 values (8 BF16 pairs) -> scale byte (returned) and 8 code bytes (lo, hi).
-__device__ __forceinline__ uint32_t nvfp4_block(const uint32_t (&w)[8], float g, float g_rcp, uint32_t& lo, uint32_t& hi) {
+__device__ __forceinline__ uint32_t nvfp4_block(const uint32_t (&w)[8], float g, const Scale* scales, uint32_t& lo, uint32_t& hi) {
   uint32_t m = 0u;
 #pragma unroll
   for (int i = 0; i < 8; ++i) m = amax2(w[i], m);
@@ -289,30 +320,13 @@ __device__ __forceinline__ uint32_t nvfp4_block(const uint32_t (&w)[8], float g,
   float bs = (amax * kRcp6) * g;
   bs = bs > 448.f ? 448.f : bs;
   const uint32_t sbits = e4m3x2(bs, 0.f) & 0xffu;
-  float d = e4m3_value(sbits) * g_rcp;
-  const bool zero = !(d > 0.f);
-  d = d < 1e-30f ? 1e-30f : d;
+  const Scale sc = scales[sbits & 0x7fu];
   lo = hi = 0u;
-  if (zero) return sbits;
-  uint32_t byte[8];
-  // a block whose quotients cannot leave FP32's range takes the short division, two values at once (a zero quotient's sign
-  // is dropped by the conversion's + 0 anyway); the rest (values near FP32's limits) the full one
-  if (amax < 1e8f) {
-    const float r = __frcp_rn(d);
-    const pair r2 = pack(r, r), d2 = pack(-d, -d);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const pair x = pack(bf16_lo(w[i]), bf16_hi(w[i])), q0 = mul2(x, r2), q1 = fma2(fma2(d2, q0, x), r2, q0);
-      float a, b;
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(q1.v));
-      byte[i] = e2m1x2(a, b);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) byte[i] = e2m1x2(__fdiv_rn(bf16_lo(w[i]), d), __fdiv_rn(bf16_hi(w[i]), d));
-  }
-  lo = __byte_perm(__byte_perm(byte[0], byte[1], 0x0040), __byte_perm(byte[2], byte[3], 0x0040), 0x5410);
-  hi = __byte_perm(__byte_perm(byte[4], byte[5], 0x0040), __byte_perm(byte[6], byte[7], 0x0040), 0x5410);
+  if (sc.d == 0.f) return sbits;
+  // Below 1e8 no quotient leaves FP32's range; BF16's smallest value, 2^-133, over less than 2^17 is not yet rounded to zero.
+  if (amax < 1e8f && sc.d < 131072.f) codes16<true, false>(w, sc, lo, hi);
+  else if (amax < 1e8f) codes16<true, true>(w, sc, lo, hi);
+  else codes16<false, true>(w, sc, lo, hi);
   return sbits;
 }
 
@@ -320,18 +334,22 @@ __device__ __forceinline__ uint32_t nvfp4_block(const uint32_t (&w)[8], float g,
 // and 96 + 8 i + w (i: which quarter), whose scale words lie side by side in the tiled layout. A lane takes one block of a
 // row: a warp reads 1024 and writes 256 consecutive bytes at a time, two rows' loads in flight at once, and the scale bytes
 // meet in shared memory and leave as 128 consecutive bytes per tile. (With four blocks to a thread a warp's load touched 32
-// lines.) The arithmetic bounds it, more than the memory: about 100 instructions a block, with the quotients in packed pairs.
-// 4096 x 8192: 22.3 us before, 18.9 now (13.1 at copy bandwidth); 16 x 28672: 5.0 and 1.9.
+// lines.) The arithmetic bounds it, more than the memory (an integer or conversion instruction takes a scheduler two clocks):
+// the quotients are in packed pairs and the scales' reciprocals in a table. 4096 x 8192: 22.3 us with four blocks to a thread, 18.6
+// without the table and with a + 0 for every quotient, 17.0 now (13.1 at copy bandwidth, 0.77 of it); 512 x 4096: 4.2 and 3.2; 16 x 28672: 5.0,
+// 1.95 and 1.8. Five CTAs per SM (48 registers): 16.3, but 1024 x 8192 7.2 instead of 6.5.
 constexpr int kQuantCols = 512, kQuantRows = 32;
 __global__ void __launch_bounds__(256) nvfp4_kernel(const __nv_bfloat16* x, long long ldx, int M, int K,
                                                     float g, float g_rcp, uint8_t* __restrict__ codes,
                                                     uint8_t* __restrict__ scales, int quads, int col_tiles, int wide_scales) {
   __shared__ __align__(16) unsigned char tile[kQuantCols / 64 * 128];   // [quad][row % 8][row / 32][block % 4]
+  __shared__ Scale known[128];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row_block = blockIdx.x / col_tiles, col_tile = blockIdx.x - row_block * col_tiles;
   const int tile_row = row_block >> 2, eight = row_block & 3;
   const int row0 = tile_row * 128 + eight * 8 + warp, k = col_tile * kQuantCols + lane * 16;
   if (tid < kQuantCols / 64 * 8) reinterpret_cast<uint4*>(tile)[tid] = make_uint4(0u, 0u, 0u, 0u);   // padding rows and blocks
+  if (tid >= 128) known[tid - 128] = scale_of((uint32_t)tid - 128u, g_rcp);
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   uint4 v[4][2];
@@ -350,7 +368,7 @@ __global__ void __launch_bounds__(256) nvfp4_kernel(const __nv_bfloat16* x, long
     if (row < M && k < K) {
       const uint32_t w[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
       uint32_t lo, hi;
-      const uint32_t scale = nvfp4_block(w, g, g_rcp, lo, hi);
+      const uint32_t scale = nvfp4_block(w, g, known, lo, hi);
       *reinterpret_cast<uint2*>(codes + (size_t)row * (K >> 1) + (k >> 1)) = make_uint2(lo, hi);
       tile[(lane >> 2) * 128 + warp * 16 + i * 4 + (lane & 3)] = (unsigned char)scale;
     }

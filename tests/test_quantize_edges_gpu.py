@@ -54,3 +54,25 @@ def test_nvfp4_at_the_edges_of_its_tiles(m, k, offset):
     assert np.array_equal(codes.cpu().numpy(), want_codes)
     assert np.array_equal(scales.cpu().numpy(), want_blocked)
     assert bool((buffer[:offset] == 0x55).all())
+
+
+@pytest.mark.parametrize("large", [7.6e5, 8.1e5, 9.9e7, 1.01e8, 3e38])        # about scales of 2^17 and values of 1e8 the division changes its way
+@pytest.mark.parametrize("input_scale", [2688.0 / 8.0, 2e-5, 1e25])
+def test_nvfp4_blocks_of_tiny_values_beside_large_ones(large, input_scale):
+    """Quotients that FP32 rounds to zero, negative ones and negative zeros among them, beside a block's largest value."""
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(40, 1024, generator=g) * torch.exp2(torch.randint(-149, -80, (40, 1024), generator=g).float())
+    x[:, 3::16] = -0.0
+    x[::2, 7::16] = large
+    x[1::4, 9::16] = -large * torch.rand(10, 64, generator=g)
+    x = x.to(torch.bfloat16)
+    codes = torch.full((40, 512), 0x55, dtype=torch.uint8, device="cuda")
+    scales = torch.full((oc.blocked_numel(40, 1024),), 0x55, dtype=torch.uint8, device="cuda")
+    s, r = np.float32(input_scale), np.float32(1.0) / np.float32(input_scale)
+    xd = x.cuda()
+    assert cabi.load().dg_enqueue_quantize_nvfp4(_ptr(xd), 1024, 40, 1024, ctypes.c_float(s), ctypes.c_float(r), _ptr(codes),
+                                                 _ptr(scales), None) == 0
+    torch.cuda.synchronize()
+    want_codes, want_blocked = qo.nvfp4_blocked(x, input_scale)
+    assert np.array_equal(codes.cpu().numpy(), want_codes)
+    assert np.array_equal(scales.cpu().numpy(), want_blocked)
