@@ -33,3 +33,29 @@ def test_runs_that_cross_rows(n, k, dtype):
 def test_matrices_around_one_run_per_sm(n, k, dtype):
     """Below 1024 output vectors per SM a CTA takes 256 of them."""
     test_runs_that_cross_rows(n, k, dtype)
+
+
+@pytest.mark.parametrize("n,k", [(40, 1024), (1500, 2048)])             # in one launch the other way of the two
+def test_a_chain_of_calls_reads_what_the_one_before_wrote(n, k):
+    """The kernels start before the previous one of the stream has finished."""
+    import crit_kernels_b200
+    kernel = crit_kernels_b200.get_kernel("crit-labs/decode-gemv", version=1)
+    mats = [tuple(t.cuda() for t in wl.cfg_nvfp4(n, k, seed=s)) for s in range(2)]
+    want = []
+    for m in mats:
+        w = kernel.decode(*m, torch.empty(n, k, dtype=torch.bfloat16, device="cuda"))
+        torch.cuda.synchronize()
+        q, scale = kernel.quantize_fp8_rows(w, torch.empty(n, k, dtype=torch.uint8, device="cuda"), torch.empty(n, device="cuda"))
+        torch.cuda.synchronize()
+        want.append((w, q, scale))
+    now = tuple(torch.empty_like(t) for t in mats[0])
+    got = [tuple(torch.zeros_like(t) for t in want[0]) for _ in range(12)]
+    for i, (w, q, scale) in enumerate(got):
+        for t, source in zip(now, mats[i % 2]):
+            t.copy_(source)
+        kernel.decode(*now, w)
+        kernel.quantize_fp8_rows(w, q, scale)
+        kernel.decode(*mats[(i + 1) % 2], w)                            # may not overtake the call that reads w
+    torch.cuda.synchronize()
+    for i, (w, q, scale) in enumerate(got):
+        assert torch.equal(w, want[(i + 1) % 2][0]) and torch.equal(q, want[i % 2][1]) and torch.equal(scale, want[i % 2][2])
