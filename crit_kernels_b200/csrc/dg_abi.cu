@@ -201,7 +201,13 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
   // (a batch shares one ring and one resident area between GEMVs of different K: only the smaller ones stay resident)
   // (one row's activations are a thirtieth of a stage: not worth a lower tile)
   const int room = dg::kSmemLimit - dg::kSmemHeader;
-  const bool may_reside = allow_resident && dg::resident_capable(fmt, M) && K % 64 == 0 &&
+  // Where a CTA's range is short, bringing and converting all activations before its first product takes longer than windows (us
+  // resident and in windows: NVFP4 600 x 8192 with 4 rows 7.7 and 6.4, 3 rows 7.1 and 6.2, 2 rows 6.2 and 6.1, one 5.35 and 6.1; 4096 x 8192, 28
+  // matrix rows per CTA, 4 rows 9.8 and 8.65, one 7.8 and 8.4; 1152 x 2048 with 1 / 4 rows 3.55 / 3.9 and 3.3 / 3.4; FP8 4096 x 4096 with
+  // 3 / 4 rows 6.4 / 6.5 and 6.3 / 6.3, 2368 x 8192 with 4 rows 8.1 and 8.5).
+  const bool short_range = grid == 0 && ((all_rows <= 48 && M >= 4) || (all_rows <= 32 && M == 3)) && (fmt == dg::FMT_NVFP4 || row_steps <= 8);
+  const bool shortest = grid == 0 && fmt == dg::FMT_NVFP4 && all_rows * row_steps <= 32;
+  const bool may_reside = !short_range && !shortest && allow_resident && dg::resident_capable(fmt, M) && K % 64 == 0 &&
                           resident_bytes <= (grid > 0 ? dg::kResidentLimit / 2 - 15 * 1024 : dg::kResidentLimit) &&
                           (M > 1 || 3 * 56 * (dg::weight_pitch(fmt, 2) + dg::scale_pitch(fmt, 2)) + resident_bytes <= room);
   int best_cost = 0, best_merit = 0;
@@ -259,7 +265,8 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
   }
   if (p.tile_rows == 0) return false;
   // Small launches: a stage for every window, in half of the shared memory, so that the next launch's CTA fits beside.
-  if (grid == 0 && dg::small_capable(fmt, M) && all_rows <= dg::kSmallRows && K % 64 == 0 && p.scale_mode != dg::SCALES_DIRECT &&
+  if (grid == 0 && dg::small_capable(M) && all_rows <= dg::kSmallRows &&
+      (fmt != dg::FMT_NVFP4 || (all_rows * row_steps <= dg::kSmallNvfp4 && !p.pairs)) && K % 64 == 0 && p.scale_mode != dg::SCALES_DIRECT &&
       p.scale_mode != dg::SCALES_BLOCKED && force_steps == 0) {
     const int steps = fmt == dg::FMT_BF16 || row_steps == 1 ? 1 : 2, windows = std::max(2, ceil_div(row_steps, steps));
     const int rows = regions * ceil_div(all_rows / regions, dg::kBoxRows) * dg::kBoxRows;

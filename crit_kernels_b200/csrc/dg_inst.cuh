@@ -10,8 +10,8 @@
   reinterpret_cast<const void*>(                                                                                                 \
       &dg::gemv_kernel<FMT, NT, dg::resident_capable(FMT, M), (FMT) == dg::FMT_BF16 ? 1 : STEPS, SMALL, XT>)
 #define DG_STEPS(FMT, STEPS, SMALL, XT)                                                                                          \
-  DG_ROWS(DG_K(FMT, 1, 1, STEPS, dg::small_capable(FMT, 1) && SMALL, XT),                                                        \
-          DG_K(FMT, 1, 5, STEPS, dg::small_capable(FMT, 5) && SMALL, XT), DG_K(FMT, 2, 9, STEPS, false, XT))
+  DG_ROWS(DG_K(FMT, 1, 1, STEPS, dg::small_capable(1) && SMALL, XT),                                                        \
+          DG_K(FMT, 1, 5, STEPS, dg::small_capable(5) && SMALL, XT), DG_K(FMT, 2, 9, STEPS, false, XT))
 #define DG_TABLE(NAME, FMT, XT)                                                                                                  \
   const void* const NAME[4][16] = {DG_STEPS(FMT, 1, false, XT), DG_STEPS(FMT, 2, false, XT), DG_STEPS(FMT, 1, true, XT),         \
                                    DG_STEPS(FMT, 2, true, XT)};

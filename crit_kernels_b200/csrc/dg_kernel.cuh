@@ -50,8 +50,12 @@ constexpr int kThreads = 32 * (kConsumers + 1 + kFinishers);
 // two fit on an SM: the next launch of the stream then waits there for this one to finish, its barriers set up and its weights
 // on their way into L2.
 constexpr int kSmallThreads = 32 * (kConsumers + 2), kSmallRows = 32;
-// (NVFP4's decoding does not fit their 96 registers: 4096 x 4096 at one row took 6.3 us with them, 5.5 without.)
-__host__ __device__ constexpr bool small_capable(int fmt, int m) { return fmt != FMT_NVFP4 && m <= 8; }
+// NVFP4's decoding spills some of their 96 registers, so that only what is very short, in matrix rows times steps of a CTA's share,
+// is faster (us without and with, one row / eight: 1024 x 1024 3.68 / 3.48 and 3.35 / 2.95, 4700 x 1024 3.9 / 3.9 and 3.5 / 3.3, 1100 x 8192, 64
+// of them, 5.66 / 6.7 and 5.4 / 6.7, 3072 x 3072, 72, 4.84 / 5.29 and 4.51 / 5.31; 4700 x 2560, 96, 5.67 / 5.79 and 5.70 / 5.75, four rows
+// 6.09 and 6.21; 2368 x 8192, 128, 6.09 and 6.48).
+__host__ __device__ constexpr bool small_capable(int m) { return m <= 8; }
+constexpr int kSmallNvfp4 = 72;
 constexpr int kSmallSmem = 111 * 1024;     // dynamic shared memory: 228 KB for two, less 1 KB and the static part each
 constexpr int kBoxRows = 8;                // tile rows come in multiples of these
 constexpr int kGroupRows = 16;             // rows of one mma tile

@@ -15,7 +15,11 @@ MAKE = {"nvfp4": wl.cfg_nvfp4, "fp8": wl.cfg_fp8, "mxfp8": wl.cfg_mxfp8}
 @pytest.mark.parametrize("fmt,n,k", [
     ("nvfp4", 148 * 56, 2048), ("nvfp4", 148 * 64 - 5, 8192), ("nvfp4", 148 * 41, 15360), ("nvfp4", 148 * 56 - 1, 16384),
     ("nvfp4", 1300, 28672), ("nvfp4", 148 * 20, 1056), ("nvfp4", 148 * 70, 1056), ("fp8", 148 * 56, 4096), ("fp8", 148 * 50, 8192),
-    ("fp8", 148 * 20, 528), ("fp8", 148 * 70, 528), ("mxfp8", 148 * 56, 8192)])
+    ("fp8", 148 * 20, 528), ("fp8", 148 * 70, 528), ("mxfp8", 148 * 56, 8192),
+    # small NVFP4 launches (up to 72 matrix rows times steps) and what is just none; ranges in which up to four rows have windows or not
+    ("nvfp4", 1, 64), ("nvfp4", 149, 1024), ("nvfp4", 148 * 8, 4096), ("nvfp4", 148 * 8 + 1, 4096), ("nvfp4", 148 * 24, 3072),
+    ("nvfp4", 148 * 24 + 1, 3072), ("nvfp4", 148 * 8, 9216), ("nvfp4", 148 * 32, 2048), ("nvfp4", 148 * 48, 1024), ("nvfp4", 148 * 48 + 1, 1024),
+    ("fp8", 148 * 32, 4096), ("fp8", 148 * 32 + 1, 4096), ("fp8", 148 * 32, 4160)])
 def test_launches_at_the_edges_of_the_plans(fmt, n, k):
     host = MAKE[fmt](n, k, seed=n + k)
     t = tuple(part.cuda() for part in host)
