@@ -174,7 +174,10 @@ int resident_bytes_of(int fmt, int M, int nblk) {
 //                   in two steps 12.65 / 14.35 / 14.9 us, one tile in one step 11.7 / 12.45 / 13.15; FP8 with 4 rows 17.3 and
 //                   14.8), and from 16 steps of K on two steps are worth more than a third stage where the ring does not have
 //                   to hold a finished tile's sums as well (8192 x 28672 NVFP4, 4 rows: three stages of 40 rows 41.8, two of 56
-//                   31.2; 8 rows: one step 32.6, two 31.7)
+//                   31.2). NVFP4 from five rows on: one, but for the shortest ranges. Its windows of activations leave two steps
+//                   only low tiles (57344 x 8192, 5 rows 66.4 and 61.6 us; gate_up with SwiGLU had tiles of 16 columns), and a layer's
+//                   projections are one kernel then: three layers at 8 rows take 374 us with two steps for K = 28672, 366 without
+//                   (31.1 and 32.1 alone), with SwiGLU in gate_up 419 and 371.5
 //   stages          as many as fit in shared memory, at most kMaxStages
 // Activations stay resident where that leaves three stages of two steps (from three rows on, where they would take a fifth
 // and more of a stage, also with four stages of one); otherwise a window of them passes through every stage.
@@ -228,6 +231,7 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
                                                                : steps == 2 && row_steps == 1 && fmt != dg::FMT_BF16) continue;
     int need = grid > 0 || force_steps > 0 ? 2 : attempt == 0 ? 3 : attempt == 1 ? (M >= 3 ? 4 : dg::kMaxStages + 1)
                                                : attempt == 2 ? 3 : 2;
+    if (grid == 0 && force_steps == 0 && fmt == dg::FMT_NVFP4 && M >= 5 && steps == 2 && all_rows > 32) continue;
     const bool one_step_tile = fmt != dg::FMT_BF16 && one_tile_fits(resident, 1, resident ? 4 : 3);
     if (steps == 2 && fmt != dg::FMT_BF16 && row_steps > 1 && !one_tile_fits(resident, 2, 3)) {
       if (!resident && row_steps >= 16 && one_tile_fits(false, 2, 2)) need = 2;
