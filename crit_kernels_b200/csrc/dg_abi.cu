@@ -84,8 +84,9 @@ bool encode_rows(CUtensorMap* map, const void* base, int rows, int row_bytes, in
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   });
 }
-// The activations [M][K] (16-bit elements, rows ldx apart, K a multiple of 64) as [K / 64][M][64], box = `blocks` of them.
+// The activations [M][K] (16-bit elements, rows ldx apart, of K the whole multiples of 64) as [K / 64][M][64], box = `blocks` of them.
 bool encode_activations(CUtensorMap* map, const void* base, int M, int K, int ldx, int blocks, bool swizzled) {
+  K &= ~63;
   const int row = M > 1 ? ldx : K;     // (one row may come with any distance to a next one)
   return kept_map(map, MapKey{base, ((long long)M << 32) | K, row, swizzled ? -blocks : -blocks - 4096}, [&](EncodeTiled fn, CUtensorMap* out) {
     const cuuint64_t dims[3] = {64, (cuuint64_t)M, (cuuint64_t)(K / 64)};
@@ -311,8 +312,13 @@ int prepare(int fmt, Params& p, int M, int& ctas, int& smem, int grid = 0, bool 
        (!encode_rows(&p.tmap_sc, p.scales, matrix_rows, p.scale_row_bytes, full_rows, sc_box) ||
         !encode_rows(&p.tmap_sc_last, p.scales, matrix_rows, p.scale_row_bytes, p.last_rows, sc_box))))
     return (int)cudaErrorNotSupported;
-  if (p.x_mode != dg::X_COPIED) {
-    const int step_blocks = kFormats[fmt].x_row / 128, steps = ceil_div(p.row_bytes, kFormats[fmt].step);
+  const int step_blocks = kFormats[fmt].x_row / 128;
+  if (p.x_mode == dg::X_COPIED) {
+    // (rows of any distance, none at all among them, may come to the copying warps)
+    p.x_box_steps = p.K / 64 >= p.steps * step_blocks && (M == 1 || p.ldx > 0) &&
+                    encode_activations(&p.tmap_x, p.x, M, p.K, p.ldx, p.steps * step_blocks, true) ? p.steps : 0;
+  } else {
+    const int steps = ceil_div(p.row_bytes, kFormats[fmt].step);
     p.x_box_steps = std::min(steps, 256 / step_blocks);           // whole boxes only: the space ends with the last step
     while (steps % p.x_box_steps) --p.x_box_steps;
     const bool resident = p.x_mode == dg::X_RESIDENT;

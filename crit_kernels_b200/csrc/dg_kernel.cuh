@@ -143,8 +143,8 @@ struct Params {
   int pairs;
   // Activations: X_RESIDENT (resident_capable; the kernel's dynamic shared memory holds, x_res_off bytes in, the steps of
   // M x XROW bytes, unswizzled, FP16), or a
-  // window of them in every ring stage, by one tensor copy (X_TENSOR) or, where K is no multiple of 64, by the copying
-  // warps (X_COPIED).
+  // window of them in every ring stage, by one tensor copy (X_TENSOR). Where K is no multiple of 64 (X_COPIED) the copying warps bring
+  // the windows that a row ends in (see tensor_windows).
   int x_mode, x_res_off;
   unsigned long long* trace; // diagnostic (dg_set_trace): kTraceSlots time stamps per CTA, or null
   unsigned long long wait_limit_ns;   // every wait in the kernel gives up after this long (status word, then leaves)
@@ -159,9 +159,9 @@ struct Params {
   // Tensor maps over the weight rows and the row-major scale rows as 8-byte elements: box = one window and its padding of
   // a full tile's rows (per region, see Walk), or of last_rows rows. Rows are 16-byte multiples apart, as the encoder asks.
   alignas(64) CUtensorMap tmap_w, tmap_w_last, tmap_sc, tmap_sc_last;
-  int x_box_steps;           // X_RESIDENT: steps of one copy of the activations
-  // The activations as [K / 64][M][64 elements]. X_TENSOR: 128-byte swizzled, box = the blocks of one window; X_RESIDENT: as
-  // they are, box = those of x_box_steps steps.
+  int x_box_steps;           // X_RESIDENT: steps of one copy of the activations; X_COPIED: 0 where there is no map for a window
+  // The activations as [K / 64][M][64 elements]. X_TENSOR, X_COPIED: 128-byte swizzled, box = the blocks of one window (X_COPIED: a map
+  // only where a row has one); X_RESIDENT: as they are, box = those of x_box_steps steps.
   alignas(64) CUtensorMap tmap_x;
 };
 
@@ -357,22 +357,33 @@ __device__ __forceinline__ void copy_resident(const Params& p, const Params& map
     tensor3_g2s(smem_addr(smem) + (uint32_t)(p.x_res_off + st * bytes), &maps.tmap_x, st * (XROW / 128), bars.x);
 }
 
+// Windows whose activations one tensor copy brings: all, or where K is no multiple of 64 those that lie within the rows (past their end a
+// copy would bring the next row's values). The three copying warps, 16 bytes a copy, cannot keep up with more than a few rows: us at
+// 12490 x 5088 with 8 / 16 rows, all windows by them and only the last: NVFP4 24.0 / 37.9 and 15.2 / 23.4, FP8 19.0 / 45.3 and 16.2 / 28.4,
+// MXFP8 22.7 / 42.6 and 17.3 / 22.6, BF16 24.1 / 36.2 and 23.5 / 26.8; NVFP4 40000 x 8160 93 / 144 and 56 / 81.
+template <int FMT, int STEPS>
+__device__ __forceinline__ int tensor_windows(const Params& p) {
+  constexpr int WINDOW = STEPS * Format<FMT>::XROW / 2;                   // elements
+  return p.x_mode == X_TENSOR ? (p.K + WINDOW - 1) / WINDOW : p.x_mode == X_COPIED && p.x_box_steps ? p.K / WINDOW : 0;
+}
+
 // A kernel's first activations, the moment the previous kernel of the stream has finished (the finishing warp has nothing else
 // to do then): the resident ones, or those of the windows that fill the ring.
 template <int FMT, int STEPS>
 __device__ __forceinline__ void start_activations(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars) {
   constexpr int X_BLOCKS = STEPS * Format<FMT>::XROW / 128;
-  if ((threadIdx.x & 31) == 0 && p.x_mode != X_COPIED) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.tmap_x) : "memory");
+  const int by_tensor = tensor_windows<FMT, STEPS>(p);
+  if ((threadIdx.x & 31) == 0 && (by_tensor > 0 || p.x_mode == X_RESIDENT)) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.tmap_x) : "memory");
   const Walk wk(p, STEPS * Format<FMT>::STEP);
   griddep_wait();
   if ((threadIdx.x & 31) != 0) return;
   if (p.x_mode == X_RESIDENT && wk.ntiles > 0) copy_resident<FMT>(p, maps, smem, bars);
-  if (p.x_mode != X_TENSOR) return;
+  if (by_tensor == 0) return;
   const uint32_t at = smem_addr(smem) + kSmemHeader +
                       (uint32_t)x_offset(p.tile_rows * (weight_pitch(FMT, STEPS) + scale_pitch(FMT, STEPS)));
   const int windows = min(p.stages, wk.ntiles * wk.nwin);
   for (int i = 0, win = 0; i < windows; ++i) {
-    tensor3_g2s(at + (uint32_t)i * p.stage_bytes, &maps.tmap_x, win * X_BLOCKS, bars.full + 8u * i);
+    if (win < by_tensor) tensor3_g2s(at + (uint32_t)i * p.stage_bytes, &maps.tmap_x, win * X_BLOCKS, bars.full + 8u * i);
     if (++win == wk.nwin) win = 0;
   }
 }
@@ -407,9 +418,13 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
   // activations by tensor copy: a window at a time
   constexpr int X_BLOCKS = STEPS * XROW / 128;
   const uint32_t x_off = (uint32_t)x_offset(p.tile_rows * (W_ROW + SC_ROW));
-  const uint32_t x_bytes = p.x_mode == X_TENSOR ? (uint32_t)(X_BLOCKS * 128 * p.M) : 0u;
+  const uint32_t x_bytes = (uint32_t)(X_BLOCKS * 128 * p.M);
+  const int by_tensor = tensor_windows<FMT, STEPS>(p);
   auto activations = [&](int at, int win) {
-    if (x_bytes && lane == 31) tensor3_g2s(ring + (uint32_t)at * stage_bytes + x_off, &maps.tmap_x, win * X_BLOCKS, bars.full + 8u * at);
+    if (win >= by_tensor || lane != 31) return;
+    // (the copying warps may have written there before)
+    if (p.x_mode == X_COPIED) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tensor3_g2s(ring + (uint32_t)at * stage_bytes + x_off, &maps.tmap_x, win * X_BLOCKS, bars.full + 8u * at);
   };
   // or all at once: when nobody reads the previous GEMV's any more, which is known once the last of its stages is empty
   bool x_due = p.x_mode == X_RESIDENT && wk.ntiles > 0 && !first;
@@ -432,7 +447,7 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
     const bool full_tile = cols == wk.cap;
     const CUtensorMap* const map_w = full_tile ? &maps.tmap_w : &maps.tmap_w_last;
     const CUtensorMap* const map_sc = full_tile ? &maps.tmap_sc : &maps.tmap_sc_last;
-    const uint32_t bytes = x_bytes + wk.regions * (full_tile ? wk.cap : p.last_rows) * (uint32_t)(W_ROW + (staged ? SC_ROW : 0));
+    const uint32_t bytes = wk.regions * (full_tile ? wk.cap : p.last_rows) * (uint32_t)(W_ROW + (staged ? SC_ROW : 0));
     // lanes 0, 1: the regions' weights; 2, 3: their scales
     const int region = lane & 1, n0 = region * wk.pairs + col0, row0 = region * wk.cap;
     for (int win = 0; win < wk.nwin; ++win) {
@@ -444,7 +459,7 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
         while ((int)(clock64() - start) < due) {}
       }
       const uint32_t full = bars.full + 8u * s, stage = ring + (uint32_t)s * stage_bytes;
-      if (lane == 0) mbar_arrive_expect_tx(full, bytes);
+      if (lane == 0) mbar_arrive_expect_tx(full, bytes + (win < by_tensor ? x_bytes : 0u));
       __syncwarp();
       if (!first || filled > stages) activations(s, win);
       if (region < wk.regions) {
@@ -583,6 +598,7 @@ __device__ __forceinline__ bool feed_activations(const Params& p, unsigned char*
   const StageLayout<FMT, STEPS> lay(p);
   const int lane = threadIdx.x & 31;
   const bool gathered = scales_gathered<FMT>(p);
+  const int by_tensor = tensor_windows<FMT, STEPS>(p);
   const uint32_t ring = smem_addr(smem) + kSmemHeader;
   for (int t = 0; t < wk.ntiles; ++t) {
     int col0, cols;
@@ -597,7 +613,7 @@ __device__ __forceinline__ bool feed_activations(const Params& p, unsigned char*
       if constexpr (Format<FMT>::SCB != 0) {
         if (gathered) stored = gather_scales<FMT, STEPS>(p, wk, stage + lay.sc_off, col0, cols, win, warp, lane);
       }
-      if (p.x_mode == X_COPIED) stored |= copy_activations<FMT, STEPS>(p, stage + lay.x_off, win, warp, lane);
+      if (p.x_mode == X_COPIED && win >= by_tensor) stored |= copy_activations<FMT, STEPS>(p, stage + lay.x_off, win, warp, lane);
       if (stored) {
         asm volatile("cp.async.wait_all;" ::: "memory");
         mbar_arrive(full);
