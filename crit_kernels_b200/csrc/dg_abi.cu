@@ -359,9 +359,9 @@ int launch(int table, int fmt, Params& p, int M, cudaStream_t stream) {
   }
   void* args[] = {&p};
   // Up to four rows whose activations come in windows run the kernel for five to eight, the bits being the same: its code for such
-  // windows is the better one (NVFP4 8192 x 28672, one row 32.5 us in the kernel for up to four and 30.5 in this one, 2731 x 5152 7.72
-  // and 7.09), but for copied windows in more than one tile per CTA (9000 x 8224, one row 16.3 and 16.45).
-  const bool windows = p.x_mode == dg::X_TENSOR || (p.x_mode == dg::X_COPIED && ceil_div(p.N, ctas) <= p.tile_rows);
+  // windows is the better one (NVFP4 8192 x 28672, one row 32.5 us in the kernel for up to four and 30.5 in this one, 12490 x 5088 with one /
+  // four rows 13.5 / 14.1 and 12.7 / 13.4, 20000 x 1056 10.8 / 11.2 and 9.7 / 10.1; FP8 20000 x 9200 35.3 / 35.6 and 34.1 / 34.4).
+  const bool windows = p.x_mode != dg::X_RESIDENT;
   const int rows = windows ? std::max(M, 5) : M;
   return launch_pdl(kTables[table][p.steps - 1 + 2 * p.small][rows - 1], args, ctas, p.small ? dg::kSmallThreads : dg::kThreads, smem,
                     stream);
