@@ -233,6 +233,9 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
     int need = grid > 0 || force_steps > 0 ? 2 : attempt == 0 ? 3 : attempt == 1 ? (M >= 3 ? 4 : dg::kMaxStages + 1)
                                                : attempt == 2 ? 3 : 2;
     if (grid == 0 && force_steps == 0 && fmt == dg::FMT_NVFP4 && M >= 5 && steps == 2 && all_rows > 32) continue;
+    // (from 13 rows on the windows of FP8 leave three stages of two steps 40 rows only: us with 16 rows so and in one step, 12288 x 5120 22.8 and
+    // 18.3, 28672 x 8192 56.5 and 54.8, 20000 x 2048 14.2 and 13.2; with 12 rows 12288 x 5120 17.3 and 18.0; one tile, 8192 x 8192, 16.1 and 16.8)
+    if (grid == 0 && force_steps == 0 && fmt == dg::FMT_FP8 && M >= 13 && steps == 2 && all_rows > 64) continue;
     const bool one_step_tile = fmt != dg::FMT_BF16 && one_tile_fits(resident, 1, resident ? 4 : 3);
     if (steps == 2 && fmt != dg::FMT_BF16 && row_steps > 1 && !one_tile_fits(resident, 2, 3)) {
       if (!resident && row_steps >= 16 && one_tile_fits(false, 2, 2)) need = 2;

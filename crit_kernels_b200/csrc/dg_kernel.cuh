@@ -224,8 +224,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // Weights and scales are read once and leave L2 first. Otherwise they drive out what the next launches need again, the kernels' code
 // above all: a launch of another kernel than the one before took 1.4 to 4.2 us longer than one of the same (its instructions came
 // from HBM, in competition with the weights), now 0.7 to 1.9. us before and after: NVFP4 57344 x 8192 with 1 / 8 / 16 rows 53.1 / 63.9 /
-// 90.9 and 51.3 / 62.6 / 88.5, 8192 x 8192 with one row 11.4 and 10.8; FP8 8192 x 8192 with one row 13.0 and 12.45; a pass over four layers
-// of four projections, 16 / 4 rows, 382 (two layers) / 535 and 348 / 487.
+// 90.9 and 51.3 / 62.6 / 88.5; FP8 28672 x 8192 with 1 / 8 rows 40.2 / 44.8 and 38.3 / 42.6; four layers of four projections at 4 rows 535 and
+// 487, two at 16 rows 382 and 348. (Small matrices that keep the usual order: NVFP4 4096 x 4096, one row, eager 5.60 and 5.40.)
 __device__ __forceinline__ uint64_t read_once() {
   uint64_t policy;
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
