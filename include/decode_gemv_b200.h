@@ -223,8 +223,10 @@ DG_API unsigned long long dg_set_wait_limit_ns(unsigned long long limit_ns);
 
 /* Tells the library whether weights (codes, block scales staged with them, BF16 weights) are static: not written by
  * any kernel of the stream that can still be in flight when a GEMV starts. Every GEMV kernel is launched with
- * programmatic dependent launch and lets its own successor start at once, so a GEMV may begin while the kernel before
- * it, and in a run of GEMVs the ones before that, are still finishing; it always waits for all of them before it
+ * programmatic dependent launch. The GEMV kernels, the quantizers and dg_enqueue_swiglu let their own successor start
+ * at once, so a GEMV may begin while the kernel before it, and in a run of such kernels the ones before that, are
+ * still finishing (codes that dg_enqueue_quantize_fp8_rows has just written are not static for the GEMV behind it); the
+ * dequantizer lets nobody start before it has ended (a matrix it has written is). A GEMV always waits for all of them before it
  * reads activations, row / inverse scales or directly-read block scales and before it writes. With enabled = 1 it
  * starts streaming weights before that wait, which hides its start-up behind the previous kernels' tails (what a
  * decode stack with resident weights wants); with 0 (the default) nothing is read before the wait, which is correct

@@ -59,3 +59,64 @@ def test_a_chain_of_calls_reads_what_the_one_before_wrote(n, k):
     torch.cuda.synchronize()
     for i, (w, q, scale) in enumerate(got):
         assert torch.equal(w, want[(i + 1) % 2][0]) and torch.equal(q, want[i % 2][1]) and torch.equal(scale, want[i % 2][2])
+
+
+@pytest.mark.parametrize("n,k", [(300, 1024), (4096, 4096)])            # in one launch the other way of the two
+def test_a_matrix_just_dequantized_is_static_for_the_next_gemv(n, k):
+    """With static weights a GEMV reads its matrix before it waits for the kernel in front of it."""
+    import crit_kernels_b200
+    kernel = crit_kernels_b200.get_kernel("crit-labs/decode-gemv", version=1)
+    mats = [tuple(t.cuda() for t in wl.cfg_nvfp4(n, k, seed=s)) for s in range(2)]
+    x = wl.activations(3, k, seed=2).cuda()
+    want = []
+    for m in mats:
+        w = kernel.decode(*m, torch.empty(n, k, dtype=torch.bfloat16, device="cuda"))
+        torch.cuda.synchronize()
+        want.append(kernel.gemv_bf16(x, w, torch.empty(3, n, device="cuda")))
+        torch.cuda.synchronize()
+    w = torch.zeros(n, k, dtype=torch.bfloat16, device="cuda")
+    got = [torch.zeros(3, n, device="cuda") for _ in range(12)]
+    previous = cabi.load().dg_set_static_weights(1)
+    try:
+        for i, out in enumerate(got):
+            kernel.decode(*mats[i % 2], w)
+            kernel.gemv_bf16(x, w, out)
+        torch.cuda.synchronize()
+    finally:
+        cabi.load().dg_set_static_weights(previous)
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2]), i
+    assert cabi.load().dg_take_status() == 0
+
+
+@pytest.mark.parametrize("n,k", [(40, 1024), (1500, 2048)])
+def test_factors_and_codes_that_the_kernel_before_writes(n, k):
+    """Kernels of the package that let the dequantizer start early write what it reads: the FP8 quantizer its factors, the NVFP4
+    quantizer its codes, others with every call."""
+    import crit_kernels_b200
+    kernel = crit_kernels_b200.get_kernel("crit-labs/decode-gemv", version=1)
+    codes, scales, _ = (t.cuda() for t in wl.cfg_nvfp4(n, k, seed=5))
+    g = torch.Generator().manual_seed(n)
+    rows = [(torch.randn(n, k, generator=g) * 2.0 ** i).to(torch.bfloat16).cuda() for i in range(3)]
+    tiles = torch.empty(oc.blocked_numel(n, k), dtype=torch.uint8, device="cuda")
+    q, factor, now = torch.empty(n, k, dtype=torch.uint8, device="cuda"), torch.empty(n, device="cuda"), torch.empty_like(codes)
+    new = lambda: (torch.zeros(n, k, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, k, dtype=torch.bfloat16, device="cuda"))
+
+    def chain(i, out, between):
+        kernel.quantize_fp8_rows(rows[i % 3], q, factor)
+        between()
+        kernel.decode(codes, scales, factor, out[0])
+        between()
+        kernel.quantize_nvfp4(rows[(i + 1) % 3], 2688.0 / (8.0 + i % 3), now, tiles)
+        between()
+        kernel.decode(now, scales, factor, out[1])
+        between()
+    want = [new() for _ in range(9)]
+    for i, out in enumerate(want):
+        chain(i, out, torch.cuda.synchronize)
+    got = [new() for _ in range(9)]
+    for i, out in enumerate(got):
+        chain(i, out, lambda: None)
+    torch.cuda.synchronize()
+    for i in range(9):
+        assert torch.equal(got[i][0], want[i][0]) and torch.equal(got[i][1], want[i][1]), i

@@ -45,3 +45,17 @@ def test_the_build_description_names_every_source():
     with open(os.path.join(os.path.dirname(CSRC), "build.toml")) as f:
         named = re.findall(r'"csrc/([^"]+)"', f.read())
     assert sorted(named) == sorted(os.listdir(CSRC))
+
+
+def test_every_kernel_launched_early_waits_and_the_dequantizer_lets_nobody_start_before_it_has_ended():
+    """A kernel launched with programmatic dependent launch reads and writes global memory behind its wait only. The dequantizer's
+    output is a weight matrix, which a GEMV told of static weights reads before its own wait, so its successor may not start early."""
+    launched = {n for n in os.listdir(CSRC) if "ProgrammaticStreamSerialization" in code(n)}
+    waiting = {"dg_abi.cu" if n == "dg_kernel.cuh" else n for n in early_starters()}     # (which launches that header's kernels)
+    assert {"dg_abi.cu", "dg_dequant.cu"} <= launched == waiting
+    text = code("dg_dequant.cu")
+    assert "launch_dependents" not in text
+    body = text[text.index("dequantize_kernel("):]
+    before, behind = body.split("griddepcontrol.wait", 1)
+    touched = r"\b(?:codes|scales|factor|out)\)?\s*\["
+    assert not re.findall(touched, before) and len(re.findall(touched, behind)) >= 6
