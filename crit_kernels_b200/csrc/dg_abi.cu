@@ -164,7 +164,14 @@ int resident_bytes_of(int fmt, int M, int nblk) {
   return row_steps * M * kFormats[fmt].x_row + ((row_steps + 15) & ~15);
 }
 
-// Launch shape: a speed choice from (format, M, N, K, SM count) only; no row's bits depend on it.
+// How row-major block scales reach a stage: by tensor copy when every window of every row starts on 16 bytes and is a multiple of 16
+// bytes long (K a multiple of 256, MXFP8 512; base on 16 bytes), else two warps copy them.
+int row_major_scales(int fmt, int K, bool on_16_bytes) {
+  if (fmt != dg::FMT_NVFP4 && fmt != dg::FMT_MXFP8) return dg::SCALES_NONE;
+  return K % (fmt == dg::FMT_NVFP4 ? 256 : 512) == 0 && on_16_bytes ? dg::SCALES_STAGED : dg::SCALES_DIRECT;
+}
+
+// Launch shape: a speed choice from (format, M, N, K, SM count, how scales travel, SwiGLU) only; no row's bits depend on it.
 //   CTAs            one per SM, fewer when the matrix has under four rows per SM
 //   tile rows       64 to 40 (less when a CTA's range is shorter): what takes the fewest eighths of 8 rows, a tile costing as much
 //                   as one eighth (its sums) plus, where its activations are converted on the way, as much as these cost
@@ -382,10 +389,7 @@ bool fill_nvfp4(Params& p, const void* x, int ldx, int x_is_bf16, const uint8_t*
   p.N = N; p.K = K;
   p.scale_row_bytes = K / 16;
   p.ct = blocked ? (K / 16 + 3) / 4 : 0;
-  // Scale rows travel by tensor copy when every window of every row starts on 16 bytes and is a multiple of 16 bytes
-  // long (K a multiple of 256, base on 16 bytes); otherwise, and for the tiled layout, two warps copy them into the stage.
-  p.scale_mode = blocked ? dg::SCALES_BLOCKED
-                         : (K % 256 == 0 && aligned(scales, 16)) ? dg::SCALES_STAGED : dg::SCALES_DIRECT;
+  p.scale_mode = blocked ? dg::SCALES_BLOCKED : row_major_scales(dg::FMT_NVFP4, K, aligned(scales, 16));
   return true;
 }
 
@@ -619,9 +623,8 @@ int dg_enqueue_fp8(const void* x, int ldx, int x_is_bf16, const uint8_t* codes, 
   p.out_kind = out_kind == 0 ? dg::OUT_F32 : (x_is_bf16 ? dg::OUT_BF16 : dg::OUT_F16);
   p.N = N; p.K = K;
   p.scale_row_bytes = K / 32;
-  p.scale_mode = !mx_scale ? dg::SCALES_NONE
-                           : (K % 512 == 0 && aligned(mx_scale, 16)) ? dg::SCALES_STAGED : dg::SCALES_DIRECT;
   const int fmt = mx_scale ? dg::FMT_MXFP8 : dg::FMT_FP8;
+  p.scale_mode = row_major_scales(fmt, K, aligned(mx_scale, 16));
   return launch((mx_scale ? 3 : 1) + (x_is_bf16 ? 0 : 1), fmt, p, M, static_cast<cudaStream_t>(stream));
 }
 
@@ -648,6 +651,7 @@ int dg_plan(int fmt, int M, int N, int K, int plan[6]) {
   if (DeviceState* st = device_state()) sms = st->sms;
   Params p{};
   p.N = N; p.K = K;
+  p.scale_mode = row_major_scales(fmt, K, true);
   int ctas = 0, smem = 0;
   if (!make_plan(fmt, M, N, K, sms, p, ctas, smem)) return (int)cudaErrorInvalidValue;
   plan[0] = ctas; plan[1] = ceil_div(p.tile_rows, dg::kGroupRows); plan[2] = p.steps; plan[3] = p.stages; plan[4] = p.stage_bytes;

@@ -201,7 +201,8 @@ DG_API int dg_enqueue_quantize_nvfp4(const void* x, long long ldx, int M, int K,
  * (decode_gemv.h:43, decode_gemv.cu:419-427); unlike it, allocates nothing and launches nothing. */
 DG_API int dg_hardware_decode(void);
 
-/* The launch a call with these sizes makes, for benches and tests: fmt 0 BF16, 1 FP8, 2 MXFP8, 3 NVFP4.
+/* The launch a call with these sizes makes, for benches and tests: fmt 0 BF16, 1 FP8, 2 MXFP8, 3 NVFP4 (block scales row
+ * major on 16 bytes; short launches with tiled or other scales, and gate_up with SwiGLU, may get another).
  * plan[0] = CTAs, [1] = groups of 16 rows in a full tile (before version 1.03: rows per consumer warp and tile), [2] =
  * 512-byte steps (BF16: 1 KB) per ring stage, [3] = ring stages, [4] = bytes per stage, [5] = dynamic shared memory bytes
  * (256 bytes of barriers, the ring, and, for FP8 / NVFP4 at few rows and small K, the activations, which then stay

@@ -114,3 +114,14 @@ def test_dequantizer_wrappers_refuse_wrong_output_types_before_any_device_work()
     assert {"decode", "decode_fp8"} <= set(k.__all__)
     with pytest.raises(AttributeError):
         k.gemv_triton
+
+
+@pytest.mark.parametrize("fmt,n,k", [("nvfp4", 1184, 1088), ("nvfp4", 1024, 1088), ("mxfp8", 1024, 1088), ("mxfp8", 1184, 1280)])
+def test_plans_know_that_gathered_scales_have_no_small_launch(fmt, n, k):
+    """Block scales of these K are copied by two warps, which the small launches (a stage for each window, two CTAs to an SM) do
+    not have: the launch is one with as many stages as fit."""
+    p = cabi.plan(fmt, 1, n, k)
+    behind = p["smem_bytes"] - (256 + p["stages"] * p["stage_bytes"])
+    assert p["stages"] == min(12, (232448 - 256 - behind) // p["stage_bytes"])
+    even = cabi.plan(fmt, 1, n, 1024)                        # (their neighbours of two windows' length)
+    assert even["stages"] == 2 and even["smem_bytes"] < 115712 // 2
