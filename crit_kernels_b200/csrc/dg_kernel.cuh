@@ -146,6 +146,7 @@ struct Params {
   // window of them in every ring stage, by one tensor copy (X_TENSOR). Where K is no multiple of 64 (X_COPIED) the copying warps bring
   // the windows that a row ends in (see tensor_windows).
   int x_mode, x_res_off;
+  int x_box_steps;           // X_RESIDENT: steps of one copy of the activations; X_COPIED: 0 where there is no map for a window
   unsigned long long* trace; // diagnostic (dg_set_trace): kTraceSlots time stamps per CTA, or null
   unsigned long long wait_limit_ns;   // every wait in the kernel gives up after this long (status word, then leaves)
   // All-gather epilogue (world >= 1, 0 = off): this rank's [M][N] results go into slot `rank` of its own
@@ -159,7 +160,6 @@ struct Params {
   // Tensor maps over the weight rows and the row-major scale rows as 8-byte elements: box = one window and its padding of
   // a full tile's rows (per region, see Walk), or of last_rows rows. Rows are 16-byte multiples apart, as the encoder asks.
   alignas(64) CUtensorMap tmap_w, tmap_w_last, tmap_sc, tmap_sc_last;
-  int x_box_steps;           // X_RESIDENT: steps of one copy of the activations; X_COPIED: 0 where there is no map for a window
   // The activations as [K / 64][M][64 elements]. X_TENSOR, X_COPIED: 128-byte swizzled, box = the blocks of one window (X_COPIED: a map
   // only where a row has one); X_RESIDENT: as they are, box = those of x_box_steps steps.
   alignas(64) CUtensorMap tmap_x;
@@ -361,23 +361,25 @@ __device__ __forceinline__ void copy_resident(const Params& p, const Params& map
 // copy would bring the next row's values). The three copying warps, 16 bytes a copy, cannot keep up with more than a few rows: us at
 // 12490 x 5088 with 8 / 16 rows, all windows by them and only the last: NVFP4 24.0 / 37.9 and 15.2 / 23.4, FP8 19.0 / 45.3 and 16.2 / 28.4,
 // MXFP8 22.7 / 42.6 and 17.3 / 22.6, BF16 24.1 / 36.2 and 23.5 / 26.8; NVFP4 40000 x 8160 93 / 144 and 56 / 81.
-template <int FMT, int STEPS>
+template <int FMT, int STEPS, bool RESIDENT>
 __device__ __forceinline__ int tensor_windows(const Params& p) {
+  if constexpr (RESIDENT) return 0;
   constexpr int WINDOW = STEPS * Format<FMT>::XROW / 2;                   // elements
   return p.x_mode == X_TENSOR ? (p.K + WINDOW - 1) / WINDOW : p.x_mode == X_COPIED && p.x_box_steps ? p.K / WINDOW : 0;
 }
 
 // A kernel's first activations, the moment the previous kernel of the stream has finished (the finishing warp has nothing else
 // to do then): the resident ones, or those of the windows that fill the ring.
-template <int FMT, int STEPS>
+template <int FMT, int STEPS, bool RESIDENT>
 __device__ __forceinline__ void start_activations(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars) {
   constexpr int X_BLOCKS = STEPS * Format<FMT>::XROW / 128;
-  const int by_tensor = tensor_windows<FMT, STEPS>(p);
-  if ((threadIdx.x & 31) == 0 && (by_tensor > 0 || p.x_mode == X_RESIDENT)) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.tmap_x) : "memory");
+  const int by_tensor = tensor_windows<FMT, STEPS, RESIDENT>(p);
+  const bool resident = RESIDENT || p.x_mode == X_RESIDENT;
+  if ((threadIdx.x & 31) == 0 && (by_tensor > 0 || resident)) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.tmap_x) : "memory");
   const Walk wk(p, STEPS * Format<FMT>::STEP);
   griddep_wait();
   if ((threadIdx.x & 31) != 0) return;
-  if (p.x_mode == X_RESIDENT && wk.ntiles > 0) copy_resident<FMT>(p, maps, smem, bars);
+  if (resident && wk.ntiles > 0) copy_resident<FMT>(p, maps, smem, bars);
   if (by_tensor == 0) return;
   const uint32_t at = smem_addr(smem) + kSmemHeader +
                       (uint32_t)x_offset(p.tile_rows * (weight_pitch(FMT, STEPS) + scale_pitch(FMT, STEPS)));
@@ -406,7 +408,7 @@ constexpr int kUnpaced = 32 * 1024, kPace = 22;   // bytes at once, bytes per cl
 // the ring fills. The ring position (stage s, its phase parity) is the caller's and
 // carries on from one GEMV of a batch to the next (`first`: its first; `wait`: the previous kernel of the stream has to be
 // waited for); `maps`: where the tensor maps are read from.
-template <int FMT, int STEPS>
+template <int FMT, int STEPS, bool RESIDENT>
 __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps, unsigned char* smem, const Bars& bars,
                                              bool first, bool wait, int& s, uint32_t& parity) {
   constexpr int SCB = Format<FMT>::SCB, WIN = STEPS * Format<FMT>::STEP, SC_WIN = STEPS * SCB;
@@ -419,7 +421,7 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
   constexpr int X_BLOCKS = STEPS * XROW / 128;
   const uint32_t x_off = (uint32_t)x_offset(p.tile_rows * (W_ROW + SC_ROW));
   const uint32_t x_bytes = (uint32_t)(X_BLOCKS * 128 * p.M);
-  const int by_tensor = tensor_windows<FMT, STEPS>(p);
+  const int by_tensor = tensor_windows<FMT, STEPS, RESIDENT>(p);
   auto activations = [&](int at, int win) {
     if (win >= by_tensor || lane != 31) return;
     // (the copying warps may have written there before)
@@ -511,8 +513,8 @@ __device__ __forceinline__ void prefetch_weights(const Params& p) {
 // The other producer warps, where they are needed: the windows' activations where no tensor copy can bring them, 16 bytes
 // (8 elements) per copy, and the scales that are gathered; then every lane's arrival, which fires when its copies have
 // landed.
-template <int FMT>
-__device__ __forceinline__ bool copies_needed(const Params& p) { return p.x_mode == X_COPIED || scales_gathered<FMT>(p); }
+template <int FMT, bool RESIDENT>
+__device__ __forceinline__ bool copies_needed(const Params& p) { return (!RESIDENT && p.x_mode == X_COPIED) || scales_gathered<FMT>(p); }
 
 // (zeros past the row's end, by stores, which the lane's arrival on the stage's barrier must follow: returns true then)
 template <int FMT, int STEPS>
@@ -591,14 +593,14 @@ __device__ __forceinline__ bool gather_scales(const Params& p, const Walk& wk, u
   return true;
 }
 
-template <int FMT, int STEPS>
+template <int FMT, int STEPS, bool RESIDENT>
 __device__ __forceinline__ bool feed_activations(const Params& p, unsigned char* smem, const Bars& bars, int warp, int& s,
                                                  uint32_t& parity) {
   const Walk wk(p, STEPS * Format<FMT>::STEP);
   const StageLayout<FMT, STEPS> lay(p);
   const int lane = threadIdx.x & 31;
   const bool gathered = scales_gathered<FMT>(p);
-  const int by_tensor = tensor_windows<FMT, STEPS>(p);
+  const int by_tensor = tensor_windows<FMT, STEPS, RESIDENT>(p);
   const uint32_t ring = smem_addr(smem) + kSmemHeader;
   for (int t = 0; t < wk.ntiles; ++t) {
     int col0, cols;
@@ -613,7 +615,7 @@ __device__ __forceinline__ bool feed_activations(const Params& p, unsigned char*
       if constexpr (Format<FMT>::SCB != 0) {
         if (gathered) stored = gather_scales<FMT, STEPS>(p, wk, stage + lay.sc_off, col0, cols, win, warp, lane);
       }
-      if (p.x_mode == X_COPIED && win >= by_tensor) stored |= copy_activations<FMT, STEPS>(p, stage + lay.x_off, win, warp, lane);
+      if (!RESIDENT && p.x_mode == X_COPIED && win >= by_tensor) stored |= copy_activations<FMT, STEPS>(p, stage + lay.x_off, win, warp, lane);
       if (stored) {
         asm volatile("cp.async.wait_all;" ::: "memory");
         mbar_arrive(full);
@@ -950,11 +952,11 @@ __device__ __forceinline__ void finish_unit(const Params& p, const Walk& wk, uin
 }
 
 enum : int { RES_NONE = 0, RES_USUAL = 1, RES_MIXED = 2 };
-// Where chunks with values outside the usual window are multiplied: nowhere (there are none); in kernels for up to four rows by
-// the usual chunks' code, which then has the columns' powers of two in registers; from five rows up, and in batched kernels unless
-// the activations are resident, in code of its own (with the powers in registers for every chunk, 28672 x 8192 NVFP4 with 8 rows
-// took 38.4 us, without 37.4, a batched pass over 32 GEMVs at one row 849, without 831; but the code of its own is one more thing
-// to fetch, which a launch for few rows pays for with a single such chunk: 4096 x 4096, one row, 7.1 and 6.4 us).
+// Where chunks with values outside the usual window are multiplied: nowhere (there are none); resident ones by the usual chunks' code,
+// which then has the columns' powers of two in registers; those that come in windows in code of its own (with the powers
+// in registers for every chunk, 28672 x 8192 NVFP4 with 8 rows took 38.4 us, without 37.4, a batched pass over 32 GEMVs at one row
+// 849, without 831; but the code of its own is one more thing to fetch, which a launch for few rows pays for with a single such
+// chunk: 4096 x 4096, one row, resident, 7.1 and 6.4 us).
 // NVFP4 28672 x 8192 at 1 / 8 / 16 rows, us: N(0, 1) activations 31.1 / 37.6 / 53.4, one value of 300 in each row 33.2 / 38.5 /
 // 54.3, all above 2^8 36.5 / 45.0 / 67.3, chunks over more than 32 binades 56.6 / 64.9 / 80.8. (As passes after the tile, from global
 // memory, they took 68 / 72 / 117, 320 / 316 / 645 and 949 / 1087 / 2158.)
@@ -962,8 +964,10 @@ enum : int { ODD_NONE = 0, ODD_SHARED = 1, ODD_APART = 2 };
 // One tile of up to 8 EIGHTS rows: the windows in turn; at the end the warp leaves its sums in the stage it has just consumed,
 // in its own chunk of each row (which no other warp reads), one FP32 per activation row, and tells the finishing warps, to
 // which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the
-// activations are resident (RES_MIXED: `spread` has the steps, modulo 32, with chunks of another exponent than the usual one).
-template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, bool SHARED, int RES>
+// activations are resident (RES_MIXED: `spread` has the steps, modulo 32, with chunks of another exponent than the usual one). FRESH:
+// the lane's places are worked out anew for every tile. Otherwise the compiler works out once what a kernel's tile codes share and
+// keeps it all the time, which costs registers (NVFP4 resident, two steps: 84 bytes a thread spilled, and none so).
+template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, int RES, bool FRESH>
 __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, const StageLayout<FMT, STEPS>& lay,
                                              unsigned char* smem, int col0, int cols, bool last, uint32_t spread, const Bars& bars, int& s, uint32_t& parity,
                                              bool first_window, bool& ok) {
@@ -973,8 +977,9 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
   constexpr bool ODD = EIGHTS % 2 != 0;       // the last group has no second half
   // BF16 activations of the formats whose weights become FP16
   constexpr bool CONVERT = FMT != FMT_BF16 && std::is_same<XT, __nv_bfloat16>::value;
-  constexpr int ODDITIES = !CONVERT || RES == RES_USUAL ? ODD_NONE : SHARED || RES == RES_MIXED ? ODD_SHARED : ODD_APART;
-  const Lane ln;
+  constexpr int ODDITIES = !CONVERT || RES == RES_USUAL ? ODD_NONE : RES == RES_MIXED ? ODD_SHARED : ODD_APART;
+  Lane ln;
+  if constexpr (FRESH) asm volatile("" : "+r"(ln.g), "+r"(ln.t), "+r"(ln.warp));
   const int M = p.M, stage_bytes = p.stage_bytes, stages = p.stages;
   if (last && p.row_scale && unit_column(wk, ln.warp) < cols) {    // (needed at the tile's end)
     const float* at = p.row_scale + col0 + unit_column(wk, ln.warp);
@@ -1074,27 +1079,16 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
       };
       if constexpr (ODDITIES == ODD_SHARED) {
         first_rows();                       // (on their way meanwhile)
-        float scale[NT];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          unscale[nt] = pack2(kWindowUnscale, kWindowUnscale);
-          scale[nt] = kWindowScale;
-        }
+        for (int nt = 0; nt < NT; ++nt) unscale[nt] = pack2(kWindowUnscale, kWindowUnscale);
         const int step = win * STEPS + st;
-        bool odd;
-        if constexpr (RES == RES_NONE) odd = outside();
-        else odd = (spread >> (step & 31) & 1u) != 0u;
-        if (__builtin_expect(odd, 0)) {
+        if (__builtin_expect((spread >> (step & 31) & 1u) != 0u, 0)) {
           uint32_t e[NT];
           bool any = false, all = true;      // are kWide
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
-            if constexpr (RES == RES_NONE) {
-              e[nt] = chunk_exp(chunk_range<NB>(b[nt]));
-            } else {
-              const int steps = (p.row_bytes + STEP - 1) / STEP;
-              e[nt] = lds_u8(bars.exps + (uint32_t)((ln.warp * steps + step) * M + min(fragment_column<FMT>(ln.g), M - 1)));
-            }
+            const int steps = (p.row_bytes + STEP - 1) / STEP;
+            e[nt] = lds_u8(bars.exps + (uint32_t)((ln.warp * steps + step) * M + min(fragment_column<FMT>(ln.g), M - 1)));
             const uint32_t wide = __ballot_sync(0xffffffffu, e[nt] == kWide);
             any |= wide != 0u;
             all &= wide == 0xffffffffu;
@@ -1103,21 +1097,12 @@ __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, co
             keep(e, true);
             multiply_wide();
             if (all) continue;
-            load_x<FMT, NT, RES != RES_NONE>(xs, xo, b);
+            load_x<FMT, NT, true>(xs, xo, b);
             first_rows();
             keep(e, false);
           }
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            unscale[nt] = column_unscale(e[nt], ln);
-            scale[nt] = exp_scale(e[nt] == kWide ? kWindowExp : e[nt]);
-          }
-        }
-        if constexpr (RES == RES_NONE) {
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int i = 0; i < NB; ++i) b[nt][i] = scaled_half2(b[nt][i], scale[nt]);
+          for (int nt = 0; nt < NT; ++nt) unscale[nt] = column_unscale(e[nt], ln);
         }
         multiply(Scaled());
       } else {
@@ -1208,12 +1193,12 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
   const Walk wk(p, STEPS * Format<FMT>::STEP);
   const StageLayout<FMT, STEPS> lay(p);
   if (first) griddep_wait();   // consumers read scales and write results in global memory: after the previous kernel
-  bool resident = false;
+  bool resident = CAN_RES;        // (a launch of its own for up to four rows whose activations come in windows has the kernel for five to eight)
   uint32_t spread = 0u;           // (see prepare_resident)
   bool ok = true;
   if (first && threadIdx.x == 0) trace_stamp(p.trace, TRACE_DEP);
   if constexpr (CAN_RES) {
-    resident = p.x_mode == X_RESIDENT;
+    if constexpr (BATCH) resident = p.x_mode == X_RESIDENT;
     if (resident && wk.ntiles > 0) {
       ok = mbar_wait(bars.x, x_parity, bars.abort_flag);
       x_parity ^= 1u;
@@ -1227,7 +1212,7 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     auto tile = [&](auto res) {
       constexpr int RES = decltype(res)::value;
       auto run = [&](auto e) {
-        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, CAN_RES && !BATCH, RES>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
+        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, RES, FMT == FMT_NVFP4 && NT == 1 && !SMALL && !(BATCH && CAN_RES)>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
                                                                   first && t == 0, ok);
       };
       const int eights = (wk.rows(cols) + 7) / 8;
@@ -1246,7 +1231,7 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
       // (the usual case in code of its own: what a launch fetches of the other costs it 0.6 us)
       if (resident && spread == 0u) tile(std::integral_constant<int, RES_USUAL>());
       else if (resident && std::is_same<XT, __nv_bfloat16>::value) tile(std::integral_constant<int, RES_MIXED>());
-      else tile(std::integral_constant<int, RES_NONE>());
+      else if constexpr (BATCH) tile(std::integral_constant<int, RES_NONE>());
     } else {
       tile(std::integral_constant<int, RES_NONE>());
     }
@@ -1418,13 +1403,13 @@ __device__ __forceinline__ Bars ring_setup(const Params& p, bool copies, unsigne
   return bars;
 }
 
-// NT: column tiles of 8 activation rows; CAN_RES: the launch may keep the activations resident (resident_capable).
+// NT: column tiles of 8 activation rows; CAN_RES: the launch keeps the activations resident (resident_capable).
 template <int FMT, int NT, bool CAN_RES, int STEPS, bool SMALL, typename XT>
 __global__ void __launch_bounds__(SMALL ? kSmallThreads : kThreads, SMALL ? 2 : 1) gemv_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t sums[kMaxStages + 1];   // and the resident activations' barrier
   __shared__ uint8_t exps[CAN_RES ? kResidentExps : 1];
-  const bool copies = !SMALL && copies_needed<FMT>(p);
+  const bool copies = !SMALL && copies_needed<FMT, CAN_RES>(p);
   const Bars bars = ring_setup(p, copies, smem, sums, exps);
   int s = 0;
   uint32_t parity = 0, x_parity = 0;
@@ -1433,14 +1418,14 @@ __global__ void __launch_bounds__(SMALL ? kSmallThreads : kThreads, SMALL ? 2 : 
     if (!p.early_weights) {
       prefetch_weights<FMT, STEPS>(p);
     }
-    feed_weights<FMT, STEPS>(p, p, smem, bars, true, !p.early_weights, s, parity);
+    feed_weights<FMT, STEPS, CAN_RES>(p, p, smem, bars, true, !p.early_weights, s, parity);
   } else if (!SMALL && warp >= kFirstCopier && copies) {
     griddep_wait();
-    feed_activations<FMT, STEPS>(p, smem, bars, warp - kFirstCopier, s, parity);
+    feed_activations<FMT, STEPS, CAN_RES>(p, smem, bars, warp - kFirstCopier, s, parity);
     if (p.world >= 1) finished_barrier();
   } else if (warp >= kFinisher) {
     // (reads scales and writes results in global memory: after the previous kernel)
-    if (warp == kFinisher) start_activations<FMT, STEPS>(p, p, smem, bars);
+    if (warp == kFinisher) start_activations<FMT, STEPS, CAN_RES>(p, p, smem, bars);
     else griddep_wait();
     if (!SMALL) finish_gemv<FMT, STEPS>(p, smem, bars, warp - kFinisher, copies ? 1 : kFinishers, s, parity);
     if (p.world >= 1) finished_barrier();
@@ -1481,9 +1466,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* _
   if (warp == kFeeder) {
     bool ok = true;
     for (int g = 0; g < count && ok; ++g)
-      ok = feed_weights<FMT, STEPS>(items[g], items[g], smem, bars, g == 0, g == 0 && !items[0].early_weights, s, parity);
+      ok = feed_weights<FMT, STEPS, false>(items[g], items[g], smem, bars, g == 0, g == 0 && !items[0].early_weights, s, parity);
   } else if (warp >= kFinisher && !(copies && warp >= kFirstCopier)) {
-    if (warp == kFinisher) start_activations<FMT, STEPS>(items[0], items[0], smem, bars);
+    if (warp == kFinisher) start_activations<FMT, STEPS, false>(items[0], items[0], smem, bars);
     else griddep_wait();
     bool ok = true;
     for (int g = 0; g < count; ++g) {
@@ -1494,7 +1479,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_batch_kernel(const Params* _
     griddep_wait();
     bool ok = true;
     for (int g = 0; g < count; ++g) {
-      if (ok) ok = feed_activations<FMT, STEPS>(items[g], smem, bars, warp - kFirstCopier, s, parity);
+      if (ok) ok = feed_activations<FMT, STEPS, false>(items[g], smem, bars, warp - kFirstCopier, s, parity);
       if (items[g].world >= 1) finished_barrier();
     }
   } else {
