@@ -307,6 +307,19 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
 
 bool aligned(const void* ptr, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(ptr) % bytes == 0; }
 
+// From this many bytes on a launch's weights and scales leave L2 first, NVFP4's always. In the usual order they drive out what the next
+// launches need, the kernels' code above all: a launch of another kernel than the one before took 1.4 to 4.2 us longer than one of
+// the same, with them first 0.7 to 1.9. But a few smaller matrices used in turn stay in L2, and leave it too early so.
+// us in the usual order and leaving first, three matrices in turn, eager / so many that they exceed L2, in a graph: BF16 3072 x 3072, one
+// row 5.0 / 5.93 and 6.0 / 5.92; FP8 4096 x 4096 4.9 / 5.55 and 5.3 / 5.3, 5120 x 4096 5.65 / 6.1 and 6.05 / 5.95, 4096 x 8192 8.3 / 8.6 and
+// 8.1 / 8.45, 28672 x 8192 40.4 and 38.4; MXFP8 5120 x 5120, two rows 8.04 / 8.11 and 8.44 / 8.07; BF16 4096 x 4096 8.13 / 8.29 and 8.08 /
+// 8.14, 8192 x 8192 23.0 and 21.9. NVFP4, which its consumers bound: 4096 x 4096 5.24 / 5.74 and 5.25 / 5.50, 8192 x 4096 7.16 / 7.74 and
+// 7.34 / 7.46, 10240 x 8192 14.05 / 13.7 and 13.3 / 13.0, four layers of four projections 488 and 464.
+constexpr long long kStreamed = 32ll << 20;
+long long weight_bytes(const Params& p) {
+  return (long long)(p.pairs ? 2 * p.pairs : p.N) * (p.row_bytes + (p.scale_mode == dg::SCALES_NONE ? 0 : p.scale_row_bytes));
+}
+
 // Everything of a launch but the launch: plan, tensor maps, process-wide settings. `grid` > 0 fixes the CTA count.
 int prepare(int fmt, Params& p, int M, int& ctas, int& smem, int grid = 0, bool allow_resident = true) {
   DeviceState* st = device_state();
@@ -335,6 +348,7 @@ int prepare(int fmt, Params& p, int M, int& ctas, int& smem, int grid = 0, bool 
     if (!encode_activations(&p.tmap_x, p.x, M, p.K, p.ldx, (resident ? p.x_box_steps : p.steps) * step_blocks, !resident))
       return (int)cudaErrorNotSupported;
   }
+  p.streamed = fmt == dg::FMT_NVFP4 || weight_bytes(p) >= kStreamed;
   p.early_weights = g_static_weights.load(std::memory_order_relaxed);
   p.wait_limit_ns = g_wait_limit_ns.load(std::memory_order_relaxed);
   return 0;

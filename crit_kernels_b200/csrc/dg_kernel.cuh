@@ -136,6 +136,7 @@ struct Params {
   int tile_rows;             // rows of a full tile (a multiple of 8; gate_up: of 16, for both regions), at most 16 * kMaxGroups
   int stage_bytes;           // bytes of one ring stage
   int early_weights;         // 1: weight copies may be issued before the previous kernel of the stream completed
+  int streamed;              // 1: weights and scales leave L2 first (see kStreamed in dg_abi.cu); NVFP4's always do
   int last_rows;             // rows of the copies of a tile that is not full (per region; a multiple of 8)
   // SwiGLU epilogue (pairs > 0): the matrix is a gate_up projection of 2 * pairs rows, gate rows [0, pairs) and up rows
   // [pairs, 2 pairs); N counts its output columns (= pairs). A tile holds row k of both halves and writes
@@ -221,25 +222,26 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity, abort_flag);
 }
-// Weights and scales are read once and leave L2 first. Otherwise they drive out what the next launches need again, the kernels' code
-// above all: a launch of another kernel than the one before took 1.4 to 4.2 us longer than one of the same (its instructions came
-// from HBM, in competition with the weights), now 0.7 to 1.9. us before and after: NVFP4 57344 x 8192 with 1 / 8 / 16 rows 53.1 / 63.9 /
-// 90.9 and 51.3 / 62.6 / 88.5; FP8 28672 x 8192 with 1 / 8 rows 40.2 / 44.8 and 38.3 / 42.6; four layers of four projections at 4 rows 535 and
-// 487, two at 16 rows 382 and 348. (Small matrices that keep the usual order: NVFP4 4096 x 4096, one row, eager 5.60 and 5.40.)
+// The policy of copies of what is read once and leaves L2 first.
 __device__ __forceinline__ uint64_t read_once() {
   uint64_t policy;
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   return policy;
 }
 // 2-D tiled tensor copy: box of the tensor map at element column x, row y.
-__device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar, uint64_t policy) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
-               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "l"(policy)
-               : "memory");
+__device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar, bool streamed, uint64_t policy) {
+  if (streamed)
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "l"(policy)
+                 : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
 }
-// The same box into L2 only.
-__device__ __forceinline__ void tensor_prefetch(const CUtensorMap* map, int x, int y, uint64_t policy) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile.L2::cache_hint [%0, {%1, %2}], %3;" ::"l"(map), "r"(x), "r"(y), "l"(policy) : "memory");
+// The same box into L2 only. (Without the hint: 4096 x 4096 NVFP4, one row, eager 5.37 with it, 5.25 without; large ones the same.)
+__device__ __forceinline__ void tensor_prefetch(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 // 3-D: from (0, 0, z) on.
 __device__ __forceinline__ void tensor3_g2s(uint32_t dst, const CUtensorMap* map, int z, uint32_t bar) {
@@ -439,6 +441,7 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
     if (lane == 0 && p.status) atomicOr(p.status, kStatusProducerTimeout);
     return false;
   };
+  const bool streamed = FMT == FMT_NVFP4 || p.streamed != 0;
   const uint64_t policy = read_once();
   if (wait) griddep_wait();   // (with everything worked out)
   int filled = 0;
@@ -465,8 +468,8 @@ __device__ __forceinline__ bool feed_weights(const Params& p, const Params& maps
       __syncwarp();
       if (!first || filled > stages) activations(s, win);
       if (region < wk.regions) {
-        if (lane < 2) tensor_g2s(stage + row0 * W_ROW, map_w, (win * WIN) >> 3, n0, full, policy);
-        else if (lane < 4 && staged) tensor_g2s(stage + sc_off + row0 * SC_ROW, map_sc, (win * SC_WIN) >> 3, n0, full, policy);
+        if (lane < 2) tensor_g2s(stage + row0 * W_ROW, map_w, (win * WIN) >> 3, n0, full, streamed, policy);
+        else if (lane < 4 && staged) tensor_g2s(stage + sc_off + row0 * SC_ROW, map_sc, (win * SC_WIN) >> 3, n0, full, streamed, policy);
       }
       if (++s == stages) { s = 0; parity ^= 1u; }
     }
@@ -500,13 +503,12 @@ __device__ __forceinline__ void prefetch_weights(const Params& p) {
   if (wk.ntiles == 0) return;
   int col0, cols;
   wk.tile(0, col0, cols);
-  const uint64_t policy = read_once();
   for (int win = 0; win < (p.small ? wk.nwin : 1); ++win)
     for (int region = 0; region < wk.regions; ++region) {
       const int n0 = region * wk.pairs + col0;
-      tensor_prefetch(cols == wk.cap ? &p.tmap_w : &p.tmap_w_last, (win * WIN) >> 3, n0, policy);
+      tensor_prefetch(cols == wk.cap ? &p.tmap_w : &p.tmap_w_last, (win * WIN) >> 3, n0);
       if (SCB != 0 && p.scale_mode == SCALES_STAGED)
-        tensor_prefetch(cols == wk.cap ? &p.tmap_sc : &p.tmap_sc_last, (win * STEPS * SCB) >> 3, n0, policy);
+        tensor_prefetch(cols == wk.cap ? &p.tmap_sc : &p.tmap_sc_last, (win * STEPS * SCB) >> 3, n0);
     }
 }
 
