@@ -281,7 +281,7 @@ bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int&
   if (p.tile_rows == 0) return false;
   // Small launches: a stage for every window, in half of the shared memory, so that the next launch's CTA fits beside.
   if (grid == 0 && dg::small_capable(M) && all_rows <= dg::kSmallRows &&
-      (fmt != dg::FMT_NVFP4 || (all_rows * row_steps <= dg::kSmallNvfp4 && !p.pairs)) && K % 64 == 0 && p.scale_mode != dg::SCALES_DIRECT &&
+      (fmt != dg::FMT_NVFP4 || (row_steps <= 2 && all_rows * row_steps <= dg::kSmallNvfp4 && !p.pairs)) && K % 64 == 0 && p.scale_mode != dg::SCALES_DIRECT &&
       p.scale_mode != dg::SCALES_BLOCKED && force_steps == 0) {
     const int steps = fmt == dg::FMT_BF16 || row_steps == 1 ? 1 : 2, windows = std::max(2, ceil_div(row_steps, steps));
     const int rows = regions * ceil_div(all_rows / regions, dg::kBoxRows) * dg::kBoxRows;

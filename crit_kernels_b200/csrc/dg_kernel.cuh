@@ -50,12 +50,15 @@ constexpr int kThreads = 32 * (kConsumers + 1 + kFinishers);
 // two fit on an SM: the next launch of the stream then waits there for this one to finish, its barriers set up and its weights
 // on their way into L2.
 constexpr int kSmallThreads = 32 * (kConsumers + 2), kSmallRows = 32;
-// NVFP4's decoding spills some of their 96 registers, so that only what is very short, in matrix rows times steps of a CTA's share,
-// is faster (us without and with, one row / eight: 1024 x 1024 3.68 / 3.48 and 3.35 / 2.95, 4700 x 1024 3.9 / 3.9 and 3.5 / 3.3, 1100 x 8192, 64
-// of them, 5.66 / 6.7 and 5.4 / 6.7, 3072 x 3072, 72, 4.84 / 5.29 and 4.51 / 5.31; 4700 x 2560, 96, 5.67 / 5.79 and 5.70 / 5.75, four rows
-// 6.09 and 6.21; 2368 x 8192, 128, 6.09 and 6.48).
+// NVFP4: only very short launches, of up to two steps of K and 48 matrix rows times steps in a CTA's share. Its decoding spills some of
+// the 96 registers, and where calls come about as fast as a launch takes, the next launch's CTAs are placed when this one has left some
+// SMs and not others; some SMs then hold two CTAs of a launch and as many hold none, and so do all launches after it, whose CTAs take
+// the places that are left. us as an ordinary and as a small launch, in a graph / eager calls: 1024 x 1024, one row 3.47 / 4.92 and
+// 2.82 / 4.93, 2368 x 2048, 32 rows times steps, 3.69 / 5.28 and 3.21 / 5.32, 3552 x 2048, 48, 4 rows 4.18 / 5.34 and 3.83 / 5.36; 1184 x
+// 6144, 48 in six steps, 2 rows 5.55 / 5.74 and 5.31 / 7.50, 2368 x 4096, 64, 8 rows 4.80 / 5.31 and 4.70 / 6.62, 2560 x 2560, 72, one row
+// 5.31 / 5.50 and 5.48 / 6.95 (129 SMs of 148 had work).
 __host__ __device__ constexpr bool small_capable(int m) { return m <= 8; }
-constexpr int kSmallNvfp4 = 72;
+constexpr int kSmallNvfp4 = 48;
 constexpr int kSmallSmem = 111 * 1024;     // dynamic shared memory: 228 KB for two, less 1 KB and the static part each
 constexpr int kBoxRows = 8;                // tile rows come in multiples of these
 constexpr int kGroupRows = 16;             // rows of one mma tile

@@ -125,3 +125,16 @@ def test_plans_know_that_gathered_scales_have_no_small_launch(fmt, n, k):
     assert p["stages"] == min(12, (232448 - 256 - behind) // p["stage_bytes"])
     even = cabi.plan(fmt, 1, n, 1024)                        # (their neighbours of two windows' length)
     assert even["stages"] == 2 and even["smem_bytes"] < 115712 // 2
+
+
+@pytest.mark.parametrize("m,n,k,small", [(1, 1024, 1024, True), (8, 148 * 16, 2048, True), (4, 148 * 24, 2048, True), (4, 148 * 24 + 1, 2048, False),
+                                         (1, 148 * 8, 3072, False), (2, 1184, 6144, False), (8, 2368, 4096, False), (1, 2560, 2560, False)])
+def test_small_nvfp4_launches_are_very_short(m, n, k, small):
+    """Two CTAs to an SM up to two steps of K (1024 values each) and 48 matrix rows times steps in a CTA's share. A longer launch takes
+    about as long as a call from Python, and calls at that pace come to lie two CTAs of a launch to an SM."""
+    p = cabi.plan("nvfp4", m, n, k)
+    behind = p["smem_bytes"] - (256 + p["stages"] * p["stage_bytes"])
+    if small:
+        assert p["smem_bytes"] <= 113664 and p["stages"] == 2           # a stage for each window, or two
+    else:
+        assert p["stages"] == min(12, (232448 - 256 - behind) // p["stage_bytes"])
