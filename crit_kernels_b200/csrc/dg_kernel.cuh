@@ -971,7 +971,9 @@ enum : int { ODD_NONE = 0, ODD_SHARED = 1, ODD_APART = 2 };
 // which the stage then belongs (the last tile: the consumers finish it, a unit each, when all have come so far). RES: the
 // activations are resident (RES_MIXED: `spread` has the steps, modulo 32, with chunks of another exponent than the usual one). FRESH:
 // the lane's places are worked out anew for every tile. Otherwise the compiler works out once what a kernel's tile codes share and
-// keeps it all the time, which costs registers (NVFP4 resident, two steps: 84 bytes a thread spilled, and none so).
+// keeps it all the time, which costs registers: the NVFP4 kernel for resident activations and two steps spilled 84 bytes a thread, and
+// none so (us without and with: 8192 x 8192, one row 10.8 and 10.55, 4096 x 4096 5.04 and 4.84, 5920 x 4096 5.73 and 5.70). The others spill
+// less, and some are slower so: one step, 8567 x 17728, two rows 24.6 and 27.0; FP16 in windows, 8567 x 17728, 8 rows 22.8 and 24.5.
 template <int FMT, int NT, int EIGHTS, int STEPS, typename XT, int RES, bool FRESH>
 __device__ __forceinline__ void consume_tile(const Params& p, const Walk& wk, const StageLayout<FMT, STEPS>& lay,
                                              unsigned char* smem, int col0, int cols, bool last, uint32_t spread, const Bars& bars, int& s, uint32_t& parity,
@@ -1217,7 +1219,7 @@ __device__ __forceinline__ bool consume_gemv(const Params& p, unsigned char* sme
     auto tile = [&](auto res) {
       constexpr int RES = decltype(res)::value;
       auto run = [&](auto e) {
-        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, RES, FMT == FMT_NVFP4 && NT == 1 && !SMALL && !(BATCH && CAN_RES)>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
+        consume_tile<FMT, NT, decltype(e)::value, STEPS, XT, RES, FMT == FMT_NVFP4 && CAN_RES && STEPS == 2 && !SMALL && !BATCH>(p, wk, lay, smem, col0, cols, t + 1 == wk.ntiles, spread, bars, s, parity,
                                                                   first && t == 0, ok);
       };
       const int eights = (wk.rows(cols) + 7) / 8;
