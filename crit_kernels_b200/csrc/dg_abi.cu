@@ -187,8 +187,9 @@ int row_major_scales(int fmt, int K, bool on_16_bytes) {
 //                   projections are one kernel then: three layers at 8 rows take 374 us with two steps for K = 28672, 366 without
 //                   (31.1 and 32.1 alone), with SwiGLU in gate_up 419 and 371.5
 //   stages          as many as fit in shared memory, at most kMaxStages
-// Activations stay resident where that leaves three stages of two steps (from three rows on, where they would take a fifth
-// and more of a stage, also with four stages of one); otherwise a window of them passes through every stage.
+// Activations stay resident (FP8, NVFP4, up to four rows) where that leaves three stages of two steps, or four of one (from three rows on,
+// where they would take a fifth and more of a stage, and where a CTA's range is one tile in stages of one step only); otherwise, and
+// where a CTA's range is short (below), a window of them passes through every stage.
 // `grid` > 0: the launch is a batch's (that many CTAs whatever N; the caller sizes the ring for all its GEMVs and
 // decides about resident activations: `allow_resident` is its wish, and no rule about stages is applied here).
 bool make_plan(int fmt, int M, int N, int K, int sms, Params& p, int& ctas, int& smem, int grid = 0,

@@ -363,8 +363,8 @@ __device__ __forceinline__ void copy_resident(const Params& p, const Params& map
 }
 
 // Windows whose activations one tensor copy brings: all, or where K is no multiple of 64 those that lie within the rows (past their end a
-// copy would bring the next row's values). The three copying warps, 16 bytes a copy, cannot keep up with more than a few rows: us at
-// 12490 x 5088 with 8 / 16 rows, all windows by them and only the last: NVFP4 24.0 / 37.9 and 15.2 / 23.4, FP8 19.0 / 45.3 and 16.2 / 28.4,
+// copy would bring the next row's values). The two copying warps, 16 bytes a copy, cannot keep up with more than a few rows: us at
+// 12490 x 5088 with 8 / 16 rows, all windows by them and only the last: NVFP4 24.0 / 37.9 and 15.2 / 23.4, FP8 19.0 / 45.3 and 16.2 / 20.8,
 // MXFP8 22.7 / 42.6 and 17.3 / 22.6, BF16 24.1 / 36.2 and 23.5 / 26.8; NVFP4 40000 x 8160 93 / 144 and 56 / 81.
 template <int FMT, int STEPS, bool RESIDENT>
 __device__ __forceinline__ int tensor_windows(const Params& p) {
