@@ -409,7 +409,7 @@ bool fill_nvfp4(Params& p, const void* x, int ldx, int x_is_bf16, const uint8_t*
 }
 
 // Head of an encoded batch (dg_encode_nvfp4_batch); the GEMVs' launch parameters follow at kBatchHead bytes.
-constexpr unsigned int kBatchMagic = 0x44474231u;   // "DGB1"
+constexpr unsigned int kBatchMagic = 0x44474232u;   // "DGB2": goes up with the layout of Params
 constexpr size_t kBatchHead = 256;
 struct BatchHead {
   unsigned int magic;
